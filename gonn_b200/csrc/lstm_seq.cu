@@ -1,0 +1,401 @@
+// A whole LSTM layer over a batch of sequences in one persistent kernel per direction (fp32).
+//
+// The recurrence is a chain of T products of B x H by H x 4H that no larger GEMM can replace: what
+// bounds it is the latency of one step, not arithmetic (B = 32, H = 512: 33.5 M multiply-adds, 0.9 us
+// of the FMA pipes).  Launched step by step (one small GEMM, one gate kernel and the tape's additions
+// per step) a step costs 70 us forward and 270 us with its backward, most of it launches and a GEMM
+// that fills 16 SMs.  Here
+//  * the recurrent weight stays in shared memory for the whole sequence: a CTA owns UT hidden units
+//    (their four gate rows forward, their column of W_hh backward) for a group of sequences;
+//  * sequences are independent, so only the CTAs of one group wait for one another: H / UT flags
+//    per group in global memory, one per CTA, each stored with release semantics after the CTA's part
+//    of h_t (or of dgates_t) is written, all polled by one warp;
+//  * within a CTA the eight warps split the contraction, a lane accumulates 4 x 4 outputs with packed
+//    fp32 multiply-adds, and the partial sums meet in shared memory in a fixed order (deterministic);
+//  * the cell state never leaves the thread that owns it except to be saved for the backward.
+// The input projections of all steps, the weight gradients and the input gradient are single
+// GEMMs outside (ops/rnn.py).  Measured at B = 32, T = 64, H = 512: 379 us forward (5.9 us a step) and
+// 474 us backward (7.4 us a step); at H = 64 a step is 2.6 us, which is the exchange alone.
+//
+// Waiting CTAs need one another to be resident: cooperative launches only.  Every wait is bounded.
+#include "common.cuh"
+
+using namespace gb;
+
+namespace {
+
+constexpr int kMB = 8;        // sequences of one sub-tile
+constexpr int kWarps = 8;
+constexpr int kThreads = kWarps * 32;
+
+__device__ __forceinline__ float sigm(float x) { return 1.f / (1.f + __expf(-x)); }
+
+// acc (two packed floats) += a * b
+__device__ __forceinline__ void ffma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+struct SeqArgs {
+  int B, T, H;
+  int sub;                    // sub-tiles of kMB sequences per CTA
+  int ug;                     // CTAs per group (hidden-unit slices)
+  const float* w;             // W_hh (4H, H)
+  const float* h0;            // (B, H) or null
+  const float* c0;            // (B, H) or null
+  unsigned int* flags;        // [groups][ug], zeroed before the launch
+  int* status;
+  // forward
+  const float* xg;            // (B, T, 4H): x W_ih^T
+  const float* bias;          // (4H) or null
+  float* out;                 // (B, T, H): h_t
+  float* cseq;                // (B, T, H): c_t
+  float* act;                 // (B, T, 4H): activated gates i, f, g, o
+  // backward (reads cseq and act)
+  const float* dout;          // (B, T, H) or null
+  const float* dcn;           // (B, H) or null: gradient of the last cell state
+  float* dgates;              // (B, T, 4H)
+  float* dc0;                 // (B, H) or null
+};
+
+// Publishes this CTA's step (`value` steps done).  Called after a __syncthreads that follows the stores.
+__device__ __forceinline__ void publish(unsigned int* flag, unsigned int value) {
+  if (threadIdx.x == 0)
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag), "r"(value) : "memory");
+}
+
+// All threads wait until every CTA of the group has published `value`; false when the budget ran out.
+__device__ __forceinline__ bool wait_group(const unsigned int* flags, int n, unsigned int value, int* abort_flag,
+                                           int* status) {
+  if (threadIdx.x < 32) {
+    const uint64_t t0 = globaltimer_ns();
+    uint32_t spins = 0;
+    for (;;) {
+      bool ok = true;
+      for (int i = (int)threadIdx.x; i < n; i += 32) {
+        unsigned int v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flags + i) : "memory");
+        ok = ok && v >= value;
+      }
+      if (__all_sync(0xffffffffu, ok)) break;
+      if ((++spins & 0xFF) == 0 && globaltimer_ns() - t0 > kWaitBudgetNs) {
+        if (threadIdx.x == 0) {
+          *abort_flag = 1;
+          set_status(status, ST_RNN_TIMEOUT, (int)value);
+        }
+        break;
+      }
+    }
+  }
+  __syncthreads();
+  return *(volatile int*)abort_flag == 0;
+}
+
+// a: kMB rows, w: N rows, both K floats with pitch K + 4 (16-byte rows four banks apart, so that the
+// 16-byte reads of eight neighbouring rows touch all banks once).  Lanes: two groups of four a-rows
+// x N/4 groups of w-rows (w row = i * N/4 + group: neighbouring lanes, neighbouring rows) x KQ
+// slices of the contraction.  part[warp][kMB * N] receives the warp's partial sums.
+template <int N>
+__device__ __forceinline__ void product(const float* __restrict__ a, const float* __restrict__ w, int K,
+                                        float* __restrict__ part) {
+  constexpr int NG = N / 4;                  // groups of w-rows
+  constexpr int KQ = 32 / (2 * NG);          // lanes that share a group pair and split k
+  static_assert(KQ >= 1, "N <= 64");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int kq = lane % KQ, ng = (lane / KQ) % NG, mg = lane / (KQ * NG);
+  const int pitch = K + 4;
+  const float* ap = a + (mg * 4) * pitch;
+  const float* wp = w + ng * pitch;
+  unsigned long long acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) acc[i][j] = 0ull;
+#pragma unroll 2
+  for (int k = (warp * KQ + kq) * 4; k < K; k += kWarps * KQ * 4) {
+    ulonglong2 av[4], wv[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) av[i] = *reinterpret_cast<const ulonglong2*>(ap + i * pitch + k);
+#pragma unroll
+    for (int j = 0; j < 4; j++) wv[j] = *reinterpret_cast<const ulonglong2*>(wp + j * NG * pitch + k);
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        ffma2(acc[i][j], av[i].x, wv[j].x);
+        ffma2(acc[i][j], av[i].y, wv[j].y);
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      float v = __uint_as_float((unsigned)(acc[i][j] & 0xffffffffull)) + __uint_as_float((unsigned)(acc[i][j] >> 32));
+#pragma unroll
+      for (int o = 1; o < KQ; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (kq == 0) part[warp * (kMB * N) + (mg * 4 + i) * N + j * NG + ng] = v;
+    }
+}
+
+// Rows b0 .. b0 + kMB - 1 of src (row stride `stride`, K floats each) into the tile; rows past B are zero.
+__device__ __forceinline__ void load_tile(float* __restrict__ tile, const float* __restrict__ src, long long stride, int K,
+                                          int b0, int B) {
+  const int k4 = K / 4, pitch = K + 4;
+  for (int i = threadIdx.x; i < kMB * k4; i += kThreads) {
+    const int r = i / k4, c = (i - r * k4) * 4;
+    float* d = tile + r * pitch + c;
+    if (src != nullptr && b0 + r < B)
+      cp_async16(d, src + (long long)(b0 + r) * stride + c);
+    else
+      *reinterpret_cast<float4*>(d) = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  cp_async_wait_all();
+}
+
+// grid: (ug, groups).  UT units per CTA: N = 4 UT weight rows, row n = gate * UT + unit.
+template <int UT>
+__global__ void __launch_bounds__(kThreads, 1) lstm_seq_fwd_kernel(const SeqArgs p) {
+  constexpr int N = 4 * UT;
+  extern __shared__ __align__(16) float sm[];
+  __shared__ int abort_flag;
+  const int H = p.H, T = p.T, pitch = H + 4;
+  float* ws = sm;                                  // [N][H + 4]
+  float* hs = ws + N * pitch;                      // [kMB][H + 4]
+  float* part = hs + kMB * pitch;                  // [kWarps][kMB * N]
+  const int u0 = blockIdx.x * UT;
+  const int bg0 = blockIdx.y * p.sub * kMB;
+  unsigned int* flags = p.flags + (long long)blockIdx.y * p.ug;
+  if (threadIdx.x == 0) abort_flag = 0;
+  for (int i = threadIdx.x; i < N * (H / 4); i += kThreads) {
+    const int n = i / (H / 4), c = (i - n * (H / 4)) * 4;
+    const int g = n / UT, u = u0 + (n - g * UT);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (u < H) v = *reinterpret_cast<const float4*>(p.w + ((long long)g * H + u) * H + c);
+    *reinterpret_cast<float4*>(ws + n * pitch + c) = v;
+  }
+  __syncthreads();
+  const int cell_m = threadIdx.x / UT, cell_u = threadIdx.x % UT;      // the cell of threads 0 .. kMB * UT - 1
+  const int u = u0 + cell_u;
+  const bool cell = threadIdx.x < kMB * UT && u < H;
+  float bias[4] = {0.f, 0.f, 0.f, 0.f};
+  if (cell && p.bias != nullptr) {
+#pragma unroll
+    for (int g = 0; g < 4; g++) bias[g] = p.bias[g * H + u];
+  }
+  for (int t = 0; t < T; t++) {
+    if (t > 0 && !wait_group(flags, p.ug, (unsigned)t, &abort_flag, p.status)) return;
+    for (int s = 0; s < p.sub; s++) {
+      const int b0 = bg0 + s * kMB, b = b0 + cell_m;
+      const bool mine = cell && b < p.B;
+      const long long row = (long long)b * T + t;
+      float pre[4] = {0.f, 0.f, 0.f, 0.f}, cp = 0.f;
+      if (mine) {                                  // in flight during the product
+#pragma unroll
+        for (int g = 0; g < 4; g++) pre[g] = __ldg(p.xg + row * 4 * H + g * H + u) + bias[g];
+        cp = t > 0 ? p.cseq[(row - 1) * H + u] : (p.c0 != nullptr ? p.c0[(long long)b * H + u] : 0.f);
+      }
+      if (t > 0 || p.h0 != nullptr) {
+        if (t > 0)
+          load_tile(hs, p.out + (long long)(t - 1) * H, (long long)T * H, H, b0, p.B);
+        else
+          load_tile(hs, p.h0, H, H, b0, p.B);
+        __syncthreads();
+        product<N>(hs, ws, H, part);
+        __syncthreads();
+        if (mine) {
+#pragma unroll
+          for (int g = 0; g < 4; g++) {
+            float v = 0.f;
+#pragma unroll
+            for (int w = 0; w < kWarps; w++) v += part[w * (kMB * N) + cell_m * N + g * UT + cell_u];
+            pre[g] += v;
+          }
+        }
+      }
+      if (mine) {
+        const float ig = sigm(pre[0]), fg = sigm(pre[1]), gg = tanhf(pre[2]), og = sigm(pre[3]);
+        const float cn = fg * cp + ig * gg;
+        p.cseq[row * H + u] = cn;
+        p.out[row * H + u] = og * tanhf(cn);
+        float* a = p.act + row * 4 * H + u;
+        a[0] = ig; a[H] = fg; a[2 * H] = gg; a[3 * H] = og;
+      }
+    }
+    __syncthreads();
+    publish(flags + blockIdx.x, (unsigned)(t + 1));
+  }
+}
+
+// grid: (ug, groups).  UT units per CTA: N = UT columns of W_hh, contraction over the 4H gates.
+template <int UT>
+__global__ void __launch_bounds__(kThreads, 1) lstm_seq_bwd_kernel(const SeqArgs p) {
+  constexpr int N = UT;
+  extern __shared__ __align__(16) float sm[];
+  __shared__ int abort_flag;
+  const int H = p.H, T = p.T, K = 4 * H, pitch = K + 4;
+  float* ws = sm;                                  // [N][4H + 4]: column u of W_hh
+  float* ds = ws + N * pitch;                      // [kMB][4H + 4]: dgates_{t+1}
+  float* part = ds + kMB * pitch;                  // [kWarps][kMB * N]
+  float* dcs = part + kWarps * kMB * N;            // [sub][kMB * N]: dc carried from step to step
+  const int u0 = blockIdx.x * UT;
+  const int bg0 = blockIdx.y * p.sub * kMB;
+  unsigned int* flags = p.flags + (long long)blockIdx.y * p.ug;
+  if (threadIdx.x == 0) abort_flag = 0;
+  for (int i = threadIdx.x; i < N * K; i += kThreads) {
+    const int n = i % UT, k = i / UT;
+    ws[n * pitch + k] = u0 + n < H ? p.w[(long long)k * H + u0 + n] : 0.f;
+  }
+  const int cell_m = threadIdx.x / UT, cell_u = threadIdx.x % UT;
+  const int u = u0 + cell_u;
+  const bool cell = threadIdx.x < kMB * UT && u < H;
+  for (int s = 0; s < p.sub; s++) {
+    const int b = bg0 + s * kMB + cell_m;
+    if (threadIdx.x < kMB * UT)
+      dcs[s * (kMB * N) + threadIdx.x] = (cell && b < p.B && p.dcn != nullptr) ? p.dcn[(long long)b * H + u] : 0.f;
+  }
+  __syncthreads();
+  for (int t = T - 1; t >= 0; t--) {
+    const bool chain = t < T - 1;
+    if (chain && !wait_group(flags, p.ug, (unsigned)(T - 1 - t), &abort_flag, p.status)) return;
+    for (int s = 0; s < p.sub; s++) {
+      const int b0 = bg0 + s * kMB, b = b0 + cell_m;
+      const bool mine = cell && b < p.B;
+      const long long row = (long long)b * T + t;
+      float dh = 0.f, ig = 0.f, fg = 0.f, gg = 0.f, og = 0.f, ct = 0.f, cp = 0.f;
+      if (mine) {
+        const float* a = p.act + row * K + u;
+        ig = __ldg(a); fg = __ldg(a + H); gg = __ldg(a + 2 * H); og = __ldg(a + 3 * H);
+        ct = __ldg(p.cseq + row * H + u);
+        cp = t > 0 ? __ldg(p.cseq + (row - 1) * H + u) : (p.c0 != nullptr ? p.c0[(long long)b * H + u] : 0.f);
+        if (p.dout != nullptr) dh = __ldg(p.dout + row * H + u);
+      }
+      if (chain) {
+        load_tile(ds, p.dgates + (long long)(t + 1) * K, (long long)T * K, K, b0, p.B);
+        __syncthreads();
+        product<N>(ds, ws, K, part);
+        __syncthreads();
+        if (mine) {
+          float v = 0.f;
+#pragma unroll
+          for (int w = 0; w < kWarps; w++) v += part[w * (kMB * N) + cell_m * N + cell_u];
+          dh += v;
+        }
+      }
+      if (mine) {
+        const float tc = tanhf(ct);
+        float* dcv = dcs + s * (kMB * N) + threadIdx.x;
+        const float dc = *dcv + dh * og * (1.f - tc * tc);
+        float* d = p.dgates + row * K + u;
+        d[0] = dc * gg * ig * (1.f - ig);
+        d[H] = dc * cp * fg * (1.f - fg);
+        d[2 * H] = dc * ig * (1.f - gg * gg);
+        d[3 * H] = dh * tc * og * (1.f - og);
+        *dcv = dc * fg;
+        if (t == 0 && p.dc0 != nullptr) p.dc0[(long long)b * H + u] = dc * fg;
+      }
+    }
+    __syncthreads();
+    publish(flags + blockIdx.x, (unsigned)(T - t));
+  }
+}
+
+constexpr int kSms = 148;
+constexpr long long kMaxSmem = 227 * 1024;
+// Each sub-tile costs a group of CTAs about 1.9 us forward and 2.9 us backward (H = 512); beyond 32 of them the
+// step-by-step GEMMs fill the GPU themselves (forward + backward over 8 steps at H = 512: B = 1024, 32
+// sub-tiles, 3.4 ms against 4.6 ms step by step; B = 2048, 7.4 against 6.1).
+constexpr int kMaxSub = 32;
+
+long long fwd_smem(int ut, int H) {
+  return 4ll * ((4ll * ut + kMB) * (H + 4) + (long long)kWarps * kMB * 4 * ut);
+}
+long long bwd_smem(int ut, int H, int sub) {
+  return 4ll * (((long long)ut + kMB) * (4ll * H + 4) + (long long)kWarps * kMB * ut + (long long)sub * kMB * ut);
+}
+
+// Units per CTA, unit slices, groups of sequences and sub-tiles per group; false when the layer does
+// not fit (the weight slices of 148 CTAs, or the exchange tile, exceed shared memory).
+// Large UT keeps the exchanged tile small against the resident weight; it is halved while that
+// gives more CTAs than half of the SMs would otherwise see.
+bool plan(int B, int H, bool bwd, int* ut, int* ug, int* groups, int* sub) {
+  if (H % 4 != 0 || H < 4) return false;
+  const int tiles = (B + kMB - 1) / kMB;
+  int best = 0;
+  for (int u = 16; u >= 4; u >>= 1) {
+    const int slices = (H + u - 1) / u;
+    if (slices > kSms) break;                     // smaller u only makes more slices
+    const int g = tiles < kSms / slices ? tiles : kSms / slices;
+    const int s = (tiles + g - 1) / g;
+    const long long need = bwd ? bwd_smem(u, H, s) : fwd_smem(u, H);
+    if (need > kMaxSmem || s > kMaxSub) continue;
+    *ut = u; *ug = slices; *sub = s; *groups = (tiles + s - 1) / s;
+    best = u;
+    if ((long long)slices * *groups >= kSms / 2) break;
+  }
+  return best != 0;
+}
+
+template <typename K>
+int launch(K kern, const SeqArgs& a, int groups, long long smem, cudaStream_t s) {
+  GB_CUDA_OK(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GB_CUDA_OK(cudaMemsetAsync(a.flags, 0, sizeof(unsigned int) * a.ug * groups, s));
+  void* args[] = {(void*)&a};
+  GB_CUDA_OK(cudaLaunchCooperativeKernel((const void*)kern, dim3(a.ug, groups), dim3(kThreads), args, (size_t)smem, s));
+  return gbh::E_OK;
+}
+
+}  // namespace
+
+// 1 when both directions of an LSTM layer of this size run as persistent kernels.
+GB_EXPORT int gb_lstm_seq_fits(int B, int H) {
+  int ut, ug, groups, sub;
+  return B > 0 && plan(B, H, false, &ut, &ug, &groups, &sub) && plan(B, H, true, &ut, &ug, &groups, &sub) ? 1 : 0;
+}
+
+// fp32.  xg (B,T,4H) = x W_ih^T, bias (4H) or null, w = W_hh (4H,H), h0 / c0 (B,H) or null; writes
+// out (B,T,H), cseq (B,T,H) and the activated gates act (B,T,4H).  flags: scratch of 148 words.
+GB_EXPORT int gb_lstm_seq_fwd(const void* xg, const void* bias, const void* w, const void* h0, const void* c0, void* out,
+                              void* cseq, void* act, void* flags, int B, int T, int H, void* stream) {
+  if (B <= 0 || T <= 0) return gbh::E_OK;
+  SeqArgs a = {};
+  int ut, groups;
+  if (!plan(B, H, false, &ut, &a.ug, &groups, &a.sub)) {
+    gbh::set_error("gb_lstm_seq_fwd: a layer of %d units does not fit", H);
+    return gbh::E_TOO_LARGE;
+  }
+  a.B = B; a.T = T; a.H = H;
+  a.w = (const float*)w; a.h0 = (const float*)h0; a.c0 = (const float*)c0;
+  a.flags = (unsigned int*)flags; a.status = gbh::status_ptr();
+  a.xg = (const float*)xg; a.bias = (const float*)bias;
+  a.out = (float*)out; a.cseq = (float*)cseq; a.act = (float*)act;
+  const long long smem = fwd_smem(ut, H);
+  cudaStream_t s = (cudaStream_t)stream;
+  if (ut == 16) return launch(lstm_seq_fwd_kernel<16>, a, groups, smem, s);
+  if (ut == 8) return launch(lstm_seq_fwd_kernel<8>, a, groups, smem, s);
+  return launch(lstm_seq_fwd_kernel<4>, a, groups, smem, s);
+}
+
+// Backward of the above: dout (B,T,H) or null, dcn (B,H) or null; writes dgates (B,T,4H), the gradient
+// of the gate pre-activations, and dc0 (B,H) when not null.
+GB_EXPORT int gb_lstm_seq_bwd(const void* w, const void* c0, const void* cseq, const void* act, const void* dout,
+                              const void* dcn, void* dgates, void* dc0, void* flags, int B, int T, int H, void* stream) {
+  if (B <= 0 || T <= 0) return gbh::E_OK;
+  SeqArgs a = {};
+  int ut, groups;
+  if (!plan(B, H, true, &ut, &a.ug, &groups, &a.sub)) {
+    gbh::set_error("gb_lstm_seq_bwd: a layer of %d units does not fit", H);
+    return gbh::E_TOO_LARGE;
+  }
+  a.B = B; a.T = T; a.H = H;
+  a.w = (const float*)w; a.c0 = (const float*)c0; a.cseq = (float*)cseq; a.act = (float*)act;
+  a.dout = (const float*)dout; a.dcn = (const float*)dcn; a.dgates = (float*)dgates; a.dc0 = (float*)dc0;
+  a.flags = (unsigned int*)flags; a.status = gbh::status_ptr();
+  const long long smem = bwd_smem(ut, H, a.sub);
+  cudaStream_t s = (cudaStream_t)stream;
+  if (ut == 16) return launch(lstm_seq_bwd_kernel<16>, a, groups, smem, s);
+  if (ut == 8) return launch(lstm_seq_bwd_kernel<8>, a, groups, smem, s);
+  return launch(lstm_seq_bwd_kernel<4>, a, groups, smem, s);
+}

@@ -5,8 +5,9 @@ Cells: ``RNNCell`` (tanh / ReLU), ``LSTMCell`` (gate order i, f, g, o; optional 
 ``RNN`` / ``LSTM`` / ``GRU``: batch-first input (B, T, F); options layers, bidirectional,
 dropout between layers, ReLU (RNN), proj_size (LSTM); children ``cells.N``, ``backcells.N``,
 ``dropout.N``.  State layout for stacks: (L * D, B, H).  Gates are computed by the fused
-Linear kernels and one fused gate kernel per cell and direction (``ops/rnn.py``); the time
-loop stays on the autograd tape.
+Linear kernels and one fused gate kernel per cell and direction (``ops/rnn.py``) with the time
+loop on the autograd tape; an fp32 LSTM layer on CUDA runs its whole sequence in one persistent
+kernel per direction where it fits and nothing observes its single steps.
 """
 from __future__ import annotations
 
@@ -146,6 +147,35 @@ def _gather_last_steps(out: torch.Tensor, lengths: Sequence[int]) -> torch.Tenso
 # ---------------------------------------------------------------------------------------
 # stacks
 # ---------------------------------------------------------------------------------------
+def _plain(m, cls) -> bool:
+    """``m`` is exactly a ``cls`` whose call is its class's forward: no hook, no replaced forward."""
+    return (type(m) is cls and "forward" not in m.__dict__ and not m._forward_hooks and not m._forward_pre_hooks
+            and not m._backward_hooks and not m._backward_pre_hooks)
+
+
+def _sequence_kernel_takes(cell, x, st0) -> bool:
+    """Whether the step-by-step calls of ``cell`` may be replaced by ``ops.rnn.lstm_sequence``: an
+    fp32 LSTM cell on CUDA without projection, nothing observing the single steps, and a layer that
+    fits the persistent kernels."""
+    g = torch.nn.modules.module
+    if (not x.is_cuda or x.dtype != torch.float32 or x.dim() != 3 or x.shape[0] == 0 or x.shape[1] == 0
+            or not _plain(cell, LSTMCell) or cell.whr is not None or not _plain(cell.wih, Linear)
+            or not _plain(cell.whh, Linear) or cell.wih.activation or cell.whh.activation or cell.whh.bias is not None
+            or g._global_forward_hooks or g._global_forward_pre_hooks or g._global_backward_hooks
+            or g._global_backward_pre_hooks):
+        return False
+    if x.shape[2] != cell.wih.in_features:
+        return False                                   # the layer's own error
+    ts = [cell.wih.weight, cell.whh.weight] + ([] if cell.wih.bias is None else [cell.wih.bias])
+    if st0 is not None:
+        ts += list(st0)
+        if any(tuple(s.shape) != (x.shape[0], cell.hidden_size) for s in st0):
+            return False
+    if any(t.dtype != torch.float32 or t.device != x.device for t in ts):
+        return False
+    return _rnn_ops.lstm_sequence_fits(x.shape[0], cell.hidden_size)
+
+
 class _RNNStack(Module):
     kind = "rnn"
 
@@ -172,6 +202,11 @@ class _RNNStack(Module):
 
     def _run_dir(self, cell, x, lengths, reverse, st0):
         B, T = x.shape[:2]
+        if lengths is None and self.kind == "lstm" and _sequence_kernel_takes(cell, x, st0):
+            h0, c0 = st0 if st0 is not None else (None, None)
+            out, c = _rnn_ops.lstm_sequence(x.flip(1) if reverse else x, cell.wih.weight, cell.wih.bias,
+                                            cell.whh.weight, h0, c0)
+            return (out.flip(1) if reverse else out), (out[:, -1], c)
         if reverse:
             x = _reverse_valid_prefix(x, lengths) if lengths is not None else x.flip(1)
         st = st0

@@ -4,6 +4,11 @@
 ``gru_gates(xg, hg, h) -> h'`` with gates r, z, n (nn/rnn.go:159-286 of the reference).
 CUDA tensors of fp32 / fp16 / bf16 run one kernel per direction; other tensors take the
 torch expression with the same formulas (the oracle of the tests).
+
+``lstm_sequence`` runs a whole fp32 LSTM layer: the input projections of all steps as one GEMM, the
+recurrence as one persistent kernel per direction (``csrc/lstm_seq.cu``), and the weight and input
+gradients as one GEMM each over all steps.  Measured forward + backward at B = 32, T = 64,
+I = H = 512: 1.34 ms, 22.6 ms step by step.
 """
 from __future__ import annotations
 
@@ -81,6 +86,81 @@ class _GRUGates(torch.autograd.Function):
         _l.call("gb_gru_gates_bwd", _l.I(_l.dtype_code(h.dtype)), _l.ptr(act), _l.ptr(h), _l.ptr(dh),
                 _l.ptr(dxg), _l.ptr(dhg), _l.ptr(dh_prev), _l.L(B), _l.I(H), _l.stream_ptr())
         return dxg, dhg, dh_prev
+
+
+def _aligned(t):
+    """Contiguous and 16-byte aligned (the persistent kernels read rows in 16-byte pieces)."""
+    if t is None:
+        return None
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+class _LSTMSequence(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, w_ih, b_ih, w_hh, h0, c0):
+        from .gemm import gemm
+        B, T, I = x.shape
+        H = w_hh.shape[1]
+        dev, s = x.device, _l.stream_ptr()
+        x2 = x.reshape(B * T, I)
+        xg = gemm(x2, w_ih, trans_b=True)
+        whh, h0, c0 = _aligned(w_hh.detach()), _aligned(h0), _aligned(c0)
+        bias = b_ih.detach().contiguous() if b_ih is not None else None
+        out = torch.empty((B, T, H), dtype=x.dtype, device=dev)
+        cseq = torch.empty_like(out)
+        act = torch.empty((B, T, 4 * H), dtype=x.dtype, device=dev)
+        flags = torch.empty(148, dtype=torch.int32, device=dev)
+        _l.call("gb_lstm_seq_fwd", _l.ptr(xg), _l.ptr(bias), _l.ptr(whh), _l.ptr(h0), _l.ptr(c0), _l.ptr(out),
+                _l.ptr(cseq), _l.ptr(act), _l.ptr(flags), _l.I(B), _l.I(T), _l.I(H), s)
+        ctx.save_for_backward(x2, w_ih, w_hh, h0, c0, out, cseq, act)
+        ctx.b_ih, ctx.xshape = b_ih, x.shape
+        ctx.set_materialize_grads(False)
+        return out, cseq[:, -1].contiguous()
+
+    @staticmethod
+    def backward(ctx, dout, dcn):
+        from .gemm import gemm
+        from .linear import emit_vector_grad, emit_weight_grad
+        x2, w_ih, w_hh, h0, c0, out, cseq, act = ctx.saved_tensors
+        B, T, H = out.shape
+        dev = out.device
+        dout = dout.contiguous() if dout is not None else None
+        dcn = dcn.contiguous() if dcn is not None else None
+        whh = _aligned(w_hh.detach())
+        dgates = torch.empty_like(act)
+        dc0 = torch.empty((B, H), dtype=out.dtype, device=dev) if ctx.needs_input_grad[5] else None
+        flags = torch.empty(148, dtype=torch.int32, device=dev)
+        _l.call("gb_lstm_seq_bwd", _l.ptr(whh), _l.ptr(c0), _l.ptr(cseq), _l.ptr(act), _l.ptr(dout), _l.ptr(dcn),
+                _l.ptr(dgates), _l.ptr(dc0), _l.ptr(flags), _l.I(B), _l.I(T), _l.I(H), _l.stream_ptr())
+        dg2 = dgates.view(B * T, 4 * H)
+        dx = dwih = db = dwhh = dh0 = None
+        # every read of a weight comes before its gradient is declared ready (ops/linear.py)
+        if ctx.needs_input_grad[0]:
+            dx = gemm(dg2, w_ih).view(ctx.xshape)
+        if ctx.needs_input_grad[4]:
+            dh0 = gemm(dgates[:, 0], w_hh)
+        if ctx.needs_input_grad[1]:
+            dwih = emit_weight_grad(w_ih, dg2, x2, True, False)
+        if ctx.b_ih is not None and ctx.needs_input_grad[2]:
+            db = emit_vector_grad(ctx.b_ih, dg2)
+        if ctx.needs_input_grad[3]:
+            # h_{t-1} of every step: the output moved on by one step
+            hprev = torch.empty_like(out)
+            hprev[:, 1:].copy_(out[:, :-1])
+            hprev[:, 0] = 0 if h0 is None else h0
+            dwhh = emit_weight_grad(w_hh, dg2, hprev.view(B * T, H), True, False)
+        return dx, dwih, db, dwhh, dh0, dc0
+
+
+def lstm_sequence_fits(B: int, H: int) -> bool:
+    """Whether a layer of ``H`` units over ``B`` sequences fits the persistent kernels."""
+    return bool(_l.lib().gb_lstm_seq_fits(_l.I(B), _l.I(H)))
+
+
+def lstm_sequence(x, w_ih, b_ih, w_hh, h0=None, c0=None):
+    """(h_1 .. h_T (B, T, H), c_T (B, H)) of an fp32 LSTM layer over (B, T, I) on CUDA."""
+    return _LSTMSequence.apply(x, w_ih, b_ih, w_hh, h0, c0)
 
 
 def lstm_gates(gates: torch.Tensor, c: torch.Tensor):

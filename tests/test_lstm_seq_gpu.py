@@ -1,0 +1,64 @@
+"""The persistent LSTM kernels (csrc/lstm_seq.cu) against the step-by-step oracle in float64."""
+import copy
+
+import pytest
+import torch
+
+from gonn_b200 import lib as L, nn
+from gonn_b200.nn import rnn as R
+
+pytestmark = pytest.mark.gpu
+
+# hidden sizes around the slices of 4 / 8 / 16 units and the exchange tile of 8 sequences, batches
+# that leave a sub-tile ragged or need several per CTA, the widest layer that fits
+SIZES = [(1, 1, 8, 4), (3, 5, 7, 20), (8, 3, 16, 64), (9, 4, 12, 68), (17, 7, 40, 132), (32, 5, 64, 512),
+         (70, 3, 24, 512), (5, 2, 16, 880)]
+
+
+def _close(a, b, tol, what):
+    a, b = a.detach().double().cpu(), b.detach()
+    err = float((a - b).norm() / b.norm().clamp_min(1e-30))
+    assert err < tol, f"{what}: relative error {err:.3g}"
+
+
+@pytest.mark.parametrize("B,T,I,H", SIZES)
+@pytest.mark.parametrize("state", [False, True])
+def test_lstm_sequence_matches_float64(B, T, I, H, state):
+    torch.manual_seed(B * 1000 + H)
+    ref = nn.LSTM(I, H, bidirectional=state, dtype=torch.float64)
+    net = copy.deepcopy(ref).float().cuda()
+    x = torch.randn(B, T, I, dtype=torch.float64)
+    D = 2 if state else 1
+    st = tuple(torch.randn(D, B, H, dtype=torch.float64) for _ in range(2)) if state else None
+    dy = torch.randn(B, T, D * H, dtype=torch.float64)
+    dh, dc = torch.randn(D, B, H, dtype=torch.float64), torch.randn(D, B, H, dtype=torch.float64)
+    xg = x.float().cuda().requires_grad_()
+    assert R._sequence_kernel_takes(net.cells[0], xg, None)
+    got, want = [], []
+    for net_, x_, conv, acc in ((net, xg, lambda t: t.float().cuda(), got),
+                                (ref, x.clone().requires_grad_(), lambda t: t, want)):
+        s_ = tuple(conv(t).requires_grad_() for t in st) if state else None
+        y, (h, c) = net_.ForwardWithState(x_, s_)
+        ((y * conv(dy)).sum() + (h * conv(dh)).sum() + (c * conv(dc)).sum()).backward()
+        acc += [("y", y), ("h", h), ("c", c), ("dx", x_.grad)] + [(n, p.grad) for n, p in net_.named_parameters()]
+        if state:
+            acc += [("dh0", s_[0].grad), ("dc0", s_[1].grad)]
+    L.assert_status_ok()
+    for (n, a), (_, b) in zip(got, want):
+        # fp32 sums of up to 4H terms and the fast-math exponential / tanh of the gate arithmetic
+        # (a few 1e-6 per step), carried through T steps
+        _close(a, b, 3e-5, n)
+
+
+def test_step_path_where_the_kernel_does_not_apply():
+    net = nn.LSTM(8, 16, device="cuda")
+    x = torch.randn(2, 3, 8, device="cuda")
+    y = net(x)
+    seen = []
+    handle = net.cells[0].register_forward_hook(lambda m, a, o: seen.append(1))
+    y2 = net(x)
+    handle.remove()
+    assert len(seen) == 3                                     # every step is observed
+    assert (y - y2).abs().max() < 1e-5
+    assert not R._sequence_kernel_takes(nn.LSTM(8, 6, device="cuda").cells[0], x, None)      # 6 % 4 != 0
+    assert not R._sequence_kernel_takes(net.cells[0].to(torch.bfloat16), x.bfloat16(), None)
