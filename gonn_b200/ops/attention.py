@@ -243,7 +243,11 @@ def _ds_workspace(device, need: int):
     return ws
 
 
-def flash_bwd(q, k, v, out, dout, lse, causal: bool, scale: float):
+def flash_bwd(q, k, v, out, dout, lse, causal: bool, scale: float, fused: bool = True):
+    """(dq, dk, dv, dqkv).  ``fused``: for equal lengths the three are slices of one (B, S, 3, H, D)
+    tensor, the gradient of a fused QKV projection; otherwise each is contiguous (dqkv is None), so that
+    the tape keeps it as the gradient of a leaf instead of copying it: at (8, 4096, 16, 128) three copies
+    of 154 us, 463 of 3190 us forward + backward."""
     q, k, v, dout = _tma_ready(q), _tma_ready(k), _tma_ready(v), _tma_ready(dout)
     B, Sq, H, D = q.shape
     Sk = k.shape[1]
@@ -252,8 +256,7 @@ def flash_bwd(q, k, v, out, dout, lse, causal: bool, scale: float):
     _l.call("gb_flash_delta", I(_l.dtype_code(q.dtype)), _l.ptr(out), _l.ptr(dout), _l.ptr(delta),
             I(B), I(H), I(Sq), I(D), *[L(s) for s in _strides3(out) + _strides3(dout)],
             _l.stream_ptr())
-    # one allocation so that dq / dk / dv can be handed on as a fused (.., 3, H, D) gradient
-    if Sq == Sk:
+    if fused and Sq == Sk:
         dqkv = torch.empty((B, Sq, 3, H, D), dtype=q.dtype, device=q.device)
         dq, dk, dv = dqkv[:, :, 0], dqkv[:, :, 1], dqkv[:, :, 2]
     else:
@@ -285,7 +288,7 @@ class _FlashAttn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         q, k, v, out, lse = ctx.saved_tensors
-        dq, dk, dv, _ = flash_bwd(q, k, v, out, dout, lse, ctx.causal, ctx.scale)
+        dq, dk, dv, _ = flash_bwd(q, k, v, out, dout, lse, ctx.causal, ctx.scale, fused=False)
         return dq, dk, dv, None, None
 
 
