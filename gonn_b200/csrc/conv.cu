@@ -21,9 +21,11 @@
 //
 // No tensor map is involved (every operand is gathered with ordinary loads from this GPU's own
 // memory), so the kernels may run inside multi-GPU jobs.  Every wait is bounded.
-#include "common.cuh"
+#include "conv.cuh"
 
 using namespace gb;
+using gbc::float_to_raw16;
+using gbc::raw16_to_float;
 
 namespace {
 
@@ -50,10 +52,6 @@ struct ConvArgs {
   long long r_per_split;   // wgrad: contraction indices per split (multiple of 64)
   int* status;
 };
-
-__device__ __forceinline__ float raw16_to_float(uint16_t u, int bf) {
-  return bf ? __uint_as_float((uint32_t)u << 16) : __half2float(__ushort_as_half(u));
-}
 
 // One 16-byte chunk (8 consecutive k) into row `row`, chunk `c8` of a K-major 128-byte-swizzled tile.
 __device__ __forceinline__ void store_chunk(uint8_t* tile, int row, int c8, const uint16_t (&v)[8]) {
@@ -339,174 +337,295 @@ conv_igemm_kernel(const ConvArgs a) {
   if (warp == 8) tmem_dealloc(tmem_base, CBN);
 }
 
-// dW[m][kk] = (beta ? dW : 0) + sum_s part[s][m][kk], in split order; written in the 16-bit type
-__global__ void conv_wgrad_finish_kernel(const float* __restrict__ part, uint16_t* __restrict__ dW, long long n,
-                                         int splits, int bf16, int beta) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    float s = beta ? raw16_to_float(dW[i], bf16) : 0.f;
-#pragma unroll 8
-    for (int sp = 0; sp < splits; sp++) s += part[(long long)sp * n + i];
-    dW[i] = bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(s)) : __half_as_ushort(__float2half_rn(s));
+// dW[m][c * T + tap] = (beta ? dW : 0) + sum_s part[s][m][kk], kk = (tap, c) when tap_major, else (c, tap).  A block
+// owns 32 consecutive elements; its eight warps add every eighth split and their sums are added in warp order
+// (deterministic).  One thread per element walked all splits alone: 9 us for 296 splits of 1728 elements.
+__global__ void __launch_bounds__(256) conv_wgrad_finish_kernel(const float* __restrict__ part, uint16_t* __restrict__ dW,
+                                                                long long n, int C, int T, int splits, int bf16, int beta,
+                                                                int tap_major) {
+  __shared__ float sm[8][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (long long b = blockIdx.x; b * 32 < n; b += gridDim.x) {
+    const long long i = b * 32 + lane;
+    float s = 0.f;
+    if (i < n) {
+#pragma unroll 4
+      for (int sp = warp; sp < splits; sp += 8) s += part[(long long)sp * n + i];
+    }
+    sm[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && i < n) {
+      const int K = C * T;
+      const long long m = i / K;
+      const int kk = (int)(i - m * K), tap = kk / C;
+      uint16_t* d = dW + (tap_major ? m * K + (long long)(kk - tap * C) * T + tap : i);
+      s = beta ? raw16_to_float(*d, bf16) : 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; w++) s += sm[w][lane];
+      *d = float_to_raw16(s, bf16);
+    }
+    __syncthreads();
   }
 }
 
-// Forward convolution with a short contraction (C * T <= 32: the first layer of an image network,
-// 3 channels x 3 x 3).  A tensor-core tile would spend its time on set-up: the implicit-GEMM kernel needs
-// about 15 us per CTA whatever the contraction length.  Here a thread owns one output position of one
-// image: it gathers its K inputs into registers once and then produces every output channel, four at a
-// time, with packed fp32 FMAs against weights that sit in shared memory as [k][channel] (one 16-byte
-// broadcast load feeds two FMA pairs).  Stores are coalesced along the positions.
+// Convolutions with a short contraction (C * T <= 32: the first layer of an image network, 3 channels x 3 x 3).
+// A tcgen05 tile would spend its time on set-up and an fp32 loop per position on its multiply-adds and their
+// weight reads (57 us forward, 97 us weight gradient at 256 x 64 channels x 900 positions); the contraction is
+// two k-steps of the warp-level mma.sync m16n8k16:
+//  * a warp takes 32 consecutive positions of the flattened batch; the index rows of those positions are
+//    contiguous in the map, so they are copied to shared memory with coalesced loads, and lane p gathers the K
+//    inputs of position p (neighbouring lanes, neighbouring addresses) into shared memory, from which the
+//    fragments are read.  Gathering the fragments directly cost eight sectors a load (43 and 55 us);
+//  * column n = 2t + e of n-tile j stands for position 8t + 2j + e, so a lane's results of the four n-tiles are eight
+//    consecutive positions of a channel (V of them at a time are aligned when V divides L).
+// Forward 22 us, weight gradient 45 us; bound by the gathers and the 29.5 MB of outputs or gradients.
 constexpr int kDirectK = 32;
-template <int KMAX>
-__global__ void __launch_bounds__(256)
-conv_direct_small_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w, const int* __restrict__ idx,
-                         const uint16_t* __restrict__ bias, uint16_t* __restrict__ y, int C, int S, int L, int T,
-                         int M, int bf16) {
-  extern __shared__ __align__(16) float sw[];          // [KMAX][M] weights, then [M] bias
-  float* sbias = sw + KMAX * M;
+constexpr int kSmallWarps = 8;
+
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2], int bf16) {
+  if (bf16)
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+  else
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// Index rows of positions p0 .. p0 + 31 into si[32 * T]: rows of consecutive positions follow one another, from the
+// end of an image's map to its beginning.  Returns the image of this lane's position.
+__device__ __forceinline__ void stage_index(int* si, const int* __restrict__ idx, long long p0, int L, int T, int& img) {
+  const int lane = threadIdx.x & 31;
+  const long long img0 = p0 / L;
+  const int l0 = (int)(p0 - img0 * L);
+  const long long LT = (long long)L * T;
+  __syncwarp();
+  for (int i = lane; i < 32 * T; i += 32) {
+    long long f = (long long)l0 * T + i;
+    while (f >= LT) f -= LT;
+    si[i] = __ldg(idx + f);
+  }
+  int l = l0 + lane;
+  img = (int)img0;
+  while (l >= L) { l -= L; img++; }
+  __syncwarp();
+}
+
+// The 32 (K of them real) inputs of this lane's position, two at a time, to put(k, v[k], v[k + 1]); image img, index rows si.
+template <typename F>
+__device__ __forceinline__ void gather_windows(const uint16_t* __restrict__ x, int img, bool live, const int* si, int C, int S, int T,
+                                               const F& put) {
   const int K = C * T;
-  for (int i = threadIdx.x; i < KMAX * M; i += blockDim.x) {
-    const int k = i / M, m = i - k * M;
-    sw[i] = k < K ? raw16_to_float(__ldg(w + (long long)m * K + k), bf16) : 0.f;
-  }
-  for (int m = threadIdx.x; m < M; m += blockDim.x) sbias[m] = bias ? raw16_to_float(__ldg(bias + m), bf16) : 0.f;
-  __syncthreads();
-  const int n = blockIdx.y;
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= L) return;
-  const uint16_t* xn = x + (long long)n * C * S;
-  float v[KMAX];
-  {
-    int c = 0, tap = 0;
+  const uint16_t* xc = x + (live ? (long long)img * C * S : 0);
+  const int* row = si + (threadIdx.x & 31) * T;
+  int tap = 0;
 #pragma unroll
-    for (int k = 0; k < KMAX; k++) {
-      float f = 0.f;
-      if (k < K) {
-        const int src = __ldg(idx + (long long)l * T + tap);
-        if (src >= 0) f = raw16_to_float(__ldg(xn + (long long)c * S + src), bf16);
-        if (++tap == T) { tap = 0; c++; }
+  for (int k = 0; k < kDirectK; k += 2) {
+    uint32_t v[2] = {0u, 0u};
+#pragma unroll
+    for (int e = 0; e < 2; e++)
+      if (k + e < K) {
+        const int src = row[tap];
+        if (live && src >= 0) v[e] = __ldg(xc + src);
+        if (++tap == T) { tap = 0; xc += S; }
       }
-      v[k] = f;
+    put(k, v[0], v[1]);
+  }
+  __syncwarp();
+}
+
+// Where the runs of V of the eight consecutive positions q0 .. q0 + 7 start in a (Nimg, M, L) tensor (channel 0), -1 past
+// the end.  V divides L, so a run never straddles images or the end.
+template <int V>
+__device__ __forceinline__ void run_starts(long long (&at)[8 / V], long long q0, long long P, int M, int L) {
+#pragma unroll
+  for (int i = 0; i < 8 / V; i++) {
+    const long long q = q0 + i * V, img = q / L;
+    at[i] = q < P ? img * M * L + (q - img * L) : -1;
+  }
+}
+// Eight values of a channel (row offset m * L), V at a time.
+template <int V>
+__device__ __forceinline__ void store8(uint16_t* __restrict__ y, const uint32_t (&v)[4], const long long (&at)[8 / V]) {
+#pragma unroll
+  for (int i = 0; i < 8 / V; i++) {
+    if (at[i] < 0) return;
+    uint16_t* d = y + at[i];
+    if constexpr (V == 8) *reinterpret_cast<uint4*>(d) = make_uint4(v[0], v[1], v[2], v[3]);
+    else if constexpr (V == 4) *reinterpret_cast<uint2*>(d) = make_uint2(v[2 * i], v[2 * i + 1]);
+    else if constexpr (V == 2) *reinterpret_cast<uint32_t*>(d) = v[i];
+    else *d = (uint16_t)(v[i / 2] >> (16 * (i & 1)));
+  }
+}
+template <int V>
+__device__ __forceinline__ void load8(const uint16_t* __restrict__ y, uint32_t (&v)[4], const long long (&at)[8 / V]) {
+#pragma unroll
+  for (int i = 0; i < 4; i++) v[i] = 0u;
+#pragma unroll
+  for (int i = 0; i < 8 / V; i++) {
+    if (at[i] < 0) return;
+    const uint16_t* d = y + at[i];
+    if constexpr (V == 8) {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(d));
+      v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+    } else if constexpr (V == 4) {
+      const uint2 u = __ldg(reinterpret_cast<const uint2*>(d));
+      v[2 * i] = u.x; v[2 * i + 1] = u.y;
+    } else if constexpr (V == 2) {
+      v[i] = __ldg(reinterpret_cast<const uint32_t*>(d));
+    } else {
+      v[i / 2] |= (uint32_t)__ldg(d) << (16 * (i & 1));
     }
   }
-  uint16_t* yn = y + (long long)n * M * L + l;
-  const float4* sw4 = reinterpret_cast<const float4*>(sw);
-  const int M4 = M >> 2;
-  for (int m4 = 0; m4 < M4; m4++) {
-    float2 a0 = make_float2(sbias[4 * m4], sbias[4 * m4 + 1]);
-    float2 a1 = make_float2(sbias[4 * m4 + 2], sbias[4 * m4 + 3]);
+}
+
+// y[n][m][l] = bias[m] + sum_k w[m][k] x[n][c(k)][idx[l][tap(k)]]: A = weights (16 channels x 16 k), B = windows (16 k x 8
+// positions).  The weights sit in shared memory in fragment order.
+template <int V>
+__global__ void __launch_bounds__(kSmallWarps * 32)
+conv_direct_small_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w, const int* __restrict__ idx,
+                         const uint16_t* __restrict__ bias, uint16_t* __restrict__ y, int Nimg, int C, int S, int L, int T,
+                         int M, int bf16) {
+  extern __shared__ __align__(16) uint32_t dsm[];
+  const int MT = (M + 15) / 16, K = C * T;
+  uint32_t* wf = dsm;                                    // [MT][2 k-steps][32 lanes][4]
+  float* sbias = reinterpret_cast<float*>(wf + MT * 256);   // [MT * 16]
+  int* si = reinterpret_cast<int*>(sbias + MT * 16) + (threadIdx.x >> 5) * 32 * (T + 17);
+  uint32_t* sp = reinterpret_cast<uint32_t*>(si + 32 * T);   // [32 positions][16 pairs of k], pitch 17
+  auto wval = [&](int m, int k) -> uint32_t { return m < M && k < K ? (uint32_t)__ldg(w + (long long)m * K + k) : 0u; };
+  for (int i = threadIdx.x; i < MT * 256; i += blockDim.x) {
+    const int r = i & 3, ln = (i >> 2) & 31, ks = (i >> 7) & 1, mt = i >> 8;
+    const int m = mt * 16 + (ln >> 2) + 8 * (r & 1), k = ks * 16 + 2 * (ln & 3) + 8 * (r >> 1);
+    wf[i] = wval(m, k) | (wval(m, k + 1) << 16);
+  }
+  for (int i = threadIdx.x; i < MT * 16; i += blockDim.x) sbias[i] = bias != nullptr && i < M ? raw16_to_float(__ldg(bias + i), bf16) : 0.f;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const long long P = (long long)Nimg * L;
+  const long long warps = (long long)gridDim.x * kSmallWarps;
+  for (long long p0 = ((long long)blockIdx.x * kSmallWarps + (threadIdx.x >> 5)) * 32; p0 < P; p0 += warps * 32) {
+    int img;
+    stage_index(si, idx, p0, L, T, img);
+    long long at[8 / V];
+    run_starts<V>(at, p0 + 8 * t, P, M, L);
+    gather_windows(x, img, p0 + lane < P, si, C, S, T, [&](int k, uint32_t lo, uint32_t hi) { sp[lane * 17 + (k >> 1)] = lo | (hi << 16); });
+    uint32_t b[4][2][2];
 #pragma unroll
-    for (int k = 0; k < KMAX; k++) {
-      const float4 wv = sw4[k * M4 + m4];
-      const float2 vv = make_float2(v[k], v[k]);
-      a0 = __ffma2_rn(make_float2(wv.x, wv.y), vv, a0);
-      a1 = __ffma2_rn(make_float2(wv.z, wv.w), vv, a1);
+    for (int j = 0; j < 4; j++) {
+      const uint32_t* row = sp + ((g >> 1) * 8 + 2 * j + (g & 1)) * 17 + t;      // position of column n = g
+#pragma unroll
+      for (int ks = 0; ks < 2; ks++)
+#pragma unroll
+        for (int r = 0; r < 2; r++) b[j][ks][r] = row[ks * 8 + r * 4];
     }
-    const float o[4] = {a0.x, a0.y, a1.x, a1.y};
+    for (int mt = 0; mt < MT; mt++) {
+      const float b0 = sbias[mt * 16 + g], b1 = sbias[mt * 16 + g + 8];
+      float c[4][4];
+      uint32_t af[2][4];
+#pragma unroll
+      for (int ks = 0; ks < 2; ks++) {
+        const uint4 u = *reinterpret_cast<const uint4*>(wf + ((mt * 2 + ks) * 32 + lane) * 4);
+        af[ks][0] = u.x; af[ks][1] = u.y; af[ks][2] = u.z; af[ks][3] = u.w;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        c[j][0] = c[j][1] = b0;
+        c[j][2] = c[j][3] = b1;
+#pragma unroll
+        for (int ks = 0; ks < 2; ks++) mma16816(c[j], af[ks], b[j][ks], bf16);
+      }
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        const int m = mt * 16 + g + 8 * r;
+        if (m >= M) continue;
+        uint32_t v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = float_to_raw16(c[j][2 * r], bf16) | ((uint32_t)float_to_raw16(c[j][2 * r + 1], bf16) << 16);
+        store8<V>(y + (long long)m * L, v, at);
+      }
+    }
+  }
+}
+
+// dW[m][k] = sum over positions p (all images) of dy[p][m] * window[p][k]: A = dy (16 channels x 16 positions), B = windows (16
+// positions x 8 k).  Slots 2t, 2t + 1 and 2t + 8, 2t + 9 of k-step s are positions 8t + 4s + {0, 1} and {2, 3} of the
+// warp's 32, so a lane reads eight consecutive values of a channel.  A warp keeps 64 (or 32) channels x 32 k in
+// registers; the CTA's warps are added in order and the CTA writes one partial matrix.  blockIdx.y: group of channels.
+template <int MT, int V>
+__global__ void __launch_bounds__(kSmallWarps * 32, 2)
+conv_wgrad_small_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ dy, const int* __restrict__ idx,
+                        float* __restrict__ part, int Nimg, int C, int S, int L, int T, int M, int bf16) {
+  extern __shared__ __align__(16) uint32_t dsm[];
+  const int K = C * T, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  int* si = reinterpret_cast<int*>(dsm) + warp * 32 * (T + 17);
+  uint16_t* sp = reinterpret_cast<uint16_t*>(si + 32 * T);   // [32 k][32 positions], pitch 34
+  const int m0 = blockIdx.y * (MT * 16);
+  float acc[MT][4][4];
+#pragma unroll
+  for (int i = 0; i < MT; i++)
 #pragma unroll
     for (int j = 0; j < 4; j++)
-      yn[(long long)(4 * m4 + j) * L] = bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(o[j]))
-                                             : __half_as_ushort(__float2half_rn(o[j]));
+#pragma unroll
+      for (int e = 0; e < 4; e++) acc[i][j][e] = 0.f;
+  const long long P = (long long)Nimg * L;
+  const long long warps = (long long)gridDim.x * kSmallWarps;
+  for (long long p0 = ((long long)blockIdx.x * kSmallWarps + warp) * 32; p0 < P; p0 += warps * 32) {
+    int img;
+    stage_index(si, idx, p0, L, T, img);
+    long long at[8 / V];
+    run_starts<V>(at, p0 + 8 * t, P, M, L);
+    gather_windows(x, img, p0 + lane < P, si, C, S, T, [&](int k, uint32_t lo, uint32_t hi) {
+      sp[k * 34 + lane] = (uint16_t)lo;
+      sp[(k + 1) * 34 + lane] = (uint16_t)hi;
+    });
+    uint32_t b[4][2][2];
+#pragma unroll
+    for (int nt = 0; nt < 4; nt++) {
+      const uint32_t* row = reinterpret_cast<const uint32_t*>(sp) + (nt * 8 + g) * 17 + 4 * t;   // positions 8t ..
+#pragma unroll
+      for (int h = 0; h < 2; h++)                        // k-steps
+#pragma unroll
+        for (int r = 0; r < 2; r++) b[nt][h][r] = row[2 * h + r];
+    }
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++) {
+      uint32_t lo[4], hi[4];
+      load8<V>(dy + (long long)(m0 + mt * 16 + g) * L, lo, at);
+      load8<V>(dy + (long long)(m0 + mt * 16 + g + 8) * L, hi, at);
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const uint32_t af[4] = {lo[2 * h], hi[2 * h], lo[2 * h + 1], hi[2 * h + 1]};
+#pragma unroll
+        for (int nt = 0; nt < 4; nt++) mma16816(acc[mt][nt], af, b[nt][h], bf16);
+      }
+    }
   }
+  __syncthreads();
+  float* red = reinterpret_cast<float*>(dsm);            // [MT * 16][32], reusing the index rows
+  for (int w = 0; w < kSmallWarps; w++) {
+    if (warp == w) {
+#pragma unroll
+      for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+        for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            float* d = red + (mt * 16 + g + 8 * (e >> 1)) * kDirectK + nt * 8 + 2 * t + (e & 1);
+            *d = w == 0 ? acc[mt][nt][e] : *d + acc[mt][nt][e];
+          }
+    }
+    __syncthreads();
+  }
+  float* out = part + ((long long)blockIdx.x * M + m0) * K;
+  for (int i = threadIdx.x; i < MT * 16 * K; i += blockDim.x) out[i] = red[(i / K) * kDirectK + i % K];
 }
 
-// Weight gradient for the same short contractions (C * T <= 32), M = 32, 64 or 128 output channels:
-//   dW[m][k] = sum over positions p (all images) of dy[p][m] * patch[p][k].
-// A CTA walks its share of the positions in tiles of 256: every thread gathers the K inputs of one
-// position and the M gradients of that position into shared memory (rows padded by four words so that
-// 16-byte accesses of consecutive rows fall into different banks), then the CTA's 256 threads form
-// 256 / M position groups of M threads; a thread accumulates a 4 (channels) x 8 (k) block of dW over its
-// group's positions with three 16-byte shared loads per 32 FMAs.  The groups are added in order at the
-// end and the CTA writes one partial matrix; conv_wgrad_finish_kernel adds the CTAs in index order.
-template <int M>
-__global__ void __launch_bounds__(256, 2)
-conv_wgrad_small_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ dy, const int* __restrict__ idx,
-                        float* __restrict__ part, int Nimg, int C, int S, int L, int T, int bf16) {
-  constexpr int KMAX = kDirectK, PS = KMAX + 4, GS = M + 4, GROUPS = 256 / M;
-  extern __shared__ __align__(16) float smw[];
-  float* sP = smw;                 // [256][PS]  patches
-  float* sG = smw + 256 * PS;      // [256][GS]  gradients
-  const int K = C * T;
-  const long long P = (long long)Nimg * L;
-  const long long per = ((P + gridDim.x - 1) / gridDim.x + 255) / 256 * 256;
-  const long long p_begin = (long long)blockIdx.x * per;
-  const long long p_end = p_begin + per < P ? p_begin + per : P;
-  const int t = threadIdx.x;
-  const int grp = t / M, tm = t % M;           // position group; 4-channel block and k block inside it
-  const int co4 = tm >> 2, kq = tm & 3;
-  float acc[4][8];
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
-  for (long long p0 = p_begin; p0 < p_end; p0 += 256) {
-    __syncthreads();                            // the previous tile has been consumed
-    {
-      const long long p = p0 + t;
-      const bool live = p < p_end;
-      const long long n = live ? p / L : 0;
-      const int l = (int)(p - n * L);
-      const uint16_t* xn = x + n * C * S;
-      float v[KMAX];
-      int c = 0, tap = 0;
-#pragma unroll
-      for (int k = 0; k < KMAX; k++) {
-        float f = 0.f;
-        if (k < K) {
-          const int src = live ? __ldg(idx + (long long)l * T + tap) : -1;
-          if (src >= 0) f = raw16_to_float(__ldg(xn + (long long)c * S + src), bf16);
-          if (++tap == T) { tap = 0; c++; }
-        }
-        v[k] = f;
-      }
-#pragma unroll
-      for (int k4 = 0; k4 < KMAX / 4; k4++)
-        *reinterpret_cast<float4*>(sP + t * PS + 4 * k4) = make_float4(v[4 * k4], v[4 * k4 + 1], v[4 * k4 + 2], v[4 * k4 + 3]);
-      const uint16_t* gn = dy + n * M * L + l;
-#pragma unroll 4
-      for (int m4 = 0; m4 < M / 4; m4++) {
-        float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (live) {
-          g.x = raw16_to_float(__ldg(gn + (long long)(4 * m4) * L), bf16);
-          g.y = raw16_to_float(__ldg(gn + (long long)(4 * m4 + 1) * L), bf16);
-          g.z = raw16_to_float(__ldg(gn + (long long)(4 * m4 + 2) * L), bf16);
-          g.w = raw16_to_float(__ldg(gn + (long long)(4 * m4 + 3) * L), bf16);
-        }
-        *reinterpret_cast<float4*>(sG + t * GS + 4 * m4) = g;
-      }
-    }
-    __syncthreads();
-    // group grp takes positions grp, grp + GROUPS, ... of the tile
-#pragma unroll 2
-    for (int q = grp; q < 256; q += GROUPS) {
-      const float4 g = *reinterpret_cast<const float4*>(sG + q * GS + 4 * co4);
-      const float4 pa = *reinterpret_cast<const float4*>(sP + q * PS + 8 * kq);
-      const float4 pb = *reinterpret_cast<const float4*>(sP + q * PS + 8 * kq + 4);
-      const float gv[4] = {g.x, g.y, g.z, g.w};
-      const float pv[8] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 8; j++) acc[i][j] = fmaf(gv[i], pv[j], acc[i][j]);
-    }
-  }
-  // add the position groups in order: group 0 writes, the others add one after another
-  __syncthreads();
-  float* red = smw;                             // [M][KMAX], reusing the tile memory
-  for (int gsel = 0; gsel < GROUPS; gsel++) {
-    if (grp == gsel) {
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-          float* dst = red + (4 * co4 + i) * KMAX + 8 * kq + j;
-          *dst = gsel == 0 ? acc[i][j] : *dst + acc[i][j];
-        }
-    }
-    __syncthreads();
-  }
-  float* out = part + (long long)blockIdx.x * M * K;
-  for (int i = t; i < M * K; i += 256) out[i] = red[(i / K) * KMAX + i % K];
+// Widest run of positions that stays aligned from image to image.
+inline int run_width(int L, const void* p) {
+  const uintptr_t a = (uintptr_t)p;
+  if (L % 8 == 0 && (a & 15) == 0) return 8;
+  if (L % 4 == 0 && (a & 7) == 0) return 4;
+  if (L % 2 == 0 && (a & 3) == 0) return 2;
+  return 1;
 }
 
 inline int wgrad_small_ctas(long long P) {
@@ -527,6 +646,14 @@ int set_attr_once() {
 }
 
 }  // namespace
+
+int gbc::launch_wgrad_finish(const float* part, uint16_t* dW, int M, int C, int T, int splits, int bf16, int beta, bool tap_major,
+                             cudaStream_t s) {
+  const long long n = (long long)M * C * T, blocks = (n + 31) / 32;
+  conv_wgrad_finish_kernel<<<(int)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, s>>>(part, dW, n, C, T, splits, bf16, beta, tap_major);
+  GB_CUDA_OK(cudaGetLastError());
+  return gbh::E_OK;
+}
 
 enum { DT_BF16 = 0, DT_F16 = 1 };
 
@@ -581,10 +708,23 @@ GB_EXPORT int gb_conv_direct_small(int dtype, const void* x, const void* w, cons
     gbh::set_error("gb_conv_direct_small: needs C * T <= %d, a channel count that is a multiple of 4, at most 65535 images", kDirectK);
     return gbh::E_BAD_ARG;
   }
-  const size_t smem = (size_t)(kDirectK + 1) * M * sizeof(float);
-  dim3 grid((L + 255) / 256, Nimg);
-  conv_direct_small_kernel<kDirectK><<<grid, 256, smem, (cudaStream_t)stream>>>(
-      (const uint16_t*)x, (const uint16_t*)w, idx, (const uint16_t*)bias, (uint16_t*)y, C, S, L, T, M, dtype == DT_BF16);
+  const int mt = (M + 15) / 16;
+  const size_t smem = (size_t)mt * 256 * 4 + mt * 16 * 4 + (size_t)kSmallWarps * 32 * (T + 17) * 4;
+  const long long blocks = ((long long)Nimg * L + 32 * kSmallWarps - 1) / (32 * kSmallWarps);
+  const int grid = (int)(blocks < 148 * 8 ? blocks : 148 * 8);
+#define GB_DS(V)                                                                                                          \
+  {                                                                                                                       \
+    GB_CUDA_OK(cudaFuncSetAttribute(conv_direct_small_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024)); \
+    conv_direct_small_kernel<V><<<grid, kSmallWarps * 32, smem, (cudaStream_t)stream>>>(                                  \
+        (const uint16_t*)x, (const uint16_t*)w, idx, (const uint16_t*)bias, (uint16_t*)y, Nimg, C, S, L, T, M, dtype == DT_BF16); \
+  }
+  switch (run_width(L, y)) {
+    case 8: GB_DS(8) break;
+    case 4: GB_DS(4) break;
+    case 2: GB_DS(2) break;
+    default: GB_DS(1)
+  }
+#undef GB_DS
   GB_CUDA_OK(cudaGetLastError());
   return gbh::E_OK;
 }
@@ -618,25 +758,25 @@ GB_EXPORT int gb_conv_wgrad(int dtype, const void* x, const void* dy, const int*
   const int splits = gb_conv_wgrad_splits(Nimg, L, M, C, T);
   const long long R = (long long)Nimg * L;
   if (wgrad_small_ok(C, T, M)) {
-    const size_t smem = (size_t)256 * ((kDirectK + 4) + (M + 4)) * sizeof(float);
     const int bf = dtype == DT_BF16;
-#define GB_WS(MM)                                                                                              \
-  {                                                                                                            \
-    static bool cfg = false;                                                                                   \
-    if (!cfg) {                                                                                                \
-      GB_CUDA_OK(cudaFuncSetAttribute(conv_wgrad_small_kernel<MM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-      cfg = true;                                                                                              \
-    }                                                                                                          \
-    conv_wgrad_small_kernel<MM><<<splits, 256, smem, (cudaStream_t)stream>>>(                                  \
-        (const uint16_t*)x, (const uint16_t*)dy, idx, part, Nimg, C, S, L, T, bf);                             \
+    const size_t idx_bytes = (size_t)kSmallWarps * 32 * (T + 17) * 4;
+#define GB_WS(MT, V)                                                                                               \
+  {                                                                                                                \
+    const size_t red = (size_t)MT * 16 * kDirectK * 4, smem = idx_bytes > red ? idx_bytes : red;                   \
+    conv_wgrad_small_kernel<MT, V><<<dim3(splits, M / (MT * 16)), kSmallWarps * 32, smem, (cudaStream_t)stream>>>( \
+        (const uint16_t*)x, (const uint16_t*)dy, idx, part, Nimg, C, S, L, T, M, bf);                              \
   }
-    if (M == 32) GB_WS(32) else if (M == 64) GB_WS(64) else GB_WS(128)
+#define GB_WV(MT)                    \
+  switch (run_width(L, dy)) {        \
+    case 8: GB_WS(MT, 8) break;      \
+    case 4: GB_WS(MT, 4) break;      \
+    case 2: GB_WS(MT, 2) break;      \
+    default: GB_WS(MT, 1)            \
+  }
+    if (M == 32) { GB_WV(2) } else { GB_WV(4) }
+#undef GB_WV
 #undef GB_WS
-    const long long nn = (long long)M * C * T;
-    conv_wgrad_finish_kernel<<<(int)((nn + 255) / 256 < 592 ? (nn + 255) / 256 : 592), 256, 0, (cudaStream_t)stream>>>(
-        part, (uint16_t*)dw, nn, splits, bf, beta);
-    GB_CUDA_OK(cudaGetLastError());
-    return gbh::E_OK;
+    return gbc::launch_wgrad_finish(part, (uint16_t*)dw, M, C, T, splits, bf, beta, false, (cudaStream_t)stream);
   }
   long long per = (R + splits - 1) / splits;
   per = (per + CBK - 1) / CBK * CBK;
@@ -651,9 +791,5 @@ GB_EXPORT int gb_conv_wgrad(int dtype, const void* x, const void* dy, const int*
   const int K = C * T;
   dim3 grid((K + CBN - 1) / CBN, (M + CBM - 1) / CBM, splits);
   conv_igemm_kernel<1><<<grid, CTHREADS, CSMEM, (cudaStream_t)stream>>>(a);
-  const long long n = (long long)M * K;
-  conv_wgrad_finish_kernel<<<(int)((n + 255) / 256 < 592 ? (n + 255) / 256 : 592), 256, 0, (cudaStream_t)stream>>>(
-      part, (uint16_t*)dw, n, splits, a.bf16, beta);
-  GB_CUDA_OK(cudaGetLastError());
-  return gbh::E_OK;
+  return gbc::launch_wgrad_finish(part, (uint16_t*)dw, M, C, T, splits, a.bf16, beta, false, (cudaStream_t)stream);
 }

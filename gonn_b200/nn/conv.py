@@ -1,7 +1,7 @@
 """Convolutions, transposed convolutions, Unfold / Fold (nn/conv.go:17-463, nn/fold.go:45-142).
 
 16-bit CUDA tensors with groups = 1 and zero padding run as implicit GEMMs on tcgen05
-(csrc/conv.cu): forward, data gradient and weight gradient gather their operands inside the
+(csrc/conv_cl.cu for channel counts that are multiples of 8, csrc/conv.cu otherwise): forward, data gradient and weight gradient gather their operands inside the
 kernel through the window index map, with the bias in the forward epilogue and the weight
 gradient as one GEMM over the whole batch.  Everything else takes the general path:
 forward = im2col by index map (no dense gather matrix) followed by one GEMM per group
@@ -105,6 +105,11 @@ class _ConvImplicit(torch.autograd.Function):
             # a contraction of at most 32 (3 channels x 3 x 3): one thread per output position, no tensor-core tile
             _l.call("gb_conv_direct_small", _l.I(_l.dtype_code(x3.dtype)), _l.ptr(xc), _l.ptr(wc), _l.ptr(didx),
                     _l.ptr(bias), _l.ptr(y), _l.I(N), _l.I(C), _l.I(S), _l.I(L), _l.I(T), _l.I(Co), _l.stream_ptr())
+        elif _l.lib().gb_conv_cl_ok(N, C, S, L, T, Co, 0):
+            # channel counts that are multiples of 8: 16-byte copies from a channels-last scratch
+            ws = torch.empty(int(_l.lib().gb_conv_cl_fwd_ws(N, C, S, T, Co)), dtype=x3.dtype, device=x3.device)
+            _l.call("gb_conv_cl_fwd", _l.I(_l.dtype_code(x3.dtype)), _l.ptr(xc), _l.ptr(wc), _l.ptr(didx), _l.ptr(bias),
+                    _l.ptr(y), _l.ptr(ws), _l.I(N), _l.I(C), _l.I(S), _l.I(L), _l.I(T), _l.I(Co), _l.stream_ptr())
         else:
             _l.call("gb_conv_igemm", _l.I(_l.dtype_code(x3.dtype)), _l.ptr(xc), _l.ptr(wc),
                     _l.ptr(_ktab(C, T, S, x3.device)), _l.ptr(didx), _l.ptr(bias), _l.ptr(y), _l.I(N), _l.I(C), _l.I(S),
@@ -126,16 +131,12 @@ class _ConvImplicit(torch.autograd.Function):
         dyc = dy.contiguous()
         dt = _l.dtype_code(xc.dtype)
         dx = dw = db = None
-        if ctx.needs_input_grad[0]:
+        need_dx, need_dw = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
+        if need_dx:
             inv = device_maps(_inverse_map(idx, S), L, xc.device, False)["idx"]
-            wt = wc.view(Co, C, T).permute(1, 0, 2).contiguous()        # (C_in, C_out * T)
             dx = torch.empty_like(xc)
-            _l.call("gb_conv_igemm", _l.I(dt), _l.ptr(dyc), _l.ptr(wt), _l.ptr(_ktab(Co, T, L, xc.device)), _l.ptr(inv),
-                    None, _l.ptr(dx), _l.I(N), _l.I(Co), _l.I(L), _l.I(S), _l.I(T), _l.I(C), _l.stream_ptr())
-        if ctx.needs_input_grad[1]:
+        if need_dw:
             didx = device_maps(idx, S, xc.device, False)["idx"]
-            splits = int(_l.lib().gb_conv_wgrad_splits(N, L, Co, C, T))
-            part = torch.empty(splits * Co * C * T, dtype=torch.float32, device=xc.device)
             w = ctx.weight_ref
             sink = getattr(w, "_gb_sink", None)
             if sink is not None:
@@ -143,9 +144,28 @@ class _ConvImplicit(torch.autograd.Function):
                 out, beta = buf, not fresh
             else:
                 out, beta = torch.empty(Co * C * T, dtype=xc.dtype, device=xc.device), False
-            _l.call("gb_conv_wgrad", _l.I(dt), _l.ptr(xc), _l.ptr(dyc), _l.ptr(_ktab(C, T, S, xc.device)), _l.ptr(didx),
-                    _l.ptr(out), _l.ptr(part), _l.I(N), _l.I(C), _l.I(S), _l.I(L), _l.I(T), _l.I(Co), _l.I(int(beta)),
-                    _l.stream_ptr())
+        # (a first layer asks for no dx and its short contraction has a kernel of its own)
+        if (need_dx or need_dw) and _l.lib().gb_conv_cl_ok(N, C, S, L, T, Co, 1):
+            ws = torch.empty(int(_l.lib().gb_conv_cl_bwd_ws(N, C, S, L, T, Co, int(need_dx), int(need_dw))), dtype=xc.dtype,
+                             device=xc.device)
+            part = (torch.empty(int(_l.lib().gb_conv_cl_part(N, C, L, T, Co)), dtype=torch.float32, device=xc.device)
+                    if need_dw else None)
+            _l.call("gb_conv_cl_bwd", _l.I(dt), _l.ptr(xc), _l.ptr(wc), _l.ptr(dyc), _l.ptr(didx if need_dw else None),
+                    _l.ptr(inv if need_dx else None), _l.ptr(dx), _l.ptr(out if need_dw else None),
+                    _l.I(int(need_dw and beta)), _l.ptr(ws), _l.ptr(part), _l.I(N), _l.I(C), _l.I(S), _l.I(L), _l.I(T),
+                    _l.I(Co), _l.stream_ptr())
+        else:
+            if need_dx:
+                wt = wc.view(Co, C, T).permute(1, 0, 2).contiguous()        # (C_in, C_out * T)
+                _l.call("gb_conv_igemm", _l.I(dt), _l.ptr(dyc), _l.ptr(wt), _l.ptr(_ktab(Co, T, L, xc.device)), _l.ptr(inv),
+                        None, _l.ptr(dx), _l.I(N), _l.I(Co), _l.I(L), _l.I(S), _l.I(T), _l.I(C), _l.stream_ptr())
+            if need_dw:
+                splits = int(_l.lib().gb_conv_wgrad_splits(N, L, Co, C, T))
+                part = torch.empty(splits * Co * C * T, dtype=torch.float32, device=xc.device)
+                _l.call("gb_conv_wgrad", _l.I(dt), _l.ptr(xc), _l.ptr(dyc), _l.ptr(_ktab(C, T, S, xc.device)), _l.ptr(didx),
+                        _l.ptr(out), _l.ptr(part), _l.I(N), _l.I(C), _l.I(S), _l.I(L), _l.I(T), _l.I(Co), _l.I(int(beta)),
+                        _l.stream_ptr())
+        if need_dw:
             if sink is not None:
                 sink.ready(w)
             else:
