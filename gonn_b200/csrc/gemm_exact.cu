@@ -3,10 +3,8 @@
 // The reference's float64 / float32 products are cuBLAS Dgemm / Sgemm calls
 // (backend/cuda/gonn_cuda.cu:147-177, 255-294, 616-622).  tcgen05 has no fp64 or fp32 form, so:
 //
-// * fp64: a double-precision tensor-core main loop (mma.sync m8n8k4 f64): 128 x 128 x 16 CTA
-//   tiles, sixteen warps of 32 x 32, operands staged through a three-deep cp.async ring in a
-//   [k][m] layout whose padding makes every fragment load conflict-free.  Results match an
-//   fp64 FMA chain in k order within a tile (1e-13-class agreement with a float64 oracle).
+// * fp64: mma.sync m16n8k8 f64 on 64 x 64 x 16 tiles.  Results match an fp64 FMA chain over k up to the order of
+//   the sum (1e-13-class agreement with a float64 oracle).
 // * fp32: each operand is split once into three bf16 planes (x = hi + mid + lo, 24 mantissa
 //   bits in total) and the six significant plane products hi*hi, hi*mid, mid*hi, hi*lo,
 //   lo*hi, mid*mid run as bf16 tcgen05 GEMMs over an extended K axis (six times the length in
@@ -41,190 +39,235 @@ namespace {
 enum { DT_BF16 = 0, DT_F16 = 1, DT_F32 = 2, DT_F64 = 3 };
 
 // ---------------------------------------------------------------------------
-// fp64: mma.sync m8n8k4
+// fp64: mma.sync m16n8k8
 // ---------------------------------------------------------------------------
-#ifndef GB_F64_BK
-#define GB_F64_BK 16        // k extent of a stage (a multiple of 16)
-#endif
-#ifndef GB_F64_STAGES
-#define GB_F64_STAGES 3
-#endif
-constexpr int DBM = 128, DBN = 128, DBK = GB_F64_BK, DSTAGES = GB_F64_STAGES;
-static_assert(DBK % 16 == 0 && DSTAGES >= 2, "stage shape");
-constexpr int DLD = DBM + 4;  // row pitch of a [k][m] stage in doubles: fragment loads hit 16 distinct bank pairs
-constexpr int DTHREADS = 512;
-constexpr int DSTAGE_DOUBLES = 2 * DBK * DLD;
+// Bound by the fp64 tensor pipe (64 multiply-adds per SM and clock).  128 x 128 tiles of one 512-thread CTA kept
+// it 68 % active: half the stalls were shared-memory instructions (8-byte fragments and 8-byte copies) and the
+// barrier that all 16 warps share, and 256 such tiles leave 14 % of two waves empty at 2048^3 (790 us, now 571; 512^3 102, now 17).  Here a CTA
+// is 64 x 64 x 16 with four warps of 32 x 32, four CTAs per SM that wait for nobody else's barrier, and
+//  * an operand whose contiguous dimension is k is staged as [8-wide k block][row][8]: 16-byte copies, and one
+//    16-byte read gives a lane the elements k = 2t and 2t + 1 of a row, which stand in the fragment's slots t and
+//    t + 4 on both sides (the order of the contraction within a block of eight is free);
+//  * the other form is staged as [k][row] with pitch 66: rows 2t and 2t + 1 are read without bank conflicts;
+//  * when the tiles alone leave SMs idle, a cluster of 2, 4 or 8 CTAs cuts K and adds its parts through
+//    distributed shared memory in rank order: no workspace, no second launch, deterministic.
+constexpr int DB = 64, DBK = 16, DSTAGES = 3;
+constexpr int DTHREADS = 128;
+constexpr int DPITCH = DB + 2;                          // [k][row] form
+constexpr int DOP = DBK * DPITCH;                       // doubles of one operand stage (the larger form)
+constexpr int DSMEM = DSTAGES * 2 * DOP * 8;
+static_assert(DB * DB <= DSTAGES * 2 * DOP, "the cluster's partial tiles reuse the stages");
 
 __device__ __forceinline__ void cp_async8(void* dst, const void* src, bool pred) {
   const int n = pred ? 8 : 0;  // src-size 0: the destination is zero-filled
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n) : "memory");
 }
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool pred) {
-  const int n = pred ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n) : "memory");
+// 16 bytes of which `bytes` (0, 8 or 16) come from memory and the rest are zero
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(c0), "+d"(c1)
-               : "d"(a), "d"(b));
-}
-// m16n8k8: A (16 x 8): a0 (g, t), a1 (g + 8, t), a2 (g, t + 4), a3 (g + 8, t + 4); B (8 x 8): b0 (t, g),
-// b1 (t + 4, g); C (16 x 8): c0, c1 (g, 2t + {0, 1}), c2, c3 (g + 8, 2t + {0, 1}); g = lane / 4, t = lane % 4.
+// A (16 x 8): a0 (g, t), a1 (g + 8, t), a2 (g, t + 4), a3 (g + 8, t + 4); B (8 x 8): b0 (t, g), b1 (t + 4, g);
+// C (16 x 8): c0, c1 (g, 2t + {0, 1}), c2, c3 (g + 8, 2t + {0, 1}); g = lane / 4, t = lane % 4.
 __device__ __forceinline__ void dmma16(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-      "{%0, %1, %2, %3};"
+  asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
       : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
       : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
-// Copies one operand tile into a [k][mn] stage.  `k_contig`: the operand is stored with k as
-// the contiguous dimension ((mn, k) row-major), so the copy transposes (8-byte pieces);
-// otherwise rows of the stage are contiguous in memory (16-byte pieces when aligned).
-__device__ __forceinline__ void load_tile(double* st, const double* src, long long ld, bool k_contig, int mn0,
-                                          int k0, int MN, int K, bool vec_ok) {
-  const int tid = threadIdx.x;
-  if (k_contig) {
-    // 128 rows x DBK k: thread -> (row = tid / 4, DBK / 4 consecutive k)
-    const int r = tid >> 2, kq = (tid & 3) * (DBK / 4);
-    const long long row = (long long)mn0 + r;
+// 64 rows (of MN) x 16 k of an operand into a stage.  KC: stored (MN, K), else (K, MN); k runs to k_end.
+template <bool KC>
+__device__ __forceinline__ void load_tile(double* st, const double* src, long long ld, int mn0, int k0, int MN, int k_end, bool vec) {
+  if (vec) {
 #pragma unroll
-    for (int i = 0; i < DBK / 4; i++) {
-      const int k = k0 + kq + i;
-      const bool ok = row < MN && k < K;
-      cp_async8(st + (kq + i) * DLD + r, ok ? src + row * ld + k : src, ok);
+    for (int i = 0; i < DB * DBK / 2 / DTHREADS; i++) {
+      const int q = threadIdx.x + i * DTHREADS;
+      if (KC) {
+        const int r = q >> 3, c = q & 7, k = k0 + 2 * c;
+        const int have = mn0 + r < MN ? min(2, max(0, k_end - k)) * 8 : 0;
+        cp_async16(st + ((c >> 2) * DB + r) * 8 + (c & 3) * 2, have ? src + (long long)(mn0 + r) * ld + k : src, have);
+      } else {
+        const int kk = q >> 5, c = (q & 31) * 2, k = k0 + kk;
+        const int have = k < k_end ? min(2, max(0, MN - mn0 - c)) * 8 : 0;
+        cp_async16(st + kk * DPITCH + c, have ? src + (long long)k * ld + mn0 + c : src, have);
+      }
     }
   } else {
-    // DBK k rows x 128 contiguous, 16 rows per pass: thread -> (k = tid / 32, four consecutive doubles)
-    const int c = (tid & 31) * 4;
 #pragma unroll
-    for (int pass = 0; pass < DBK / 16; pass++) {
-      const int kk = pass * 16 + (tid >> 5);
-      const int k = k0 + kk;
-      const double* g = src + (long long)k * ld + mn0 + c;
-      double* d = st + kk * DLD + c;
-      if (vec_ok && k < K && mn0 + c + 3 < MN) {
-        cp_async16(d, g, true);
-        cp_async16(d + 2, g + 2, true);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const bool ok = k < K && mn0 + c + i < MN;
-          cp_async8(d + i, ok ? g + i : src, ok);
-        }
-      }
+    for (int i = 0; i < DB * DBK / DTHREADS; i++) {
+      const int q = threadIdx.x + i * DTHREADS;
+      const int r = KC ? q >> 4 : q & 63, kk = KC ? q & 15 : q >> 6;
+      const bool ok = mn0 + r < MN && k0 + kk < k_end;
+      const long long at = KC ? (long long)(mn0 + r) * ld + k0 + kk : (long long)(k0 + kk) * ld + mn0 + r;
+      cp_async8(KC ? st + ((kk >> 3) * DB + r) * 8 + (kk & 7) : st + kk * DPITCH + r, ok ? src + at : src, ok);
     }
   }
 }
+// Elements k = 2t and 2t + 1 of k block kb, row r.
+template <bool KC>
+__device__ __forceinline__ void frag(const double* st, int kb, int t, int r, double& lo, double& hi) {
+  if (KC) {
+    const double2 v = *reinterpret_cast<const double2*>(st + (kb * DB + r) * 8 + 2 * t);
+    lo = v.x; hi = v.y;
+  } else {
+    lo = st[(kb * 8 + 2 * t) * DPITCH + r];
+    hi = st[(kb * 8 + 2 * t + 1) * DPITCH + r];
+  }
+}
 
-template <int SHAPE>   // 0: m8n8k4 instructions, 1: m16n8k8
-__global__ void __launch_bounds__(DTHREADS, 1)
-gemm_f64_mma_kernel(const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ C, int M, int N,
-                    int K, int transA, int transB, long long lda, long long ldb, long long ldc, long long sA,
-                    long long sB, long long sC, double alpha, int beta) {
+// grid: (row tiles * column tiles * splits, batch); a cluster is the `splits` CTAs of one tile.
+template <bool AK, bool BKC>
+__global__ void __launch_bounds__(DTHREADS, 4)
+gemm_f64_mma_kernel(const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ C, int M, int N, int K,
+                    long long lda, long long ldb, long long ldc, long long sA, long long sB, long long sC, double alpha, int beta,
+                    int splits, int k_per) {
   extern __shared__ __align__(16) double dsm[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wm = (warp >> 2) * 32, wn = (warp & 3) * 32;  // 4 x 4 warps of 32 x 32
-  const int m0 = blockIdx.y * DBM, n0 = blockIdx.x * DBN;
-  A += (long long)blockIdx.z * sA;
-  B += (long long)blockIdx.z * sB;
-  C += (long long)blockIdx.z * sC;
-  // A as stored: (M, K) row-major (k contiguous) unless transA, then (K, M)
-  // B as stored: (K, N) row-major (n contiguous) unless transB, then (N, K) (k contiguous)
-  const bool a_kc = transA == 0, b_kc = transB != 0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+  const unsigned tile = splits == 1 ? blockIdx.x : blockIdx.x / splits, tiles_n = (N + DB - 1) / DB;
+  const int rank = (int)(blockIdx.x - tile * splits);
+  const int m0 = (int)(tile / tiles_n) * DB, n0 = (int)(tile % tiles_n) * DB;
+  A += (long long)blockIdx.y * sA;
+  B += (long long)blockIdx.y * sB;
+  C += (long long)blockIdx.y * sC;
   const bool a_vec = ((lda & 1) == 0) && (((uintptr_t)A & 15) == 0);
   const bool b_vec = ((ldb & 1) == 0) && (((uintptr_t)B & 15) == 0);
-  const int nk = (K + DBK - 1) / DBK;
-
-  double acc[4][4][2];
+  const int k_begin = rank * k_per, k_end = min(K, k_begin + k_per);
+  const int nk = k_end > k_begin ? (k_end - k_begin + DBK - 1) / DBK : 0;
+  double acc[2][4][4];
 #pragma unroll
-  for (int i = 0; i < 4; i++)
+  for (int i = 0; i < 2; i++)
 #pragma unroll
-    for (int j = 0; j < 4; j++) { acc[i][j][0] = 0.0; acc[i][j][1] = 0.0; }
+    for (int j = 0; j < 4; j++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) acc[i][j][e] = 0.0;
 
   auto issue = [&](int kt) {
     if (kt < nk) {
-      double* st = dsm + (kt % DSTAGES) * DSTAGE_DOUBLES;
-      load_tile(st, A, lda, a_kc, m0, kt * DBK, M, K, a_vec);
-      load_tile(st + DBK * DLD, B, ldb, b_kc, n0, kt * DBK, N, K, b_vec);
+      double* st = dsm + (kt % DSTAGES) * 2 * DOP;
+      load_tile<AK>(st, A, lda, m0, k_begin + kt * DBK, M, k_end, a_vec);
+      load_tile<BKC>(st + DOP, B, ldb, n0, k_begin + kt * DBK, N, k_end, b_vec);
     }
-    cp_async_commit();
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
 #pragma unroll
   for (int i = 0; i < DSTAGES - 1; i++) issue(i);
-  const int fr = lane >> 2, fk = lane & 3;
   for (int kt = 0; kt < nk; kt++) {
-    cp_async_wait<DSTAGES - 2>();   // tile kt has landed (the newer groups may still be in flight)
-    __syncthreads();                // ... for every thread, and tile kt-1's stage is no longer read
+    asm volatile("cp.async.wait_group %0;" ::"n"(DSTAGES - 2) : "memory");   // tile kt has landed
+    __syncthreads();                                                         // ... for every thread; kt - 1 is no longer read
     issue(kt + DSTAGES - 1);
-    const double* sa = dsm + (kt % DSTAGES) * DSTAGE_DOUBLES;
-    const double* sb = sa + DBK * DLD;
-    if (SHAPE == 0) {
+    const double* sa = dsm + (kt % DSTAGES) * 2 * DOP;
+    const double* sb = sa + DOP;
 #pragma unroll
-      for (int ks = 0; ks < DBK; ks += 4) {
-        double af[4], bf[4];
+    for (int kb = 0; kb < DBK / 8; kb++) {
+      double af[2][4], bf[4][2];
 #pragma unroll
-        for (int i = 0; i < 4; i++) af[i] = sa[(ks + fk) * DLD + wm + i * 8 + fr];
-#pragma unroll
-        for (int j = 0; j < 4; j++) bf[j] = sb[(ks + fk) * DLD + wn + j * 8 + fr];
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-#pragma unroll
-          for (int j = 0; j < 4; j++) dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+      for (int i = 0; i < 2; i++) {
+        frag<AK>(sa, kb, t, wm + i * 16 + g, af[i][0], af[i][2]);
+        frag<AK>(sa, kb, t, wm + i * 16 + 8 + g, af[i][1], af[i][3]);
       }
-    } else {
-      // acc[2h][j] / acc[2h + 1][j] are the upper / lower 8 rows of 16-row tile h
 #pragma unroll
-      for (int ks = 0; ks < DBK; ks += 8) {
-        double af[2][4], bf[4][2];
+      for (int j = 0; j < 4; j++) frag<BKC>(sb, kb, t, wn + j * 8 + g, bf[j][0], bf[j][1]);
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-          af[h][0] = sa[(ks + fk) * DLD + wm + h * 16 + fr];
-          af[h][1] = sa[(ks + fk) * DLD + wm + h * 16 + 8 + fr];
-          af[h][2] = sa[(ks + fk + 4) * DLD + wm + h * 16 + fr];
-          af[h][3] = sa[(ks + fk + 4) * DLD + wm + h * 16 + 8 + fr];
-        }
+      for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) dmma16(acc[i][j], af[i], bf[j]);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  const bool c_vec = ((ldc & 1) == 0) && (((uintptr_t)C & 15) == 0);
+  if (splits == 1) {
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int m = m0 + wm + i * 16 + h * 8 + g;
+        if (m >= M) continue;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-          bf[j][0] = sb[(ks + fk) * DLD + wn + j * 8 + fr];
-          bf[j][1] = sb[(ks + fk + 4) * DLD + wn + j * 8 + fr];
-        }
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            double c[4] = {acc[2 * h][j][0], acc[2 * h][j][1], acc[2 * h + 1][j][0], acc[2 * h + 1][j][1]};
-            dmma16(c, af[h], bf[j]);
-            acc[2 * h][j][0] = c[0]; acc[2 * h][j][1] = c[1];
-            acc[2 * h + 1][j][0] = c[2]; acc[2 * h + 1][j][1] = c[3];
+          const int n = n0 + wn + j * 8 + 2 * t;
+          double* c = C + (long long)m * ldc + n;
+          double v0 = alpha * acc[i][j][2 * h], v1 = alpha * acc[i][j][2 * h + 1];
+          if (n + 1 < N) {
+            if (beta) { v0 += c[0]; v1 += c[1]; }
+            if (c_vec) *reinterpret_cast<double2*>(c) = make_double2(v0, v1);
+            else { c[0] = v0; c[1] = v1; }
+          } else if (n < N) {
+            if (beta) v0 += c[0];
+            c[0] = v0;
           }
+        }
       }
+    return;
+  }
+  // ---- a cluster adds its parts: every CTA leaves its tile in its own shared memory, then sums 64 / splits rows ----
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        *reinterpret_cast<double2*>(dsm + (wm + i * 16 + h * 8 + g) * DB + wn + j * 8 + 2 * t) =
+            make_double2(acc[i][j][2 * h], acc[i][j][2 * h + 1]);
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const int rows = DB / splits;
+  for (int q = threadIdx.x; q < rows * DB; q += DTHREADS) {
+    const int r = rank * rows + q / DB, n = q % DB;
+    const uint32_t local = smem_u32(dsm + r * DB + n);
+    double v = 0.0;
+    for (int p = 0; p < splits; p++) {
+      uint32_t remote;
+      double x;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(p));
+      asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(x) : "r"(remote) : "memory");
+      v += x;
+    }
+    if (m0 + r < M && n0 + n < N) {
+      double* c = C + (long long)(m0 + r) * ldc + n0 + n;
+      *c = beta ? *c + alpha * v : alpha * v;
     }
   }
-  cp_async_wait<0>();
-  // C fragment: row = lane / 4, columns 2 * (lane % 4) + {0, 1} of each 8 x 8 tile
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int m = m0 + wm + i * 8 + fr;
-    if (m >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int n = n0 + wn + j * 8 + 2 * fk;
-      double* c = C + (long long)m * ldc + n;
-      double v0 = alpha * acc[i][j][0], v1 = alpha * acc[i][j][1];
-      if (n + 1 < N) {
-        if (beta) { v0 += c[0]; v1 += c[1]; }
-        c[0] = v0; c[1] = v1;
-      } else if (n < N) {
-        if (beta) v0 += c[0];
-        c[0] = v0;
-      }
-    }
-  }
+  // nobody leaves while a peer may still read its shared memory
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+int g_f64_splits = 0;      // 0: by the rule below
+
+// CTAs per tile: K is cut while the CTAs stay within three per SM and a part keeps about a k-tile.  Measured, us for 1 | 2 | 4 |
+// 8 parts: 64 x 64 x 2048 122 | 67 | 36 | 20; 362^3 25 | 19 | 14 | 12; 512^3 33 | 23 | 17 | 17; 100^3 9 | 11 | 7.5 | 5.8; and where
+// the tiles fill the GPU, 1024^3 (256 tiles) 86 | 94 | 92 | 91, 2048^3 572 | 572 | 594 | 606.
+int f64_splits(int M, int N, int K, int batch) {
+  if (g_f64_splits) return g_f64_splits;
+  const long long tiles = (long long)((M + DB - 1) / DB) * ((N + DB - 1) / DB) * batch;
+  int s = 1;
+  while (s < 8 && tiles * s * 2 <= 3 * 148 && K / (2 * s) >= 12) s *= 2;
+  return s;
+}
+
+template <bool AK, bool BKC>
+int launch_f64(const void* A, const void* B, void* C, int M, int N, int K, int batch, long long lda, long long ldb, long long ldc,
+               long long sA, long long sB, long long sC, double alpha, int beta, cudaStream_t s) {
+  auto kern = gemm_f64_mma_kernel<AK, BKC>;
+  GB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, DSMEM));
+  const int splits = f64_splits(M, N, K, batch);
+  const int k_per = ((K + splits - 1) / splits + DBK - 1) / DBK * DBK;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)((long long)((M + DB - 1) / DB) * ((N + DB - 1) / DB) * splits), batch);
+  cfg.blockDim = dim3(DTHREADS);
+  cfg.dynamicSmemBytes = DSMEM;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = splits;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = splits > 1 ? 1 : 0;
+  GB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, (const double*)A, (const double*)B, (double*)C, M, N, K, lda, ldb, ldc, sA, sB, sC, alpha,
+                                beta, splits, k_per));
+  return gbh::E_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -269,10 +312,13 @@ __global__ void split3_kernel(const float* __restrict__ src, __nv_bfloat16* __re
 
 }  // namespace
 
-namespace { int g_f64_shape = 1; }
-// Instruction shape of the fp64 kernel: 0 = m8n8k4, 1 = m16n8k8 (default).
-GB_EXPORT int gb_gemm_f64_tune(int shape) {
-  g_f64_shape = shape ? 1 : 0;
+// CTAs that share a tile of the fp64 product: 1, 2, 4 or 8, 0 = chosen by size (for measurements and tests).
+GB_EXPORT int gb_gemm_f64_tune(int splits) {
+  if (splits != 0 && splits != 1 && splits != 2 && splits != 4 && splits != 8) {
+    gbh::set_error("gb_gemm_f64_tune: splits is 0, 1, 2, 4 or 8");
+    return gbh::E_BAD_ARG;
+  }
+  g_f64_splits = splits;
   return gbh::E_OK;
 }
 
@@ -284,26 +330,15 @@ GB_EXPORT int gb_gemm_f64(const void* A, const void* B, void* C, int M, int N, i
     gbh::set_error("gb_gemm_f64: empty problem");
     return gbh::E_BAD_ARG;
   }
-  dim3 grid((N + DBN - 1) / DBN, (M + DBM - 1) / DBM, batch);
-  if (grid.y > 65535 || grid.z > 65535) {
+  if ((long long)((M + DB - 1) / DB) * ((N + DB - 1) / DB) >= (1LL << 28) || batch > 65535) {
     gbh::set_error("gb_gemm_f64: problem too large");
     return gbh::E_TOO_LARGE;
   }
-  const size_t smem = (size_t)DSTAGES * DSTAGE_DOUBLES * sizeof(double);
-  static bool attr_set = false;
-  if (!attr_set) {
-    GB_CUDA_OK(cudaFuncSetAttribute(gemm_f64_mma_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    GB_CUDA_OK(cudaFuncSetAttribute(gemm_f64_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_set = true;
-  }
-  if (g_f64_shape == 0)
-    gemm_f64_mma_kernel<0><<<grid, DTHREADS, smem, (cudaStream_t)stream>>>(
-        (const double*)A, (const double*)B, (double*)C, M, N, K, transA, transB, lda, ldb, ldc, sA, sB, sC, alpha, beta);
-  else
-    gemm_f64_mma_kernel<1><<<grid, DTHREADS, smem, (cudaStream_t)stream>>>(
-        (const double*)A, (const double*)B, (double*)C, M, N, K, transA, transB, lda, ldb, ldc, sA, sB, sC, alpha, beta);
-  GB_CUDA_OK(cudaGetLastError());
-  return gbh::E_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (!transA && transB) return launch_f64<true, true>(A, B, C, M, N, K, batch, lda, ldb, ldc, sA, sB, sC, alpha, beta, st);
+  if (!transA) return launch_f64<true, false>(A, B, C, M, N, K, batch, lda, ldb, ldc, sA, sB, sC, alpha, beta, st);
+  if (transB) return launch_f64<false, true>(A, B, C, M, N, K, batch, lda, ldb, ldc, sA, sB, sC, alpha, beta, st);
+  return launch_f64<false, false>(A, B, C, M, N, K, batch, lda, ldb, ldc, sA, sB, sC, alpha, beta, st);
 }
 
 // Bytes of scratch gb_gemm_f32x3 needs for the split operands.
