@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import torch
 
+from . import block as _block
 from .activation import Activation, ReLU
 from .attention import MultiHeadAttention
 from .dropout import Dropout
@@ -38,6 +39,15 @@ class TransformerEncoderLayer(Module):
         self.drop2 = Dropout(dropout)
         self.dropff = Dropout(dropout)
 
+    def _no_dropout(self) -> bool:
+        """No dropout draws a mask and nothing observes one, so that they may be skipped."""
+        m = self._modules
+        for name in ("drop1", "drop2", "dropff"):
+            d = m[name]
+            if not _block.plain(d, Dropout) or self.training and d.p > 0:
+                return False
+        return True
+
     def _ff(self, x, residual=None, bias2_grad: bool = True):
         kind = getattr(self.act, "kind", None)
         plain = not (self.training and self.dropff.p > 0)
@@ -53,6 +63,11 @@ class TransformerEncoderLayer(Module):
         return y if residual is None else residual + y
 
     def forward(self, x):
+        if not torch.is_grad_enabled() and type(self) is TransformerEncoderLayer and self._no_dropout():
+            m = self._modules
+            y = _block.evaluate(x, m["attn"], m["norm1"], m["norm2"], m["ff1"], m["ff2"], m["act"], self.pre_norm, self.causal)
+            if y is not None:
+                return y
         nodrop = not (self.training and self.drop1.p > 0)
         if self.pre_norm:
             if nodrop:
