@@ -1075,6 +1075,242 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 }
 
 // ---------------------------------------------------------------------------
+// Few output tiles: 128 x 64 tiles whose K is cut over a cluster.
+//
+// A product with a few hundred rows has so few 128 x 128 tiles that most SMs idle while a handful of CTAs walk all of K
+// (77 x 768 x 3072: 6 CTAs, 48 k-blocks; 10 us of latency for 1 us of weight traffic).  Here 2, 4 or 8 CTAs of a
+// cluster share a tile: each multiplies its k-blocks into its own TMEM, leaves the fp32 partial tile in its shared
+// memory, and after a cluster barrier sums every S-th row over the cluster in rank order (distributed shared
+// memory: no workspace, no second launch, deterministic) and applies the whole epilogue to it.  One tile per
+// cluster, 99 KB of shared memory: two CTAs per SM.  Loads are plain per-CTA TMA loads.
+// ---------------------------------------------------------------------------
+struct CfgS {
+  static constexpr int BN = 64, BK = 64, STAGES = 4;
+  static constexpr int A_BYTES = BM * kSwizzleBytes, B_BYTES = BN * kSwizzleBytes, STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int PITCH = BN + 4;           // floats per row of the partial tile
+  static constexpr int BARS = STAGES * STAGE_BYTES;
+  static constexpr int BYTES = BARS + 256;
+  static constexpr int THREADS = 192;            // TMA warp, MMA warp, four epilogue warps
+  static_assert(BM * PITCH * 4 <= BARS, "the partial tile reuses the ring");
+};
+
+__device__ __forceinline__ float load16(const void* p, long long i, int bf) {
+  const uint16_t u = __ldg((const uint16_t*)p + i);
+  return bf ? __uint_as_float((uint32_t)u << 16) : __half2float(__ushort_as_half(u));
+}
+
+template <bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(CfgS::THREADS, 2)
+gemm_tcgen05_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs args) {
+  using C = CfgS;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if (smem_u32(smem) & 1023u) {      // the same in every CTA of the launch
+    if (threadIdx.x == 0) set_status(args.status, ST_BAD_INDEX, 1024);
+    return;
+  }
+  uint64_t* full_bar = (uint64_t*)(smem + C::BARS);
+  uint64_t* empty_bar = full_bar + C::STAGES;
+  uint64_t* done_bar = empty_bar + C::STAGES;
+  uint32_t* tmem_slot = (uint32_t*)(done_bar + 1);
+  volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int S = args.splits;
+  const int tile = blockIdx.x / S, rank = blockIdx.x - tile * S;
+  const int b = blockIdx.y;
+  const int m0 = (tile / args.num_n) * BM, n0 = (tile % args.num_n) * C::BN;
+  const int num_kb = (args.K + C::BK - 1) / C::BK;
+  const int kb_begin = rank * args.kb_per, kb_end = min(num_kb, kb_begin + args.kb_per);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < C::STAGES; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    mbar_init(done_bar, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, C::BN);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  if (warp == 0) {
+    if (lane == 0) {
+      bool ok = true;
+      const int ba = args.bcastA ? 0 : b, bb = args.bcastB ? 0 : b;
+      for (int kb = kb_begin, i = 0; kb < kb_end; kb++, i++) {
+        const int stage = i % C::STAGES;
+        ok = mbar_wait(&empty_bar[stage], ((i / C::STAGES) & 1) ^ 1, abort_flag, args.status, ST_GEMM_TIMEOUT, 21);
+        if (!ok) break;
+        uint8_t* sa = smem + stage * C::STAGE_BYTES;
+        uint8_t* sb = sa + C::A_BYTES;
+        mbar_expect_tx(&full_bar[stage], C::STAGE_BYTES);
+        const int k0 = kb * C::BK;
+        if (!A_MN) tma_load_3d(sa, &tmA, &full_bar[stage], k0, m0, ba);
+        else
+          for (int j = 0; j < 2; j++) tma_load_3d(sa + j * (C::BK * kSwizzleBytes), &tmA, &full_bar[stage], m0 + j * 64, k0, ba);
+        if (!B_MN) tma_load_3d(sb, &tmB, &full_bar[stage], k0, n0, bb);
+        else tma_load_3d(sb, &tmB, &full_bar[stage], n0, k0, bb);
+      }
+      if (!ok) {
+        // give copies already in flight a bounded chance to land before the ring is reused
+        uint64_t t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 2000000ull) { }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (elect_one()) {
+      const uint32_t id = make_idesc(1u, args.in_bf16 ? 1u : 0u, A_MN, B_MN, BM, C::BN);
+      for (int kb = kb_begin, i = 0; kb < kb_end; kb++, i++) {
+        const int stage = i % C::STAGES;
+        if (!mbar_wait(&full_bar[stage], (i / C::STAGES) & 1, abort_flag, args.status, ST_GEMM_TIMEOUT, 22)) break;
+        tc_fence_after();
+        const uint32_t sa = smem_u32(smem + stage * C::STAGE_BYTES), sb = sa + C::A_BYTES;
+#pragma unroll
+        for (int k = 0; k < C::BK / 16; k++) {
+          const uint64_t adesc = A_MN ? make_smem_desc_sw128(sa + k * 16 * kSwizzleBytes, C::BK * kSwizzleBytes, 1024)
+                                      : make_smem_desc_sw128(sa + k * 32, 16, 1024);
+          const uint64_t bdesc = B_MN ? make_smem_desc_sw128(sb + k * 16 * kSwizzleBytes, C::BK * kSwizzleBytes, 1024)
+                                      : make_smem_desc_sw128(sb + k * 32, 16, 1024);
+          tc_mma_f16(tmem_base, adesc, bdesc, id, i > 0 || k != 0);
+        }
+        tc_commit(&empty_bar[stage]);
+      }
+      tc_commit(done_bar);
+    }
+    __syncwarp();
+  } else {
+    // the accumulator's rows into the ring (every load has been consumed by then): thread = row
+    const bool ok = mbar_wait(done_bar, 0, abort_flag, args.status, ST_GEMM_TIMEOUT, 23);
+    const int q = warp & 3;
+    float* row = reinterpret_cast<float*>(smem) + (q * 32 + lane) * C::PITCH;
+    if (__all_sync(0xffffffffu, ok)) {
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < C::BN / 32; c++) {
+        uint32_t rr[32];
+        if (kb_end > kb_begin) {
+          tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + c * 32, rr);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; j++) rr[j] = 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(row + c * 32 + j) = make_uint4(rr[j], rr[j + 1], rr[j + 2], rr[j + 3]);
+      }
+    }
+    tc_fence_before();
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, C::BN);
+  }
+  if (S > 1) cluster_sync_all();
+  // ---- rows rank, rank + S, ... of the tile: sum over the cluster, epilogue, store; a thread takes four columns ----
+  const int rows = min(BM, args.M - m0);
+  const bool bf = args.in_bf16;
+  const int c4 = (threadIdx.x & 15) * 4;
+  float bias[4] = {0.f, 0.f, 0.f, 0.f};
+  if (args.bias) {
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (n0 + c4 + j < args.N)
+        bias[j] = args.bias_f32 ? __ldg((const float*)args.bias + n0 + c4 + j) : load16(args.bias, n0 + c4 + j, bf);
+  }
+  const bool whole = n0 + c4 + 4 <= args.N;
+  const bool c_vec = whole && ((args.ldc | args.strideC) & 3) == 0 && ((uintptr_t)args.C & 15) == 0;
+  const bool x_vec = whole && ((args.ldaux | args.strideAux) & 3) == 0 && ((uintptr_t)args.aux & 7) == 0;
+  for (int i = threadIdx.x >> 4; i * S + rank < rows; i += C::THREADS / 16) {
+    const int r = i * S + rank;
+    const uint32_t local = smem_u32(reinterpret_cast<float*>(smem) + r * C::PITCH + c4);
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (S == 1) {
+      const float4 u = *reinterpret_cast<const float4*>(reinterpret_cast<float*>(smem) + r * C::PITCH + c4);
+      v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+    } else {
+#pragma unroll 4
+      for (int p = 0; p < S; p++) {
+        uint32_t remote;
+        float4 u;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(p));
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(u.x), "=f"(u.y), "=f"(u.z), "=f"(u.w) : "r"(remote) : "memory");
+        v[0] += u.x; v[1] += u.y; v[2] += u.z; v[3] += u.w;
+      }
+    }
+    if (n0 + c4 >= args.N) continue;
+    const long long row = m0 + r;
+#pragma unroll
+    for (int j = 0; j < 4; j++) v[j] = v[j] * args.alpha + bias[j];
+    if (args.aux_mode != AUX_NONE) {
+      uint16_t* xp = (uint16_t*)args.aux + (long long)b * args.strideAux + row * args.ldaux + n0 + c4;
+      if (args.aux_mode == AUX_STORE_PRE) {
+        if (x_vec) *reinterpret_cast<uint2*>(xp) = make_uint2(pack16x(v[0], v[1], bf), pack16x(v[2], v[3], bf));
+        else
+          for (int j = 0; j < 4; j++)
+            if (n0 + c4 + j < args.N) xp[j] = (uint16_t)pack16x(v[j], 0.f, bf);
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = act_apply<float>(v[j], args.act);
+      } else {
+        float x[4] = {0.f, 0.f, 0.f, 0.f};
+        if (x_vec) {
+          const uint2 u = __ldg(reinterpret_cast<const uint2*>(xp));
+          const float2 lo = unpack16(u.x, bf), hi = unpack16(u.y, bf);
+          x[0] = lo.x; x[1] = lo.y; x[2] = hi.x; x[3] = hi.y;
+        } else {
+          for (int j = 0; j < 4; j++)
+            if (n0 + c4 + j < args.N) x[j] = load16(xp, j, bf);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          v[j] = act_apply<float>(v[j], args.act);
+          if (args.aux_mode == AUX_ADD) v[j] += x[j];
+          else if (args.aux_mode == AUX_MUL_DGELU_TANH) v[j] *= dgelu_tanh_f(x[j]);
+          else if (args.aux_mode == AUX_MUL_DRELU) v[j] = x[j] > 0.f ? v[j] : 0.f;
+          else v[j] *= dgelu_erf_f(x[j]);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; j++) v[j] = act_apply<float>(v[j], args.act);
+    }
+    if (args.out_kind == OUT_F32) {
+      float* cp = (float*)args.C + (long long)b * args.strideC + row * args.ldc + n0 + c4;
+      if (c_vec) {
+        float4 o = make_float4(v[0], v[1], v[2], v[3]);
+        if (args.beta) {
+          const float4 old = *reinterpret_cast<const float4*>(cp);
+          o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
+        }
+        *reinterpret_cast<float4*>(cp) = o;
+      } else {
+        for (int j = 0; j < 4; j++)
+          if (n0 + c4 + j < args.N) cp[j] = args.beta ? cp[j] + v[j] : v[j];
+      }
+    } else {
+      uint16_t* cp = (uint16_t*)args.C + (long long)b * args.strideC + row * args.ldc + n0 + c4;
+      const int obf = args.out_kind == OUT_BF16;
+      if (c_vec) {
+        if (args.beta) {
+          const uint2 u = *reinterpret_cast<const uint2*>(cp);
+          const float2 lo = unpack16(u.x, obf), hi = unpack16(u.y, obf);
+          v[0] += lo.x; v[1] += lo.y; v[2] += hi.x; v[3] += hi.y;
+        }
+        *reinterpret_cast<uint2*>(cp) = make_uint2(pack16x(v[0], v[1], obf), pack16x(v[2], v[3], obf));
+      } else {
+        for (int j = 0; j < 4; j++)
+          if (n0 + c4 + j < args.N) cp[j] = (uint16_t)pack16x(args.beta ? v[j] + unpack16(cp[j], obf).x : v[j], 0.f, obf);
+      }
+    }
+  }
+  if (S > 1) cluster_sync_all();   // nobody leaves while a peer may still read its shared memory
+}
+
+// ---------------------------------------------------------------------------
 // SIMT fallback for fp32 / fp64 operands (exact-precision parity paths)
 // ---------------------------------------------------------------------------
 template <typename T>
@@ -1370,6 +1606,49 @@ int launch_2cta(const TMaps& tm, const GemmArgs& args, int num_sms, cudaStream_t
   return gbh::E_OK;
 }
 
+int g_cluster_splits = 0;   // 0: by the rule of cluster_splits(); -1: off; 1, 2, 4, 8: that many CTAs per tile
+
+// CTAs per 128 x 64 tile of the cluster kernel, 0 = another kernel.  K is cut until the CTAs come to about one per SM.
+// The cluster's exchange costs 2.5 us, so it pays from four parts on, or from two where K is long.  Measured, us
+// (best | one CTA per 128 x 128 tile): 77 x 768 x 3072 6.9 (8 parts) | 14.0; 128 x 2048 x 8192 13.6 (4) | 30.3; 300 x 768 x
+// 3072 9.2 (4) | 14.2; 128 x 2048 x 2048 8.4 (4) | 11.1; 77 x 768 x 768 6.0 (8) | 7.0; 77 x 2304 x 768 7.1 (4) | 6.9;
+// 700 x 768 x 3072 13.4 (2) | 14.3; 77 x 3072 x 768 8.1 (2) | 7.0; 128 x 8192 x 2048 12.7 (2) | 11.3; 300 x 2304 x 768 10.5 (1) | 7.2.
+int cluster_splits(int M, int N, int K, int batch, int num_sms) {
+  if (g_cluster_splits < 0 || batch > 65535) return 0;
+  const long long tiles = (long long)((M + BM - 1) / BM) * ((N + CfgS::BN - 1) / CfgS::BN) * batch;
+  if (tiles >= (1LL << 28)) return 0;
+  if (g_cluster_splits > 0) return g_cluster_splits;
+  const int num_kb = (K + CfgS::BK - 1) / CfgS::BK;
+  int s = 1;
+  while (s < 8 && tiles * s * 2 <= num_sms + num_sms / 8 && num_kb >= 2 * s) s *= 2;
+  return s >= 4 || (s == 2 && num_kb >= 48) ? s : 0;
+}
+
+template <bool A_MN, bool B_MN>
+int launch_cluster(const TMaps& tm, const GemmArgs& args, cudaStream_t stream) {
+  auto kern = gemm_tcgen05_cluster_kernel<A_MN, B_MN>;
+  static bool configured = false;
+  if (!configured) {
+    GB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CfgS::BYTES));
+    configured = true;
+  }
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(args.num_m * args.num_n * args.splits, args.batch);
+  cfg.blockDim = dim3(CfgS::THREADS);
+  cfg.dynamicSmemBytes = CfgS::BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = args.splits;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = args.splits > 1 ? 1 : 0;
+  GB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tm.a, tm.b, args));
+  return gbh::E_OK;
+}
+
 // Sums the K slices of a split launch in slice order and writes the result in the
 // caller's type: C = (beta ? C : 0) + sum_s ws[s].
 template <typename TO>
@@ -1508,6 +1787,13 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
     args.out_kind = OUT_F32;
     args.beta = 0;
   }
+  const int cluster = esz == 2 && force_bn == 0 && splits == 1 && !use2 ? cluster_splits(M, N, K, batch, g_num_sms) : 0;
+  if (cluster) {
+    const int num_kb = (K + CfgS::BK - 1) / CfgS::BK;
+    bn = CfgS::BN;
+    args.splits = cluster;
+    args.kb_per = (num_kb + cluster - 1) / cluster;
+  }
   if (use2) bn = 128;   // each CTA of a pair stages 128 of the tile's 256 columns
   args.num_m = use2 ? (M + 255) / 256 : (M + BM - 1) / BM;
   args.num_n = use2 ? (N + 255) / 256 : (N + bn - 1) / bn;
@@ -1525,7 +1811,7 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
   // (and the auxiliary tensor) can be described by a tensor map and nothing is accumulated.
   args.tma_epi = 0;
   const bool f32_out = args.out_kind == OUT_F32;
-  if (esz == 2 && g_tma_epi && !args.beta && !(f32_out && (args.act != ACT_NONE || args.aux_mode != AUX_NONE))) {
+  if (esz == 2 && g_tma_epi && !cluster && !args.beta && !(f32_out && (args.act != ACT_NONE || args.aux_mode != AUX_NONE))) {
     const int osz = f32_out ? 4 : 2;
     auto mappable = [&](const void* p, long long ld, long long bs) {
       return (((uintptr_t)p & 15) == 0) && (ld * osz % 16 == 0) && (bs * osz % 16 == 0);
@@ -1586,6 +1872,12 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
     if (rc) return rc;
   }
   int rc;
+  if (cluster) {
+    if (!a_mn && !b_mn) return launch_cluster<false, false>(tm, args, stream);
+    if (!a_mn && b_mn) return launch_cluster<false, true>(tm, args, stream);
+    if (a_mn && !b_mn) return launch_cluster<true, false>(tm, args, stream);
+    return launch_cluster<true, true>(tm, args, stream);
+  }
   if (use2) {
     if (!a_mn && !b_mn) rc = launch_2cta<false, false>(tm, args, g_num_sms, stream);
     else if (!a_mn && b_mn) rc = launch_2cta<false, true>(tm, args, g_num_sms, stream);
@@ -1633,6 +1925,11 @@ GB_EXPORT int gb_gemm_simt_tiled(int on) {
 // Enables (1) or disables (0) the automatic choice of the two-CTA kernel.
 GB_EXPORT int gb_gemm_use_2cta(int on) {
   g_use_2cta = on;
+  return 0;
+}
+// CTAs per tile of the cluster kernel for products with few tiles: 0 by size, -1 never, 1, 2, 4 or 8.
+GB_EXPORT int gb_gemm_cluster_tune(int splits) {
+  if (splits == -1 || splits == 0 || splits == 1 || splits == 2 || splits == 4 || splits == 8) g_cluster_splits = splits;
   return 0;
 }
 // Enables (1) or disables (0) split-K for products with few output tiles.
