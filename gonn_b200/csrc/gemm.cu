@@ -66,7 +66,12 @@ struct GemmArgs {
   int bcastA, bcastB;  // operand shared by every batch entry (batch stride 0)
   int group_m;         // row blocks per rasterisation group
   int tma_epi;         // 1: results leave through shared memory and TMA stores (16-bit outputs)
+  int num_kb;          // k-blocks of a tile, over all plane products
   int splits, kb_per;  // split-K: slice s of a tile covers k-blocks [s * kb_per, (s + 1) * kb_per)
+  // planes > 0: the operands are stacks of three planes of kb_plane k-blocks; a slice runs its part of K through every
+  // plane product p, planes (plane_a >> 4p) & 15 and (plane_b >> 4p) & 15, one after another (csrc/gemm_exact.cu)
+  int planes, kb_plane;
+  uint32_t plane_a, plane_b;
   int* status;
 };
 
@@ -124,6 +129,50 @@ __device__ __forceinline__ Unit decode_unit(int t, const GemmArgs& args) {
   tile_coords(t2 - u.b * tiles_per_batch, args.num_m, args.num_n, args.group_m, u.mb, u.nb);
   return u;
 }
+
+// The k-blocks of slice s.  PL: plane products (a template parameter of the kernels: at run time the distinction cost the
+// ordinary products 1 to 3 %).
+template <bool PL>
+__device__ __forceinline__ void slice_range(const GemmArgs& args, int s, int& begin, int& end) {
+  begin = s * args.kb_per;
+  if (PL) {
+    const int per = args.kb_per / args.planes;                          // of each plane
+    end = begin + args.planes * max(0, min(per, args.kb_plane - s * per));
+  } else {
+    end = min(args.num_kb, begin + args.kb_per);
+  }
+}
+// Walks the k-blocks of slice s: position along K and the third coordinate of either operand's tensor map.  (Stepped, not
+// computed from the index: two divisions per k-block in the thread that issues the loads cost 20 % of a plane product.)
+template <bool PL>
+struct KWalk {
+  int k0, a, b, i, len, p, first;
+  __device__ __forceinline__ KWalk(const GemmArgs& args, int s, int block_k, int batch) {
+    a = args.bcastA ? 0 : batch;
+    b = args.bcastB ? 0 : batch;
+    first = s * args.kb_per * block_k;
+    if (PL) {
+      const int per = args.kb_per / args.planes;
+      first = s * per * block_k;
+      len = min(per, args.kb_plane - s * per);
+      i = 0;
+      p = 0;
+      a = a * 3 + (int)(args.plane_a & 15u);
+      b = b * 3 + (int)(args.plane_b & 15u);
+    }
+    k0 = first;
+  }
+  __device__ __forceinline__ void next(const GemmArgs& args, int block_k) {
+    k0 += block_k;
+    if (PL && ++i == len) {
+      a += (int)((args.plane_a >> (4 * p + 4)) & 15u) - (int)((args.plane_a >> (4 * p)) & 15u);
+      b += (int)((args.plane_b >> (4 * p + 4)) & 15u) - (int)((args.plane_b >> (4 * p)) & 15u);
+      p++;
+      i = 0;
+      k0 = first;
+    }
+  }
+};
 
 template <typename T>
 __device__ __forceinline__ float act_apply(float v, int act) {
@@ -601,7 +650,7 @@ __device__ __forceinline__ bool epilogue_tile_tma(const GemmArgs& args, const Ep
 
 // ESZ: operand element size (2 = bf16/fp16, 1 = int8).  A_MN / B_MN: operand
 // is MN-major.  BN: tile width.
-template <int ESZ, bool A_MN, bool B_MN, int BN, int EW>
+template <int ESZ, bool A_MN, bool B_MN, int BN, int EW, bool PL>
 __global__ void __launch_bounds__(64 + 32 * EW, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmX,
@@ -627,7 +676,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int num_kb = (args.K + C::BK - 1) / C::BK;
   const int num_tiles = args.num_m * args.num_n * args.batch * args.splits;
 
   if (threadIdx.x == 0) {
@@ -668,15 +716,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         const Unit u = decode_unit(t, args);
         const int b = u.b;
         const int m0 = u.mb * BM, n0 = u.nb * BN;
-        const int kb_end = min(num_kb, (u.s + 1) * args.kb_per);
-        for (int kb = u.s * args.kb_per; kb < kb_end; kb++) {
+        int kb_begin, kb_end;
+        slice_range<PL>(args, u.s, kb_begin, kb_end);
+        KWalk<PL> kw(args, u.s, C::BK, b);
+        for (int kb = kb_begin; kb < kb_end; kb++) {
           ok = mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, args.status, ST_GEMM_TIMEOUT, 1);
           if (!ok) break;
           uint8_t* sa = smem + stage * C::STAGE_BYTES;
           uint8_t* sb = sa + C::A_BYTES;
           mbar_expect_tx(&full_bar[stage], C::STAGE_BYTES);
-          const int k0 = kb * C::BK;
-          const int ba = args.bcastA ? 0 : b, bb = args.bcastB ? 0 : b;
+          const int k0 = kw.k0, ba = kw.a, bb = kw.b;
+          kw.next(args, C::BK);
           if (!A_MN) {
             tma_load_3d(sa, &tmA, &full_bar[stage], k0, m0, ba);
           } else {
@@ -730,7 +780,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * BN;
         const int slice = t / (num_tiles / args.splits);
-        const int kb_begin = slice * args.kb_per, kb_end = min(num_kb, kb_begin + args.kb_per);
+        int kb_begin, kb_end;
+        slice_range<PL>(args, slice, kb_begin, kb_end);
         for (int kb = kb_begin; kb < kb_end; kb++) {
           ok = mbar_wait(&full_bar[stage], phase, abort_flag, args.status, ST_GEMM_TIMEOUT, 3);
           if (!ok) break;
@@ -879,7 +930,7 @@ struct Cfg2 {
   static constexpr int TMEM_COLS = 512;
 };
 
-template <bool A_MN, bool B_MN, int EW>
+template <bool A_MN, bool B_MN, int EW, bool PL>
 __global__ void __launch_bounds__(64 + 32 * EW, 1)
 gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                          const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmX,
@@ -908,7 +959,6 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   const uint32_t cta = cluster_ctarank();      // 0: leader (issues the MMAs), 1: peer
   const int pair = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
-  const int num_kb = (args.K + C::BK - 1) / C::BK;
   // num_m / num_n count 256 x 256 pair tiles here
   const int num_tiles = args.num_m * args.num_n * args.batch * args.splits;
 
@@ -952,8 +1002,10 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         const int b = u.b;
         const int m0 = u.mb * 256 + (int)cta * 128;   // this CTA's rows of A
         const int n0 = u.nb * 256 + (int)cta * 128;   // this CTA's columns of B
-        const int kb_end = min(num_kb, (u.s + 1) * args.kb_per);
-        for (int kb = u.s * args.kb_per; kb < kb_end; kb++) {
+        int kb_begin, kb_end;
+        slice_range<PL>(args, u.s, kb_begin, kb_end);
+        KWalk<PL> kw(args, u.s, C::BK, b);
+        for (int kb = kb_begin; kb < kb_end; kb++) {
           ok = mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, args.status, ST_GEMM_TIMEOUT, 11);
           if (!ok) break;
           uint8_t* sa = smem + stage * C::STAGE_BYTES;
@@ -961,8 +1013,8 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           // bytes of both CTAs land on the leader's barrier
           const uint32_t fb = smem_u32(&full_bar[stage]) & ~kPeerBit;
           if (cta == 0) mbar_expect_tx(&full_bar[stage], 2 * C::STAGE_BYTES);
-          const int k0 = kb * C::BK;
-          const int ba = args.bcastA ? 0 : b, bb = args.bcastB ? 0 : b;
+          const int k0 = kw.k0, ba = kw.a, bb = kw.b;
+          kw.next(args, C::BK);
           if (!A_MN) {
             tma_load_3d_2sm(sa, &tmA, fb, k0, m0, ba);
           } else {
@@ -1000,7 +1052,8 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * 256;
         const int slice = t / (num_tiles / args.splits);
-        const int kb_begin = slice * args.kb_per, kb_end = min(num_kb, kb_begin + args.kb_per);
+        int kb_begin, kb_end;
+        slice_range<PL>(args, slice, kb_begin, kb_end);
         for (int kb = kb_begin; kb < kb_end; kb++) {
           ok = mbar_wait(&full_bar[stage], phase, abort_flag, args.status, ST_GEMM_TIMEOUT, 13);
           if (!ok) break;
@@ -1099,7 +1152,7 @@ __device__ __forceinline__ float load16(const void* p, long long i, int bf) {
   return bf ? __uint_as_float((uint32_t)u << 16) : __half2float(__ushort_as_half(u));
 }
 
-template <bool A_MN, bool B_MN>
+template <bool A_MN, bool B_MN, bool PL>
 __global__ void __launch_bounds__(CfgS::THREADS, 2)
 gemm_tcgen05_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs args) {
   using C = CfgS;
@@ -1118,8 +1171,8 @@ gemm_tcgen05_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
   const int tile = blockIdx.x / S, rank = blockIdx.x - tile * S;
   const int b = blockIdx.y;
   const int m0 = (tile / args.num_n) * BM, n0 = (tile % args.num_n) * C::BN;
-  const int num_kb = (args.K + C::BK - 1) / C::BK;
-  const int kb_begin = rank * args.kb_per, kb_end = min(num_kb, kb_begin + args.kb_per);
+  int kb_begin, kb_end;
+  slice_range<PL>(args, rank, kb_begin, kb_end);
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; s++) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     mbar_init(done_bar, 1);
@@ -1139,7 +1192,7 @@ gemm_tcgen05_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
   if (warp == 0) {
     if (lane == 0) {
       bool ok = true;
-      const int ba = args.bcastA ? 0 : b, bb = args.bcastB ? 0 : b;
+      KWalk<PL> kw(args, rank, C::BK, b);
       for (int kb = kb_begin, i = 0; kb < kb_end; kb++, i++) {
         const int stage = i % C::STAGES;
         ok = mbar_wait(&empty_bar[stage], ((i / C::STAGES) & 1) ^ 1, abort_flag, args.status, ST_GEMM_TIMEOUT, 21);
@@ -1147,7 +1200,8 @@ gemm_tcgen05_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
         uint8_t* sa = smem + stage * C::STAGE_BYTES;
         uint8_t* sb = sa + C::A_BYTES;
         mbar_expect_tx(&full_bar[stage], C::STAGE_BYTES);
-        const int k0 = kb * C::BK;
+        const int k0 = kw.k0, ba = kw.a, bb = kw.b;
+        kw.next(args, C::BK);
         if (!A_MN) tma_load_3d(sa, &tmA, &full_bar[stage], k0, m0, ba);
         else
           for (int j = 0; j < 2; j++) tma_load_3d(sa + j * (C::BK * kSwizzleBytes), &tmA, &full_bar[stage], m0 + j * 64, k0, ba);
@@ -1538,11 +1592,11 @@ struct TMaps {
   CUtensorMap a, b, c, x;  // operands, output, auxiliary tensor
 };
 
-template <int ESZ, bool A_MN, bool B_MN, int BN, int EW>
+template <int ESZ, bool A_MN, bool B_MN, int BN, int EW, bool PL>
 int launch_tc_ew(const TMaps& tm, const GemmArgs& args, int num_sms, cudaStream_t stream) {
   using C = Cfg<ESZ, BN>;
   using SL = SmemLayout<ESZ, C::RING_BYTES, EW>;
-  auto kern = gemm_tcgen05_kernel<ESZ, A_MN, B_MN, BN, EW>;
+  auto kern = gemm_tcgen05_kernel<ESZ, A_MN, B_MN, BN, EW, PL>;
   static bool configured = false;
   if (!configured) {
     GB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SL::BYTES));
@@ -1557,8 +1611,10 @@ int launch_tc_ew(const TMaps& tm, const GemmArgs& args, int num_sms, cudaStream_
 
 template <int ESZ, bool A_MN, bool B_MN, int BN>
 int launch_tc(const TMaps& tm, const GemmArgs& args, int num_sms, cudaStream_t stream) {
-  if (g_epi_warps == 4) return launch_tc_ew<ESZ, A_MN, B_MN, BN, 4>(tm, args, num_sms, stream);
-  return launch_tc_ew<ESZ, A_MN, B_MN, BN, 8>(tm, args, num_sms, stream);
+  if constexpr (ESZ == 2)
+    if (args.planes > 0) return launch_tc_ew<ESZ, A_MN, B_MN, BN, 8, true>(tm, args, num_sms, stream);
+  if (g_epi_warps == 4) return launch_tc_ew<ESZ, A_MN, B_MN, BN, 4, false>(tm, args, num_sms, stream);
+  return launch_tc_ew<ESZ, A_MN, B_MN, BN, 8, false>(tm, args, num_sms, stream);
 }
 
 template <int ESZ, int BN>
@@ -1577,10 +1633,10 @@ int dispatch_major(bool a_mn, bool b_mn, const TMaps& tm, const GemmArgs& args, 
 
 int g_use_2cta = 1;
 
-template <bool A_MN, bool B_MN>
-int launch_2cta(const TMaps& tm, const GemmArgs& args, int num_sms, cudaStream_t stream) {
+template <bool A_MN, bool B_MN, bool PL>
+int launch_2cta_t(const TMaps& tm, const GemmArgs& args, int num_sms, cudaStream_t stream) {
   using SL = SmemLayout<2, Cfg2::RING_BYTES, 8>;
-  auto kern = gemm_tcgen05_2cta_kernel<A_MN, B_MN, 8>;
+  auto kern = gemm_tcgen05_2cta_kernel<A_MN, B_MN, 8, PL>;
   static bool configured = false;
   if (!configured) {
     GB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SL::BYTES));
@@ -1606,6 +1662,12 @@ int launch_2cta(const TMaps& tm, const GemmArgs& args, int num_sms, cudaStream_t
   return gbh::E_OK;
 }
 
+template <bool A_MN, bool B_MN>
+int launch_2cta(const TMaps& tm, const GemmArgs& args, int num_sms, cudaStream_t stream) {
+  return args.planes > 0 ? launch_2cta_t<A_MN, B_MN, true>(tm, args, num_sms, stream)
+                         : launch_2cta_t<A_MN, B_MN, false>(tm, args, num_sms, stream);
+}
+
 int g_cluster_splits = 0;   // 0: by the rule of cluster_splits(); -1: off; 1, 2, 4, 8: that many CTAs per tile
 
 // CTAs per 128 x 64 tile of the cluster kernel, 0 = another kernel.  K is cut until the CTAs come to about one per SM.
@@ -1624,9 +1686,9 @@ int cluster_splits(int M, int N, int K, int batch, int num_sms) {
   return s >= 4 || (s == 2 && num_kb >= 48) ? s : 0;
 }
 
-template <bool A_MN, bool B_MN>
-int launch_cluster(const TMaps& tm, const GemmArgs& args, cudaStream_t stream) {
-  auto kern = gemm_tcgen05_cluster_kernel<A_MN, B_MN>;
+template <bool A_MN, bool B_MN, bool PL>
+int launch_cluster_t(const TMaps& tm, const GemmArgs& args, cudaStream_t stream) {
+  auto kern = gemm_tcgen05_cluster_kernel<A_MN, B_MN, PL>;
   static bool configured = false;
   if (!configured) {
     GB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CfgS::BYTES));
@@ -1649,11 +1711,16 @@ int launch_cluster(const TMaps& tm, const GemmArgs& args, cudaStream_t stream) {
   return gbh::E_OK;
 }
 
+template <bool A_MN, bool B_MN>
+int launch_cluster(const TMaps& tm, const GemmArgs& args, cudaStream_t stream) {
+  return args.planes > 0 ? launch_cluster_t<A_MN, B_MN, true>(tm, args, stream) : launch_cluster_t<A_MN, B_MN, false>(tm, args, stream);
+}
+
 // Sums the K slices of a split launch in slice order and writes the result in the
-// caller's type: C = (beta ? C : 0) + sum_s ws[s].
+// caller's type: C = (beta ? C : 0) + sum_s ws[s] (+ an fp32 bias).
 template <typename TO>
-__global__ void splitk_finish_kernel(const float* __restrict__ ws, TO* __restrict__ C, int M, int N, int batch,
-                                     int splits, long long ldc, long long strideC, int beta) {
+__global__ void splitk_finish_kernel(const float* __restrict__ ws, TO* __restrict__ C, const float* __restrict__ bias, int M, int N,
+                                     int batch, int splits, long long ldc, long long strideC, int beta) {
   const long long per = (long long)M * N;
   const long long total = per * batch;
   for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < total;
@@ -1676,6 +1743,7 @@ __global__ void splitk_finish_kernel(const float* __restrict__ ws, TO* __restric
       m = r / N;
       n = r - m * N;
     }
+    if (bias != nullptr) { a.x += bias[n]; a.y += bias[n + 1]; a.z += bias[n + 2]; a.w += bias[n + 3]; }
     TO* c = C + b * strideC + m * ldc + n;
     if (sizeof(TO) == 2 && (((uintptr_t)c & 7) == 0)) {
       // four 16-bit results as one 8-byte access
@@ -1720,7 +1788,9 @@ int g_tma_epi = 1;
 // Builds the two tensor maps and launches.  esz: 2 (bf16/fp16) or 1 (int8).
 int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, int transB,
             long long lda, long long ldb, long long sA, long long sB, int force_bn,
-            cudaStream_t stream, void* workspace = nullptr, long long workspace_bytes = 0) {
+            cudaStream_t stream, void* workspace = nullptr, long long workspace_bytes = 0, int planes = 0) {
+  // planes > 0: A and B are stacks of three planes, sA / sB elements apart (batch entries 3 sA / 3 sB apart, 0: shared), and
+  // `planes` plane products run along K
   if (g_num_sms == 0) {
     int dev = 0;
     GB_CUDA_OK(cudaGetDevice(&dev));
@@ -1728,7 +1798,12 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
   }
   const bool a_mn = transA != 0;  // stored K x M
   const bool b_mn = transB == 0;  // stored K x N
-  const int M = args.M, N = args.N, K = args.K, batch = args.batch;
+  const int M = args.M, N = args.N, batch = args.batch;
+  const int atom_k = kSwizzleBytes / esz, kb_plane = (args.K + atom_k - 1) / atom_k;
+  args.num_kb = kb_plane * (planes > 0 ? planes : 1);
+  args.planes = planes;
+  args.kb_plane = kb_plane;
+  const int Kreal = args.K, K = planes > 0 ? args.num_kb * atom_k : args.K;   // K: length of the contraction
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) {
     gbh::set_error("gemm: empty problem M=%d N=%d K=%d batch=%d", M, N, K, batch);
     return gbh::E_BAD_ARG;
@@ -1757,7 +1832,7 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
   args.splits = 1;
   args.kb_per = (K + atom - 1) / atom;
   int splits = 1;
-  const bool plain = args.bias == nullptr && args.act == ACT_NONE && args.aux_mode == AUX_NONE;
+  const bool plain = (args.bias == nullptr || (planes > 0 && args.bias_f32)) && args.act == ACT_NONE && args.aux_mode == AUX_NONE;
   const bool big = 2.0 * M * N * (double)K * batch >= 8e9;  // below this the second launch costs more than it saves
   if (esz == 2 && g_splitk && force_bn == 0 && plain && big && workspace != nullptr && (N & 3) == 0 &&
       M >= 128 && N >= 128) {
@@ -1774,13 +1849,12 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
   void* user_C = args.C;
   const long long user_ldc = args.ldc, user_strideC = args.strideC;
   const int user_out = args.out_kind, user_beta = args.beta;
+  const float* user_bias = splits > 1 ? (const float*)args.bias : nullptr;
   if (splits > 1) {
-    const int num_kb = (K + atom - 1) / atom;
-    args.splits = splits;
-    args.kb_per = (num_kb + splits - 1) / splits;
-    if ((long long)(splits - 1) * args.kb_per >= num_kb) {  // the last slice would be empty
-      args.splits = splits = (num_kb + args.kb_per - 1) / args.kb_per;
-    }
+    args.bias = nullptr;
+    const int per = (kb_plane + splits - 1) / splits;
+    args.splits = splits = (kb_plane + per - 1) / per;      // (the last slice would be empty otherwise)
+    args.kb_per = per * (planes > 0 ? planes : 1);
     args.C = workspace;
     args.ldc = N;
     args.strideC = (long long)M * N;
@@ -1789,10 +1863,9 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
   }
   const int cluster = esz == 2 && force_bn == 0 && splits == 1 && !use2 ? cluster_splits(M, N, K, batch, g_num_sms) : 0;
   if (cluster) {
-    const int num_kb = (K + CfgS::BK - 1) / CfgS::BK;
     bn = CfgS::BN;
     args.splits = cluster;
-    args.kb_per = (num_kb + cluster - 1) / cluster;
+    args.kb_per = (kb_plane + cluster - 1) / cluster * (planes > 0 ? planes : 1);
   }
   if (use2) bn = 128;   // each CTA of a pair stages 128 of the tile's 256 columns
   args.num_m = use2 ? (M + 255) / 256 : (M + BM - 1) / BM;
@@ -1841,15 +1914,16 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
     uint64_t dims[3], strides[2];
     uint32_t box[3];
     if (!a_mn) {
-      dims[0] = K; dims[1] = M; dims[2] = batch;
+      dims[0] = Kreal; dims[1] = M; dims[2] = batch;
       box[0] = atom; box[1] = BM; box[2] = 1;
     } else {
-      dims[0] = M; dims[1] = K; dims[2] = batch;
+      dims[0] = M; dims[1] = Kreal; dims[2] = batch;
       box[0] = atom; box[1] = atom; box[2] = 1;
     }
     strides[0] = (uint64_t)lda * esz;
-    args.bcastA = (batch > 1 && sA == 0);
+    args.bcastA = planes > 0 ? args.bcastA : (batch > 1 && sA == 0);
     if (batch == 1 || args.bcastA) dims[2] = 1;
+    if (planes > 0) dims[2] *= 3;
     strides[1] = (uint64_t)(dims[2] > 1 ? sA : (long long)dims[1] * lda) * esz;
     int rc = gbh::encode_tmap(&tmA, dt, 3, A, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
@@ -1858,15 +1932,16 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
     uint64_t dims[3], strides[2];
     uint32_t box[3];
     if (!b_mn) {
-      dims[0] = K; dims[1] = N; dims[2] = batch;
+      dims[0] = Kreal; dims[1] = N; dims[2] = batch;
       box[0] = atom; box[1] = bn; box[2] = 1;
     } else {
-      dims[0] = N; dims[1] = K; dims[2] = batch;
+      dims[0] = N; dims[1] = Kreal; dims[2] = batch;
       box[0] = atom; box[1] = atom; box[2] = 1;
     }
     strides[0] = (uint64_t)ldb * esz;
-    args.bcastB = (batch > 1 && sB == 0);
+    args.bcastB = planes > 0 ? args.bcastB : (batch > 1 && sB == 0);
     if (batch == 1 || args.bcastB) dims[2] = 1;
+    if (planes > 0) dims[2] *= 3;
     strides[1] = (uint64_t)(dims[2] > 1 ? sB : (long long)dims[1] * ldb) * esz;
     int rc = gbh::encode_tmap(&tmB, dt, 3, B, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
@@ -1896,13 +1971,13 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
     const int grid = (int)(quads + 255) / 256 < g_num_sms * 8 ? (int)((quads + 255) / 256) : g_num_sms * 8;
     const float* ws = (const float*)workspace;
     if (user_out == OUT_F32)
-      splitk_finish_kernel<float><<<grid, 256, 0, stream>>>(ws, (float*)user_C, M, N, batch, splits, user_ldc,
+      splitk_finish_kernel<float><<<grid, 256, 0, stream>>>(ws, (float*)user_C, user_bias, M, N, batch, splits, user_ldc,
                                                             user_strideC, user_beta);
     else if (user_out == OUT_BF16)
-      splitk_finish_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(ws, (__nv_bfloat16*)user_C, M, N, batch,
+      splitk_finish_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(ws, (__nv_bfloat16*)user_C, user_bias, M, N, batch,
                                                                     splits, user_ldc, user_strideC, user_beta);
     else
-      splitk_finish_kernel<__half><<<grid, 256, 0, stream>>>(ws, (__half*)user_C, M, N, batch, splits,
+      splitk_finish_kernel<__half><<<grid, 256, 0, stream>>>(ws, (__half*)user_C, user_bias, M, N, batch, splits,
                                                              user_ldc, user_strideC, user_beta);
     GB_CUDA_OK(cudaGetLastError());
   }
@@ -1976,6 +2051,23 @@ GB_EXPORT int gb_gemm16(const void* A, const void* B, void* C, const void* bias,
   a.in_bf16 = in_dtype == DT_BF16;
   return gemm_tc(2, A, B, a, transA, transB, lda, ldb, sA, sB, force_bn, (cudaStream_t)stream, workspace,
                  workspace_bytes);
+}
+
+// fp32 C = alpha * op(A) op(B) (+ C) (+ bias[N]) from stacks of three bf16 planes: A (batch or 1, 3, rows, lda), B likewise,
+// plane_a / plane_b elements between planes.  `planes` products, product p of planes (order_a >> 4p) & 15 and
+// (order_b >> 4p) & 15, are added in that order into one fp32 accumulator.  (Called by gb_gemm_f32x3.)
+int gemm_bf16_planes(const void* A, const void* B, float* C, const float* bias, int M, int N, int K, int batch, int transA,
+                     int transB, long long lda, long long ldb, long long ldc, long long plane_a, long long plane_b, int bcastA,
+                     int bcastB, long long sC, int planes, uint32_t order_a, uint32_t order_b, float alpha, int beta,
+                     void* workspace, long long workspace_bytes, cudaStream_t stream) {
+  GemmArgs a;
+  memset(&a, 0, sizeof(a));
+  a.M = M; a.N = N; a.K = K; a.batch = batch;
+  a.C = C; a.bias = bias; a.bias_f32 = 1;
+  a.ldc = ldc; a.strideC = sC; a.alpha = alpha; a.beta = beta;
+  a.out_kind = OUT_F32; a.in_bf16 = 1;
+  a.bcastA = bcastA; a.bcastB = bcastB; a.plane_a = order_a; a.plane_b = order_b;
+  return gemm_tc(2, A, B, a, transA, transB, lda, ldb, plane_a, plane_b, 0, stream, workspace, workspace_bytes, planes);
 }
 
 // int8 x int8 -> int32 GEMM with the dequantising epilogue of the reference's

@@ -6,11 +6,11 @@
 // * fp64: mma.sync m16n8k8 f64 on 64 x 64 x 16 tiles.  Results match an fp64 FMA chain over k up to the order of
 //   the sum (1e-13-class agreement with a float64 oracle).
 // * fp32: each operand is split once into three bf16 planes (x = hi + mid + lo, 24 mantissa
-//   bits in total) and the six significant plane products hi*hi, hi*mid, mid*hi, hi*lo,
-//   lo*hi, mid*mid run as bf16 tcgen05 GEMMs over an extended K axis (six times the length in
-//   total, in three passes by magnitude class), with fp32 accumulation in tensor memory.  The
-//   dropped products are below 2^-24 of the result, the rounding level of an fp32 product itself.  Non-finite inputs keep their value in the hi
-//   plane and contribute zero to the others.
+//   bits in total) and the six significant plane products lo hi, hi lo, mid mid, mid hi, hi mid, hi hi
+//   run as one bf16 tcgen05 launch, in that order into one fp32 accumulator; the planes are the third
+//   dimension of the operands' tensor maps.  The dropped products are below 2^-24 of the result, the
+//   rounding level of an fp32 product itself.  Non-finite inputs keep their value in the hi plane and
+//   contribute zero to the others.  3000 x 4096 x 1024: 115 us (240 as three launches that added to C).
 //
 // The in-library benchmark loops at the end mirror the reference's (gonn_cuda.cu:255-294,
 // 532-592, 673-690): operands allocated once, five untimed calls, `iters` calls between two
@@ -24,6 +24,10 @@ extern "C" int gb_gemm16(const void* A, const void* B, void* C, const void* bias
                          long long ldc, long long ldaux, long long sA, long long sB, long long sC, long long sAux,
                          int in_dtype, int out_dtype, int act, int aux_mode, int beta, float alpha, int force_bn,
                          void* workspace, long long workspace_bytes, void* stream);
+int gemm_bf16_planes(const void* A, const void* B, float* C, const float* bias, int M, int N, int K, int batch, int transA,
+                     int transB, long long lda, long long ldb, long long ldc, long long plane_a, long long plane_b, int bcastA,
+                     int bcastB, long long sC, int planes, uint32_t order_a, uint32_t order_b, float alpha, int beta,
+                     void* workspace, long long workspace_bytes, cudaStream_t stream);
 extern "C" int gb_gemm_simt(const void* A, const void* B, void* C, int M, int N, int K, int batch, int transA,
                             int transB, long long lda, long long ldb, long long ldc, long long sA, long long sB,
                             long long sC, int dtype, double alpha, int beta, void* stream);
@@ -273,40 +277,41 @@ int launch_f64(const void* A, const void* B, void* C, int M, int N, int K, int b
 // ---------------------------------------------------------------------------
 // fp32 as three bf16 planes
 // ---------------------------------------------------------------------------
-// Plane order along the extended K axis: A side (hi, hi, mid, hi, lo, mid), B side
-// (hi, mid, hi, lo, hi, mid): position p of one multiplies position p of the other.
-__constant__ int c_plane_a[6] = {0, 0, 1, 0, 2, 1};
-__constant__ int c_plane_b[6] = {0, 1, 0, 2, 0, 1};
-
-// src: (rows, cols) fp32 with row pitch ld.  k_contig: cols is the K axis and the six planes sit
-// side by side in a row of 6 * Kp (Kp = cols padded to a multiple of 8, zero filled);
-// otherwise rows is the K axis and the planes are stacked: plane p occupies rows [p * rows, (p+1) * rows).
-__global__ void split3_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long rows,
-                              long long cols, long long ld, long long cols_p, int k_contig, int b_side,
-                              long long src_batch, long long dst_batch) {
+// Plane p of the result holds the p-th bf16 part of src (rows, cols; row pitch ld): dst [3][rows][cols_p], cols_p = cols
+// rounded up to 8, zero filled.  Bound by memory: 4 bytes read and 6 written per element; a thread turns eight
+// neighbouring elements into three 16-byte stores.  (Six planes in the order of the products, two bytes at a time
+// with a 64-bit division per element, took 267 us for the six operands of a 3000 x 1024 x 4096 layer; this takes 65.)
+__global__ void __launch_bounds__(256) split3_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, int rows, int cols,
+                                                     long long ld, int cols_p, long long src_batch, int vec) {
   src += (long long)blockIdx.z * src_batch;
-  dst += (long long)blockIdx.z * dst_batch;
-  const long long total = rows * cols_p;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long r = i / cols_p, c = i - r * cols_p;
-    float x = c < cols ? src[r * ld + c] : 0.f;
-    __nv_bfloat16 pl[3];
-    if (isfinite(x)) {
-      pl[0] = __float2bfloat16_rn(x);
-      const float r1 = x - __bfloat162float(pl[0]);
-      pl[1] = __float2bfloat16_rn(r1);
-      pl[2] = __float2bfloat16_rn(r1 - __bfloat162float(pl[1]));
+  const long long plane = (long long)rows * cols_p;
+  dst += (long long)blockIdx.z * 3 * plane;
+  const int per_row = cols_p / 8;
+  const unsigned total = (unsigned)rows * (unsigned)per_row;      // < 2^31: the operands' 16-bit planes fit 4 GiB
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const unsigned r = i / (unsigned)per_row;
+    const int c = (int)(i - r * per_row) * 8;
+    const float* s = src + (long long)r * ld + c;
+    float x[8];
+    if (vec && c + 8 <= cols) {
+      const float4 u = __ldg(reinterpret_cast<const float4*>(s)), v = __ldg(reinterpret_cast<const float4*>(s) + 1);
+      x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
     } else {
-      pl[0] = __float2bfloat16_rn(x);
-      pl[1] = pl[2] = __float2bfloat16_rn(0.f);
-    }
 #pragma unroll
-    for (int p = 0; p < 6; p++) {
-      const __nv_bfloat16 v = pl[b_side ? c_plane_b[p] : c_plane_a[p]];
-      if (k_contig) dst[r * (6 * cols_p) + p * cols_p + c] = v;
-      else dst[((long long)p * rows + r) * cols_p + c] = v;
+      for (int j = 0; j < 8; j++) x[j] = c + j < cols ? __ldg(s + j) : 0.f;
     }
+    __align__(16) __nv_bfloat16 pl[3][8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const bool fin = isfinite(x[j]);
+      pl[0][j] = __float2bfloat16_rn(x[j]);
+      const float r1 = fin ? x[j] - __bfloat162float(pl[0][j]) : 0.f;
+      pl[1][j] = __float2bfloat16_rn(r1);
+      pl[2][j] = __float2bfloat16_rn(r1 - __bfloat162float(pl[1][j]));
+    }
+    __nv_bfloat16* d = dst + (long long)r * cols_p + c;
+#pragma unroll
+    for (int p = 0; p < 3; p++) *reinterpret_cast<uint4*>(d + p * plane) = *reinterpret_cast<const uint4*>(pl[p]);
   }
 }
 
@@ -344,14 +349,13 @@ GB_EXPORT int gb_gemm_f64(const void* A, const void* B, void* C, int M, int N, i
 // Bytes of scratch gb_gemm_f32x3 needs for the split operands.
 GB_EXPORT long long gb_gemm_f32x3_workspace(int M, int N, int K, int batch) {
   const long long Kp = (K + 7) / 8 * 8, Mp = (M + 7) / 8 * 8, Np = (N + 7) / 8 * 8;
-  // either layout of an operand fits in 6 * Kp * (padded other dimension) elements
-  return 2LL * batch * 6 * Kp * (Mp > Np ? Mp : Np) * 2 + 256;
+  const long long a = M * Kp > K * Mp ? M * Kp : K * Mp, b = N * Kp > K * Np ? N * Kp : K * Np;   // either storage form
+  return 2LL * batch * 3 * (a + b) + 256;
 }
 
-// fp32 GEMM through three bf16 planes per operand (see the file header).  workspace:
-// gb_gemm_f32x3_workspace() bytes; split_ws / split_ws_bytes: optional split-K scratch handed
-// on to the bf16 GEMM.
-GB_EXPORT int gb_gemm_f32x3(const void* A, const void* B, void* C, int M, int N, int K, int batch, int transA,
+// fp32 GEMM through three bf16 planes per operand (see the file header).  bias: fp32 [N] or null.  workspace:
+// gb_gemm_f32x3_workspace() bytes; split_ws / split_ws_bytes: optional split-K scratch handed on to the bf16 GEMM.
+GB_EXPORT int gb_gemm_f32x3(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int batch, int transA,
                             int transB, long long lda, long long ldb, long long ldc, long long sA, long long sB,
                             long long sC, float alpha, int beta, void* workspace, long long workspace_bytes,
                             void* split_ws, long long split_ws_bytes, void* stream) {
@@ -360,50 +364,29 @@ GB_EXPORT int gb_gemm_f32x3(const void* A, const void* B, void* C, int M, int N,
     return gbh::E_BAD_ARG;
   }
   cudaStream_t s = (cudaStream_t)stream;
-  const long long Kp = (K + 7) / 8 * 8, Mp = (M + 7) / 8 * 8, Np = (N + 7) / 8 * 8;
+  const bool share_a = batch > 1 && sA == 0, share_b = batch > 1 && sB == 0;
+  // an operand as stored: (rows, cols)
+  const int ar = transA ? K : M, ac = transA ? M : K, br = transB ? N : K, bc = transB ? K : N;
+  const long long acp = (ac + 7) / 8 * 8, bcp = (bc + 7) / 8 * 8;
+  const long long plane_a = ar * acp, plane_b = br * bcp;
   __nv_bfloat16* a3 = (__nv_bfloat16*)workspace;
-  const long long a_elems = 6 * Kp * Mp, b_elems = 6 * Kp * Np;
-  __nv_bfloat16* b3 = a3 + (long long)batch * a_elems;
-  const int ba = sA ? batch : 1, bb = sB ? batch : 1;
-  long long lda3, ldb3;
-  // A as stored: (M, K) (k contiguous) unless transA, then (K, M)
-  if (!transA) {
-    split3_kernel<<<dim3(592, 1, ba), 256, 0, s>>>((const float*)A, a3, M, K, lda, Kp, 1, 0, sA, a_elems);
-    lda3 = 6 * Kp;
-  } else {
-    split3_kernel<<<dim3(592, 1, ba), 256, 0, s>>>((const float*)A, a3, K, M, lda, Mp, 0, 0, sA, a_elems);
-    lda3 = Mp;
-  }
-  if (transB) {  // stored (N, K): k contiguous
-    split3_kernel<<<dim3(592, 1, bb), 256, 0, s>>>((const float*)B, b3, N, K, ldb, Kp, 1, 1, sB, b_elems);
-    ldb3 = 6 * Kp;
-  } else {
-    split3_kernel<<<dim3(592, 1, bb), 256, 0, s>>>((const float*)B, b3, K, N, ldb, Np, 0, 1, sB, b_elems);
-    ldb3 = Np;
-  }
+  __nv_bfloat16* b3 = a3 + 3 * plane_a * (share_a ? 1 : batch);
+  auto split = [&](const void* src, __nv_bfloat16* dst, int rows, int cols, long long ld, long long cols_p, long long sb, int n) {
+    const int vec = (ld & 3) == 0 && (sb & 3) == 0 && (((uintptr_t)src) & 15) == 0;
+    const long long blocks = (rows * (cols_p / 8) + 255) / 256;
+    split3_kernel<<<dim3((unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 1, n), 256, 0, s>>>((const float*)src, dst, rows, cols, ld,
+                                                                                               (int)cols_p, sb, vec);
+  };
+  split(A, a3, ar, ac, lda, acp, sA, share_a ? 1 : batch);
+  split(B, b3, br, bc, ldb, bcp, sB, share_b ? 1 : batch);
   GB_CUDA_OK(cudaGetLastError());
-  // Both operands must agree on where plane p starts along the extended K axis: at p * Kp when
-  // the planes sit side by side, at p * K when they are stacked; so the stacked form needs Kp == K.
-  const bool stacked_a = transA != 0, stacked_b = transB == 0;
-  if ((stacked_a || stacked_b) && Kp != K) {
-    gbh::set_error("gb_gemm_f32x3: K must be a multiple of 8 unless both operands are K-contiguous");
-    return gbh::E_BAD_ARG;
-  }
-  // Three passes over sub-ranges of the extended K axis, smallest terms first, each added to C
-  // by the epilogue's fp32 add: (hi*lo, lo*hi, mid*mid), then (hi*mid, mid*hi), then hi*hi.  The
-  // tensor core aligns every product with its accumulator before adding; keeping terms of one
-  // magnitude class per accumulator is what preserves the low planes' contribution.
-  const int first_plane[3] = {3, 1, 0}, planes[3] = {3, 2, 1};
-  for (int pass = 0; pass < 3; pass++) {
-    const long long koff = (long long)first_plane[pass] * Kp;
-    const __nv_bfloat16* ap = a3 + (stacked_a ? koff * lda3 : koff);
-    const __nv_bfloat16* bp = b3 + (stacked_b ? koff * ldb3 : koff);
-    const int rc = gb_gemm16(ap, bp, C, nullptr, 0, nullptr, M, N, (int)(planes[pass] * Kp), batch, transA, transB,
-                             lda3, ldb3, ldc, 0, sA ? a_elems : 0, sB ? b_elems : 0, sC, 0, DT_BF16, DT_F32, 0, 0,
-                             pass == 0 ? beta : 1, alpha, 0, split_ws, split_ws_bytes, stream);
-    if (rc != 0) return rc;
-  }
-  return gbh::E_OK;
+  // Planes 0, 1, 2 = hi, mid, lo.  One launch and one accumulator for all six products, from the smallest to the largest:
+  // lo hi, hi lo, mid mid, then mid hi, hi mid, then hi hi.  The tensor core truncates each sum at its accumulator's last
+  // bit, so the small products must be in before the large ones; the error is then that of the hi hi chain alone
+  // (relative to 64 bits at 3000 x 4096 x 1024: 1.0e-6 in this order in one accumulator, in two and in three).
+  // A slice of a split K runs all six products over its part of K, which shortens that chain.
+  return gemm_bf16_planes(a3, b3, (float*)C, (const float*)bias, M, N, K, batch, transA, transB, acp, bcp, ldc, plane_a, plane_b,
+                          share_a, share_b, sC, 6, 0x001102u, 0x010120u, alpha, beta, split_ws, split_ws_bytes, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -452,7 +435,7 @@ GB_EXPORT double gb_bench_matmul(int m, int k, int n, int iters, int dtype) {
     ms = bench_loop(iters, [&] { return gb_gemm_f64(A, B, C, m, n, k, 1, 0, 0, k, n, n, 0, 0, 0, 1.0, 0, nullptr); });
   else if (dtype == DT_F32)
     ms = bench_loop(iters, [&] {
-      return gb_gemm_f32x3(A, B, C, m, n, k, 1, 0, 0, k, n, n, 0, 0, 0, 1.f, 0, ws, ws_bytes, nullptr, 0, nullptr);
+      return gb_gemm_f32x3(A, B, C, nullptr, m, n, k, 1, 0, 0, k, n, n, 0, 0, 0, 1.f, 0, ws, ws_bytes, nullptr, 0, nullptr);
     });
   else
     ms = bench_loop(iters, [&] {

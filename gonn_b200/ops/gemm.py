@@ -172,7 +172,17 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         raise ValueError(f"gemm: out has shape {tuple(out.shape)}, expected {oshape}")
 
     if native_simt:
-        if bias is not None or ACT[act] or (aux is not None and AUX[aux_mode]):
+        need = 0                        # scratch of the plane path, 0 = another kernel
+        if (a.dtype == torch.float32 and out.dtype == torch.float32 and _FP32_MODE == "bf16x3"
+                and 2.0 * M * N * K * batch >= 2.0 ** 28 and M >= 128 and N >= 128
+                and (K % 8 == 0 or (not trans_a and trans_b)) and out.stride(-2) % 4 == 0
+                and out.data_ptr() % 16 == 0):
+            need = int(_l.lib().gb_gemm_f32x3_workspace(M, N, K, batch))
+            need = need if need <= (4 << 30) else 0
+        # the plane path adds an fp32 bias in its epilogue
+        bias_in = (bias is None or need > 0 and bias.dtype == torch.float32 and bias.device == a.device and bias.numel() == N
+                   and bias.is_contiguous())
+        if not bias_in or ACT[act] or (aux is not None and AUX[aux_mode]):
             # exact-precision path: epilogue evaluated with tensor ops
             tmp = gemm(a, b, trans_a=trans_a, trans_b=trans_b, alpha=alpha)
             return _epilogue_torch(tmp, bias, act, aux, aux_mode, beta, out)
@@ -186,20 +196,15 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
                     _l.I(int(trans_a)), _l.I(int(trans_b)), _l.L(lda), _l.L(ldb), _l.L(out.stride(-2)), _l.L(sA),
                     _l.L(sB), _l.L(sC), _l.D(alpha), _l.I(int(beta)), _l.stream_ptr())
             return out
-        if (a.dtype == torch.float32 and out.dtype == torch.float32 and _FP32_MODE == "bf16x3"
-                and 2.0 * M * N * K * batch >= 2.0 ** 28 and M >= 128 and N >= 128
-                and (K % 8 == 0 or (not trans_a and trans_b)) and out.stride(-2) % 4 == 0
-                and out.data_ptr() % 16 == 0):
-            need = int(_l.lib().gb_gemm_f32x3_workspace(M, N, K, batch))
-            if need <= (4 << 30):
-                ws3 = _x3_workspace(a.device, need)
-                ws = _workspace(a.device) if M * N * batch * 4 * 2 <= _WS_BYTES else None
-                _l.call("gb_gemm_f32x3", _l.ptr(a2), _l.ptr(b2), _l.ptr(out), _l.I(M), _l.I(N), _l.I(K),
-                        _l.I(batch), _l.I(int(trans_a)), _l.I(int(trans_b)), _l.L(lda), _l.L(ldb),
-                        _l.L(out.stride(-2)), _l.L(sA), _l.L(sB), _l.L(sC), _l.F(alpha), _l.I(int(beta)),
-                        _l.ptr(ws3), _l.L(ws3.numel()), _l.ptr(ws), _l.L(_WS_BYTES if ws is not None else 0),
-                        _l.stream_ptr())
-                return out
+        if need:
+            ws3 = _x3_workspace(a.device, need)
+            ws = _workspace(a.device) if M * N * batch * 4 * 2 <= _WS_BYTES else None
+            _l.call("gb_gemm_f32x3", _l.ptr(a2), _l.ptr(b2), _l.ptr(out), _l.ptr(bias), _l.I(M), _l.I(N), _l.I(K),
+                    _l.I(batch), _l.I(int(trans_a)), _l.I(int(trans_b)), _l.L(lda), _l.L(ldb),
+                    _l.L(out.stride(-2)), _l.L(sA), _l.L(sB), _l.L(sC), _l.F(alpha), _l.I(int(beta)),
+                    _l.ptr(ws3), _l.L(ws3.numel()), _l.ptr(ws), _l.L(_WS_BYTES if ws is not None else 0),
+                    _l.stream_ptr())
+            return out
         _l.call("gb_gemm_simt", _l.ptr(a2), _l.ptr(b2), _l.ptr(out), _l.I(M), _l.I(N), _l.I(K),
                 _l.I(batch), _l.I(int(trans_a)), _l.I(int(trans_b)), _l.L(lda), _l.L(ldb),
                 _l.L(out.stride(-2)), _l.L(sA), _l.L(sB), _l.L(sC), _l.I(_l.dtype_code(a.dtype)),

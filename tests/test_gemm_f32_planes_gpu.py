@@ -1,0 +1,40 @@
+"""fp32 products as bf16 planes (csrc/gemm_exact.cu): one launch for the six plane products, K slices, the fused bias."""
+import pytest
+import torch
+
+from gonn_b200 import lib as L
+from gonn_b200.ops.gemm import gemm
+
+pytestmark = pytest.mark.gpu
+
+
+# one tile row, K that 64 does not divide (K % 8 == 0 where an operand is stored along K), split and cluster sizes, two-CTA tiles
+@pytest.mark.parametrize("M,N,K,ta,tb", [(128, 256, 4100, False, True), (333, 512, 1000, False, False), (136, 132, 8200, True, False),
+                                         (1100, 768, 520, True, True), (3000, 1028, 264, False, True)])
+@pytest.mark.parametrize("bias,beta", [(False, False), (True, False), (True, True), (False, True)])
+def test_against_float64(M, N, K, ta, tb, bias, beta):
+    torch.manual_seed(K)
+    a, b = torch.randn((K, M) if ta else (M, K)), torch.randn((N, K) if tb else (K, N))
+    bv = torch.randn(N) * K ** 0.5 if bias else None
+    want = (a.t() if ta else a).double() @ (b.t() if tb else b).double()
+    out = torch.randn(M, N).cuda() if beta else None
+    if bias:
+        want = want + bv.double()
+    if beta:
+        want = want + out.double().cpu()
+    got = gemm(a.cuda(), b.cuda(), trans_a=ta, trans_b=tb, bias=None if bv is None else bv.cuda(), out=out, beta=beta)
+    L.assert_status_ok()
+    # planes drop less than 2^-24 of each product; the accumulator truncates once per 16 products: K / 16 units of 2^-24
+    # of a partial sum at worst, half that on average over the chain
+    assert float((got.double().cpu() - want).norm() / want.norm()) < (K / 32 + 4) * 2.0 ** -24
+
+
+def test_batches_share_an_operand_and_infinities_stay_in_their_row():
+    a, b = torch.randn(3, 256, 512), torch.randn(512, 512)
+    a[1, 5, 7] = float("inf")
+    got = gemm(a.cuda(), b.cuda()).cpu()
+    want = a.double() @ b.double()
+    fin = torch.ones(3, 256, dtype=torch.bool)
+    fin[1, 5] = False
+    assert not got[~fin].isfinite().any()      # (the planes of b have both signs)
+    assert float((got[fin].double() - want[fin]).norm() / want[fin].norm()) < 20 * 2.0 ** -24
