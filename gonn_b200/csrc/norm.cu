@@ -671,6 +671,105 @@ norm_fwd_pipe_kernel(const T* __restrict__ x, const TW* __restrict__ w, const TW
   }
 }
 
+// V weights (16-byte aligned), or a constant where there are none.
+template <typename TW, int V>
+__device__ __forceinline__ void load_params(const TW* p, int vi, float none, float2* f) {
+  constexpr int PER = IO<TW>::V;          // elements of one 16-byte load
+  using Raw = typename IO<TW>::Raw;
+#pragma unroll
+  for (int i = 0; i < V / PER; i++) {
+    if (p != nullptr) Pairs<TW>::unpack(__ldg(reinterpret_cast<const Raw*>(p) + vi * (V / PER) + i), f + i * (PER / 2));
+    else
+#pragma unroll
+      for (int j = 0; j < PER / 2; j++) f[i * (PER / 2) + j] = f2(none);
+  }
+}
+
+// Forward, rows of at most 256 vectors: one warp per row, the whole row in registers, every load in flight at once and
+// nothing shared.  Bound by memory and launch latency; the ring of the kernel above needs several tiles per CTA to pay
+// for its barriers and leaves only 3 x 148 rows in work (us here | there: 8192 rows of 2048 bf16 9.9 | 19.2, 16 384 of 768
+// 9.1 | 12.7, 77 of 768 2.3 | 3.6, 131 072 of 2048 164 | 249, which is 6.5 TB/s).
+template <typename T, typename TW, int VPT, bool RMS>
+__global__ void __launch_bounds__(128)
+norm_fwd_warp_kernel(const T* __restrict__ x, const TW* __restrict__ w, const TW* __restrict__ b, T* __restrict__ y,
+                     float* __restrict__ mean_out, float* __restrict__ rstd_out, long long rows, int D, float eps) {
+  constexpr int V = IO<T>::V;
+  constexpr int NP2 = Pairs<T>::NP2;
+  using Raw = typename IO<T>::Raw;
+  const int lane = threadIdx.x & 31, nvec = D / V;
+  const float invD = 1.f / (float)D;
+  for (long long row = (long long)blockIdx.x * 4 + (threadIdx.x >> 5); row < rows; row += (long long)gridDim.x * 4) {
+    const T* xr = x + row * D;
+    Raw raw[VPT];
+#pragma unroll
+    for (int i = 0; i < VPT; i++)
+      if (lane + 32 * i < nvec) raw[i] = __ldg(reinterpret_cast<const Raw*>(xr) + lane + 32 * i);
+    float2 f[VPT][NP2];
+#pragma unroll
+    for (int i = 0; i < VPT; i++) {
+      if (lane + 32 * i < nvec) Pairs<T>::unpack(raw[i], f[i]);
+      else
+#pragma unroll
+        for (int j = 0; j < NP2; j++) f[i][j] = f2(0.f);
+    }
+    float mean = 0.f, rstd, shiftv = 0.f;
+    float2 a = f2(0.f), q = f2(0.f);
+    float K = 0.f;
+    if (RMS) {
+#pragma unroll
+      for (int i = 0; i < VPT; i++)
+#pragma unroll
+        for (int j = 0; j < NP2; j++) q = __ffma2_rn(f[i][j], f[i][j], q);
+    } else {
+      // sums of (x - K) and (x - K)^2, K = the row's first element (see the kernel above)
+      K = __shfl_sync(0xffffffffu, f[0][0].x, 0);
+      const float2 nk = f2(-K);
+#pragma unroll
+      for (int i = 0; i < VPT; i++)
+        if (lane + 32 * i < nvec) {
+#pragma unroll
+          for (int j = 0; j < NP2; j++) {
+            f[i][j] = __fadd2_rn(f[i][j], nk);
+            a = __fadd2_rn(a, f[i][j]);
+            q = __ffma2_rn(f[i][j], f[i][j], q);
+          }
+        }
+    }
+    float s0 = a.x + a.y, s1 = q.x + q.y;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      if (!RMS) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+    }
+    if (RMS) {
+      rstd = rsqrtf(s1 * invD + eps);
+    } else {
+      const float m = s0 * invD;
+      mean = K + m;
+      rstd = rsqrtf(fmaxf(s1 * invD - m * m, 0.f) + eps);
+      shiftv = -m * rstd;
+    }
+    if (lane == 0) {
+      if (mean_out) mean_out[row] = mean;
+      rstd_out[row] = rstd;
+    }
+    Raw* yr = reinterpret_cast<Raw*>(y + row * D);
+    const float2 rs = f2(rstd), sv = f2(shiftv);
+#pragma unroll
+    for (int i = 0; i < VPT; i++) {
+      const int vi = lane + 32 * i;
+      if (vi < nvec) {
+        float2 o[NP2], wv[NP2], bv[NP2];
+        load_params<TW, V>(w, vi, 1.f, wv);
+        load_params<TW, V>(RMS ? nullptr : b, vi, 0.f, bv);
+#pragma unroll
+        for (int j = 0; j < NP2; j++) o[j] = __ffma2_rn(__ffma2_rn(f[i][j], rs, sv), wv[j], bv[j]);
+        yr[vi] = Pairs<T>::pack(o);
+      }
+    }
+  }
+}
+
 // Backward: dx per row; dgamma / dbeta accumulate per thread over the rows its group
 // visits, are combined over the groups of the CTA through shared memory in group order and
 // written to part[blockIdx.x][NP][D]; norm_param_reduce_kernel adds the CTAs in index order.
@@ -853,26 +952,6 @@ inline PipePlan pipe_plan(size_t row_bytes, int NG, int nsrc, size_t extra_bytes
 
 // (threads per row, vectors per thread) by row width in 16-byte vectors.  The backward keeps
 // 16 fp32 accumulators per vector in registers, so it spreads a row over more threads.
-#define GB_PIPE_DISPATCH(X)      \
-  if (nvec <= 32) X(32, 1)       \
-  else if (nvec <= 64) X(32, 2)  \
-  else if (nvec <= 96) X(32, 3)  \
-  else if (nvec <= 128) X(64, 2) \
-  else if (nvec <= 192) X(64, 3) \
-  else if (nvec <= 256) X(128, 2)\
-  else if (nvec <= 384) X(128, 3)\
-  else if (nvec <= 512) X(256, 2)\
-  else if (nvec <= 768) X(256, 3)\
-  else X(256, 4)
-#define GB_PIPE_DISPATCH_BWD(X)  \
-  if (nvec <= 32) X(32, 1)       \
-  else if (nvec <= 64) X(32, 2)  \
-  else if (nvec <= 128) X(64, 2) \
-  else if (nvec <= 256) X(128, 2)\
-  else if (nvec <= 512) X(256, 2)\
-  else if (nvec <= 768) X(256, 3)\
-  else X(256, 4)
-
 #define GB_PIPE_DISPATCH_RES(X)  \
   if (nvec <= 32) X(32, 1)       \
   else if (nvec <= 64) X(64, 1)  \
@@ -896,7 +975,22 @@ int norm_fwd_t(const void* x, const void* w, const void* b, void* y, float* mean
   constexpr int V = IO<T>::V;
   const bool aligned = (D % V == 0) && ((((uintptr_t)x | (uintptr_t)y) & 15) == 0);
   const int nvec = D / V;
-  if (aligned && nvec <= 1024 && g_norm_pipe) {
+  if (aligned && nvec <= 256 && g_norm_pipe && (((uintptr_t)w | (uintptr_t)b) & 15) == 0) {
+    const long long blocks = (rows + 3) / 4;
+#define GB_FWDW(VPT)                                                                                               \
+  norm_fwd_warp_kernel<T, TW, VPT, RMS><<<(unsigned)(blocks < (1 << 20) ? blocks : (1 << 20)), 128, 0, s>>>(       \
+      (const T*)x, (const TW*)w, (const TW*)b, (T*)y, mean, rstd, rows, D, eps)
+    if (nvec <= 32) GB_FWDW(1);
+    else if (nvec <= 64) GB_FWDW(2);
+    else if (nvec <= 96) GB_FWDW(3);
+    else if (nvec <= 128) GB_FWDW(4);
+    else if (nvec <= 192) GB_FWDW(6);
+    else GB_FWDW(8);
+#undef GB_FWDW
+    GB_CUDA_OK(cudaGetLastError());
+    return gbh::E_OK;
+  }
+  if (aligned && nvec > 256 && nvec <= 1024 && g_norm_pipe) {
     int rc = 1;
 #define GB_FWDP(G, VPT)                                                                                  \
     {                                                                                                    \
@@ -916,7 +1010,10 @@ int norm_fwd_t(const void* x, const void* w, const void* b, void* y, float* mean
         rc = 0;                                                                                          \
       }                                                                                                  \
     }
-    GB_PIPE_DISPATCH(GB_FWDP)
+    if (nvec <= 384) GB_FWDP(128, 3)
+    else if (nvec <= 512) GB_FWDP(256, 2)
+    else if (nvec <= 768) GB_FWDP(256, 3)
+    else GB_FWDP(256, 4)
 #undef GB_FWDP
     if (rc == 0) {
       GB_CUDA_OK(cudaGetLastError());

@@ -1,0 +1,27 @@
+"""The warp-per-row norm forward (csrc/norm.cu): every vector count per lane, ragged rows, weights it cannot load whole."""
+import pytest
+import torch
+
+from gonn_b200 import lib as L
+from gonn_b200.ops import norm as N
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype,wdtype", [(torch.bfloat16, torch.bfloat16), (torch.float16, torch.float32), (torch.float32, torch.float32)])
+@pytest.mark.parametrize("nvec", [1, 31, 33, 64, 65, 97, 129, 192, 193, 256, 257])
+@pytest.mark.parametrize("rms", [False, True])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_forward(dtype, wdtype, nvec, rms, shift):
+    D, rows = nvec * (4 if dtype == torch.float32 else 8), 7
+    torch.manual_seed(nvec)
+    x = (torch.randn(rows, D) * 3 + 50 * (not rms)).to(dtype)             # a mean far above the spread
+    w, b = (torch.randn(D + 1)[shift:shift + D].to(wdtype) for _ in range(2))
+    wc, bc = (torch.empty(D + 1, dtype=wdtype, device="cuda")[shift:shift + D].copy_(t) for t in (w, b))
+    got = (N.rms_norm(x.cuda(), wc, 1e-6) if rms else N.layer_norm(x.cuda(), wc, bc, 1e-5)).double().cpu()
+    L.assert_status_ok()
+    want = N.norm_ref(x.double(), w.double(), None if rms else b.double(), 1e-6 if rms else 1e-5, rms)
+    # one rounding of the result; the fp32 sums of the shifted row stay far below it (fp32: 2^-24 per term, D terms, and the
+    # cancellation of the offset, 50 / 3 of it)
+    tol = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 1e-5}[dtype]
+    assert float((got - want).norm() / want.norm()) < tol
