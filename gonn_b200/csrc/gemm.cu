@@ -1368,7 +1368,7 @@ gemm_tcgen05_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
 // SIMT fallback for fp32 / fp64 operands (exact-precision parity paths)
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void gemm_simt_kernel(const T* __restrict__ A, const T* __restrict__ B, T* __restrict__ C,
+__global__ void gemm_simt_kernel(const T* __restrict__ A, const T* __restrict__ B, T* __restrict__ C, const T* __restrict__ bias,
                                  int M, int N, int K, int transA, int transB, long long lda,
                                  long long ldb, long long ldc, long long sA, long long sB,
                                  long long sC, T alpha, int beta) {
@@ -1427,7 +1427,7 @@ __global__ void gemm_simt_kernel(const T* __restrict__ A, const T* __restrict__ 
       int gn = n0 + tx * 4 + j;
       if (gn >= N) continue;
       T* p = C + (long long)gm * ldc + gn;
-      T v = alpha * acc[i][j];
+      T v = alpha * acc[i][j] + (bias != nullptr ? bias[gn] : T(0));
       *p = beta ? (*p + v) : v;
     }
   }
@@ -1440,7 +1440,7 @@ __global__ void gemm_simt_kernel(const T* __restrict__ A, const T* __restrict__ 
 // buffers; the next tile travels global -> registers while the current one is multiplied.
 template <typename T, int TM, int TN, int BK>
 __global__ void __launch_bounds__(256, 2)
-gemm_simt_tiled_kernel(const T* __restrict__ A, const T* __restrict__ B, T* __restrict__ C, int M,
+gemm_simt_tiled_kernel(const T* __restrict__ A, const T* __restrict__ B, T* __restrict__ C, const T* __restrict__ bias, int M,
                        int N, int K, int transA, int transB, long long lda, long long ldb,
                        long long ldc, long long sA, long long sB, long long sC, T alpha, int beta) {
   constexpr int VEC = 16 / (int)sizeof(T);
@@ -1551,12 +1551,15 @@ gemm_simt_tiled_kernel(const T* __restrict__ A, const T* __restrict__ B, T* __re
         const int gn = n0 + h * 16 * VEC + tx * VEC;
         if (gn >= N) continue;
         T* p = C + (long long)gm * ldc + gn;
+        T add[VEC];
+#pragma unroll
+        for (int v = 0; v < VEC; v++) add[v] = bias != nullptr && gn + v < N ? __ldg(bias + gn + v) : T(0);
         if (vec_ok && gn + VEC <= N) {
           Vec o;
           if (beta) o = *reinterpret_cast<const Vec*>(p);
 #pragma unroll
           for (int v = 0; v < VEC; v++) {
-            const T r = alpha * acc[i][h * VEC + v];
+            const T r = alpha * acc[i][h * VEC + v] + add[v];
             o.v[v] = beta ? (o.v[v] + r) : r;
           }
           *reinterpret_cast<Vec*>(p) = o;
@@ -1564,7 +1567,7 @@ gemm_simt_tiled_kernel(const T* __restrict__ A, const T* __restrict__ B, T* __re
 #pragma unroll
           for (int v = 0; v < VEC; v++) {
             if (gn + v >= N) continue;
-            const T r = alpha * acc[i][h * VEC + v];
+            const T r = alpha * acc[i][h * VEC + v] + add[v];
             p[v] = beta ? (p[v] + r) : r;
           }
         }
@@ -1576,13 +1579,13 @@ gemm_simt_tiled_kernel(const T* __restrict__ A, const T* __restrict__ B, T* __re
 int g_simt_tiled = 1;   // 0 selects the plain 64 x 64 kernel above
 
 template <typename T, int TM, int TN, int BK>
-void launch_simt_tiled(const void* A, const void* B, void* C, int M, int N, int K, int batch,
+void launch_simt_tiled(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int batch,
                        int transA, int transB, long long lda, long long ldb, long long ldc,
                        long long sA, long long sB, long long sC, double alpha, int beta,
                        cudaStream_t stream) {
   dim3 grid((N + 16 * TN - 1) / (16 * TN), (M + 16 * TM - 1) / (16 * TM), batch);
   gemm_simt_tiled_kernel<T, TM, TN, BK><<<grid, 256, 0, stream>>>(
-      (const T*)A, (const T*)B, (T*)C, M, N, K, transA, transB, lda, ldb, ldc, sA, sB, sC, (T)alpha,
+      (const T*)A, (const T*)B, (T*)C, (const T*)bias, M, N, K, transA, transB, lda, ldb, ldc, sA, sB, sC, (T)alpha,
       beta);
 }
 
@@ -1668,7 +1671,7 @@ int launch_2cta(const TMaps& tm, const GemmArgs& args, int num_sms, cudaStream_t
                          : launch_2cta_t<A_MN, B_MN, false>(tm, args, num_sms, stream);
 }
 
-int g_cluster_splits = 0;   // 0: by the rule of cluster_splits(); -1: off; 1, 2, 4, 8: that many CTAs per tile
+thread_local int g_cluster_splits = 0;   // 0: by the rule of cluster_splits(); -1: off; 1, 2, 4, 8: that many CTAs per tile
 
 // CTAs per 128 x 64 tile of the cluster kernel, 0 = another kernel.  K is cut until the CTAs come to about one per SM.
 // The cluster's exchange costs 2.5 us, so it pays from four parts on, or from two where K is long.  Measured, us
@@ -2094,8 +2097,8 @@ GB_EXPORT int gb_gemm_i8(const void* A, const void* B, void* C, const float* bia
   return gemm_tc(1, A, B, a, 0, 1, lda, ldb, 0, 0, 0, (cudaStream_t)stream);
 }
 
-// fp32 / fp64 SIMT GEMM (exact-precision paths).
-GB_EXPORT int gb_gemm_simt(const void* A, const void* B, void* C, int M, int N, int K, int batch,
+// fp32 / fp64 SIMT GEMM (exact-precision paths).  bias: length N in the operands' type, or null.
+GB_EXPORT int gb_gemm_simt(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int batch,
                            int transA, int transB, long long lda, long long ldb, long long ldc,
                            long long sA, long long sB, long long sC, int dtype, double alpha,
                            int beta, void* stream) {
@@ -2115,22 +2118,22 @@ GB_EXPORT int gb_gemm_simt(const void* A, const void* B, void* C, int M, int N, 
     const bool big = big_tiles >= 120;
     cudaStream_t st = (cudaStream_t)stream;
     if (dtype == DT_F32) {
-      if (big) launch_simt_tiled<float, 8, 8, 16>(A, B, C, M, N, K, batch, transA, transB, lda, ldb, ldc, sA, sB, sC, alpha, beta, st);
-      else launch_simt_tiled<float, 4, 4, 16>(A, B, C, M, N, K, batch, transA, transB, lda, ldb, ldc, sA, sB, sC, alpha, beta, st);
+      if (big) launch_simt_tiled<float, 8, 8, 16>(A, B, C, bias, M, N, K, batch, transA, transB, lda, ldb, ldc, sA, sB, sC, alpha, beta, st);
+      else launch_simt_tiled<float, 4, 4, 16>(A, B, C, bias, M, N, K, batch, transA, transB, lda, ldb, ldc, sA, sB, sC, alpha, beta, st);
     } else {
-      if (big) launch_simt_tiled<double, 8, 4, 8>(A, B, C, M, N, K, batch, transA, transB, lda, ldb, ldc, sA, sB, sC, alpha, beta, st);
-      else launch_simt_tiled<double, 4, 4, 8>(A, B, C, M, N, K, batch, transA, transB, lda, ldb, ldc, sA, sB, sC, alpha, beta, st);
+      if (big) launch_simt_tiled<double, 8, 4, 8>(A, B, C, bias, M, N, K, batch, transA, transB, lda, ldb, ldc, sA, sB, sC, alpha, beta, st);
+      else launch_simt_tiled<double, 4, 4, 8>(A, B, C, bias, M, N, K, batch, transA, transB, lda, ldb, ldc, sA, sB, sC, alpha, beta, st);
     }
     GB_CUDA_OK(cudaGetLastError());
     return gbh::E_OK;
   }
   if (dtype == DT_F32) {
     gemm_simt_kernel<float><<<grid, 256, 0, (cudaStream_t)stream>>>(
-        (const float*)A, (const float*)B, (float*)C, M, N, K, transA, transB, lda, ldb, ldc, sA, sB,
+        (const float*)A, (const float*)B, (float*)C, (const float*)bias, M, N, K, transA, transB, lda, ldb, ldc, sA, sB,
         sC, (float)alpha, beta);
   } else if (dtype == DT_F64) {
     gemm_simt_kernel<double><<<grid, 256, 0, (cudaStream_t)stream>>>(
-        (const double*)A, (const double*)B, (double*)C, M, N, K, transA, transB, lda, ldb, ldc, sA,
+        (const double*)A, (const double*)B, (double*)C, (const double*)bias, M, N, K, transA, transB, lda, ldb, ldc, sA,
         sB, sC, alpha, beta);
   } else {
     gbh::set_error("gb_gemm_simt: dtype must be fp32 or fp64");

@@ -28,9 +28,6 @@ int gemm_bf16_planes(const void* A, const void* B, float* C, const float* bias, 
                      int transB, long long lda, long long ldb, long long ldc, long long plane_a, long long plane_b, int bcastA,
                      int bcastB, long long sC, int planes, uint32_t order_a, uint32_t order_b, float alpha, int beta,
                      void* workspace, long long workspace_bytes, cudaStream_t stream);
-extern "C" int gb_gemm_simt(const void* A, const void* B, void* C, int M, int N, int K, int batch, int transA,
-                            int transB, long long lda, long long ldb, long long ldc, long long sA, long long sB,
-                            long long sC, int dtype, double alpha, int beta, void* stream);
 extern "C" int gb_binary(int op, int dtype, const void* a, const void* b, void* c, long long n, int rank,
                          const long long* shape, const long long* sa, const long long* sb, void* stream);
 extern "C" int gb_flash_fwd(int dtype, const void* q, const void* k, const void* v, void* o, float* lse, int B, int H,
@@ -236,7 +233,7 @@ gemm_f64_mma_kernel(const double* __restrict__ A, const double* __restrict__ B, 
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-int g_f64_splits = 0;      // 0: by the rule below
+thread_local int g_f64_splits = 0;      // 0: by the rule below
 
 // CTAs per tile: K is cut while the CTAs stay within three per SM and a part keeps about a k-tile.  Measured, us for 1 | 2 | 4 |
 // 8 parts: 64 x 64 x 2048 122 | 67 | 36 | 20; 362^3 25 | 19 | 14 | 12; 512^3 33 | 23 | 17 | 17; 100^3 9 | 11 | 7.5 | 5.8; and where

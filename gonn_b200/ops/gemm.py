@@ -179,9 +179,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
                 and out.data_ptr() % 16 == 0):
             need = int(_l.lib().gb_gemm_f32x3_workspace(M, N, K, batch))
             need = need if need <= (4 << 30) else 0
-        # the plane path adds an fp32 bias in its epilogue
-        bias_in = (bias is None or need > 0 and bias.dtype == torch.float32 and bias.device == a.device and bias.numel() == N
-                   and bias.is_contiguous())
+        f64_mma = a.dtype == torch.float64 and M >= 64 and N >= 64 and K >= 16
+        # the plane and SIMT kernels add a bias of the operands' type in their epilogue (as separate tensor
+        # operations an addition and a copy: six of the 38 launches of a small classifier's training step)
+        bias_in = bias is None or (not f64_mma and bias.dtype == a.dtype == out.dtype and bias.device == a.device
+                                   and bias.numel() == N and bias.dim() == 1 and bias.is_contiguous())
         if not bias_in or ACT[act] or (aux is not None and AUX[aux_mode]):
             # exact-precision path: epilogue evaluated with tensor ops
             tmp = gemm(a, b, trans_a=trans_a, trans_b=trans_b, alpha=alpha)
@@ -191,7 +193,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         sA = a2.stride(0) if a2.dim() == 3 and a2.shape[0] > 1 else 0
         sB = b2.stride(0) if b2.dim() == 3 and b2.shape[0] > 1 else 0
         sC = out.stride(0) if batched else 0
-        if a.dtype == torch.float64 and M >= 64 and N >= 64 and K >= 16:
+        if f64_mma:
             _l.call("gb_gemm_f64", _l.ptr(a2), _l.ptr(b2), _l.ptr(out), _l.I(M), _l.I(N), _l.I(K), _l.I(batch),
                     _l.I(int(trans_a)), _l.I(int(trans_b)), _l.L(lda), _l.L(ldb), _l.L(out.stride(-2)), _l.L(sA),
                     _l.L(sB), _l.L(sC), _l.D(alpha), _l.I(int(beta)), _l.stream_ptr())
@@ -205,7 +207,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
                     _l.ptr(ws3), _l.L(ws3.numel()), _l.ptr(ws), _l.L(_WS_BYTES if ws is not None else 0),
                     _l.stream_ptr())
             return out
-        _l.call("gb_gemm_simt", _l.ptr(a2), _l.ptr(b2), _l.ptr(out), _l.I(M), _l.I(N), _l.I(K),
+        _l.call("gb_gemm_simt", _l.ptr(a2), _l.ptr(b2), _l.ptr(out), _l.ptr(bias), _l.I(M), _l.I(N), _l.I(K),
                 _l.I(batch), _l.I(int(trans_a)), _l.I(int(trans_b)), _l.L(lda), _l.L(ldb),
                 _l.L(out.stride(-2)), _l.L(sA), _l.L(sB), _l.L(sC), _l.I(_l.dtype_code(a.dtype)),
                 _l.D(alpha), _l.I(int(beta)), _l.stream_ptr())

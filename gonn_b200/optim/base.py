@@ -105,13 +105,16 @@ class Optimizer:
     Step = step
 
     def zero_grad(self, set_to_none: bool = False):
+        grads = []
         for g in self.groups:
             for p in g.params:
                 if p.grad is not None:
                     if set_to_none:
                         p.grad = None
                     else:
-                        p.grad.zero_()
+                        grads.append(p.grad)
+        if grads:
+            torch._foreach_zero_(grads)        # one launch, not one per parameter
 
     ZeroGrad = zero_grad
 

@@ -38,3 +38,14 @@ def test_batches_share_an_operand_and_infinities_stay_in_their_row():
     fin[1, 5] = False
     assert not got[~fin].isfinite().any()      # (the planes of b have both signs)
     assert float((got[fin].double() - want[fin]).norm() / want[fin].norm()) < 20 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 3), (64, 10, 128), (65, 67, 40), (30, 130, 17), (1500, 1200, 33)])
+def test_bias_of_the_simt_kernel(dtype, M, N, K):
+    a, b, bias = torch.randn(M, K, dtype=dtype), torch.randn(N, K, dtype=dtype), torch.randn(N, dtype=dtype)
+    out = torch.randn(M, N, dtype=dtype)
+    got = gemm(a.cuda(), b.cuda(), trans_b=True, bias=bias.cuda(), out=out.cuda(), beta=True)
+    want = a.double() @ b.double().t() + bias.double() + out.double()
+    # rounding of K products and sums
+    assert float((got.double().cpu() - want).norm() / want.norm()) < 4 * (K + 2) ** 0.5 * torch.finfo(dtype).eps
