@@ -19,6 +19,10 @@ struct GArgs {
   const unsigned char* kpm;     // [B, Tk], 1 = padded key, or null
   double p_drop;
   unsigned long long seed;
+  // fp64, head size <= 64, optional: dS^T (B * H, Tk, Tq) with both lengths rounded up to 64, written by the dK / dV
+  // role; the dQ role is then its product with K
+  double* dS;
+  long long ds_rows, ds_ld;
 };
 
 __device__ __forceinline__ uint4 philox(uint4 ctr, uint2 key) {

@@ -1,7 +1,7 @@
 // Double-precision attention on the fp64 tensor instructions (mma.sync m16n8k8 f64), head size <= 64: the
 // three roles of attn_general.cu (forward, dQ, dK/dV) with the same masks, padding and dropout.
 //
-// What bounds it: 7 products of T x T x D forward + backward-with-recomputation on a pipe of 64 fused
+// What bounds it: 7 products of T x T x D forward and backward (9 where the backward recomputes dS for dQ) on a pipe of 64 fused
 // multiply-adds per SM and clock (and one exponential per score and pass, 15 of them each).  The SIMT kernel
 // spent its time in shared-memory reads (a 16-byte read feeds eight multiply-adds); here a fragment read of
 // 16 bytes a lane feeds 32.
@@ -272,6 +272,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_f64_kernel(const GArgs a) {
           const double dpd = keep ? dp[j][e] * keep_scale : 0.0;
           s[j][e] = p * (dpd - delta) * a.scale;
           dp[j][e] = keep ? p * keep_scale : 0.0;
+          if (MODE == MODE_DKV && a.dS != nullptr && valid) a.dS[((long long)bh * a.ds_rows + row) * a.ds_ld + col] = s[j][e];
         }
       }
     // ---- FWD: acc += p V   DQ: acc += ds K   DKV: acc += ds Q, acc2 += p' dO ----
@@ -373,6 +374,91 @@ __global__ void __launch_bounds__(kThreads, 2) attn_f64_kernel(const GArgs a) {
   }
 }
 
+// dQ = dS K from the dS^T that the dK / dV role left in memory: one product instead of three and the exponentials.  A
+// warp owns 16 queries; tiles of 32 keys, [key][query] and [key][column], pitch 4 mod 16: conflict-free fragments.
+// Bound by the fp64 pipe and the read of dS^T (268 MB at 16 heads of 2048, causal: backward 1507 -> 1092 us).
+template <int DT>
+struct DqShape {
+  static constexpr int C = DT * 8, P = C + 4, ROWS = 64, PS = ROWS + 4, TK = 32;
+  static constexpr int STAGE = TK * (P + PS), BYTES = 2 * STAGE * 8;
+};
+template <int DT>
+__global__ void __launch_bounds__(kThreads, 3) attn_f64_dq_ds_kernel(const GArgs a) {
+  using S = DqShape<DT>;
+  constexpr int P = S::P, PS = S::PS, TK = S::TK;
+  extern __shared__ __align__(16) double fsm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const bool pure_causal = a.causal && a.mask == nullptr && a.kpm == nullptr;
+  const long long lin = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
+  const long long heads = (long long)gridDim.y * gridDim.z;
+  const int rank = (int)(lin / heads), bh = (int)(lin - rank * heads), b = bh / a.H, h = bh - b * a.H;
+  const int row0 = (pure_causal ? (int)gridDim.x - 1 - rank : rank) * S::ROWS;      // longest first
+  const int t_end = pure_causal ? min(a.Tk, row0 + S::ROWS) : a.Tk;
+  const double* ds = a.dS + (long long)bh * a.ds_rows * a.ds_ld + row0;
+  auto issue = [&](int st, int t0) {
+    if (t0 < t_end) {
+      double* ts = fsm + st * S::STAGE;
+      for (int i = threadIdx.x; i < TK * (S::ROWS / 2); i += kThreads) {      // rows of dS^T are 64-padded and aligned
+        const int r = i / (S::ROWS / 2), c = (i - r * (S::ROWS / 2)) * 2;
+        const bool ok = t0 + r < a.Tk;
+        cp_async16(ts + r * PS + c, ok ? ds + (long long)(t0 + r) * a.ds_ld + c : ds, ok);
+      }
+      issue_rows<S::C, P>(ts + TK * PS, a.K, a.k_s, b, h, t0, TK, a.Tk, a.D);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  double acc[DT][4];
+#pragma unroll
+  for (int n = 0; n < DT; n++)
+#pragma unroll
+    for (int e = 0; e < 4; e++) acc[n][e] = 0.0;
+  issue(0, 0);
+  const int q = row0 + warp * 16 + g;
+  for (int t0 = 0, st = 0; t0 < t_end; t0 += TK, st ^= 1) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    issue(st ^ 1, t0 + TK);
+    const double* ts = fsm + st * S::STAGE + t * PS + warp * 16 + g;
+    const double* tk = fsm + st * S::STAGE + TK * PS + t * P + g;
+    // above the diagonal of pure causal attention nothing was written (queries past Tq: never written either, their rows of
+    // dQ are not stored)
+    const bool diagonal = pure_causal && t0 + TK - 1 > row0 + warp * 16;
+#pragma unroll
+    for (int k = 0; k < TK; k += 8) {
+      double a0 = ts[k * PS], a1 = ts[k * PS + 8], a2 = ts[(k + 4) * PS], a3 = ts[(k + 4) * PS + 8];
+      if (diagonal) {
+        const int key = t0 + k + t;
+        a0 = key > q ? 0.0 : a0;
+        a1 = key > q + 8 ? 0.0 : a1;
+        a2 = key + 4 > q ? 0.0 : a2;
+        a3 = key + 4 > q + 8 ? 0.0 : a3;
+      }
+#pragma unroll
+      for (int n = 0; n < DT; n++) dmma(acc[n], a0, a1, a2, a3, tk[k * P + n * 8], tk[(k + 4) * P + n * 8]);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+    if (q + 8 * r >= a.Tq) continue;
+    double* o = (double*)a.dQ + (long long)b * a.dq_s[0] + (long long)(q + 8 * r) * a.dq_s[1] + (long long)h * a.dq_s[2];
+#pragma unroll
+    for (int n = 0; n < DT; n++)
+#pragma unroll
+      for (int e = 0; e < 2; e++)
+        if (n * 8 + 2 * t + e < a.D) o[n * 8 + 2 * t + e] = acc[n][2 * r + e];
+  }
+}
+
+template <int DT>
+int launch_dq_ds(const GArgs& a, cudaStream_t s) {
+  auto k = attn_f64_dq_ds_kernel<DT>;
+  GB_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, DqShape<DT>::BYTES));
+  k<<<dim3((a.Tq + 63) / 64, a.H, a.B), kThreads, DqShape<DT>::BYTES, s>>>(a);
+  GB_CUDA_OK(cudaGetLastError());
+  return gbh::E_OK;
+}
+
 int g_f64_split = 0;      // 0: by the rule below; 1, 2, 4: that many warps per row group
 
 template <int MODE, int DT, int KW, int NT>
@@ -417,6 +503,8 @@ int launch_mode(const GArgs& a, cudaStream_t s) {
 
 int gba::launch_f64(int mode, const GArgs& a, cudaStream_t s) {
   if (mode == MODE_FWD) return launch_mode<MODE_FWD>(a, s);
+  if (mode == MODE_DQ && a.dS != nullptr)
+    return a.D <= 16 ? launch_dq_ds<2>(a, s) : a.D <= 32 ? launch_dq_ds<4>(a, s) : launch_dq_ds<8>(a, s);
   if (mode == MODE_DQ) return launch_mode<MODE_DQ>(a, s);
   return launch_mode<MODE_DKV>(a, s);
 }

@@ -445,11 +445,13 @@ GB_EXPORT int gb_attn_keep_mask(unsigned char* out, int B, int H, int Tq, int Tk
 
 // mode 0: forward (writes O and LSE); 1: dQ; 2: dK and dV (modes 1 and 2 first need delta: mode 3 computes
 // it from O and dO).  ptrs: Q, K, V, dO, O, dQ, dK, dV (unused ones null); strides: 8 triples (b, s, h) in the
+// ds (may be null): fp64 heads of up to 64 columns, B * H * ceil64(Tk) * ceil64(Tq) doubles, 16-byte aligned: mode 2 leaves dS^T
+// there and mode 1, called after it, reads it instead of recomputing it.
 // same order.  lse / delta: (B, H, Tq) in fp32 (fp64 for fp64 tensors).  mask: additive fp32 (Tq, Tk) or null; kpm: bytes (B, Tk), non-zero = padded key, or null.
 GB_EXPORT int gb_attn_general(int mode, int dtype, void* const* ptrs, const long long* strides, void* lse,
                               void* delta, int B, int H, int Tq, int Tk, int D, double scale, int causal,
                               const float* mask, const unsigned char* kpm, double p_drop, long long seed,
-                              void* stream) {
+                              void* ds, long long ds_bytes, void* stream) {
   if (D < 1 || D > 128 || B <= 0 || H <= 0 || Tq <= 0 || Tk <= 0 || B > 65535 || H > 65535) {
     gbh::set_error("gb_attn_general: bad shape (head size 1..128)");
     return gbh::E_BAD_ARG;
@@ -470,6 +472,15 @@ GB_EXPORT int gb_attn_general(int mode, int dtype, void* const* ptrs, const long
   a.B = B; a.H = H; a.Tq = Tq; a.Tk = Tk; a.D = D;
   a.scale = scale; a.causal = causal; a.mask = mask; a.kpm = kpm; a.p_drop = p_drop;
   a.seed = (unsigned long long)seed;
+  if (ds != nullptr && dtype == DT_F64 && D <= kF64MaxHead) {
+    a.dS = (double*)ds;
+    a.ds_rows = (Tk + 63LL) / 64 * 64;
+    a.ds_ld = (Tq + 63LL) / 64 * 64;
+    if (ds_bytes < 8 * a.ds_rows * a.ds_ld * B * H || ((uintptr_t)ds & 15)) {
+      gbh::set_error("gb_attn_general: the dS workspace is too small or not aligned");
+      return gbh::E_BAD_ARG;
+    }
+  }
   if (mode == 3) {
     const long long warps = (long long)B * H * Tq;
     const int grid = (int)((warps * 32 + 255) / 256 < 148 * 16 ? (warps * 32 + 255) / 256 : 148 * 16);

@@ -64,7 +64,7 @@ def masked_attention_ref(q, k, v, causal=False, scale=None, attn_mask=None, key_
     return torch.matmul(p, vf).permute(0, 2, 1, 3).to(q.dtype)
 
 
-def _general_call(mode, tensors, lse, delta, B, H, Tq, Tk, D, scale, causal, mask, kpm, p_drop, seed):
+def _general_call(mode, tensors, lse, delta, B, H, Tq, Tk, D, scale, causal, mask, kpm, p_drop, seed, ds=None):
     import ctypes
     dt = None
     ptrs, strides = [], []
@@ -80,7 +80,22 @@ def _general_call(mode, tensors, lse, delta, B, H, Tq, Tk, D, scale, causal, mas
     sarr = (_l.L * 24)(*strides)
     _l.call("gb_attn_general", _l.I(mode), _l.I(_l.dtype_code(dt)), parr, sarr, _l.ptr(lse), _l.ptr(delta), _l.I(B),
             _l.I(H), _l.I(Tq), _l.I(Tk), _l.I(D), _l.D(scale), _l.I(int(causal)), _l.ptr(mask), _l.ptr(kpm),
-            _l.D(p_drop), _l.L(seed), _l.stream_ptr())
+            _l.D(p_drop), _l.L(seed), _l.ptr(ds), _l.L(0 if ds is None else ds.numel()), _l.stream_ptr())
+
+
+def _general_backward(ts, lse, delta, *common):
+    """delta, dQ and dK / dV of the general kernels.  fp64 heads of up to 64 columns hand dS from the dK / dV kernel to the
+    dQ kernel where the workspace allows it (see ``_ds_workspace``) and the problem is large enough for the coarser
+    blocks of that product.  Measured backward, us, with it | recomputing: 16 x 2048 x 64 causal 1092 | 1507, 16 x 2048 x 16 967 | 1369,
+    8 x 512 x 64 119 | 140, 2 x 1024 x 64 causal 178 | 201, 4 x 512 x 16 causal 79 | 71, 2 x 128 x 64 63 | 62."""
+    B, H, Tq, Tk, D = common[:5]
+    q = ts[0]
+    _general_call(3, ts, lse, delta, *common)
+    ds = None
+    if q.dtype == torch.float64 and D <= 64 and B * H * Tq * Tk >= DS_MIN_SCORES:
+        ds = _ds_workspace(q.device, 8 * B * H * ((Tk + 63) // 64 * 64) * ((Tq + 63) // 64 * 64))
+    for mode in ((1, 2) if ds is None else (2, 1)):
+        _general_call(mode, ts, lse, delta, *common, ds)
 
 
 class _GeneralAttn(torch.autograd.Function):
@@ -111,9 +126,7 @@ class _GeneralAttn(torch.autograd.Function):
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         ts = [q, k, v, dout, out, dq, dk, dv]
         common = (B, H, Tq, Tk, D, scale, causal, mask, kpm, p_drop, seed)
-        _general_call(3, ts, lse, delta, *common)
-        _general_call(1, ts, lse, delta, *common)
-        _general_call(2, ts, lse, delta, *common)
+        _general_backward(ts, lse, delta, *common)
         return dq, dk, dv, None, None, None, None, None, None
 
 
@@ -138,8 +151,7 @@ def general_bwd(q, k, v, out, dout, lse, causal: bool, scale: float):
     delta = torch.empty((B, H, Tq), dtype=st, device=q.device)
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
     ts = [q, k, v, dout, out, dq, dk, dv]
-    for mode in (3, 1, 2):
-        _general_call(mode, ts, lse, delta, B, H, Tq, Tk, D, scale, causal, None, None, 0.0, 0)
+    _general_backward(ts, lse, delta, B, H, Tq, Tk, D, scale, causal, None, None, 0.0, 0)
     return dq, dk, dv
 
 
@@ -219,6 +231,7 @@ def flash_fwd(q, k, v, causal: bool, scale: float, out=None):
 # that recomputes the scores.  Problems whose dS^T is larger than the limit take the two-pass path.
 DS_SPILL_LIMIT_BYTES = 1 << 32          # the kernel's 32-bit offsets allow no more
 _ds_ws = {}
+DS_MIN_SCORES = 3 << 19                 # fp64: smaller problems recompute the scores
 
 
 def set_ds_spill_limit(nbytes: int) -> None:

@@ -20,6 +20,13 @@ def split(request):
     L.call("gb_attn_f64_tune", L.I(0))
 
 
+@pytest.fixture(params=[True, False])
+def spill(request, monkeypatch):
+    """dQ from the dS that the dK / dV kernel left in memory, or recomputed."""
+    monkeypatch.setattr(A, "DS_MIN_SCORES", 0 if request.param else 1 << 62)
+    return request.param
+
+
 def _check(B, H, Tq, Tk, D, causal, masks, p_drop, strided=False):
     torch.manual_seed(Tq * 7 + Tk * 3 + D)
     mk = lambda n: torch.randn(B, n, H, D, dtype=torch.float64)
@@ -56,18 +63,18 @@ def _check(B, H, Tq, Tk, D, causal, masks, p_drop, strided=False):
 
 @pytest.mark.parametrize("B,H,Tq,Tk,D", SHAPES)
 @pytest.mark.parametrize("causal", [False, True])
-def test_plain(split, B, H, Tq, Tk, D, causal):
+def test_plain(split, spill, B, H, Tq, Tk, D, causal):
     _check(B, H, Tq, Tk, D, causal, False, 0.0)
 
 
 @pytest.mark.parametrize("p_drop", [0.0, 0.3])
 @pytest.mark.parametrize("causal", [False, True])
-def test_masks_and_dropout(split, causal, p_drop):
+def test_masks_and_dropout(split, spill, causal, p_drop):
     _check(2, 2, 70, 50, 24, causal and False, True, p_drop)
     _check(2, 2, 45, 45, 64, causal, False, p_drop)
 
 
-def test_unaligned_strides(split):
+def test_unaligned_strides(split, spill):
     _check(1, 2, 40, 40, 15, True, False, 0.0, strided=True)
 
 
