@@ -7,15 +7,19 @@
 // that fills 16 SMs.  Here
 //  * the recurrent weight stays in shared memory for the whole sequence: a CTA owns UT hidden units
 //    (their four gate rows forward, their column of W_hh backward) for a group of sequences;
-//  * sequences are independent, so only the CTAs of one group wait for one another: H / UT flags
-//    per group in global memory, one per CTA, each stored with release semantics after the CTA's part
-//    of h_t (or of dgates_t) is written, all polled by one warp;
+//  * sequences are independent, so only the CTAs of one group wait for one another.  Forward: h_t travels as 64-bit
+//    words {value, step + 1} in a buffer of two steps by turns; a reader loads the words it needs and repeats those whose
+//    step is not there yet, so that no flag, fence or second round trip stands between a product and the next (a flag
+//    per CTA with release semantics: 6.3 us a step, this 4.2).  A word of step t is overwritten by step t + 2, whose writer
+//    has read step t + 1 from every CTA of its group, and each of those had read step t before.  Backward (four
+//    times the data): H / UT flags per group, one per CTA, stored with release semantics after the CTA's part of
+//    dgates_t is written, all polled by one warp;
 //  * within a CTA the eight warps split the contraction, a lane accumulates 4 x 4 outputs with packed
 //    fp32 multiply-adds, and the partial sums meet in shared memory in a fixed order (deterministic);
 //  * the cell state never leaves the thread that owns it except to be saved for the backward.
 // The input projections of all steps, the weight gradients and the input gradient are single
-// GEMMs outside (ops/rnn.py).  Measured at B = 32, T = 64, H = 512: 379 us forward (5.9 us a step) and
-// 474 us backward (7.4 us a step); at H = 64 a step is 2.6 us, which is the exchange alone.
+// GEMMs outside (ops/rnn.py).  Measured at B = 32, T = 64, H = 512: 267 us forward (4.2 us a step) and
+// 475 us backward (7.4 us a step); at H = 64 a step is 2.6 us, which is the exchange alone.
 //
 // Waiting CTAs need one another to be resident: cooperative launches only.  Every wait is bounded.
 #include "common.cuh"
@@ -54,6 +58,7 @@ struct SeqArgs {
   float* out;                 // (B, T, H): h_t
   float* cseq;                // (B, T, H): c_t
   float* act;                 // (B, T, 4H): activated gates i, f, g, o
+  unsigned long long* xch;    // [2][B][H] words of the exchange, zeroed before the launch
   // backward (reads cseq and act)
   const float* dout;          // (B, T, H) or null
   const float* dcn;           // (B, H) or null: gradient of the last cell state
@@ -155,6 +160,57 @@ __device__ __forceinline__ void load_tile(float* __restrict__ tile, const float*
   cp_async_wait_all();
 }
 
+// h of the step whose words carry `step` (its index + 1), rows b0 .. b0 + kMB - 1, into the tile; rows past B are zero.  False when
+// the budget of the wait ran out (for any thread of the CTA: ends with a barrier).
+__device__ __forceinline__ bool receive_tile(float* __restrict__ tile, const unsigned long long* __restrict__ xch, unsigned step, int H,
+                                             int b0, int B, int* abort_flag, int* status) {
+  constexpr int U = 8;
+  const int h2 = H / 2, pitch = H + 4, total = kMB * h2;
+  for (int i0 = threadIdx.x; i0 < total; i0 += kThreads * U) {
+    unsigned long long w[U][2];
+    unsigned todo = 0;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int i = i0 + u * kThreads, r = i / h2;
+      if (i < total && b0 + r < B) todo |= 1u << u;
+    }
+    const unsigned mine = todo;
+    uint64_t t0 = 0;
+    for (uint32_t spins = 0; todo != 0; spins++) {
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (todo >> u & 1u) {
+          const int i = i0 + u * kThreads, r = i / h2;
+          const unsigned long long* src = xch + (long long)(b0 + r) * H + 2 * (i - r * h2);
+          asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(w[u][0]), "=l"(w[u][1]) : "l"(src) : "memory");
+        }
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if ((unsigned)(w[u][0] >> 32) == step && (unsigned)(w[u][1] >> 32) == step) todo &= ~(1u << u);
+      if (todo != 0 && (spins & 0xFF) == 0xFF) {
+        if (t0 == 0) t0 = globaltimer_ns();
+        if (*(volatile int*)abort_flag) break;
+        if (globaltimer_ns() - t0 > kWaitBudgetNs) {
+          *(volatile int*)abort_flag = 1;
+          set_status(status, ST_RNN_TIMEOUT, (int)step);
+          break;
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int i = i0 + u * kThreads, r = i / h2;
+      if (i < total) {
+        const float2 v = mine >> u & 1u ? make_float2(__uint_as_float((unsigned)w[u][0]), __uint_as_float((unsigned)w[u][1]))
+                                        : make_float2(0.f, 0.f);
+        *reinterpret_cast<float2*>(tile + r * pitch + 2 * (i - r * h2)) = v;
+      }
+    }
+  }
+  __syncthreads();
+  return *(volatile int*)abort_flag == 0;
+}
+
 // grid: (ug, groups).  UT units per CTA: N = 4 UT weight rows, row n = gate * UT + unit.
 template <int UT>
 __global__ void __launch_bounds__(kThreads, 1) lstm_seq_fwd_kernel(const SeqArgs p) {
@@ -167,7 +223,6 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_fwd_kernel(const SeqArgs
   float* part = hs + kMB * pitch;                  // [kWarps][kMB * N]
   const int u0 = blockIdx.x * UT;
   const int bg0 = blockIdx.y * p.sub * kMB;
-  unsigned int* flags = p.flags + (long long)blockIdx.y * p.ug;
   if (threadIdx.x == 0) abort_flag = 0;
   for (int i = threadIdx.x; i < N * (H / 4); i += kThreads) {
     const int n = i / (H / 4), c = (i - n * (H / 4)) * 4;
@@ -186,7 +241,6 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_fwd_kernel(const SeqArgs
     for (int g = 0; g < 4; g++) bias[g] = p.bias[g * H + u];
   }
   for (int t = 0; t < T; t++) {
-    if (t > 0 && !wait_group(flags, p.ug, (unsigned)t, &abort_flag, p.status)) return;
     for (int s = 0; s < p.sub; s++) {
       const int b0 = bg0 + s * kMB, b = b0 + cell_m;
       const bool mine = cell && b < p.B;
@@ -198,11 +252,12 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_fwd_kernel(const SeqArgs
         cp = t > 0 ? p.cseq[(row - 1) * H + u] : (p.c0 != nullptr ? p.c0[(long long)b * H + u] : 0.f);
       }
       if (t > 0 || p.h0 != nullptr) {
-        if (t > 0)
-          load_tile(hs, p.out + (long long)(t - 1) * H, (long long)T * H, H, b0, p.B);
-        else
+        if (t > 0) {
+          if (!receive_tile(hs, p.xch + (long long)((t - 1) & 1) * p.B * H, (unsigned)t, H, b0, p.B, &abort_flag, p.status)) return;
+        } else {
           load_tile(hs, p.h0, H, H, b0, p.B);
-        __syncthreads();
+          __syncthreads();
+        }
         product<N>(hs, ws, H, part);
         __syncthreads();
         if (mine) {
@@ -218,14 +273,17 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_fwd_kernel(const SeqArgs
       if (mine) {
         const float ig = sigm(pre[0]), fg = sigm(pre[1]), gg = tanhf(pre[2]), og = sigm(pre[3]);
         const float cn = fg * cp + ig * gg;
+        const float h = og * tanhf(cn);
+        if (t + 1 < T)        // first: the others wait for it
+          asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p.xch + ((long long)(t & 1) * p.B + b) * H + u),
+                       "l"((unsigned long long)__float_as_uint(h) | (unsigned long long)(t + 1) << 32)
+                       : "memory");
+        p.out[row * H + u] = h;
         p.cseq[row * H + u] = cn;
-        p.out[row * H + u] = og * tanhf(cn);
         float* a = p.act + row * 4 * H + u;
         a[0] = ig; a[H] = fg; a[2 * H] = gg; a[3 * H] = og;
       }
     }
-    __syncthreads();
-    publish(flags + blockIdx.x, (unsigned)(t + 1));
   }
 }
 
@@ -341,7 +399,8 @@ bool plan(int B, int H, bool bwd, int* ut, int* ug, int* groups, int* sub) {
 template <typename K>
 int launch(K kern, const SeqArgs& a, int groups, long long smem, cudaStream_t s) {
   GB_CUDA_OK(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  GB_CUDA_OK(cudaMemsetAsync(a.flags, 0, sizeof(unsigned int) * a.ug * groups, s));
+  if (a.xch != nullptr) GB_CUDA_OK(cudaMemsetAsync(a.xch, 0, 16ll * a.B * a.H, s));
+  else GB_CUDA_OK(cudaMemsetAsync(a.flags, 0, sizeof(unsigned int) * a.ug * groups, s));
   void* args[] = {(void*)&a};
   GB_CUDA_OK(cudaLaunchCooperativeKernel((const void*)kern, dim3(a.ug, groups), dim3(kThreads), args, (size_t)smem, s));
   return gbh::E_OK;
@@ -356,9 +415,9 @@ GB_EXPORT int gb_lstm_seq_fits(int B, int H) {
 }
 
 // fp32.  xg (B,T,4H) = x W_ih^T, bias (4H) or null, w = W_hh (4H,H), h0 / c0 (B,H) or null; writes
-// out (B,T,H), cseq (B,T,H) and the activated gates act (B,T,4H).  flags: scratch of 148 words.
+// out (B,T,H), cseq (B,T,H) and the activated gates act (B,T,4H).  xch: scratch of 2 * B * H 64-bit words, 16-byte aligned.
 GB_EXPORT int gb_lstm_seq_fwd(const void* xg, const void* bias, const void* w, const void* h0, const void* c0, void* out,
-                              void* cseq, void* act, void* flags, int B, int T, int H, void* stream) {
+                              void* cseq, void* act, void* xch, int B, int T, int H, void* stream) {
   if (B <= 0 || T <= 0) return gbh::E_OK;
   SeqArgs a = {};
   int ut, groups;
@@ -368,7 +427,7 @@ GB_EXPORT int gb_lstm_seq_fwd(const void* xg, const void* bias, const void* w, c
   }
   a.B = B; a.T = T; a.H = H;
   a.w = (const float*)w; a.h0 = (const float*)h0; a.c0 = (const float*)c0;
-  a.flags = (unsigned int*)flags; a.status = gbh::status_ptr();
+  a.xch = (unsigned long long*)xch; a.status = gbh::status_ptr();
   a.xg = (const float*)xg; a.bias = (const float*)bias;
   a.out = (float*)out; a.cseq = (float*)cseq; a.act = (float*)act;
   const long long smem = fwd_smem(ut, H);
@@ -378,7 +437,7 @@ GB_EXPORT int gb_lstm_seq_fwd(const void* xg, const void* bias, const void* w, c
   return launch(lstm_seq_fwd_kernel<4>, a, groups, smem, s);
 }
 
-// Backward of the above: dout (B,T,H) or null, dcn (B,H) or null; writes dgates (B,T,4H), the gradient
+// Backward of the above (flags: scratch of 148 words): dout (B,T,H) or null, dcn (B,H) or null; writes dgates (B,T,4H), the gradient
 // of the gate pre-activations, and dc0 (B,H) when not null.
 GB_EXPORT int gb_lstm_seq_bwd(const void* w, const void* c0, const void* cseq, const void* act, const void* dout,
                               const void* dcn, void* dgates, void* dc0, void* flags, int B, int T, int H, void* stream) {

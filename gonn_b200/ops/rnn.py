@@ -8,7 +8,7 @@ torch expression with the same formulas (the oracle of the tests).
 ``lstm_sequence`` runs a whole fp32 LSTM layer: the input projections of all steps as one GEMM, the
 recurrence as one persistent kernel per direction (``csrc/lstm_seq.cu``), and the weight and input
 gradients as one GEMM each over all steps.  Measured forward + backward at B = 32, T = 64,
-I = H = 512: 1.34 ms, 22.6 ms step by step.
+I = H = 512: 0.96 ms, 22.6 ms step by step.
 """
 from __future__ import annotations
 
@@ -110,9 +110,9 @@ class _LSTMSequence(torch.autograd.Function):
         out = torch.empty((B, T, H), dtype=x.dtype, device=dev)
         cseq = torch.empty_like(out)
         act = torch.empty((B, T, 4 * H), dtype=x.dtype, device=dev)
-        flags = torch.empty(148, dtype=torch.int32, device=dev)
+        xch = torch.empty(2 * B * H, dtype=torch.int64, device=dev)
         _l.call("gb_lstm_seq_fwd", _l.ptr(xg), _l.ptr(bias), _l.ptr(whh), _l.ptr(h0), _l.ptr(c0), _l.ptr(out),
-                _l.ptr(cseq), _l.ptr(act), _l.ptr(flags), _l.I(B), _l.I(T), _l.I(H), s)
+                _l.ptr(cseq), _l.ptr(act), _l.ptr(xch), _l.I(B), _l.I(T), _l.I(H), s)
         ctx.save_for_backward(x2, w_ih, w_hh, h0, c0, out, cseq, act)
         ctx.b_ih, ctx.xshape = b_ih, x.shape
         ctx.set_materialize_grads(False)
