@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_bwd_kernel(const SeqArgs
 }
 
 constexpr int kSms = 148;
-constexpr long long kMaxSmem = 227 * 1024;
+constexpr long long kMaxSmem = 227 * 1024 - 16;      // what a block may take, less the kernels' static abort flag
 // Each sub-tile costs a group of CTAs about 1.9 us forward and 2.9 us backward (H = 512); beyond 32 of them the
 // step-by-step GEMMs fill the GPU themselves (forward + backward over 8 steps at H = 512: B = 1024, 32
 // sub-tiles, 3.4 ms against 4.6 ms step by step; B = 2048, 7.4 against 6.1).
@@ -408,6 +408,12 @@ int launch(K kern, const SeqArgs& a, int groups, long long smem, cudaStream_t s)
 
 }  // namespace
 
+// Dynamic shared memory of a CTA of either direction, 0 when the layer does not fit (for tests).
+GB_EXPORT int gb_lstm_seq_smem(int B, int H, int bwd) {
+  int ut, ug, groups, sub;
+  if (B <= 0 || !plan(B, H, bwd != 0, &ut, &ug, &groups, &sub)) return 0;
+  return (int)(bwd ? bwd_smem(ut, H, sub) : fwd_smem(ut, H));
+}
 // 1 when both directions of an LSTM layer of this size run as persistent kernels.
 GB_EXPORT int gb_lstm_seq_fits(int B, int H) {
   int ut, ug, groups, sub;

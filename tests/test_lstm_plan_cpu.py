@@ -1,0 +1,28 @@
+"""Which LSTM layers the persistent kernels accept (host code of csrc/lstm_seq.cu; no GPU needed)."""
+import pytest
+
+from gonn_b200 import lib as L
+
+pytestmark = pytest.mark.skipif(not L.available(), reason="the native library is not built")
+
+BLOCK = 227 * 1024        # shared memory of a block of sm_100a, static and dynamic together
+
+
+def test_accepted_layers_leave_room_for_static_shared_memory():
+    l = L.lib()
+    widest = 0
+    for H in range(4, 1100, 4):
+        for B in range(1, 602, 8):                 # a plan depends on the batch through its tiles of 8 sequences
+            if not l.gb_lstm_seq_fits(L.I(B), L.I(H)):
+                continue
+            for bwd in (0, 1):
+                dyn = int(l.gb_lstm_seq_smem(L.I(B), L.I(H), L.I(bwd)))
+                # both kernels hold a 4-byte static flag beside it
+                assert 0 < dyn <= BLOCK - 4, (B, H, bwd, dyn)
+                widest = max(widest, dyn)
+    assert widest > BLOCK - 2048                   # the boundary is in the range above
+
+
+@pytest.mark.parametrize("B,H", [(20, 896), (50, 892), (85, 888), (115, 884), (150, 880), (180, 876), (210, 872), (245, 868)])
+def test_layers_that_would_need_the_whole_block_are_refused(B, H):
+    assert not L.lib().gb_lstm_seq_fits(L.I(B), L.I(H))

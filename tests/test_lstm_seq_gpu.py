@@ -62,3 +62,20 @@ def test_step_path_where_the_kernel_does_not_apply():
     assert (y - y2).abs().max() < 1e-5
     assert not R._sequence_kernel_takes(nn.LSTM(8, 6, device="cuda").cells[0], x, None)      # 6 % 4 != 0
     assert not R._sequence_kernel_takes(net.cells[0].to(torch.bfloat16), x.bfloat16(), None)
+
+
+@pytest.mark.parametrize("B,H", [(20, 896), (150, 880)])
+def test_layers_at_the_limit_of_shared_memory_train(B, H):
+    """Layers whose backward would need a whole block's shared memory beside its static flag take the steps."""
+    torch.manual_seed(H)
+    net = nn.LSTM(16, H, device="cuda")
+    x = torch.randn(B, 2, 16, device="cuda", requires_grad=True)
+    y = net(x)
+    y.sum().backward()
+    ref = copy.deepcopy(net).double().cpu()
+    xr = x.detach().double().cpu().requires_grad_()
+    yr = ref(xr)
+    yr.sum().backward()
+    L.assert_status_ok()
+    _close(y, yr, 3e-5, "y")
+    _close(x.grad, xr.grad, 3e-5, "dx")
