@@ -381,6 +381,7 @@ __global__ void __launch_bounds__(256) conv_wgrad_finish_kernel(const float* __r
 // Forward 22 us, weight gradient 45 us; bound by the gathers and the 29.5 MB of outputs or gradients.
 constexpr int kDirectK = 32;
 constexpr int kSmallWarps = 8;
+constexpr int kSmallSmem = 96 * 1024;   // limit of the dynamic shared memory: windows of 32 taps alone take 49 KB
 
 __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2], int bf16) {
   if (bf16)
@@ -714,7 +715,7 @@ GB_EXPORT int gb_conv_direct_small(int dtype, const void* x, const void* w, cons
   const int grid = (int)(blocks < 148 * 8 ? blocks : 148 * 8);
 #define GB_DS(V)                                                                                                          \
   {                                                                                                                       \
-    GB_CUDA_OK(cudaFuncSetAttribute(conv_direct_small_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024)); \
+    GB_CUDA_OK(cudaFuncSetAttribute(conv_direct_small_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem)); \
     conv_direct_small_kernel<V><<<grid, kSmallWarps * 32, smem, (cudaStream_t)stream>>>(                                  \
         (const uint16_t*)x, (const uint16_t*)w, idx, (const uint16_t*)bias, (uint16_t*)y, Nimg, C, S, L, T, M, dtype == DT_BF16); \
   }
@@ -763,6 +764,7 @@ GB_EXPORT int gb_conv_wgrad(int dtype, const void* x, const void* dy, const int*
 #define GB_WS(MT, V)                                                                                               \
   {                                                                                                                \
     const size_t red = (size_t)MT * 16 * kDirectK * 4, smem = idx_bytes > red ? idx_bytes : red;                   \
+    GB_CUDA_OK(cudaFuncSetAttribute(conv_wgrad_small_kernel<MT, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem)); \
     conv_wgrad_small_kernel<MT, V><<<dim3(splits, M / (MT * 16)), kSmallWarps * 32, smem, (cudaStream_t)stream>>>( \
         (const uint16_t*)x, (const uint16_t*)dy, idx, part, Nimg, C, S, L, T, M, bf);                              \
   }

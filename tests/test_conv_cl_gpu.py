@@ -45,3 +45,26 @@ def test_padding_and_tiles_ignore_non_finite_neighbours():
     y = net(x)
     assert y[0].isfinite().all() and y[2].isfinite().all() and not y[1, :, :2, :2].isfinite().all()
     assert y[1, :, 2:, 2:].isfinite().all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("Co", [32, 64, 128, 372])
+@pytest.mark.parametrize("case", ["conv1d_32", "conv2d_4x8"])
+def test_windows_of_32_taps(dtype, Co, case):
+    """One input channel and 32 taps: the longest windows of the short-contraction kernels (49 KB of shared memory)."""
+    torch.manual_seed(Co)
+    kw = dict(dtype=dtype, device="cuda")
+    net = nn.Conv1d(1, Co, 32, **kw) if case == "conv1d_32" else nn.Conv2d(1, Co, (4, 8), **kw)
+    x = torch.randn(*((3, 1, 75) if case == "conv1d_32" else (3, 1, 9, 13)), device="cuda").to(dtype).requires_grad_()
+    y = net(x)
+    dy = torch.randn_like(y)
+    y.backward(dy)
+    L.assert_status_ok()
+    xr, wr, br = (t.detach().double().cpu().requires_grad_() for t in (x, net.weight, net.bias))
+    conv = torch.nn.functional.conv1d if case == "conv1d_32" else torch.nn.functional.conv2d
+    want = conv(xr, wr.view(Co, *((1, 32) if case == "conv1d_32" else (1, 4, 8))), br)
+    want.backward(dy.double().cpu())
+    tol = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11      # one rounding of exact products' fp32 sums
+    for n, a, b in (("y", y, want), ("dx", x.grad, xr.grad), ("dw", net.weight.grad, wr.grad), ("db", net.bias.grad, br.grad)):
+        err = float((a.detach().double().cpu() - b.detach()).norm() / b.detach().norm())
+        assert err < tol, f"{n}: {err:.3g}"
