@@ -56,6 +56,7 @@ struct SeqArgs {
   const float* xg;            // (B, T, 4H): x W_ih^T
   const float* bias;          // (4H) or null
   float* out;                 // (B, T, H): h_t
+  float* hprev;               // (B, T, H) or null: h_{t-1}, for the gradient of W_hh
   float* cseq;                // (B, T, H): c_t
   float* act;                 // (B, T, 4H): activated gates i, f, g, o
   unsigned long long* xch;    // [2][B][H] words of the exchange, zeroed before the launch
@@ -279,6 +280,10 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_fwd_kernel(const SeqArgs
                        "l"((unsigned long long)__float_as_uint(h) | (unsigned long long)(t + 1) << 32)
                        : "memory");
         p.out[row * H + u] = h;
+        if (p.hprev != nullptr) {
+          if (t + 1 < T) p.hprev[(row + 1) * H + u] = h;
+          if (t == 0) p.hprev[row * H + u] = p.h0 != nullptr ? p.h0[(long long)b * H + u] : 0.f;
+        }
         p.cseq[row * H + u] = cn;
         float* a = p.act + row * 4 * H + u;
         a[0] = ig; a[H] = fg; a[2 * H] = gg; a[3 * H] = og;
@@ -421,9 +426,10 @@ GB_EXPORT int gb_lstm_seq_fits(int B, int H) {
 }
 
 // fp32.  xg (B,T,4H) = x W_ih^T, bias (4H) or null, w = W_hh (4H,H), h0 / c0 (B,H) or null; writes
-// out (B,T,H), cseq (B,T,H) and the activated gates act (B,T,4H).  xch: scratch of 2 * B * H 64-bit words, 16-byte aligned.
+// out (B,T,H), cseq (B,T,H), the activated gates act (B,T,4H) and, when hprev is not null, h_{t-1} of every step there (a buffer of
+// its own, so that the caller of the layer may change out).  xch: scratch of 2 * B * H 64-bit words, 16-byte aligned.
 GB_EXPORT int gb_lstm_seq_fwd(const void* xg, const void* bias, const void* w, const void* h0, const void* c0, void* out,
-                              void* cseq, void* act, void* xch, int B, int T, int H, void* stream) {
+                              void* hprev, void* cseq, void* act, void* xch, int B, int T, int H, void* stream) {
   if (B <= 0 || T <= 0) return gbh::E_OK;
   SeqArgs a = {};
   int ut, groups;
@@ -435,7 +441,7 @@ GB_EXPORT int gb_lstm_seq_fwd(const void* xg, const void* bias, const void* w, c
   a.w = (const float*)w; a.h0 = (const float*)h0; a.c0 = (const float*)c0;
   a.xch = (unsigned long long*)xch; a.status = gbh::status_ptr();
   a.xg = (const float*)xg; a.bias = (const float*)bias;
-  a.out = (float*)out; a.cseq = (float*)cseq; a.act = (float*)act;
+  a.out = (float*)out; a.hprev = (float*)hprev; a.cseq = (float*)cseq; a.act = (float*)act;
   const long long smem = fwd_smem(ut, H);
   cudaStream_t s = (cudaStream_t)stream;
   if (ut == 16) return launch(lstm_seq_fwd_kernel<16>, a, groups, smem, s);

@@ -110,26 +110,28 @@ class _LSTMSequence(torch.autograd.Function):
         out = torch.empty((B, T, H), dtype=x.dtype, device=dev)
         cseq = torch.empty_like(out)
         act = torch.empty((B, T, 4 * H), dtype=x.dtype, device=dev)
+        # the backward reads h_{t-1} from a buffer of its own: the output belongs to the caller, who may change it in place
+        hprev = torch.empty_like(out) if ctx.needs_input_grad[3] else None
         xch = torch.empty(2 * B * H, dtype=torch.int64, device=dev)
         _l.call("gb_lstm_seq_fwd", _l.ptr(xg), _l.ptr(bias), _l.ptr(whh), _l.ptr(h0), _l.ptr(c0), _l.ptr(out),
-                _l.ptr(cseq), _l.ptr(act), _l.ptr(xch), _l.I(B), _l.I(T), _l.I(H), s)
-        ctx.save_for_backward(x2, w_ih, w_hh, h0, c0, out, cseq, act)
+                _l.ptr(hprev), _l.ptr(cseq), _l.ptr(act), _l.ptr(xch), _l.I(B), _l.I(T), _l.I(H), s)
+        ctx.save_for_backward(x2, w_ih, w_hh, c0, hprev, cseq, act)
         ctx.b_ih, ctx.xshape = b_ih, x.shape
         ctx.set_materialize_grads(False)
-        return out, cseq[:, -1].contiguous()
+        return out, cseq[:, -1].clone()
 
     @staticmethod
     def backward(ctx, dout, dcn):
         from .gemm import gemm
         from .linear import emit_vector_grad, emit_weight_grad
-        x2, w_ih, w_hh, h0, c0, out, cseq, act = ctx.saved_tensors
-        B, T, H = out.shape
-        dev = out.device
+        x2, w_ih, w_hh, c0, hprev, cseq, act = ctx.saved_tensors
+        B, T, H = cseq.shape
+        dev = cseq.device
         dout = dout.contiguous() if dout is not None else None
         dcn = dcn.contiguous() if dcn is not None else None
         whh = _aligned(w_hh.detach())
         dgates = torch.empty_like(act)
-        dc0 = torch.empty((B, H), dtype=out.dtype, device=dev) if ctx.needs_input_grad[5] else None
+        dc0 = torch.empty((B, H), dtype=cseq.dtype, device=dev) if ctx.needs_input_grad[5] else None
         flags = torch.empty(148, dtype=torch.int32, device=dev)
         _l.call("gb_lstm_seq_bwd", _l.ptr(whh), _l.ptr(c0), _l.ptr(cseq), _l.ptr(act), _l.ptr(dout), _l.ptr(dcn),
                 _l.ptr(dgates), _l.ptr(dc0), _l.ptr(flags), _l.I(B), _l.I(T), _l.I(H), _l.stream_ptr())
@@ -145,10 +147,6 @@ class _LSTMSequence(torch.autograd.Function):
         if ctx.b_ih is not None and ctx.needs_input_grad[2]:
             db = emit_vector_grad(ctx.b_ih, dg2)
         if ctx.needs_input_grad[3]:
-            # h_{t-1} of every step: the output moved on by one step
-            hprev = torch.empty_like(out)
-            hprev[:, 1:].copy_(out[:, :-1])
-            hprev[:, 0] = 0 if h0 is None else h0
             dwhh = emit_weight_grad(w_hh, dg2, hprev.view(B * T, H), True, False)
         return dx, dwih, db, dwhh, dh0, dc0
 

@@ -79,3 +79,27 @@ def test_layers_at_the_limit_of_shared_memory_train(B, H):
     L.assert_status_ok()
     _close(y, yr, 3e-5, "y")
     _close(x.grad, xr.grad, 3e-5, "dx")
+
+
+@pytest.mark.parametrize("edit", [lambda t: t.relu_(), lambda t: t.mul_(2.0), lambda t: t[:, 0].zero_()])
+@pytest.mark.parametrize("layers,bidirectional,state", [(1, False, False), (1, False, True), (2, True, False)])
+def test_the_output_may_be_changed_in_place(edit, layers, bidirectional, state):
+    """The backward keeps nothing that the caller of a layer gets: in-place work on the output differentiates."""
+    torch.manual_seed(5)
+    ref = nn.LSTM(12, 20, layers, bidirectional=bidirectional, dtype=torch.float64)
+    net = copy.deepcopy(ref).float().cuda()
+    x = torch.randn(3, 5, 12, dtype=torch.float64)
+    D = (2 if bidirectional else 1) * layers
+    st = tuple(torch.randn(D, 3, 20, dtype=torch.float64) for _ in range(2)) if state else None
+    grads = []
+    for m, conv in ((net, lambda t: t.float().cuda()), (ref, lambda t: t.clone())):
+        xi = conv(x).requires_grad_()
+        y, (h, c) = m.ForwardWithState(xi, None if st is None else tuple(conv(t) for t in st))
+        edit(y)
+        edit(h)
+        edit(c)
+        (y.sum() + (h * h).sum() + c.sum()).backward()
+        grads.append([y, h, c, xi.grad] + [p.grad for p in m.parameters()])
+    L.assert_status_ok()
+    for a, b in zip(*grads):
+        _close(a, b, 3e-5, "in-place")
