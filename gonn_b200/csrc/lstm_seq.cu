@@ -53,14 +53,15 @@ struct SeqArgs {
   unsigned int* flags;        // [groups][ug], zeroed before the launch
   int* status;
   // forward
-  const float* xg;            // (B, T, 4H): x W_ih^T
+  float* xg;                  // (B, T, 4H): x W_ih^T; with a tape replaced by the activated gates i, f, g, o
   const float* bias;          // (4H) or null
-  float* out;                 // (B, T, H): h_t
-  float* hprev;               // (B, T, H) or null: h_{t-1}, for the gradient of W_hh
-  float* cseq;                // (B, T, H): c_t
-  float* act;                 // (B, T, 4H): activated gates i, f, g, o
+  float* out;                 // (B, T, H): h_t; without a tape sequences out_sb elements apart
+  long long out_sb;
+  float* hprev;               // tape: (B, T, H): h_{t-1}, for the gradient of W_hh
+  float* cseq;                // tape: (B, T, H): c_t; without one (B, H): the cell state, replaced in every step
   unsigned long long* xch;    // [2][B][H] words of the exchange, zeroed before the launch
-  // backward (reads cseq and act)
+  // backward (reads cseq, (B, T, H), and act)
+  const float* act;           // (B, T, 4H): activated gates
   const float* dout;          // (B, T, H) or null
   const float* dcn;           // (B, H) or null: gradient of the last cell state
   float* dgates;              // (B, T, 4H)
@@ -212,8 +213,9 @@ __device__ __forceinline__ bool receive_tile(float* __restrict__ tile, const uns
   return *(volatile int*)abort_flag == 0;
 }
 
-// grid: (ug, groups).  UT units per CTA: N = 4 UT weight rows, row n = gate * UT + unit.
-template <int UT>
+// grid: (ug, groups).  UT units per CTA: N = 4 UT weight rows, row n = gate * UT + unit.  TAPE: a backward follows (a template
+// parameter and the stores in this order: with strides and flags at run time a step takes 0.2 us longer).
+template <int UT, bool TAPE>
 __global__ void __launch_bounds__(kThreads, 1) lstm_seq_fwd_kernel(const SeqArgs p) {
   constexpr int N = 4 * UT;
   extern __shared__ __align__(16) float sm[];
@@ -249,8 +251,8 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_fwd_kernel(const SeqArgs
       float pre[4] = {0.f, 0.f, 0.f, 0.f}, cp = 0.f;
       if (mine) {                                  // in flight during the product
 #pragma unroll
-        for (int g = 0; g < 4; g++) pre[g] = __ldg(p.xg + row * 4 * H + g * H + u) + bias[g];
-        cp = t > 0 ? p.cseq[(row - 1) * H + u] : (p.c0 != nullptr ? p.c0[(long long)b * H + u] : 0.f);
+        for (int g = 0; g < 4; g++) pre[g] = p.xg[row * 4 * H + g * H + u] + bias[g];   // (not __ldg: this thread writes there)
+        cp = t > 0 ? p.cseq[(TAPE ? row - 1 : (long long)b) * H + u] : (p.c0 != nullptr ? p.c0[(long long)b * H + u] : 0.f);
       }
       if (t > 0 || p.h0 != nullptr) {
         if (t > 0) {
@@ -279,14 +281,14 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_fwd_kernel(const SeqArgs
           asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p.xch + ((long long)(t & 1) * p.B + b) * H + u),
                        "l"((unsigned long long)__float_as_uint(h) | (unsigned long long)(t + 1) << 32)
                        : "memory");
-        p.out[row * H + u] = h;
-        if (p.hprev != nullptr) {
+        p.out[(TAPE ? row * H : b * p.out_sb + (long long)t * H) + u] = h;
+        p.cseq[(TAPE ? row : (long long)b) * H + u] = cn;
+        if (TAPE) {
+          float* a = p.xg + row * 4 * H + u;
+          a[0] = ig; a[H] = fg; a[2 * H] = gg; a[3 * H] = og;
           if (t + 1 < T) p.hprev[(row + 1) * H + u] = h;
           if (t == 0) p.hprev[row * H + u] = p.h0 != nullptr ? p.h0[(long long)b * H + u] : 0.f;
         }
-        p.cseq[row * H + u] = cn;
-        float* a = p.act + row * 4 * H + u;
-        a[0] = ig; a[H] = fg; a[2 * H] = gg; a[3 * H] = og;
       }
     }
   }
@@ -425,11 +427,12 @@ GB_EXPORT int gb_lstm_seq_fits(int B, int H) {
   return B > 0 && plan(B, H, false, &ut, &ug, &groups, &sub) && plan(B, H, true, &ut, &ug, &groups, &sub) ? 1 : 0;
 }
 
-// fp32.  xg (B,T,4H) = x W_ih^T, bias (4H) or null, w = W_hh (4H,H), h0 / c0 (B,H) or null; writes
-// out (B,T,H), cseq (B,T,H), the activated gates act (B,T,4H) and, when hprev is not null, h_{t-1} of every step there (a buffer of
-// its own, so that the caller of the layer may change out).  xch: scratch of 2 * B * H 64-bit words, 16-byte aligned.
-GB_EXPORT int gb_lstm_seq_fwd(const void* xg, const void* bias, const void* w, const void* h0, const void* c0, void* out,
-                              void* hprev, void* cseq, void* act, void* xch, int B, int T, int H, void* stream) {
+// fp32.  xg (B,T,4H) = x W_ih^T, bias (4H) or null, w = W_hh (4H,H), h0 / c0 (B,H) or null; writes out (B,T,H), whose sequences are
+// out_sb elements apart.  For a backward (hprev not null): h_{t-1} of every step in hprev (B,T,H) (a buffer of its own, so that the
+// caller of the layer may change out), all cell states in c (B,T,H), and the activated gates in the place of xg.  Without one
+// (hprev null): only the last cell state, in c (B,H), which may be c0.  xch: scratch of 2 * B * H 64-bit words, 16-byte aligned.
+GB_EXPORT int gb_lstm_seq_fwd(void* xg, const void* bias, const void* w, const void* h0, const void* c0, void* out, long long out_sb,
+                              void* hprev, void* c, void* xch, int B, int T, int H, void* stream) {
   if (B <= 0 || T <= 0) return gbh::E_OK;
   SeqArgs a = {};
   int ut, groups;
@@ -440,13 +443,22 @@ GB_EXPORT int gb_lstm_seq_fwd(const void* xg, const void* bias, const void* w, c
   a.B = B; a.T = T; a.H = H;
   a.w = (const float*)w; a.h0 = (const float*)h0; a.c0 = (const float*)c0;
   a.xch = (unsigned long long*)xch; a.status = gbh::status_ptr();
-  a.xg = (const float*)xg; a.bias = (const float*)bias;
-  a.out = (float*)out; a.hprev = (float*)hprev; a.cseq = (float*)cseq; a.act = (float*)act;
+  a.xg = (float*)xg; a.bias = (const float*)bias;
+  a.out = (float*)out; a.out_sb = out_sb; a.hprev = (float*)hprev; a.cseq = (float*)c;
+  if (hprev != nullptr && out_sb != (long long)T * H) {
+    gbh::set_error("gb_lstm_seq_fwd: a contiguous output is needed where a backward follows");
+    return gbh::E_BAD_ARG;
+  }
   const long long smem = fwd_smem(ut, H);
   cudaStream_t s = (cudaStream_t)stream;
-  if (ut == 16) return launch(lstm_seq_fwd_kernel<16>, a, groups, smem, s);
-  if (ut == 8) return launch(lstm_seq_fwd_kernel<8>, a, groups, smem, s);
-  return launch(lstm_seq_fwd_kernel<4>, a, groups, smem, s);
+  if (hprev != nullptr) {
+    if (ut == 16) return launch(lstm_seq_fwd_kernel<16, true>, a, groups, smem, s);
+    if (ut == 8) return launch(lstm_seq_fwd_kernel<8, true>, a, groups, smem, s);
+    return launch(lstm_seq_fwd_kernel<4, true>, a, groups, smem, s);
+  }
+  if (ut == 16) return launch(lstm_seq_fwd_kernel<16, false>, a, groups, smem, s);
+  if (ut == 8) return launch(lstm_seq_fwd_kernel<8, false>, a, groups, smem, s);
+  return launch(lstm_seq_fwd_kernel<4, false>, a, groups, smem, s);
 }
 
 // Backward of the above (flags: scratch of 148 words): dout (B,T,H) or null, dcn (B,H) or null; writes dgates (B,T,4H), the gradient
@@ -461,7 +473,7 @@ GB_EXPORT int gb_lstm_seq_bwd(const void* w, const void* c0, const void* cseq, c
     return gbh::E_TOO_LARGE;
   }
   a.B = B; a.T = T; a.H = H;
-  a.w = (const float*)w; a.c0 = (const float*)c0; a.cseq = (float*)cseq; a.act = (float*)act;
+  a.w = (const float*)w; a.c0 = (const float*)c0; a.cseq = (float*)cseq; a.act = (const float*)act;
   a.dout = (const float*)dout; a.dcn = (const float*)dcn; a.dgates = (float*)dgates; a.dc0 = (float*)dc0;
   a.flags = (unsigned int*)flags; a.status = gbh::status_ptr();
   const long long smem = bwd_smem(ut, H, a.sub);

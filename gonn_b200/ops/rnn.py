@@ -96,25 +96,43 @@ def _aligned(t):
     return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
+# Without a tape the projections of the whole input (four times the output) live for a moment only: longer sequences go in
+# pieces of at most this many bytes, each from the state that the one before it left.
+PROJECTION_BYTES = 256 << 20
+
+
+def _lstm_forward(x, w_ih, b_ih, w_hh, h0, c0, tape: bool):
+    """(out (B, T, H), c, hprev, gates): with ``tape`` c and hprev are (B, T, H) and gates (B * T, 4H), what the backward reads;
+    without it c is the last cell state (B, H) and nothing else is kept."""
+    from .gemm import gemm
+    B, T, I = x.shape
+    H = w_hh.shape[1]
+    dev, s = x.device, _l.stream_ptr()
+    whh, h0, c0 = _aligned(w_hh.detach()), _aligned(h0), _aligned(c0)
+    bias = b_ih.detach().contiguous() if b_ih is not None else None
+    out = torch.empty((B, T, H), dtype=x.dtype, device=dev)
+    xch = torch.empty(2 * B * H, dtype=torch.int64, device=dev)
+    steps = T if tape else max(1, min(T, PROJECTION_BYTES // (16 * B * H)))
+    hprev = torch.empty_like(out) if tape else None
+    c = torch.empty_like(out) if tape else torch.empty((B, H), dtype=x.dtype, device=dev)
+    xg = None
+    for t in range(0, T, steps):
+        n = min(steps, T - t)
+        xg = gemm(x[:, t:t + n].reshape(B * n, I), w_ih, trans_b=True,
+                  out=None if xg is None or n < steps else xg)
+        _l.call("gb_lstm_seq_fwd", _l.ptr(xg), _l.ptr(bias), _l.ptr(whh), _l.ptr(h0), _l.ptr(c0), _l.ptr(out[:, t]), _l.L(T * H),
+                _l.ptr(hprev), _l.ptr(c), _l.ptr(xch), _l.I(B), _l.I(n), _l.I(H), s)
+        if t + n < T:
+            h0, c0 = _aligned(out[:, t + n - 1]), c
+    return out, c, hprev, xg
+
+
 class _LSTMSequence(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w_ih, b_ih, w_hh, h0, c0):
-        from .gemm import gemm
-        B, T, I = x.shape
-        H = w_hh.shape[1]
-        dev, s = x.device, _l.stream_ptr()
-        x2 = x.reshape(B * T, I)
-        xg = gemm(x2, w_ih, trans_b=True)
-        whh, h0, c0 = _aligned(w_hh.detach()), _aligned(h0), _aligned(c0)
-        bias = b_ih.detach().contiguous() if b_ih is not None else None
-        out = torch.empty((B, T, H), dtype=x.dtype, device=dev)
-        cseq = torch.empty_like(out)
-        act = torch.empty((B, T, 4 * H), dtype=x.dtype, device=dev)
         # the backward reads h_{t-1} from a buffer of its own: the output belongs to the caller, who may change it in place
-        hprev = torch.empty_like(out) if ctx.needs_input_grad[3] else None
-        xch = torch.empty(2 * B * H, dtype=torch.int64, device=dev)
-        _l.call("gb_lstm_seq_fwd", _l.ptr(xg), _l.ptr(bias), _l.ptr(whh), _l.ptr(h0), _l.ptr(c0), _l.ptr(out),
-                _l.ptr(hprev), _l.ptr(cseq), _l.ptr(act), _l.ptr(xch), _l.I(B), _l.I(T), _l.I(H), s)
+        x2, c0 = x.reshape(-1, x.shape[2]), _aligned(c0)
+        out, cseq, hprev, act = _lstm_forward(x2.view(x.shape), w_ih, b_ih, w_hh, h0, c0, True)
         ctx.save_for_backward(x2, w_ih, w_hh, c0, hprev, cseq, act)
         ctx.b_ih, ctx.xshape = b_ih, x.shape
         ctx.set_materialize_grads(False)
@@ -130,24 +148,23 @@ class _LSTMSequence(torch.autograd.Function):
         dout = dout.contiguous() if dout is not None else None
         dcn = dcn.contiguous() if dcn is not None else None
         whh = _aligned(w_hh.detach())
-        dgates = torch.empty_like(act)
+        dgates = torch.empty_like(act)                     # (B * T, 4H)
         dc0 = torch.empty((B, H), dtype=cseq.dtype, device=dev) if ctx.needs_input_grad[5] else None
         flags = torch.empty(148, dtype=torch.int32, device=dev)
         _l.call("gb_lstm_seq_bwd", _l.ptr(whh), _l.ptr(c0), _l.ptr(cseq), _l.ptr(act), _l.ptr(dout), _l.ptr(dcn),
                 _l.ptr(dgates), _l.ptr(dc0), _l.ptr(flags), _l.I(B), _l.I(T), _l.I(H), _l.stream_ptr())
-        dg2 = dgates.view(B * T, 4 * H)
         dx = dwih = db = dwhh = dh0 = None
         # every read of a weight comes before its gradient is declared ready (ops/linear.py)
         if ctx.needs_input_grad[0]:
-            dx = gemm(dg2, w_ih).view(ctx.xshape)
+            dx = gemm(dgates, w_ih).view(ctx.xshape)
         if ctx.needs_input_grad[4]:
-            dh0 = gemm(dgates[:, 0], w_hh)
+            dh0 = gemm(dgates.view(B, T, 4 * H)[:, 0], w_hh)
         if ctx.needs_input_grad[1]:
-            dwih = emit_weight_grad(w_ih, dg2, x2, True, False)
+            dwih = emit_weight_grad(w_ih, dgates, x2, True, False)
         if ctx.b_ih is not None and ctx.needs_input_grad[2]:
-            db = emit_vector_grad(ctx.b_ih, dg2)
+            db = emit_vector_grad(ctx.b_ih, dgates)
         if ctx.needs_input_grad[3]:
-            dwhh = emit_weight_grad(w_hh, dg2, hprev.view(B * T, H), True, False)
+            dwhh = emit_weight_grad(w_hh, dgates, hprev.view(B * T, H), True, False)
         return dx, dwih, db, dwhh, dh0, dc0
 
 
@@ -158,7 +175,9 @@ def lstm_sequence_fits(B: int, H: int) -> bool:
 
 def lstm_sequence(x, w_ih, b_ih, w_hh, h0=None, c0=None):
     """(h_1 .. h_T (B, T, H), c_T (B, H)) of an fp32 LSTM layer over (B, T, I) on CUDA."""
-    return _LSTMSequence.apply(x, w_ih, b_ih, w_hh, h0, c0)
+    if torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x, w_ih, b_ih, w_hh, h0, c0)):
+        return _LSTMSequence.apply(x, w_ih, b_ih, w_hh, h0, c0)
+    return _lstm_forward(x, w_ih, b_ih, w_hh, h0, c0, False)[:2]
 
 
 def lstm_gates(gates: torch.Tensor, c: torch.Tensor):

@@ -103,3 +103,38 @@ def test_the_output_may_be_changed_in_place(edit, layers, bidirectional, state):
     L.assert_status_ok()
     for a, b in zip(*grads):
         _close(a, b, 3e-5, "in-place")
+
+
+@pytest.mark.parametrize("state", [False, True])
+@pytest.mark.parametrize("T", [1, 6, 7, 8, 50])
+def test_evaluation_in_pieces(monkeypatch, T, state):
+    """Without a tape a sequence may run in pieces (here of 7 steps): the outputs and the last states of a whole one."""
+    B, I, H = 5, 24, 64
+    net = nn.LSTM(I, H, 2, bidirectional=True, device="cuda")
+    x = torch.randn(B, T, I, device="cuda")
+    st = tuple(torch.randn(4, B, H, device="cuda") for _ in range(2)) if state else None
+    want, (h, c) = net.ForwardWithState(x, st)                       # with a tape
+    monkeypatch.setattr(R._rnn_ops, "PROJECTION_BYTES", 7 * 16 * B * H + 1)
+    with torch.no_grad():
+        got, (h2, c2) = net.ForwardWithState(x, st)
+    L.assert_status_ok()
+    for n, a, b in (("y", got, want), ("h", h2, h), ("c", c2, c)):
+        # the same kernel; the projections of fewer rows may be summed in another order
+        assert a.shape == b.shape and not a.requires_grad
+        _close(a, b.double().cpu(), 2e-6, n)
+
+
+def test_evaluation_keeps_neither_gates_nor_cell_states(monkeypatch):
+    B, T, I, H = 64, 512, 16, 128
+    net = nn.LSTM(I, H, device="cuda")
+    x = torch.randn(B, T, I, device="cuda")
+    piece = 8 << 20
+    monkeypatch.setattr(R._rnn_ops, "PROJECTION_BYTES", piece)
+    with torch.no_grad():
+        net(x)
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        y = net(x)
+    # the output and two pieces of the projections (one of them the ragged last); the states are small
+    assert torch.cuda.max_memory_allocated() - before < y.numel() * 4 + 2 * piece + (4 << 20)
