@@ -53,13 +53,28 @@ _FP32_MODE = "bf16x3"
 
 def set_fp32_gemm_mode(mode: str) -> str:
     """``"bf16x3"`` (default): large fp32 products run on the tensor cores as three bf16 planes
-    per operand (error at the rounding level of an fp32 product); ``"simt"``: always the
-    register-tiled fp32 FMA kernel.  Returns the previous mode."""
+    per operand; ``"simt"``: always the register-tiled fp32 FMA kernel.  The planes themselves lose less than the rounding
+    of an fp32 product, but the tensor core truncates its fp32 accumulator once per 16 products.  Relative error
+    (2-norm, normal inputs | inputs of one sign) against 64 bits, planes and FMA: K = 1024 9.9e-7 | 1.7e-6 and 5.7e-7 | 4.3e-7,
+    K = 4096 4.4e-6 | 1.1e-5 and 1.2e-6 | 8.4e-7; with few tiles K is cut into slices of their own accumulators
+    (1024^3 2.4e-7 | 3.2e-7).  Returns the previous mode."""
     global _FP32_MODE
     if mode not in ("bf16x3", "simt"):
         raise ValueError("fp32 GEMM mode must be 'bf16x3' or 'simt'")
     old, _FP32_MODE = _FP32_MODE, mode
     return old
+
+
+def _plane_chain(M: int, N: int, K: int, batch: int) -> int:
+    """How much of K one launch of the plane kernel adds up.  The tensor core truncates its accumulator, so the error
+    grows with that length.  The largest products (vocabulary heads, squares above 13 000), which used to take the fp32
+    FMA kernel, go in pieces that are added in fp32 outside, short enough to stay below the error of an FMA chain of
+    their K.  Relative error against 64 bits on normal inputs | inputs of one sign, and time, of 4096 x 50304 x 4096: one
+    accumulator 4.4e-6 | 1.1e-5, 7.1 ms; FMA 1.2e-6 | 8.4e-7, 40 ms; pieces of 512 4.8e-7 | 7.1e-7, 11 ms; of 256
+    2.5e-7 | 3.2e-7, 17 ms; of 128 1.6e-7 | 1.6e-7, 27 ms.  (FMA at K = 2048: 8.1e-7 | 6.0e-7, at 1024: 5.7e-7 | 4.3e-7.)"""
+    if 24 * batch * (-(-K // 8) * 8) * (-(-max(M, N) // 8) * 8) < 1 << 32:
+        return K
+    return min(K, 512 if K >= 4096 else 256 if K >= 1024 else 128)
 
 
 def _x3_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
@@ -177,7 +192,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
                 and 2.0 * M * N * K * batch >= 2.0 ** 28 and M >= 128 and N >= 128
                 and (K % 8 == 0 or (not trans_a and trans_b)) and out.stride(-2) % 4 == 0
                 and out.data_ptr() % 16 == 0):
-            need = int(_l.lib().gb_gemm_f32x3_workspace(M, N, K, batch))
+            chain = _plane_chain(M, N, K, batch)
+            need = int(_l.lib().gb_gemm_f32x3_workspace(M, N, chain, batch))
             need = need if need <= (4 << 30) else 0
         f64_mma = a.dtype == torch.float64 and M >= 64 and N >= 64 and K >= 16
         # the plane and SIMT kernels add a bias of the operands' type in their epilogue (as separate tensor
@@ -201,11 +217,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         if need:
             ws3 = _x3_workspace(a.device, need)
             ws = _workspace(a.device) if M * N * batch * 4 * 2 <= _WS_BYTES else None
-            _l.call("gb_gemm_f32x3", _l.ptr(a2), _l.ptr(b2), _l.ptr(out), _l.ptr(bias), _l.I(M), _l.I(N), _l.I(K),
-                    _l.I(batch), _l.I(int(trans_a)), _l.I(int(trans_b)), _l.L(lda), _l.L(ldb),
-                    _l.L(out.stride(-2)), _l.L(sA), _l.L(sB), _l.L(sC), _l.F(alpha), _l.I(int(beta)),
-                    _l.ptr(ws3), _l.L(ws3.numel()), _l.ptr(ws), _l.L(_WS_BYTES if ws is not None else 0),
-                    _l.stream_ptr())
+            for k in range(0, K, chain):
+                ak, bk = a2.data_ptr() + 4 * k * (lda if trans_a else 1), b2.data_ptr() + 4 * k * (1 if trans_b else ldb)
+                _l.call("gb_gemm_f32x3", _l.P(ak), _l.P(bk), _l.ptr(out), _l.ptr(bias if k == 0 else None), _l.I(M), _l.I(N),
+                        _l.I(min(chain, K - k)), _l.I(batch), _l.I(int(trans_a)), _l.I(int(trans_b)), _l.L(lda), _l.L(ldb),
+                        _l.L(out.stride(-2)), _l.L(sA), _l.L(sB), _l.L(sC), _l.F(alpha), _l.I(int(beta or k > 0)),
+                        _l.ptr(ws3), _l.L(ws3.numel()), _l.ptr(ws), _l.L(_WS_BYTES if ws is not None else 0),
+                        _l.stream_ptr())
             return out
         _l.call("gb_gemm_simt", _l.ptr(a2), _l.ptr(b2), _l.ptr(out), _l.ptr(bias), _l.I(M), _l.I(N), _l.I(K),
                 _l.I(batch), _l.I(int(trans_a)), _l.I(int(trans_b)), _l.L(lda), _l.L(ldb),

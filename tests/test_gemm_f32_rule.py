@@ -1,0 +1,54 @@
+"""How fp32 products run as bf16 planes (ops/gemm.py): the rule on the CPU, its error on a GPU."""
+import pytest
+import torch
+
+from gonn_b200 import lib as L
+from gonn_b200.ops import gemm as G
+
+
+@pytest.mark.parametrize("M,N,K,batch,chain", [
+    (3000, 4096, 1024, 1, 1024), (4096, 4096, 4096, 1, 4096), (128, 4096, 4096, 1, 4096),
+    (512, 512, 512, 1, 512), (128, 128, 128, 64, 128),
+    # vocabulary heads and the largest squares: no less exact than the FMA kernel
+    (4096, 50304, 4096, 1, 512), (50304, 4096, 4096, 1, 512), (16384, 16384, 16384, 1, 512), (13368, 13368, 13368, 1, 13368),
+    (13384, 13384, 13384, 1, 512), (128, 43688, 4096, 1, 4096), (128, 43696, 4096, 1, 512), (1024, 1024, 1024, 170, 1024),
+    (1024, 1024, 1024, 171, 256), (200, 10 ** 6, 200, 1, 128), (200, 10 ** 7, 100, 1, 100)])
+def test_rule(M, N, K, batch, chain):
+    assert G._plane_chain(M, N, K, batch) == chain
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("draw", [torch.randn, torch.rand])
+@pytest.mark.parametrize("M,N,K,ta,tb", [(128, 43696, 4096, False, True), (43700, 128, 4104, True, False), (136, 60000, 3000, False, False),
+                                         (128, 176000, 1024, False, True), (300000, 130, 600, True, True)])
+def test_the_largest_products_are_no_less_exact_than_fma(draw, M, N, K, ta, tb):
+    assert 0 < G._plane_chain(M, N, K, 1) < K
+    a, b = draw(*((K, M) if ta else (M, K)), device="cuda"), draw(*((N, K) if tb else (K, N)), device="cuda")
+    want = (a.t() if ta else a).double() @ (b.t() if tb else b).double()
+    err = {}
+    for mode in ("bf16x3", "simt"):
+        old = G.set_fp32_gemm_mode(mode)
+        try:
+            err[mode] = float((G.gemm(a, b, trans_a=ta, trans_b=tb).double() - want).norm() / want.norm())
+        finally:
+            G.set_fp32_gemm_mode(old)
+    assert err["bf16x3"] <= err["simt"], err
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ta,tb", [(False, True), (False, False), (True, False), (True, True)])
+@pytest.mark.parametrize("bias,beta,batch", [(True, False, 1), (False, True, 1), (True, True, 1), (False, True, 3)])
+def test_pieces(monkeypatch, ta, tb, bias, beta, batch):
+    """K in pieces with a ragged last one: bias once, the old result once, alpha in every piece."""
+    M, N, K = 333, 516, 1004 if (not ta and tb) else 1000
+    monkeypatch.setattr(G, "_plane_chain", lambda *s: 256)
+    one = (lambda *s: torch.randn(batch, *s)) if batch > 1 else torch.randn
+    a, b, bv = one(*((K, M) if ta else (M, K))), one(*((N, K) if tb else (K, N))), 30 * torch.randn(N)
+    out = 30 * one(M, N)
+    want = -0.5 * ((a.transpose(-1, -2) if ta else a).double() @ (b.transpose(-1, -2) if tb else b).double())
+    want = want + (bv.double() if bias else 0) + (out.double() if beta else 0)
+    got = G.gemm(a.cuda(), b.cuda(), trans_a=ta, trans_b=tb, alpha=-0.5, bias=bv.cuda() if bias else None,
+                 out=out.cuda(), beta=beta)
+    L.assert_status_ok()
+    # every accumulator truncates 6 x 16 sums and every piece is rounded once: below 2^-20 together
+    assert float((got.double().cpu() - want).norm() / want.norm()) < 2.0 ** -20
