@@ -9,8 +9,8 @@
 //   bits in total) and the six significant plane products lo hi, hi lo, mid mid, mid hi, hi mid, hi hi
 //   run as one bf16 tcgen05 launch, in that order into one fp32 accumulator; the planes are the third
 //   dimension of the operands' tensor maps.  The dropped products are below 2^-24 of the result, the
-//   rounding level of an fp32 product itself.  Non-finite inputs keep their value in the hi plane and
-//   contribute zero to the others.  3000 x 4096 x 1024: 115 us (240 as three launches that added to C).
+//   rounding level of an fp32 product itself.  Infinities and NaN give what they give in fp32 (split3_kernel).
+//   3000 x 4096 x 1024: 115 us (240 as three launches that added to C).
 //
 // The in-library benchmark loops at the end mirror the reference's (gonn_cuda.cu:255-294,
 // 532-592, 673-690): operands allocated once, five untimed calls, `iters` calls between two
@@ -278,6 +278,10 @@ int launch_f64(const void* A, const void* B, void* C, int M, int N, int K, int b
 // rounded up to 8, zero filled.  Bound by memory: 4 bytes read and 6 written per element; a thread turns eight
 // neighbouring elements into three 16-byte stores.  (Six planes in the order of the products, two bytes at a time
 // with a 64-bit division per element, took 267 us for the six operands of a 3000 x 1024 x 4096 layer; this takes 65.)
+// An infinity or NaN stands in the lo plane, which meets the other operand's hi plane alone, so that no product with a
+// lo or mid part of the other sign turns it into NaN; the hi plane holds +-1 in its place, with which an infinity of the other
+// operand gets its sign.  (In the hi plane an infinity times an ordinary row gave NaN.)  A finite value that would round
+// to infinity in bf16 is cut to bf16's largest value and keeps the rest in the other planes.
 __global__ void __launch_bounds__(256) split3_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, int rows, int cols,
                                                      long long ld, int cols_p, long long src_batch, int vec) {
   src += (long long)blockIdx.z * src_batch;
@@ -301,10 +305,11 @@ __global__ void __launch_bounds__(256) split3_kernel(const float* __restrict__ s
 #pragma unroll
     for (int j = 0; j < 8; j++) {
       const bool fin = isfinite(x[j]);
-      pl[0][j] = __float2bfloat16_rn(x[j]);
+      const float top = __uint_as_float(0x7f7f0000u);                 // bf16's largest value
+      pl[0][j] = __float2bfloat16_rn(fin ? fminf(fmaxf(x[j], -top), top) : copysignf(1.f, x[j]));
       const float r1 = fin ? x[j] - __bfloat162float(pl[0][j]) : 0.f;
       pl[1][j] = __float2bfloat16_rn(r1);
-      pl[2][j] = __float2bfloat16_rn(r1 - __bfloat162float(pl[1][j]));
+      pl[2][j] = __float2bfloat16_rn(fin ? r1 - __bfloat162float(pl[1][j]) : x[j]);
     }
     __nv_bfloat16* d = dst + (long long)r * cols_p + c;
 #pragma unroll

@@ -49,3 +49,51 @@ def test_bias_of_the_simt_kernel(dtype, M, N, K):
     want = a.double() @ b.double().t() + bias.double() + out.double()
     # rounding of K products and sums
     assert float((got.double().cpu() - want).norm() / want.norm()) < 4 * (K + 2) ** 0.5 * torch.finfo(dtype).eps
+
+
+@pytest.mark.parametrize("ta,tb", [(False, True), (False, False), (True, False), (True, True)])
+def test_infinities_nan_and_the_largest_values_as_in_fp32(ta, tb):
+    """Every entry is finite, an infinity of one sign or NaN exactly where an fp32 product has it."""
+    torch.manual_seed(3)
+    M, N, K = 264, 520, 2048
+    a, b = torch.randn(M, K), torch.randn(K, N)
+    inf, big = float("inf"), torch.finfo(torch.float32).max
+    a[3, 5] = inf                       # meets ordinary values of both signs
+    a[4, 6] = -inf
+    b[5, 7] = 0.0                       # inf * 0
+    a[9, 10], b[10, 11] = inf, -inf     # both sides at one k
+    a[12, 20], a[12, 21] = inf, inf     # two of them: NaN where their partners' signs differ
+    a[15, 1] = float("nan")
+    b[100, 200] = float("nan")
+    b[101, 300] = inf
+    a[30, 40], a[31, 41], a[32, 42] = big, -big, -3.4e38          # masks of the type's lowest value
+    b[40] *= 1e-3
+    b[41] *= 1e-3
+    b[42] *= 1e-3
+    a[50, 60], b[60, 70] = 3.395e38, 1.0      # between bf16's largest value and the rounding to infinity
+    put = lambda t, tr: (t.t().contiguous().cuda().t() if tr else t.cuda())
+    got = gemm(put(a, ta).t() if ta else a.cuda(), put(b, tb).t() if tb else b.cuda(), trans_a=ta, trans_b=tb).cpu()
+    want = a @ b
+    L.assert_status_ok()
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got == inf, want == inf) and torch.equal(got == -inf, want == -inf)
+    fin = want.isfinite()
+    exact = a.double() @ b.double()
+    assert not fin.all() and fin[30].sum() > 0 and fin[32].sum() > 0
+    for rows in (slice(30, 33), slice(50, 51), slice(60, M)):
+        f = fin[rows]
+        err = float((got[rows][f].double() - exact[rows][f]).norm() / exact[rows][f].norm())
+        assert err < (K / 32 + 4) * 2.0 ** -24, err
+
+
+def test_split_values_add_up():
+    """A product with the identity returns the operand: finite values of all sizes, the largest ones among them."""
+    n = 1024
+    x = torch.randn(n, n) * torch.logspace(-30, 38, n)[:, None]
+    x[:, 0], x[:, 1], x[:, 2] = torch.finfo(torch.float32).max, -3.4e38, 3.3961775e38
+    x = x.clamp(-torch.finfo(torch.float32).max, torch.finfo(torch.float32).max)
+    got = gemm(x.cuda(), torch.eye(n).cuda()).cpu()
+    # three roundings to 8 bits leave nothing of a 24-bit value; the accumulator, aligned to the hi part, which may lie in the
+    # binade above, cuts each of the two sums by less than 2^-23 of it
+    assert got.isfinite().all()
+    assert float(((got.double() - x.double()) / x.double()).abs().max()) <= 2.0 ** -22

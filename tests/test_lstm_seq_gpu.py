@@ -138,3 +138,14 @@ def test_evaluation_keeps_neither_gates_nor_cell_states(monkeypatch):
         y = net(x)
     # the output and two pieces of the projections (one of them the ragged last); the states are small
     assert torch.cuda.max_memory_allocated() - before < y.numel() * 4 + 2 * piece + (4 << 20)
+
+
+@pytest.mark.parametrize("value", [float("inf"), -float("inf"), 3.4e38, -3.4e38])
+def test_an_infinite_input_saturates_the_gates(value):
+    """The projections of the whole input are large enough for the plane products: an infinity must arrive as one."""
+    net = nn.LSTM(512, 512, device="cuda")
+    x = torch.randn(32, 64, 512, device="cuda")
+    x[3, 2, 5] = value
+    with torch.no_grad():
+        y = net(x)
+    assert y.isfinite().all()
