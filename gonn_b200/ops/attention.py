@@ -85,7 +85,7 @@ def _general_call(mode, tensors, lse, delta, B, H, Tq, Tk, D, scale, causal, mas
 
 def _general_backward(ts, lse, delta, *common):
     """delta, dQ and dK / dV of the general kernels.  fp64 heads of up to 64 columns hand dS from the dK / dV kernel to the
-    dQ kernel where the workspace allows it (see ``_ds_workspace``) and the problem is large enough for the coarser
+    dQ kernel where memory (at most ``DS_SPILL_LIMIT_BYTES``) allows it and the problem is large enough for the coarser
     blocks of that product.  Measured backward, us, with it | recomputing: 16 x 2048 x 64 causal 1092 | 1507, 16 x 2048 x 16 967 | 1369,
     8 x 512 x 64 119 | 140, 2 x 1024 x 64 causal 178 | 201, 4 x 512 x 16 causal 79 | 71, 2 x 128 x 64 63 | 62."""
     B, H, Tq, Tk, D = common[:5]
@@ -93,7 +93,14 @@ def _general_backward(ts, lse, delta, *common):
     _general_call(3, ts, lse, delta, *common)
     ds = None
     if q.dtype == torch.float64 and D <= 64 and B * H * Tq * Tk >= DS_MIN_SCORES:
-        ds = _ds_workspace(q.device, 8 * B * H * ((Tk + 63) // 64 * 64) * ((Tq + 63) // 64 * 64))
+        need = 8 * B * H * ((Tk + 63) // 64 * 64) * ((Tq + 63) // 64 * 64)
+        if need <= DS_SPILL_LIMIT_BYTES:
+            # of this call alone: these kernels never needed scratch, so none outlives the call, and where the memory
+            # is not there the scores are recomputed
+            try:
+                ds = torch.empty(need, dtype=torch.uint8, device=q.device)
+            except torch.OutOfMemoryError:
+                pass
     for mode in ((1, 2) if ds is None else (2, 1)):
         _general_call(mode, ts, lse, delta, *common, ds)
 

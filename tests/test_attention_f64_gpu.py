@@ -88,3 +88,38 @@ def test_rows_without_finite_scores_and_nan():
     q2[0, 5, 0, 0] = float("nan")
     out = A.general_attention(q2, k, v, False, 1.0)
     assert out[:, 5].isnan().all() and out[:, :5].isfinite().all() and out[:, 6:].isfinite().all()
+
+
+def test_the_handed_over_ds_lives_for_one_call(monkeypatch):
+    """The fp64 backward leaves no workspace behind, and without memory for it gives the same gradients."""
+    monkeypatch.setattr(A, "DS_MIN_SCORES", 0)
+    q, k, v = (torch.randn(2, 300, 2, 32, dtype=torch.float64, device="cuda", requires_grad=True) for _ in range(3))
+    dy = torch.randn(2, 300, 2, 32, dtype=torch.float64, device="cuda")
+    need = 8 * 4 * 320 * 320
+    out = A.flash_attention(q, k, v, causal=True)
+
+    def gradients():
+        return torch.autograd.grad(out, (q, k, v), dy, retain_graph=True)
+
+    del_me = gradients()
+    del del_me
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    with_ds = gradients()
+    assert torch.cuda.max_memory_allocated() - before >= need                     # it was used
+    kept = sum(g.numel() * 8 for g in with_ds)
+    assert torch.cuda.memory_allocated() - before <= kept + 4096                  # and given back
+    empty = torch.empty
+
+    def no_room(*size, **kw):
+        if kw.get("dtype") is torch.uint8:
+            raise torch.OutOfMemoryError("no room")
+        return empty(*size, **kw)
+
+    monkeypatch.setattr(torch, "empty", no_room)
+    without = gradients()
+    monkeypatch.setattr(torch, "empty", empty)
+    L.assert_status_ok()
+    for a, b in zip(with_ds, without):
+        assert float((a - b).norm() / b.norm()) < 5e-14                           # (as in _check)
