@@ -671,14 +671,15 @@ norm_fwd_pipe_kernel(const T* __restrict__ x, const TW* __restrict__ w, const TW
   }
 }
 
-// V weights (16-byte aligned), or a constant where there are none.
-template <typename TW, int V>
+// V weights (16-byte aligned; SHARED: in shared memory), or a constant where there are none.
+template <typename TW, int V, bool SHARED>
 __device__ __forceinline__ void load_params(const TW* p, int vi, float none, float2* f) {
   constexpr int PER = IO<TW>::V;          // elements of one 16-byte load
   using Raw = typename IO<TW>::Raw;
 #pragma unroll
   for (int i = 0; i < V / PER; i++) {
-    if (p != nullptr) Pairs<TW>::unpack(__ldg(reinterpret_cast<const Raw*>(p) + vi * (V / PER) + i), f + i * (PER / 2));
+    const Raw* at = reinterpret_cast<const Raw*>(p) + vi * (V / PER) + i;
+    if (p != nullptr) Pairs<TW>::unpack(SHARED ? *at : __ldg(at), f + i * (PER / 2));
     else
 #pragma unroll
       for (int j = 0; j < PER / 2; j++) f[i * (PER / 2) + j] = f2(none);
@@ -688,8 +689,10 @@ __device__ __forceinline__ void load_params(const TW* p, int vi, float none, flo
 // Forward, rows of at most 256 vectors: one warp per row, the whole row in registers, every load in flight at once and
 // nothing shared.  Bound by memory and launch latency; the ring of the kernel above needs several tiles per CTA to pay
 // for its barriers and leaves only 3 x 148 rows in work (us here | there: 8192 rows of 2048 bf16 9.9 | 19.2, 16 384 of 768
-// 9.1 | 12.7, 77 of 768 2.3 | 3.6, 131 072 of 2048 164 | 249, which is 6.5 TB/s).
-template <typename T, typename TW, int VPT, bool RMS>
+// 9.1 | 12.7, 77 of 768 2.3 | 3.6, 131 072 of 2048 164 | 249, which is 6.5 TB/s).  STAGED: weights that are not 16-byte aligned are
+// copied to shared memory first, by about as many CTAs as run at a time (here | the kernel above: bf16 16 384 x 1024 14.5 |
+// 20.7, 131 072 x 2048 233 | 256, 131 072 x 768 81 | 78, fp32 131 072 x 768 139 | 151).
+template <typename T, typename TW, int VPT, bool RMS, bool STAGED>
 __global__ void __launch_bounds__(128)
 norm_fwd_warp_kernel(const T* __restrict__ x, const TW* __restrict__ w, const TW* __restrict__ b, T* __restrict__ y,
                      float* __restrict__ mean_out, float* __restrict__ rstd_out, long long rows, int D, float eps) {
@@ -698,6 +701,29 @@ norm_fwd_warp_kernel(const T* __restrict__ x, const TW* __restrict__ w, const TW
   using Raw = typename IO<T>::Raw;
   const int lane = threadIdx.x & 31, nvec = D / V;
   const float invD = 1.f / (float)D;
+  extern __shared__ __align__(16) uint8_t warp_sm[];      // STAGED: weights, bias
+  if (STAGED) {
+    TW* sw = reinterpret_cast<TW*>(warp_sm);
+    TW* sb = sw + D;                                      // D is a multiple of 16 bytes of either type
+    for (int i0 = threadIdx.x; i0 < D; i0 += 128 * 8) {   // sixteen loads in flight
+      TW t[2][8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const int i = i0 + 128 * j;
+        if (i < D && w != nullptr) t[0][j] = w[i];
+        if (!RMS && i < D && b != nullptr) t[1][j] = b[i];
+      }
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const int i = i0 + 128 * j;
+        if (i < D && w != nullptr) sw[i] = t[0][j];
+        if (!RMS && i < D && b != nullptr) sb[i] = t[1][j];
+      }
+    }
+    __syncthreads();
+    if (w != nullptr) w = sw;
+    if (b != nullptr) b = sb;
+  }
   for (long long row = (long long)blockIdx.x * 4 + (threadIdx.x >> 5); row < rows; row += (long long)gridDim.x * 4) {
     const T* xr = x + row * D;
     Raw raw[VPT];
@@ -760,8 +786,8 @@ norm_fwd_warp_kernel(const T* __restrict__ x, const TW* __restrict__ w, const TW
       const int vi = lane + 32 * i;
       if (vi < nvec) {
         float2 o[NP2], wv[NP2], bv[NP2];
-        load_params<TW, V>(w, vi, 1.f, wv);
-        load_params<TW, V>(RMS ? nullptr : b, vi, 0.f, bv);
+        load_params<TW, V, STAGED>(w, vi, 1.f, wv);
+        load_params<TW, V, STAGED>(RMS ? nullptr : b, vi, 0.f, bv);
 #pragma unroll
         for (int j = 0; j < NP2; j++) o[j] = __ffma2_rn(__ffma2_rn(f[i][j], rs, sv), wv[j], bv[j]);
         yr[vi] = Pairs<T>::pack(o);
@@ -975,17 +1001,23 @@ int norm_fwd_t(const void* x, const void* w, const void* b, void* y, float* mean
   constexpr int V = IO<T>::V;
   const bool aligned = (D % V == 0) && ((((uintptr_t)x | (uintptr_t)y) & 15) == 0);
   const int nvec = D / V;
-  if (aligned && nvec <= 256 && g_norm_pipe && (((uintptr_t)w | (uintptr_t)b) & 15) == 0) {
-    const long long blocks = (rows + 3) / 4;
-#define GB_FWDW(VPT)                                                                                               \
-  norm_fwd_warp_kernel<T, TW, VPT, RMS><<<(unsigned)(blocks < (1 << 20) ? blocks : (1 << 20)), 128, 0, s>>>(       \
+  if (aligned && nvec <= 256 && g_norm_pipe) {
+    const bool staged = (((uintptr_t)w | (uintptr_t)b) & 15) != 0;
+    const long long blocks = (rows + 3) / 4, most = staged ? 148 * (nvec <= 128 ? 16 : 8) : 1 << 20;
+    const size_t smem = staged ? 2 * (size_t)D * sizeof(TW) : 0;
+#define GB_FWDW_(VPT, STAGED)                                                                              \
+  norm_fwd_warp_kernel<T, TW, VPT, RMS, STAGED><<<(unsigned)(blocks < most ? blocks : most), 128, smem, s>>>( \
       (const T*)x, (const TW*)w, (const TW*)b, (T*)y, mean, rstd, rows, D, eps)
-    if (nvec <= 32) GB_FWDW(1);
-    else if (nvec <= 64) GB_FWDW(2);
-    else if (nvec <= 96) GB_FWDW(3);
-    else if (nvec <= 128) GB_FWDW(4);
-    else if (nvec <= 192) GB_FWDW(6);
-    else GB_FWDW(8);
+#define GB_FWDW(VPT)              \
+  if (staged) GB_FWDW_(VPT, true); \
+  else GB_FWDW_(VPT, false)
+    if (nvec <= 32) { GB_FWDW(1); }
+    else if (nvec <= 64) { GB_FWDW(2); }
+    else if (nvec <= 96) { GB_FWDW(3); }
+    else if (nvec <= 128) { GB_FWDW(4); }
+    else if (nvec <= 192) { GB_FWDW(6); }
+    else { GB_FWDW(8); }
+#undef GB_FWDW_
 #undef GB_FWDW
     GB_CUDA_OK(cudaGetLastError());
     return gbh::E_OK;
