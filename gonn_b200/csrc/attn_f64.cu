@@ -15,7 +15,7 @@
 // Work split: KW warps of a CTA share 16 rows and take different rows of each tile (their sums meet in
 // shared memory in a fixed order), 4 / KW row groups per CTA.  KW = 1 reuses a tile four times; small
 // problems leave SMs idle that way and take KW = 2 or 4 (launch_split).
-// Measured at 16 heads x 2048, D = 64, causal: forward 562 us (784 SIMT), dQ 651 (1906), dK / dV 812 (2220); the
+// Measured at 16 heads x 2048, D = 64, causal: forward 562 us (784 SIMT), dQ 623 (1906), dK / dV 791 (2220); the
 // fp64 pipe is 57 - 70 % active (ncu), the rest is the exponentials' dependent chains, which the two
 // warps per scheduler that 250 registers allow do not cover.
 #include "attn_args.cuh"
@@ -479,14 +479,18 @@ int launch_one(const GArgs& a, cudaStream_t s) {
 //   8 x 1024, D = 64 (128)                                    241/256/322 | 177/182/233 | 223/211/256
 //   8 x 1024, D = 64, causal (128)                            239/256/322 | 159/159/202 | 113/106/128
 //   8 x 512, D = 64 (64)                                      123/133/166 |  80/ 75/ 94 |  66/ 59/ 71
+// and for full GPUs, forward / dK and dV, KW = 1 | 2:
+//   8 x 512 x 16, causal (1024) 310/461 | 364/450     4 x 1024 x 16 (1024) 1133/1748 | 1198/1661
+//   2 x 2048 x 16, causal (1024) 1050/1612 | 1165/1578    1 x 2048 x 16 (512) 1138/1798 | 1284/1832
 // KW = 1 needs 1.5 waves of two CTAs per SM and the long accumulation of wide heads to pay for its coarse
-// blocks; KW = 4 pays while KW = 2 leaves SMs without a second CTA (causal blocks are half as long on average).
+// blocks, and pays in the forward alone, whose row state (running maximum and sum) every merge has to bring
+// together; KW = 4 pays while KW = 2 leaves SMs without a second CTA (causal blocks are half as long on average).
 template <int MODE, int DT>
 int launch_split(const GArgs& a, cudaStream_t s) {
   const int rows = MODE == MODE_DKV ? a.Tk : a.Tq;
   const long long blocks64 = (long long)((rows + 63) / 64) * a.H * a.B;
   const int kw = g_f64_split ? g_f64_split
-                             : blocks64 >= 444 && a.D > 32 ? 1 : blocks64 >= (a.causal ? 200 : 100) ? 2 : 4;
+                             : MODE == MODE_FWD && blocks64 >= 444 && a.D > 32 ? 1 : blocks64 >= (a.causal ? 200 : 100) ? 2 : 4;
   if (kw == 1) return launch_one<MODE, DT, 1, MODE == MODE_FWD ? 4 : 2>(a, s);   // 104 KB: two CTAs per SM
   if (kw == 2) return launch_one<MODE, DT, 2, 2>(a, s);
   return launch_one<MODE, DT, 4, 1>(a, s);
