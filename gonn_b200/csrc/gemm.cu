@@ -1673,11 +1673,15 @@ int launch_2cta(const TMaps& tm, const GemmArgs& args, int num_sms, cudaStream_t
 
 thread_local int g_cluster_splits = 0;   // 0: by the rule of cluster_splits(); -1: off; 1, 2, 4, 8: that many CTAs per tile
 
-// CTAs per 128 x 64 tile of the cluster kernel, 0 = another kernel.  K is cut until the CTAs come to about one per SM.
-// The cluster's exchange costs 2.5 us, so it pays from four parts on, or from two where K is long.  Measured, us
-// (best | one CTA per 128 x 128 tile): 77 x 768 x 3072 6.9 (8 parts) | 14.0; 128 x 2048 x 8192 13.6 (4) | 30.3; 300 x 768 x
-// 3072 9.2 (4) | 14.2; 128 x 2048 x 2048 8.4 (4) | 11.1; 77 x 768 x 768 6.0 (8) | 7.0; 77 x 2304 x 768 7.1 (4) | 6.9;
-// 700 x 768 x 3072 13.4 (2) | 14.3; 77 x 3072 x 768 8.1 (2) | 7.0; 128 x 8192 x 2048 12.7 (2) | 11.3; 300 x 2304 x 768 10.5 (1) | 7.2.
+// CTAs per 128 x 64 tile of the cluster kernel, 0 = another kernel.  K is cut until the CTAs come to about one per SM; from 16
+// tiles on, eight CTAs of a cluster no longer find SMs of their own and take four.  The exchange costs 1 to 2.5 us with the
+// rows of a tile, so K must be long enough to pay for it.  Measured, us (parts: time | one CTA per 128 x 128 tile):
+//   77 x 768 x 3072 8: 6.9 | 14.0   77 x 768 x 768 8: 6.0 | 7.0   64 x 576 x 512 8: 5.6 | 6.0   128 x 832 x 768 8: 7.0 | 7.0
+//   256^3 4: 6.5 | 5.4   512^3 4: 7.0 | 6.3   128 x 512 x 640 8: 6.8 | 6.7   64 x 784 x 256 4: 5.7 | 5.3
+//   128 x 1280 x 1024 8: 8.0, 4: 7.3 | 7.8   512 x 320 x 768 8: 8.6, 4: 7.1 | 7.1   128 x 1280 x 4096 8: 9.6, 4: 10.1 | 17.3
+//   32 x 2304 x 512 4: 5.7 | 6.2   77 x 2304 x 640 4: 6.8 | 6.7   77 x 2304 x 768 4: 7.0 | 7.0   256 x 1024 x 768 4: 7.3 | 7.1
+//   64 x 2624 x 768 4: 7.2 | 6.9   77 x 2304 x 1024 4: 7.0 | 7.8   128 x 2048 x 8192 4: 13.6 | 30.3
+//   700 x 768 x 3072 2: 13.4 | 14.3   77 x 3072 x 768 2: 8.1 | 7.0   128 x 8192 x 2048 2: 12.7 | 11.3   300 x 2304 x 768 1: 10.5 | 7.2
 int cluster_splits(int M, int N, int K, int batch, int num_sms) {
   if (g_cluster_splits < 0 || batch > 65535) return 0;
   const long long tiles = (long long)((M + BM - 1) / BM) * ((N + CfgS::BN - 1) / CfgS::BN) * batch;
@@ -1685,8 +1689,12 @@ int cluster_splits(int M, int N, int K, int batch, int num_sms) {
   if (g_cluster_splits > 0) return g_cluster_splits;
   const int num_kb = (K + CfgS::BK - 1) / CfgS::BK;
   int s = 1;
-  while (s < 8 && tiles * s * 2 <= num_sms + num_sms / 8 && num_kb >= 2 * s) s *= 2;
-  return s >= 4 || (s == 2 && num_kb >= 48) ? s : 0;
+  while (s < 8 && tiles * s * 2 <= num_sms + num_sms / 8) s *= 2;
+  if (s == 8 && tiles >= 16 && num_kb < 48) s = 4;
+  int least = 48;                                          // k-blocks
+  if (s == 8) least = M <= 80 ? 8 : 12;
+  if (s == 4) least = M <= 64 && tiles * s <= num_sms ? 8 : 14;
+  return s >= 2 && num_kb >= least ? s : 0;
 }
 
 template <bool A_MN, bool B_MN, bool PL>
@@ -2010,6 +2018,8 @@ GB_EXPORT int gb_gemm_cluster_tune(int splits) {
   if (splits == -1 || splits == 0 || splits == 1 || splits == 2 || splits == 4 || splits == 8) g_cluster_splits = splits;
   return 0;
 }
+// CTAs that share a tile of this 16-bit product on a whole B200, 0: not a product of the cluster kernel (for tests).
+GB_EXPORT int gb_gemm_cluster_parts(int M, int N, int K, int batch) { return cluster_splits(M, N, K, batch, 148); }
 // Enables (1) or disables (0) split-K for products with few output tiles.
 GB_EXPORT int gb_gemm_splitk(int on) {
   g_splitk = on;
