@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(256) conv_wgrad_finish_kernel(const float* __r
 //    fragments are read.  Gathering the fragments directly cost eight sectors a load (43 and 55 us);
 //  * column n = 2t + e of n-tile j stands for position 8t + 2j + e, so a lane's results of the four n-tiles are eight
 //    consecutive positions of a channel (V of them at a time are aligned when V divides L).
-// Forward 22 us, weight gradient 45 us; bound by the gathers and the 29.5 MB of outputs or gradients.
+// Forward 23 us, weight gradient 35 us; bound by the gathers and the 29.5 MB of outputs or gradients.
 constexpr int kDirectK = 32;
 constexpr int kSmallWarps = 8;
 constexpr int kSmallSmem = 96 * 1024;   // limit of the dynamic shared memory: windows of 32 taps alone take 49 KB
@@ -392,27 +392,51 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// Index rows of positions p0 .. p0 + 31 into si[32 * T]: rows of consecutive positions follow one another, from the
-// end of an image's map to its beginning.  Returns the image of this lane's position.
-__device__ __forceinline__ void stage_index(int* si, const int* __restrict__ idx, long long p0, int L, int T, int& img) {
+// Position p0 of a warp's 32 as (image, position in the image).  The first ones are below 2^31 (148 * 8 CTAs of 256), and so are the
+// strides from one to the next: no 64-bit division.
+struct SmallPos {
+  int img;
+  unsigned l;
+  __device__ __forceinline__ SmallPos(unsigned p, unsigned L) : img((int)(p / L)), l(p % L) {}
+  __device__ __forceinline__ void advance(const SmallPos& by, unsigned L) {
+    img += by.img;
+    l += by.l;
+    if (l >= L) { l -= L; img++; }
+  }
+};
+
+// Index rows of the 32 positions from `at` on into si[32 * T]: rows of consecutive positions follow one another, from the
+// end of an image's map to its beginning.  img, l: this lane's position.
+__device__ __forceinline__ void stage_index(int* si, const int* __restrict__ idx, const SmallPos& at, unsigned L, int T, int& img, unsigned& l) {
   const int lane = threadIdx.x & 31;
-  const long long img0 = p0 / L;
-  const int l0 = (int)(p0 - img0 * L);
   const long long LT = (long long)L * T;
   __syncwarp();
-  for (int i = lane; i < 32 * T; i += 32) {
-    long long f = (long long)l0 * T + i;
-    while (f >= LT) f -= LT;
-    si[i] = __ldg(idx + f);
+  for (int j0 = 0; j0 < T; j0 += 8) {                      // eight loads in flight: one at a time, T load latencies in a row
+    int v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+      if (j0 + j < T) {
+        long long f = (long long)at.l * T + (j0 + j) * 32 + lane;
+        if (f >= LT) {                                     // past the end by less than 32 T <= 1024
+          const unsigned past = (unsigned)(f - LT);
+          f = past < LT ? past : past % (unsigned)LT;
+        }
+        v[j] = __ldg(idx + f);
+      }
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+      if (j0 + j < T) si[(j0 + j) * 32 + lane] = v[j];
   }
-  int l = l0 + lane;
-  img = (int)img0;
+  l = at.l + lane;
+  img = at.img;
   while (l >= L) { l -= L; img++; }
   __syncwarp();
 }
 
-// The 32 (K of them real) inputs of this lane's position, two at a time, to put(k, v[k], v[k + 1]); image img, index rows si.
-template <typename F>
+// The 32 (K of them real) inputs of this lane's position, two at a time, to put(k, v[k], v[k + 1]); image img, index rows si.  B
+// loads are in flight together: put writes shared memory, past which the compiler moves no later index read (64 images, 3 x
+// 31 x 31 to 64 channels, forward 28.3 -> 10.5 us with this, the batched index rows and the wide stores below).
+template <int B, typename F>
 __device__ __forceinline__ void gather_windows(const uint16_t* __restrict__ x, int img, bool live, const int* si, int C, int S, int T,
                                                const F& put) {
   const int K = C * T;
@@ -420,28 +444,35 @@ __device__ __forceinline__ void gather_windows(const uint16_t* __restrict__ x, i
   const int* row = si + (threadIdx.x & 31) * T;
   int tap = 0;
 #pragma unroll
-  for (int k = 0; k < kDirectK; k += 2) {
-    uint32_t v[2] = {0u, 0u};
+  for (int k0 = 0; k0 < kDirectK; k0 += B) {
+    uint32_t v[B];
 #pragma unroll
-    for (int e = 0; e < 2; e++)
-      if (k + e < K) {
+    for (int e = 0; e < B; e++) {
+      v[e] = 0u;
+      if (k0 + e < K) {
         const int src = row[tap];
         if (live && src >= 0) v[e] = __ldg(xc + src);
         if (++tap == T) { tap = 0; xc += S; }
       }
-    put(k, v[0], v[1]);
+    }
+#pragma unroll
+    for (int e = 0; e < B; e += 2) put(k0 + e, v[e], v[e + 1]);
   }
   __syncwarp();
 }
 
-// Where the runs of V of the eight consecutive positions q0 .. q0 + 7 start in a (Nimg, M, L) tensor (channel 0), -1 past
+// Where the runs of V of the eight consecutive positions from `at` + 8t on start in a (Nimg, M, L) tensor (channel 0), -1 past
 // the end.  V divides L, so a run never straddles images or the end.
 template <int V>
-__device__ __forceinline__ void run_starts(long long (&at)[8 / V], long long q0, long long P, int M, int L) {
+__device__ __forceinline__ void run_starts(long long (&start)[8 / V], const SmallPos& at, int t, int Nimg, int M, unsigned L) {
+  unsigned l = at.l + 8 * t;
+  int img = at.img;
+  while (l >= L) { l -= L; img++; }
 #pragma unroll
   for (int i = 0; i < 8 / V; i++) {
-    const long long q = q0 + i * V, img = q / L;
-    at[i] = q < P ? img * M * L + (q - img * L) : -1;
+    start[i] = img < Nimg ? (long long)img * M * L + l : -1;
+    l += V;
+    if (l >= L) { l -= L; img++; }
   }
 }
 // Eight values of a channel (row offset m * L), V at a time.
@@ -492,6 +523,16 @@ conv_direct_small_kernel(const uint16_t* __restrict__ x, const uint16_t* __restr
   float* sbias = reinterpret_cast<float*>(wf + MT * 256);   // [MT * 16]
   int* si = reinterpret_cast<int*>(sbias + MT * 16) + (threadIdx.x >> 5) * 32 * (T + 17);
   uint32_t* sp = reinterpret_cast<uint32_t*>(si + 32 * T);   // [32 positions][16 pairs of k], pitch 17
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const unsigned first = (blockIdx.x * kSmallWarps + (threadIdx.x >> 5)) * 32u, stride = gridDim.x * kSmallWarps * 32u;
+  SmallPos at(first, L);
+  const SmallPos by(stride, L);
+  int img;
+  unsigned l;
+  auto fetch = [&]() {                                     // index rows and windows of the warp's positions into sp
+    stage_index(si, idx, at, L, T, img, l);
+    gather_windows<32>(x, img, img < Nimg, si, C, S, T, [&](int k, uint32_t lo, uint32_t hi) { sp[lane * 17 + (k >> 1)] = lo | (hi << 16); });
+  };
   auto wval = [&](int m, int k) -> uint32_t { return m < M && k < K ? (uint32_t)__ldg(w + (long long)m * K + k) : 0u; };
   for (int i = threadIdx.x; i < MT * 256; i += blockDim.x) {
     const int r = i & 3, ln = (i >> 2) & 31, ks = (i >> 7) & 1, mt = i >> 8;
@@ -499,16 +540,11 @@ conv_direct_small_kernel(const uint16_t* __restrict__ x, const uint16_t* __restr
     wf[i] = wval(m, k) | (wval(m, k + 1) << 16);
   }
   for (int i = threadIdx.x; i < MT * 16; i += blockDim.x) sbias[i] = bias != nullptr && i < M ? raw16_to_float(__ldg(bias + i), bf16) : 0.f;
+  if (at.img < Nimg) fetch();                              // in flight with the weights
   __syncthreads();
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const long long P = (long long)Nimg * L;
-  const long long warps = (long long)gridDim.x * kSmallWarps;
-  for (long long p0 = ((long long)blockIdx.x * kSmallWarps + (threadIdx.x >> 5)) * 32; p0 < P; p0 += warps * 32) {
-    int img;
-    stage_index(si, idx, p0, L, T, img);
-    long long at[8 / V];
-    run_starts<V>(at, p0 + 8 * t, P, M, L);
-    gather_windows(x, img, p0 + lane < P, si, C, S, T, [&](int k, uint32_t lo, uint32_t hi) { sp[lane * 17 + (k >> 1)] = lo | (hi << 16); });
+  while (at.img < Nimg) {
+    long long run[8 / V];
+    run_starts<V>(run, at, t, Nimg, M, L);
     uint32_t b[4][2][2];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
@@ -518,6 +554,8 @@ conv_direct_small_kernel(const uint16_t* __restrict__ x, const uint16_t* __restr
 #pragma unroll
         for (int r = 0; r < 2; r++) b[j][ks][r] = row[ks * 8 + r * 4];
     }
+    const bool live = img < Nimg;
+    uint16_t* yl = y + (live ? (long long)img * M * L + l : 0);     // this lane's position, channel 0
     for (int mt = 0; mt < MT; mt++) {
       const float b0 = sbias[mt * 16 + g], b1 = sbias[mt * 16 + g + 8];
       float c[4][4];
@@ -534,16 +572,36 @@ conv_direct_small_kernel(const uint16_t* __restrict__ x, const uint16_t* __restr
 #pragma unroll
         for (int ks = 0; ks < 2; ks++) mma16816(c[j], af[ks], b[j][ks], bf16);
       }
+      if (V <= 2) __syncwarp();                            // the windows, or the block before, have been read
 #pragma unroll
       for (int r = 0; r < 2; r++) {
         const int m = mt * 16 + g + 8 * r;
-        if (m >= M) continue;
+        if (V > 2 && m >= M) continue;
         uint32_t v[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) v[j] = float_to_raw16(c[j][2 * r], bf16) | ((uint32_t)float_to_raw16(c[j][2 * r + 1], bf16) << 16);
-        store8<V>(y + (long long)m * L, v, at);
+        if (V > 2) {
+          store8<V>(y + (long long)m * L, v, run);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; j++) sp[(g + 8 * r) * 17 + 4 * t + j] = v[j];
+        }
+      }
+      if (V <= 2) {
+        // planes that no wide run divides: the block of 16 channels turns around in shared memory, so that a store takes 32
+        // consecutive positions (64 images of 8 x 28 x 28 to 32 channels, 2 x 2: runs of two bytes 17.4 us, this 8.9)
+        __syncwarp();
+        const uint16_t* sh = reinterpret_cast<const uint16_t*>(sp) + lane;
+        const int rows = min(16, M - mt * 16);
+        if (live) {
+          uint16_t* d = yl + (long long)mt * 16 * L;
+#pragma unroll 4
+          for (int r = 0; r < rows; r++) d[(long long)r * L] = sh[r * 34];
+        }
       }
     }
+    at.advance(by, L);
+    if (at.img < Nimg) fetch();
   }
 }
 
@@ -567,14 +625,15 @@ conv_wgrad_small_kernel(const uint16_t* __restrict__ x, const uint16_t* __restri
     for (int j = 0; j < 4; j++)
 #pragma unroll
       for (int e = 0; e < 4; e++) acc[i][j][e] = 0.f;
-  const long long P = (long long)Nimg * L;
-  const long long warps = (long long)gridDim.x * kSmallWarps;
-  for (long long p0 = ((long long)blockIdx.x * kSmallWarps + warp) * 32; p0 < P; p0 += warps * 32) {
+  SmallPos at((blockIdx.x * kSmallWarps + warp) * 32u, L);
+  const SmallPos by(gridDim.x * kSmallWarps * 32u, L);
+  for (; at.img < Nimg; at.advance(by, L)) {
     int img;
-    stage_index(si, idx, p0, L, T, img);
-    long long at[8 / V];
-    run_starts<V>(at, p0 + 8 * t, P, M, L);
-    gather_windows(x, img, p0 + lane < P, si, C, S, T, [&](int k, uint32_t lo, uint32_t hi) {
+    unsigned l;
+    stage_index(si, idx, at, L, T, img, l);
+    long long run[8 / V];
+    run_starts<V>(run, at, t, Nimg, M, L);
+    gather_windows<MT == 4 ? 8 : 16>(x, img, img < Nimg, si, C, S, T, [&](int k, uint32_t lo, uint32_t hi) {
       sp[k * 34 + lane] = (uint16_t)lo;
       sp[(k + 1) * 34 + lane] = (uint16_t)hi;
     });
@@ -590,8 +649,8 @@ conv_wgrad_small_kernel(const uint16_t* __restrict__ x, const uint16_t* __restri
 #pragma unroll
     for (int mt = 0; mt < MT; mt++) {
       uint32_t lo[4], hi[4];
-      load8<V>(dy + (long long)(m0 + mt * 16 + g) * L, lo, at);
-      load8<V>(dy + (long long)(m0 + mt * 16 + g + 8) * L, hi, at);
+      load8<V>(dy + (long long)(m0 + mt * 16 + g) * L, lo, run);
+      load8<V>(dy + (long long)(m0 + mt * 16 + g + 8) * L, hi, run);
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         const uint32_t af[4] = {lo[2 * h], hi[2 * h], lo[2 * h + 1], hi[2 * h + 1]};
