@@ -367,7 +367,16 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_bwd_kernel(const SeqArgs
   }
 }
 
-constexpr int kSms = 148;
+constexpr int kSms = 148;       // of a whole B200; also the words of the flags' scratch
+// SMs of the current device: all CTAs of a cooperative launch need one each.  (No device, as in host-side tests: a whole B200.)
+int device_sms() {
+  int dev, n;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return kSms;
+  }
+  return n < kSms ? n : kSms;
+}
 constexpr long long kMaxSmem = 227 * 1024 - 16;      // what a block may take, less the kernels' static abort flag
 // Each sub-tile costs a group of CTAs about 1.9 us forward and 2.9 us backward (H = 512); beyond 32 of them the
 // step-by-step GEMMs fill the GPU themselves (forward + backward over 8 steps at H = 512: B = 1024, 32
@@ -382,23 +391,23 @@ long long bwd_smem(int ut, int H, int sub) {
 }
 
 // Units per CTA, unit slices, groups of sequences and sub-tiles per group; false when the layer does
-// not fit (the weight slices of 148 CTAs, or the exchange tile, exceed shared memory).
+// not fit (the weight slices of `sms` CTAs, or the exchange tile, exceed shared memory).
 // Large UT keeps the exchanged tile small against the resident weight; it is halved while that
 // gives more CTAs than half of the SMs would otherwise see.
-bool plan(int B, int H, bool bwd, int* ut, int* ug, int* groups, int* sub) {
+bool plan(int sms, int B, int H, bool bwd, int* ut, int* ug, int* groups, int* sub) {
   if (H % 4 != 0 || H < 4) return false;
   const int tiles = (B + kMB - 1) / kMB;
   int best = 0;
   for (int u = 16; u >= 4; u >>= 1) {
     const int slices = (H + u - 1) / u;
-    if (slices > kSms) break;                     // smaller u only makes more slices
-    const int g = tiles < kSms / slices ? tiles : kSms / slices;
+    if (slices > sms) break;                      // smaller u only makes more slices
+    const int g = tiles < sms / slices ? tiles : sms / slices;
     const int s = (tiles + g - 1) / g;
     const long long need = bwd ? bwd_smem(u, H, s) : fwd_smem(u, H);
     if (need > kMaxSmem || s > kMaxSub) continue;
     *ut = u; *ug = slices; *sub = s; *groups = (tiles + s - 1) / s;
     best = u;
-    if ((long long)slices * *groups >= kSms / 2) break;
+    if ((long long)slices * *groups >= sms / 2) break;
   }
   return best != 0;
 }
@@ -418,14 +427,16 @@ int launch(K kern, const SeqArgs& a, int groups, long long smem, cudaStream_t s)
 // Dynamic shared memory of a CTA of either direction, 0 when the layer does not fit (for tests).
 GB_EXPORT int gb_lstm_seq_smem(int B, int H, int bwd) {
   int ut, ug, groups, sub;
-  if (B <= 0 || !plan(B, H, bwd != 0, &ut, &ug, &groups, &sub)) return 0;
+  if (B <= 0 || !plan(kSms, B, H, bwd != 0, &ut, &ug, &groups, &sub)) return 0;
   return (int)(bwd ? bwd_smem(ut, H, sub) : fwd_smem(ut, H));
 }
-// 1 when both directions of an LSTM layer of this size run as persistent kernels.
-GB_EXPORT int gb_lstm_seq_fits(int B, int H) {
+// 1 when both directions of an LSTM layer of this size run as persistent kernels on that many SMs ...
+GB_EXPORT int gb_lstm_seq_fits_on(int sms, int B, int H) {
   int ut, ug, groups, sub;
-  return B > 0 && plan(B, H, false, &ut, &ug, &groups, &sub) && plan(B, H, true, &ut, &ug, &groups, &sub) ? 1 : 0;
+  return B > 0 && plan(sms, B, H, false, &ut, &ug, &groups, &sub) && plan(sms, B, H, true, &ut, &ug, &groups, &sub) ? 1 : 0;
 }
+// ... and on the current device.
+GB_EXPORT int gb_lstm_seq_fits(int B, int H) { return gb_lstm_seq_fits_on(device_sms(), B, H); }
 
 // fp32.  xg (B,T,4H) = x W_ih^T, bias (4H) or null, w = W_hh (4H,H), h0 / c0 (B,H) or null; writes out (B,T,H), whose sequences are
 // out_sb elements apart.  For a backward (hprev not null): h_{t-1} of every step in hprev (B,T,H) (a buffer of its own, so that the
@@ -436,7 +447,7 @@ GB_EXPORT int gb_lstm_seq_fwd(void* xg, const void* bias, const void* w, const v
   if (B <= 0 || T <= 0) return gbh::E_OK;
   SeqArgs a = {};
   int ut, groups;
-  if (!plan(B, H, false, &ut, &a.ug, &groups, &a.sub)) {
+  if (!plan(device_sms(), B, H, false, &ut, &a.ug, &groups, &a.sub)) {
     gbh::set_error("gb_lstm_seq_fwd: a layer of %d units does not fit", H);
     return gbh::E_TOO_LARGE;
   }
@@ -468,7 +479,7 @@ GB_EXPORT int gb_lstm_seq_bwd(const void* w, const void* c0, const void* cseq, c
   if (B <= 0 || T <= 0) return gbh::E_OK;
   SeqArgs a = {};
   int ut, groups;
-  if (!plan(B, H, true, &ut, &a.ug, &groups, &a.sub)) {
+  if (!plan(device_sms(), B, H, true, &ut, &a.ug, &groups, &a.sub)) {
     gbh::set_error("gb_lstm_seq_bwd: a layer of %d units does not fit", H);
     return gbh::E_TOO_LARGE;
   }

@@ -26,3 +26,14 @@ def test_accepted_layers_leave_room_for_static_shared_memory():
 @pytest.mark.parametrize("B,H", [(20, 896), (50, 892), (85, 888), (115, 884), (150, 880), (180, 876), (210, 872), (245, 868)])
 def test_layers_that_would_need_the_whole_block_are_refused(B, H):
     assert not L.lib().gb_lstm_seq_fits(L.I(B), L.I(H))
+
+
+def test_fewer_sms_fit_fewer_layers():
+    """Every CTA of the cooperative launch needs an SM of its own: on a part of a GPU the steps take over."""
+    l = L.lib()
+    fits = lambda sms, B, H: bool(l.gb_lstm_seq_fits_on(L.I(sms), L.I(B), L.I(H)))
+    assert fits(148, 32, 512) and fits(32, 32, 512) and not fits(31, 32, 512)     # 32 slices of 16 units
+    assert fits(148, 5, 880) and not fits(100, 5, 880)                            # 110 slices of 8 units
+    assert fits(1, 1, 16) and not fits(1, 300, 16)                                # one CTA, 32 tiles of 8 sequences at most
+    for H in (64, 512, 800):
+        assert [fits(s, 64, H) for s in range(1, 149)] == sorted(fits(s, 64, H) for s in range(1, 149))
