@@ -34,7 +34,7 @@ def _check(B, H, Tq, Tk, D, causal, masks, p_drop, strided=False):
     mask = kpm = None
     if masks:
         mask = torch.randn(Tq, Tk).masked_fill(torch.rand(Tq, Tk) < 0.2, float("-inf"))
-        mask[:, -1] = 0.5                                       # no row without a finite score
+        mask[:, 0] = 0.5                                        # no row without a finite score, causal ones neither
         kpm = torch.rand(B, Tk) < 0.2
     scale = 0.37
     qc, kc, vc = (t.cuda().requires_grad_() for t in (q, k, v))
@@ -70,7 +70,9 @@ def test_plain(split, spill, B, H, Tq, Tk, D, causal):
 @pytest.mark.parametrize("p_drop", [0.0, 0.3])
 @pytest.mark.parametrize("causal", [False, True])
 def test_masks_and_dropout(split, spill, causal, p_drop):
-    _check(2, 2, 70, 50, 24, causal and False, True, p_drop)
+    # (a mask beside the causal flag: no tile is skipped, and dS above the diagonal counts)
+    _check(2, 2, 70, 50, 24, causal, True, p_drop)
+    _check(1, 2, 130, 130, 40, causal, True, p_drop)
     _check(2, 2, 45, 45, 64, causal, False, p_drop)
 
 
