@@ -86,6 +86,15 @@ def _ktab(C, T, S, device):
     return t
 
 
+def _scratch(n: int, dtype, device):
+    """Scratch of the channels-last kernels; None where memory is short, and the gathers of csrc/conv.cu, which need none, take
+    the product."""
+    try:
+        return torch.empty(n, dtype=dtype, device=device)
+    except torch.OutOfMemoryError:
+        return None
+
+
 class _ConvImplicit(torch.autograd.Function):
     """Convolution as implicit GEMMs (csrc/conv.cu): forward, data gradient and weight gradient
     gather their operands inside the kernels; no (N, L, C*T) column tensor exists."""
@@ -101,13 +110,16 @@ class _ConvImplicit(torch.autograd.Function):
         wc = weight.contiguous()
         didx = device_maps(idx, S, x3.device, False)["idx"]
         y = torch.empty((N, Co, L), dtype=x3.dtype, device=x3.device)
-        if _l.lib().gb_conv_direct_ok(C, T, Co):
+        ws = None
+        direct = _l.lib().gb_conv_direct_ok(C, T, Co)
+        if not direct and _l.lib().gb_conv_cl_ok(N, C, S, L, T, Co, 0):
+            ws = _scratch(int(_l.lib().gb_conv_cl_fwd_ws(N, C, S, T, Co)), x3.dtype, x3.device)
+        if direct:
             # a contraction of at most 32 (3 channels x 3 x 3): one thread per output position, no tensor-core tile
             _l.call("gb_conv_direct_small", _l.I(_l.dtype_code(x3.dtype)), _l.ptr(xc), _l.ptr(wc), _l.ptr(didx),
                     _l.ptr(bias), _l.ptr(y), _l.I(N), _l.I(C), _l.I(S), _l.I(L), _l.I(T), _l.I(Co), _l.stream_ptr())
-        elif _l.lib().gb_conv_cl_ok(N, C, S, L, T, Co, 0):
+        elif ws is not None:
             # channel counts that are multiples of 8: 16-byte copies from a channels-last scratch
-            ws = torch.empty(int(_l.lib().gb_conv_cl_fwd_ws(N, C, S, T, Co)), dtype=x3.dtype, device=x3.device)
             _l.call("gb_conv_cl_fwd", _l.I(_l.dtype_code(x3.dtype)), _l.ptr(xc), _l.ptr(wc), _l.ptr(didx), _l.ptr(bias),
                     _l.ptr(y), _l.ptr(ws), _l.I(N), _l.I(C), _l.I(S), _l.I(L), _l.I(T), _l.I(Co), _l.stream_ptr())
         else:
@@ -145,9 +157,10 @@ class _ConvImplicit(torch.autograd.Function):
             else:
                 out, beta = torch.empty(Co * C * T, dtype=xc.dtype, device=xc.device), False
         # (a first layer asks for no dx and its short contraction has a kernel of its own)
+        ws = None
         if (need_dx or need_dw) and _l.lib().gb_conv_cl_ok(N, C, S, L, T, Co, 1):
-            ws = torch.empty(int(_l.lib().gb_conv_cl_bwd_ws(N, C, S, L, T, Co, int(need_dx), int(need_dw))), dtype=xc.dtype,
-                             device=xc.device)
+            ws = _scratch(int(_l.lib().gb_conv_cl_bwd_ws(N, C, S, L, T, Co, int(need_dx), int(need_dw))), xc.dtype, xc.device)
+        if ws is not None:
             part = (torch.empty(int(_l.lib().gb_conv_cl_part(N, C, L, T, Co)), dtype=torch.float32, device=xc.device)
                     if need_dw else None)
             _l.call("gb_conv_cl_bwd", _l.I(dt), _l.ptr(xc), _l.ptr(wc), _l.ptr(dyc), _l.ptr(didx if need_dw else None),

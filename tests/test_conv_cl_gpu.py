@@ -68,3 +68,39 @@ def test_windows_of_32_taps(dtype, Co, case):
     for n, a, b in (("y", y, want), ("dx", x.grad, xr.grad), ("dw", net.weight.grad, wr.grad), ("db", net.bias.grad, br.grad)):
         err = float((a.detach().double().cpu() - b.detach()).norm() / b.detach().norm())
         assert err < tol, f"{n}: {err:.3g}"
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_without_memory_for_the_channels_last_copies(monkeypatch, dtype):
+    """The kernels that need no scratch take a convolution for which it cannot be had."""
+    from gonn_b200.nn import conv
+    net = nn.Conv2d(24, 40, 3, 1, 1, dtype=dtype, device="cuda")
+    x = torch.randn(5, 24, 11, 9, device="cuda").to(dtype).requires_grad_()
+    y = net(x)
+    dy = torch.randn_like(y)
+    want = [y] + list(torch.autograd.grad(y, [x, *net.parameters()], dy))
+    seen = []
+    L.set_call_hook(lambda name, fn, args: (seen.append(name), fn(*args))[1])
+    monkeypatch.setattr(conv, "_scratch", lambda *a: None)
+    try:
+        y = net(x)
+        got = [y] + list(torch.autograd.grad(y, [x, *net.parameters()], dy))
+    finally:
+        L.set_call_hook(None)
+    L.assert_status_ok()
+    assert "gb_conv_igemm" in seen and not any(n.startswith("gb_conv_cl") for n in seen)
+    tol = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11      # one rounding of the result on either side
+    for a, b in zip(got, want):
+        a, b = a.detach().double(), b.detach().double()
+        assert float((a - b).norm() / b.norm()) < 2 * tol
+
+
+def test_scratch_is_none_when_memory_runs_out(monkeypatch):
+    from gonn_b200.nn import conv
+
+    def no_room(*a, **kw):
+        raise torch.OutOfMemoryError("no room")
+
+    assert conv._scratch(8, torch.bfloat16, "cuda").numel() == 8
+    monkeypatch.setattr(torch, "empty", no_room)
+    assert conv._scratch(8, torch.bfloat16, "cuda") is None
