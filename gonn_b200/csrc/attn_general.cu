@@ -445,9 +445,9 @@ GB_EXPORT int gb_attn_keep_mask(unsigned char* out, int B, int H, int Tq, int Tk
 
 // mode 0: forward (writes O and LSE); 1: dQ; 2: dK and dV (modes 1 and 2 first need delta: mode 3 computes
 // it from O and dO).  ptrs: Q, K, V, dO, O, dQ, dK, dV (unused ones null); strides: 8 triples (b, s, h) in the
-// ds (may be null): fp64 heads of up to 64 columns, B * H * ceil64(Tk) * ceil64(Tq) doubles, 16-byte aligned: mode 2 leaves dS^T
-// there and mode 1, called after it, reads it instead of recomputing it.
-// same order.  lse / delta: (B, H, Tq) in fp32 (fp64 for fp64 tensors).  mask: additive fp32 (Tq, Tk) or null; kpm: bytes (B, Tk), non-zero = padded key, or null.
+// same order.  lse / delta: (B, H, Tq) in fp32 (fp64 for fp64 tensors).  mask: additive fp32 (Tq, Tk) or null; kpm: bytes (B, Tk),
+// non-zero = padded key, or null.  ds (may be null): fp64 heads of up to 64 columns, B * H * ceil64(Tk) * ceil64(Tq) doubles,
+// 16-byte aligned: mode 2 leaves dS^T there and mode 1, called after it, reads it instead of recomputing it.
 GB_EXPORT int gb_attn_general(int mode, int dtype, void* const* ptrs, const long long* strides, void* lse,
                               void* delta, int B, int H, int Tq, int Tk, int D, double scale, int causal,
                               const float* mask, const unsigned char* kpm, double p_drop, long long seed,

@@ -751,10 +751,11 @@ GB_EXPORT int gb_conv_igemm(int dtype, const void* x, const void* w, const int* 
   return gbh::E_OK;
 }
 
-// Whether gb_conv_direct_small takes a forward convolution: a contraction of at most 32 and a channel
-// count that is a multiple of 4 whose weights fit in 48 KB of shared memory.
+// Whether gb_conv_direct_small takes a forward convolution: a contraction of at most 32 and a channel count that is a
+// multiple of 4 and at most 372 (the weights of 372 channels in fragment order, 26 KB, and the windows of eight warps, 50 KB
+// at 32 taps, fit its limit; more channels fill the 128-wide tiles of the other kernels).
 GB_EXPORT int gb_conv_direct_ok(int C, int T, int M) {
-  return C * T <= kDirectK && (M & 3) == 0 && M > 0 && (long long)(kDirectK + 1) * M * 4 <= 48 * 1024;
+  return C * T <= kDirectK && (M & 3) == 0 && M > 0 && M <= 372;
 }
 
 // The forward of gb_conv_igemm for the shapes gb_conv_direct_ok accepts (same arguments, no ktab).

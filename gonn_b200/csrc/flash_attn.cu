@@ -850,7 +850,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       tc_fence_after();
       constexpr int W = HD * 4 / C::EW;  // columns of dV / dK per warp
       const int cw = (group * 2 + half) * W;
-        uint16_t* dvrow = (uint16_t*)args.dV + (long long)b * args.dv_sb + (long long)kvrow * args.dv_ss +
+      uint16_t* dvrow = (uint16_t*)args.dV + (long long)b * args.dv_sb + (long long)kvrow * args.dv_ss +
                         (long long)h * args.dv_sh + cw;
       uint16_t* dkrow = (uint16_t*)args.dK + (long long)b * args.dk_sb + (long long)kvrow * args.dk_ss +
                         (long long)h * args.dk_sh + cw;

@@ -96,8 +96,9 @@ def _scratch(n: int, dtype, device):
 
 
 class _ConvImplicit(torch.autograd.Function):
-    """Convolution as implicit GEMMs (csrc/conv.cu): forward, data gradient and weight gradient
-    gather their operands inside the kernels; no (N, L, C*T) column tensor exists."""
+    """Convolution as implicit GEMMs: forward, data gradient and weight gradient read their operands through the window index
+    map inside the kernels; no (N, L, C*T) column tensor exists.  csrc/conv_cl.cu takes channel counts that are multiples of
+    8 from channels-last copies, csrc/conv.cu the others, and contractions of at most 32 without a tcgen05 tile."""
 
     @staticmethod
     def forward(ctx, x3, weight, bias, idx, S, L):
@@ -115,7 +116,7 @@ class _ConvImplicit(torch.autograd.Function):
         if not direct and _l.lib().gb_conv_cl_ok(N, C, S, L, T, Co, 0):
             ws = _scratch(int(_l.lib().gb_conv_cl_fwd_ws(N, C, S, T, Co)), x3.dtype, x3.device)
         if direct:
-            # a contraction of at most 32 (3 channels x 3 x 3): one thread per output position, no tensor-core tile
+            # a contraction of at most 32 (3 channels x 3 x 3): a warp per 32 positions and two k-steps of mma.sync
             _l.call("gb_conv_direct_small", _l.I(_l.dtype_code(x3.dtype)), _l.ptr(xc), _l.ptr(wc), _l.ptr(didx),
                     _l.ptr(bias), _l.ptr(y), _l.I(N), _l.I(C), _l.I(S), _l.I(L), _l.I(T), _l.I(Co), _l.stream_ptr())
         elif ws is not None:

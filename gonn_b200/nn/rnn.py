@@ -17,6 +17,7 @@ import torch
 
 from ..ops import elementwise as _ew
 from ..ops import rnn as _rnn_ops
+from .block import plain as _plain
 from .dropout import Dropout
 from .embedding import Embedding
 from .linear import Linear
@@ -147,12 +148,6 @@ def _gather_last_steps(out: torch.Tensor, lengths: Sequence[int]) -> torch.Tenso
 # ---------------------------------------------------------------------------------------
 # stacks
 # ---------------------------------------------------------------------------------------
-def _plain(m, cls) -> bool:
-    """``m`` is exactly a ``cls`` whose call is its class's forward: no hook, no replaced forward."""
-    return (type(m) is cls and "forward" not in m.__dict__ and not m._forward_hooks and not m._forward_pre_hooks
-            and not m._backward_hooks and not m._backward_pre_hooks)
-
-
 def _sequence_kernel_takes(cell, x, st0) -> bool:
     """Whether the step-by-step calls of ``cell`` may be replaced by ``ops.rnn.lstm_sequence``: an
     fp32 LSTM cell on CUDA without projection, nothing observing the single steps, and a layer that

@@ -8,7 +8,10 @@ torch expression with the same formulas (the oracle of the tests).
 ``lstm_sequence`` runs a whole fp32 LSTM layer: the input projections of all steps as one GEMM, the
 recurrence as one persistent kernel per direction (``csrc/lstm_seq.cu``), and the weight and input
 gradients as one GEMM each over all steps.  Measured forward + backward at B = 32, T = 64,
-I = H = 512: 0.96 ms, 22.6 ms step by step.
+I = H = 512: 0.96 ms, 22.6 ms step by step.  The products of all steps are large enough for the bf16 planes (``ops/gemm.py``),
+where those of one step were FMA sums; the layer's error against 64 bits, which the fast-math gates set, is the same
+within 2 % up to 64 x 64 steps (output 5.5e-6, dx 3.9e-6 against 4.0e-6, dW_ih 3.9e-6, dW_hh 6.2e-6) and
+up to 6 % larger where a gradient sums 8192 rows (32 x 256 steps: dx 4.2e-6 against 4.0e-6).
 """
 from __future__ import annotations
 

@@ -112,8 +112,8 @@ def test_fp32_three_plane_gemm(ta, tb, shape, status_ok):
     err = ((c.double() - ref).abs() / scale).max().item()
     err_simt = ((c_simt.double() - ref).abs() / scale).max().item()
     assert c.dtype == torch.float32
-    # both within a few units of 2^-24 of the summed magnitude (the three passes by magnitude
-    # class are what keeps the plane scheme there: one pass over all six products loses the low planes)
+    # both within a few units of 2^-24 of the summed magnitude (the small plane products are added first: after the
+    # large ones they would fall below the accumulator's last bit)
     assert err < 1e-6, (err, err_simt)
     assert err_simt < 1e-6, err_simt
 
