@@ -19,6 +19,7 @@
 // fp64 pipe is 57 - 70 % active (ncu), the rest is the exponentials' dependent chains, which the two
 // warps per scheduler that 250 registers allow do not cover.
 #include "attn_args.cuh"
+#include "f64_mma.cuh"
 
 using namespace gb;
 using namespace gba;
@@ -26,22 +27,6 @@ using namespace gba;
 namespace {
 
 constexpr int kWarps = 4, kThreads = kWarps * 32;
-
-__device__ __forceinline__ void cp_async8(void* dst, const void* src, bool pred) {
-  const int n = pred ? 8 : 0;  // src-size 0: the destination is zero-filled
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool pred) {
-  const int n = pred ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n) : "memory");
-}
-// A (16 x 8): a0 (g, t), a1 (g + 8, t), a2 (g, t + 4), a3 (g + 8, t + 4); B (8 x 8): b0 (t, g), b1 (t + 4, g);
-// C (16 x 8): c0, c1 (g, 2t + {0, 1}), c2, c3 (g + 8, 2t + {0, 1}); g = lane / 4, t = lane % 4.
-__device__ __forceinline__ void dmma(double (&c)[4], double a0, double a1, double a2, double a3, double b0, double b1) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-      : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(b0), "d"(b1));
-}
 
 // n rows of D columns (rows r0 .. of tensor p, batch b, head h) into a tile of pitch P; rows past `limit` and
 // the columns D .. C - 1 become zero.
@@ -54,13 +39,13 @@ __device__ __forceinline__ void issue_rows(double* dst, const void* p, const lon
     for (int i = threadIdx.x; i < n * (C / 2); i += kThreads) {
       const int r = i / (C / 2), c = (i - r * (C / 2)) * 2;
       const bool ok = r0 + r < limit && c < D;
-      cp_async16(dst + r * P + c, ok ? base + (long long)(r0 + r) * s[1] + c : base, ok);
+      cp_async16(dst + r * P + c, ok ? base + (long long)(r0 + r) * s[1] + c : base, ok ? 16 : 0);
     }
   } else {
     for (int i = threadIdx.x; i < n * C; i += kThreads) {
       const int r = i / C, c = i - r * C;
       const bool ok = r0 + r < limit && c < D;
-      cp_async8(dst + r * P + c, ok ? base + (long long)(r0 + r) * s[1] + c : base, ok);
+      cp_async8(dst + r * P + c, ok ? base + (long long)(r0 + r) * s[1] + c : base, ok ? 8 : 0);
     }
   }
 }
@@ -125,7 +110,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_f64_kernel(const GArgs a) {
         for (int i = threadIdx.x; i < 2 * TK; i += kThreads) {
           const int q = t0 + (i < TK ? i : i - TK);
           const double* src = i < TK ? LSEp : Deltap;
-          cp_async8(ls + i, q < a.Tq ? src + q : src, q < a.Tq);
+          cp_async8(ls + i, q < a.Tq ? src + q : src, q < a.Tq ? 8 : 0);
         }
       } else {
         issue_rows<S::C, P>(ta, a.K, a.k_s, b, h, t0, TK, a.Tk, a.D);
@@ -401,7 +386,7 @@ __global__ void __launch_bounds__(kThreads, 3) attn_f64_dq_ds_kernel(const GArgs
       for (int i = threadIdx.x; i < TK * (S::ROWS / 2); i += kThreads) {      // rows of dS^T are 64-padded and aligned
         const int r = i / (S::ROWS / 2), c = (i - r * (S::ROWS / 2)) * 2;
         const bool ok = t0 + r < a.Tk;
-        cp_async16(ts + r * PS + c, ok ? ds + (long long)(t0 + r) * a.ds_ld + c : ds, ok);
+        cp_async16(ts + r * PS + c, ok ? ds + (long long)(t0 + r) * a.ds_ld + c : ds, ok ? 16 : 0);
       }
       issue_rows<S::C, P>(ts + TK * PS, a.K, a.k_s, b, h, t0, TK, a.Tk, a.D);
     }

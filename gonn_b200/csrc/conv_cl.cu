@@ -42,11 +42,6 @@ struct ClArgs {
   int* status;
 };
 
-__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool ok) {
-  const int n = ok ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
-}
-
 // MODE 0: forward / dgrad (grid: position tiles, M tiles); MODE 1: wgrad (grid: (tap, c) tiles, M tiles, splits)
 template <int MODE>
 __global__ void __launch_bounds__(THREADS, 2) conv_cl_kernel(const ClArgs a) {
@@ -153,10 +148,10 @@ __global__ void __launch_bounds__(THREADS, 2) conv_cl_kernel(const ClArgs a) {
           const uint32_t off = r * 128 + ((c8 ^ (r & 7)) << 4);
           if (m0 + 32 * i < a.M) {                         // rows of the accumulator past M are never read
             const bool live = m0 + r < a.M && k < K;
-            cp16(sa + off, a.W + (live ? (long long)(m0 + r) * K + k : 0), live);
+            cp_async16(sa + off, a.W + (live ? (long long)(m0 + r) * K + k : 0), live ? 16 : 0);
           }
           const int s = tap < a.T ? sidx[tap * BN + r] : -1;
-          cp16(sb + off, a.X + (s >= 0 ? (long long)s * a.C + c : 0), s >= 0);
+          cp_async16(sb + off, a.X + (s >= 0 ? (long long)s * a.C + c : 0), s >= 0 ? 16 : 0);
         }
         c += BK;
         while (c >= a.C) { c -= a.C; tap++; }
@@ -171,9 +166,9 @@ __global__ void __launch_bounds__(THREADS, 2) conv_cl_kernel(const ClArgs a) {
             const int m = m0 + h * 64 + c8 * 8;
             if (m0 + h * 64 < a.M) {
               const bool live = m < a.M && p0 + r < k_end;
-              cp16(sa + h * (TILE / 2) + off, a.DY + (live ? (p0 + r) * a.M + m : 0), live);
+              cp_async16(sa + h * (TILE / 2) + off, a.DY + (live ? (p0 + r) * a.M + m : 0), live ? 16 : 0);
             }
-            cp16(sb + h * (TILE / 2) + off, a.X + (src[i][h] >= 0 ? (long long)src[i][h] * a.C + c_h[h] : 0), src[i][h] >= 0);
+            cp_async16(sb + h * (TILE / 2) + off, a.X + (src[i][h] >= 0 ? (long long)src[i][h] * a.C + c_h[h] : 0), src[i][h] >= 0 ? 16 : 0);
           }
         }
       }

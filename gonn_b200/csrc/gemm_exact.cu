@@ -15,7 +15,7 @@
 // The in-library benchmark loops at the end mirror the reference's (gonn_cuda.cu:255-294,
 // 532-592, 673-690): operands allocated once, five untimed calls, `iters` calls between two
 // events, milliseconds per call returned.
-#include "common.cuh"
+#include "f64_mma.cuh"
 
 using namespace gb;
 
@@ -59,23 +59,6 @@ constexpr int DOP = DBK * DPITCH;                       // doubles of one operan
 constexpr int DSMEM = DSTAGES * 2 * DOP * 8;
 static_assert(DB * DB <= DSTAGES * 2 * DOP, "the cluster's partial tiles reuse the stages");
 
-__device__ __forceinline__ void cp_async8(void* dst, const void* src, bool pred) {
-  const int n = pred ? 8 : 0;  // src-size 0: the destination is zero-filled
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(n) : "memory");
-}
-// 16 bytes of which `bytes` (0, 8 or 16) come from memory and the rest are zero
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
-}
-
-// A (16 x 8): a0 (g, t), a1 (g + 8, t), a2 (g, t + 4), a3 (g + 8, t + 4); B (8 x 8): b0 (t, g), b1 (t + 4, g);
-// C (16 x 8): c0, c1 (g, 2t + {0, 1}), c2, c3 (g + 8, 2t + {0, 1}); g = lane / 4, t = lane % 4.
-__device__ __forceinline__ void dmma16(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
-}
-
 // 64 rows (of MN) x 16 k of an operand into a stage.  KC: stored (MN, K), else (K, MN); k runs to k_end.
 template <bool KC>
 __device__ __forceinline__ void load_tile(double* st, const double* src, long long ld, int mn0, int k0, int MN, int k_end, bool vec) {
@@ -100,7 +83,7 @@ __device__ __forceinline__ void load_tile(double* st, const double* src, long lo
       const int r = KC ? q >> 4 : q & 63, kk = KC ? q & 15 : q >> 6;
       const bool ok = mn0 + r < MN && k0 + kk < k_end;
       const long long at = KC ? (long long)(mn0 + r) * ld + k0 + kk : (long long)(k0 + kk) * ld + mn0 + r;
-      cp_async8(KC ? st + ((kk >> 3) * DB + r) * 8 + (kk & 7) : st + kk * DPITCH + r, ok ? src + at : src, ok);
+      cp_async8(KC ? st + ((kk >> 3) * DB + r) * 8 + (kk & 7) : st + kk * DPITCH + r, ok ? src + at : src, ok ? 8 : 0);
     }
   }
 }
@@ -172,7 +155,7 @@ gemm_f64_mma_kernel(const double* __restrict__ A, const double* __restrict__ B, 
 #pragma unroll
       for (int i = 0; i < 2; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) dmma16(acc[i][j], af[i], bf[j]);
+        for (int j = 0; j < 4; j++) dmma(acc[i][j], af[i][0], af[i][1], af[i][2], af[i][3], bf[j][0], bf[j][1]);
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");

@@ -38,9 +38,6 @@ __device__ __forceinline__ float sigm(float x) { return 1.f / (1.f + __expf(-x))
 __device__ __forceinline__ void ffma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 struct SeqArgs {
@@ -155,7 +152,7 @@ __device__ __forceinline__ void load_tile(float* __restrict__ tile, const float*
     const int r = i / k4, c = (i - r * k4) * 4;
     float* d = tile + r * pitch + c;
     if (src != nullptr && b0 + r < B)
-      cp_async16(d, src + (long long)(b0 + r) * stride + c);
+      cp_async16(d, src + (long long)(b0 + r) * stride + c, 16);
     else
       *reinterpret_cast<float4*>(d) = make_float4(0.f, 0.f, 0.f, 0.f);
   }
