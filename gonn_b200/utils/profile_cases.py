@@ -12,6 +12,8 @@
                                                                        # B S H D: masked + dropout attention, fwd and bwd
     python -m gonn_b200.utils.profile_cases suite                      # one launch or two of every other kernel family
     python -m gonn_b200.utils.profile_cases suite2                     # ... and of the families `suite` leaves out
+    python -m gonn_b200.utils.profile_cases suite3                     # LSTM layer, convolutions, few-tile and exact products,
+                                                                       # norm rows, fp64 attention
 
 Each case allocates a few hundred MB at most, runs three warm-up launches and
 then five timed launches (CUDA events), and prints one line with the time and the
@@ -261,6 +263,31 @@ def main(argv):
             flash_bwd(q, k, v, o, torch.randn_like(o), lse, True, 0.125)
             torch.cuda.synchronize()
         print("suite2 done")
+    elif kind == "suite3":
+        # A whole LSTM layer, channels-last and short-contraction convolutions, a 16-bit product of few tiles, fp32 and fp64
+        # products, norm rows of one warp each and fp64 attention with its dS hand-over.
+        from .. import nn
+        from ..ops.attention import flash_attention
+        from ..ops.norm import rms_norm
+        bf = torch.bfloat16
+        for rep in range(2):
+            lstm = nn.LSTM(512, 512, device=dev)
+            lstm(torch.randn(32, 64, 512, device=dev, requires_grad=True)).sum().backward()
+            for ci, co, hw in ((64, 128, 15), (3, 64, 32)):
+                conv = nn.Conv2d(ci, co, 3, dtype=bf, device=dev)
+                conv(torch.randn(256, ci, hw, hw, device=dev, dtype=bf, requires_grad=ci > 3)).sum().backward()
+            gemm(torch.randn(77, 3072, device=dev, dtype=bf), torch.randn(768, 3072, device=dev, dtype=bf), trans_b=True)
+            gemm(torch.randn(3000, 1024, device=dev), torch.randn(4096, 1024, device=dev), trans_b=True)
+            a = torch.randn(2048, 2048, device=dev, dtype=torch.float64)
+            gemm(a, a)
+            x = torch.randn(65536, 768, device=dev, dtype=bf)
+            w, b = torch.randn(768, device=dev, dtype=bf), torch.randn(768, device=dev, dtype=bf)
+            layer_norm(x, w, b)
+            rms_norm(x, w)
+            q, k, v = (torch.randn(1, 2048, 16, 64, device=dev, dtype=torch.float64, requires_grad=True) for _ in range(3))
+            flash_attention(q, k, v, causal=True).sum().backward()
+            torch.cuda.synchronize()
+        print("suite3 done")
     elif kind == "step":
         n = int(argv[1]) // 8 * 8
         from ..distributed.nvlink import SymmetricMemory
