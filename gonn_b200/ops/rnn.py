@@ -105,37 +105,39 @@ PROJECTION_BYTES = 256 << 20
 
 
 def _lstm_forward(x, w_ih, b_ih, w_hh, h0, c0, tape: bool):
-    """(out (B, T, H), c, hprev, gates): with ``tape`` c and hprev are (B, T, H) and gates (B * T, 4H), what the backward reads;
-    without it c is the last cell state (B, H) and nothing else is kept."""
+    """(out (B, T, H), c, hprev, gates, x2): with ``tape`` c and hprev are (B, T, H), gates (B * T, 4H) and x2 the input's rows, what the
+    backward reads; without it c is the last cell state (B, H) and nothing else is kept."""
     from .gemm import gemm
     B, T, I = x.shape
     H = w_hh.shape[1]
+    steps = T if tape or 16 * B * T * H <= PROJECTION_BYTES else max(1, PROJECTION_BYTES // (16 * B * H))
+    # the product first: the rest of the host's work hides behind it
+    x2 = (x if steps == T else x[:, :steps]).reshape(B * steps, I)
+    xg = gemm(x2, w_ih, trans_b=True)
     dev, s = x.device, _l.stream_ptr()
     whh, h0, c0 = _aligned(w_hh.detach()), _aligned(h0), _aligned(c0)
     bias = b_ih.detach().contiguous() if b_ih is not None else None
     out = torch.empty((B, T, H), dtype=x.dtype, device=dev)
     xch = torch.empty(2 * B * H, dtype=torch.int64, device=dev)
-    steps = T if tape else max(1, min(T, PROJECTION_BYTES // (16 * B * H)))
-    hprev = torch.empty_like(out) if tape else None
-    c = torch.empty_like(out) if tape else torch.empty((B, H), dtype=x.dtype, device=dev)
-    xg = None
+    hprev = torch.empty((B, T, H), dtype=x.dtype, device=dev) if tape else None
+    c = torch.empty((B, T, H) if tape else (B, H), dtype=x.dtype, device=dev)
     for t in range(0, T, steps):
         n = min(steps, T - t)
-        xg = gemm(x[:, t:t + n].reshape(B * n, I), w_ih, trans_b=True,
-                  out=None if xg is None or n < steps else xg)
-        _l.call("gb_lstm_seq_fwd", _l.ptr(xg), _l.ptr(bias), _l.ptr(whh), _l.ptr(h0), _l.ptr(c0), _l.ptr(out[:, t]), _l.L(T * H),
-                _l.ptr(hprev), _l.ptr(c), _l.ptr(xch), _l.I(B), _l.I(n), _l.I(H), s)
+        if t > 0:
+            xg = gemm(x[:, t:t + n].reshape(B * n, I), w_ih, trans_b=True, out=xg if n == steps else None)
+        _l.call("gb_lstm_seq_fwd", _l.ptr(xg), _l.ptr(bias), _l.ptr(whh), _l.ptr(h0), _l.ptr(c0), _l.P(out.data_ptr() + 4 * t * H),
+                _l.L(T * H), _l.ptr(hprev), _l.ptr(c), _l.ptr(xch), _l.I(B), _l.I(n), _l.I(H), s)
         if t + n < T:
             h0, c0 = _aligned(out[:, t + n - 1]), c
-    return out, c, hprev, xg
+    return out, c, hprev, xg, x2
 
 
 class _LSTMSequence(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w_ih, b_ih, w_hh, h0, c0):
         # the backward reads h_{t-1} from a buffer of its own: the output belongs to the caller, who may change it in place
-        x2, c0 = x.reshape(-1, x.shape[2]), _aligned(c0)
-        out, cseq, hprev, act = _lstm_forward(x2.view(x.shape), w_ih, b_ih, w_hh, h0, c0, True)
+        c0 = _aligned(c0)
+        out, cseq, hprev, act, x2 = _lstm_forward(x, w_ih, b_ih, w_hh, h0, c0, True)
         ctx.save_for_backward(x2, w_ih, w_hh, c0, hprev, cseq, act)
         ctx.b_ih, ctx.xshape = b_ih, x.shape
         ctx.set_materialize_grads(False)
@@ -176,9 +178,17 @@ def lstm_sequence_fits(B: int, H: int) -> bool:
     return bool(_l.lib().gb_lstm_seq_fits(_l.I(B), _l.I(H)))
 
 
+def _transformed() -> bool:
+    """Forward-mode tangents, a function transform, tracing or compilation: these must see the autograd function."""
+    return bool(torch.autograd.forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None
+                or torch.jit.is_tracing() or torch.compiler.is_compiling())
+
+
 def lstm_sequence(x, w_ih, b_ih, w_hh, h0=None, c0=None):
     """(h_1 .. h_T (B, T, H), c_T (B, H)) of an fp32 LSTM layer over (B, T, I) on CUDA."""
-    if torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x, w_ih, b_ih, w_hh, h0, c0)):
+    if (torch.is_grad_enabled() and (x.requires_grad or w_ih.requires_grad or w_hh.requires_grad
+                                     or any(t is not None and t.requires_grad for t in (b_ih, h0, c0)))
+            or _transformed()):
         return _LSTMSequence.apply(x, w_ih, b_ih, w_hh, h0, c0)
     return _lstm_forward(x, w_ih, b_ih, w_hh, h0, c0, False)[:2]
 

@@ -149,3 +149,17 @@ def test_an_infinite_input_saturates_the_gates(value):
     with torch.no_grad():
         y = net(x)
     assert y.isfinite().all()
+
+
+def test_tangents_and_transforms_are_not_dropped_without_a_tape():
+    """Forward-mode tangents and vmap reach the autograd function, which refuses them, also where no gradient is recorded."""
+    net = nn.LSTM(12, 20, device="cuda")
+    x = torch.randn(3, 5, 12, device="cuda")
+    fw = torch.autograd.forward_ad
+    with torch.no_grad(), fw.dual_level():
+        with pytest.raises(Exception):
+            net(fw.make_dual(x, torch.ones_like(x)))
+    with torch.no_grad(), pytest.raises(Exception):
+        torch.func.vmap(net)(torch.randn(2, 3, 5, 12, device="cuda"))
+    with torch.no_grad():
+        assert net(x).isfinite().all()
