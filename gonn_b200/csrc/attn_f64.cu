@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_f64_kernel(const GArgs a) {
 
 // dQ = dS K from the dS^T that the dK / dV role left in memory: one product instead of three and the exponentials.  A
 // warp owns 16 queries; tiles of 32 keys, [key][query] and [key][column], pitch 4 mod 16: conflict-free fragments.
-// Bound by the fp64 pipe and the read of dS^T (268 MB at 16 heads of 2048, causal: backward 1507 -> 1092 us).
+// Bound by the fp64 pipe and the read of dS^T (268 MB at 16 heads of 2048, causal: backward 1438 -> 1024 us).
 template <int DT>
 struct DqShape {
   static constexpr int C = DT * 8, P = C + 4, ROWS = 64, PS = ROWS + 4, TK = 32;

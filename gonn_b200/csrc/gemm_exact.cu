@@ -44,7 +44,7 @@ enum { DT_BF16 = 0, DT_F16 = 1, DT_F32 = 2, DT_F64 = 3 };
 // ---------------------------------------------------------------------------
 // Bound by the fp64 tensor pipe (64 multiply-adds per SM and clock).  128 x 128 tiles of one 512-thread CTA kept
 // it 68 % active: half the stalls were shared-memory instructions (8-byte fragments and 8-byte copies) and the
-// barrier that all 16 warps share, and 256 such tiles leave 14 % of two waves empty at 2048^3 (790 us, now 571; 512^3 102, now 17).  Here a CTA
+// barrier that all 16 warps share, and 256 such tiles leave 14 % of two waves empty at 2048^3 (790 us, now 558; 512^3 102, now 17).  Here a CTA
 // is 64 x 64 x 16 with four warps of 32 x 32, four CTAs per SM that wait for nobody else's barrier, and
 //  * an operand whose contiguous dimension is k is staged as [8-wide k block][row][8]: 16-byte copies, and one
 //    16-byte read gives a lane the elements k = 2t and 2t + 1 of a row, which stand in the fragment's slots t and

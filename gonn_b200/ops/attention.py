@@ -86,7 +86,7 @@ def _general_call(mode, tensors, lse, delta, B, H, Tq, Tk, D, scale, causal, mas
 def _general_backward(ts, lse, delta, *common):
     """delta, dQ and dK / dV of the general kernels.  fp64 heads of up to 64 columns hand dS from the dK / dV kernel to the
     dQ kernel where memory (at most ``DS_SPILL_LIMIT_BYTES``) allows it and the problem is large enough for the coarser
-    blocks of that product.  Measured backward, us, with it | recomputing: 16 x 2048 x 64 causal 1092 | 1507, 16 x 2048 x 16 967 | 1369,
+    blocks of that product.  Measured backward, us, with it | recomputing: 16 x 2048 x 64 causal 1024 | 1438, 16 x 2048 x 16 971 | 1374,
     8 x 512 x 64 119 | 140, 2 x 1024 x 64 causal 178 | 201, 4 x 512 x 16 causal 79 | 71, 2 x 128 x 64 63 | 62."""
     B, H, Tq, Tk, D = common[:5]
     q = ts[0]
