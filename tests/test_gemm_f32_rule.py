@@ -52,3 +52,22 @@ def test_pieces(monkeypatch, ta, tb, bias, beta, batch):
     L.assert_status_ok()
     # every accumulator truncates 6 x 16 sums and every piece is rounded once: below 2^-20 together
     assert float((got.double().cpu() - want).norm() / want.norm()) < 2.0 ** -20
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,factor", [(1024, 1024, 1024, 1.0), (1024, 1024, 4096, 1.0), (3000, 4096, 1024, 2.0),
+                                          (2048, 2048, 2048, 3.0), (4096, 4096, 4096, 4.5)])
+def test_error_relative_to_the_fma_kernel(M, N, K, factor):
+    """One accumulator truncates K / 16 sums where an FMA chain rounds K: measured ratios on normal inputs 1.7 at K = 1024, 2.6 at
+    2048, 3.8 at 4096, and below 0.5 where few tiles cut K into slices."""
+    torch.manual_seed(K)
+    a, b = torch.randn(M, K, device="cuda"), torch.randn(K, N, device="cuda")
+    want = a.double() @ b.double()
+    err = {}
+    for mode in ("bf16x3", "simt"):
+        old = G.set_fp32_gemm_mode(mode)
+        try:
+            err[mode] = float((G.gemm(a, b).double() - want).norm() / want.norm())
+        finally:
+            G.set_fp32_gemm_mode(old)
+    assert err["bf16x3"] <= factor * err["simt"], err
