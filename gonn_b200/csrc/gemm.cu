@@ -88,13 +88,13 @@ struct Cfg {
 };
 
 // Dynamic shared memory of both kernels (the base must be 1024-byte aligned, which the
-// kernels check):  [operand ring] [epilogue staging: 2 x 2 KB per epilogue warp, 16-bit
-// path only] [512 B of barriers] [per-column epilogue constants, double buffered].
-template <int ESZ, int RING, int EW>
+// kernels check):  [operand ring] [epilogue staging: 2 x 2 KB per epilogue warp, not in the
+// one-CTA int8 kernel] [512 B of barriers] [per-column epilogue constants, double buffered].
+template <int ESZ, int RING, int EW, bool STAGED = ESZ == 2>
 struct SmemLayout {
   static constexpr int kStageBuf = 2048;  // 32 rows x 64 B, 64-byte swizzle
   static constexpr int OFF_STAGING = RING;
-  static constexpr int STAGING = ESZ == 2 ? EW * 2 * kStageBuf : 0;
+  static constexpr int STAGING = STAGED ? EW * 2 * kStageBuf : 0;
   static constexpr int OFF_BARS = OFF_STAGING + STAGING;
   static constexpr int OFF_COLS = OFF_BARS + 512;
   static constexpr int COL_BYTES = (ESZ == 1 ? 3 : 1) * 2 * 256 * 4;
@@ -225,6 +225,34 @@ __device__ __forceinline__ EpiCtx make_epi_ctx(const GemmArgs& args, int warp, i
   return c;
 }
 
+// The constants of a tile's columns into shared memory (double buffered by tile parity): bias, and for int8 scales and row sums.
+template <int ESZ, int BN, int EW>
+__device__ __forceinline__ void stage_columns(const GemmArgs& args, const EpiCtx& cx, int buf, int n0) {
+  for (int e = cx.et; e < BN; e += 32 * EW) {
+    const int col = n0 + e;
+    float bv = 0.f;
+    if (args.bias && col < args.N) {
+      if (args.bias_f32) bv = __ldg((const float*)args.bias + col);
+      else {
+        uint32_t u = __ldg((const uint16_t*)args.bias + col);
+        bv = args.in_bf16 ? __uint_as_float(u << 16) : __half2float(__ushort_as_half((unsigned short)u));
+      }
+    }
+    cx.s_bias[buf * 256 + e] = bv;
+    if (ESZ == 1) {
+      float sw = 1.f;
+      int rs = 0;
+      if (col < args.N) {
+        sw = args.q_per_channel ? __ldg(args.q_sw + col) : __ldg(args.q_sw);
+        rs = args.q_rowsum ? __ldg(args.q_rowsum + col) : 0;
+      }
+      cx.s_qsw[buf * 256 + e] = sw;
+      cx.s_qrs[buf * 256 + e] = rs;
+    }
+  }
+  asm volatile("bar.sync 1, %0;" ::"n"(32 * EW) : "memory");
+}
+
 // Epilogue of one 128-row x BN-column accumulator held in this CTA's TMEM at column
 // `tmem_acc`: everything that does not depend on the accumulator (bias, residual / saved
 // pre-activation) is fetched BEFORE waiting for the MMAs, so those latencies overlap the
@@ -235,7 +263,7 @@ __device__ __forceinline__ bool epilogue_tile(const GemmArgs& args, const EpiCtx
                                               volatile int* abort_flag) {
   constexpr int COLS = BN / (EW / 4);  // columns per thread per tile
   constexpr int NCH = COLS / 32;
-  const int q = cx.q, half = cx.half, et = cx.et, lane = cx.lane;
+  const int q = cx.q, half = cx.half, lane = cx.lane;
   const bool vec_ok = cx.vec_ok, aux_vec_ok = cx.aux_vec_ok, aux_in = cx.aux_in, has_cols = cx.has_cols;
   const float q_sx = cx.q_sx;
   const int q_zx = cx.q_zx;
@@ -246,32 +274,7 @@ __device__ __forceinline__ bool epilogue_tile(const GemmArgs& args, const EpiCtx
     const bool row_ok = row < args.M;
     const int cbase = n0 + half * COLS;  // first column of this thread
     // ---- per-column constants into shared memory (double buffered by tile parity) ----
-    if (has_cols) {
-      for (int e2 = et; e2 < BN; e2 += 32 * EW) {
-        const int et_ = e2;
-        const int col = n0 + et_;
-        float bv = 0.f;
-        if (args.bias && col < args.N) {
-          if (args.bias_f32) bv = __ldg((const float*)args.bias + col);
-          else {
-            uint32_t u = __ldg((const uint16_t*)args.bias + col);
-            bv = args.in_bf16 ? __uint_as_float(u << 16) : __half2float(__ushort_as_half((unsigned short)u));
-          }
-        }
-        s_bias[buf * 256 + et_] = bv;
-        if (ESZ == 1) {
-          float sw = 1.f;
-          int rs = 0;
-          if (col < args.N) {
-            sw = args.q_per_channel ? __ldg(args.q_sw + col) : __ldg(args.q_sw);
-            rs = args.q_rowsum ? __ldg(args.q_rowsum + col) : 0;
-          }
-          s_qsw[buf * 256 + et_] = sw;
-          s_qrs[buf * 256 + et_] = rs;
-        }
-      }
-      asm volatile("bar.sync 1, %0;" ::"n"(32 * EW) : "memory");
-    }
+    if (has_cols) stage_columns<ESZ, BN, EW>(args, cx, buf, n0);
     // ---- prefetch the first chunk of the auxiliary input (next chunks: one ahead) ----
     const bool aux_fast = aux_in && aux_vec_ok && row_ok && (cbase + COLS <= args.N);
     const uint4* aux_row = reinterpret_cast<const uint4*>(
@@ -474,7 +477,7 @@ struct EpiStage {
 // input (residual, saved pre-activation) arrives the same way, one chunk ahead, and the
 // result overwrites it in place.  With a second output (saved pre-activation) buffer 0 holds
 // the result and buffer 1 the pre-activation.
-template <int BN, int EW>
+template <int ESZ, int BN, int EW>
 __device__ __forceinline__ bool epilogue_tile_tma(const GemmArgs& args, const EpiCtx& cx, EpiStage& st,
                                                   const CUtensorMap* tmC, const CUtensorMap* tmX, int buf, int b,
                                                   int m0, int n0, uint32_t tmem_acc, uint64_t* tfull,
@@ -482,7 +485,7 @@ __device__ __forceinline__ bool epilogue_tile_tma(const GemmArgs& args, const Ep
   constexpr int COLS = BN / (EW / 4);
   constexpr int NCH = COLS / 32;
   static_assert(NCH % 2 == 0, "chunks alternate between two staging buffers");
-  const int q = cx.q, half = cx.half, et = cx.et, lane = cx.lane;
+  const int q = cx.q, half = cx.half, lane = cx.lane;
   float* s_bias = cx.s_bias;
   const int mrow0 = m0 + q * 32;
   const int cbase = n0 + half * COLS;
@@ -490,21 +493,7 @@ __device__ __forceinline__ bool epilogue_tile_tma(const GemmArgs& args, const Ep
   const bool aux_in = cx.aux_in;
   const bool two_out = args.aux_mode == AUX_STORE_PRE;
   const int out_bf = args.out_kind == OUT_BF16;
-  if (args.bias) {
-    for (int e2 = et; e2 < BN; e2 += 32 * EW) {
-      const int col = n0 + e2;
-      float bv = 0.f;
-      if (col < args.N) {
-        if (args.bias_f32) bv = __ldg((const float*)args.bias + col);
-        else {
-          uint32_t u = __ldg((const uint16_t*)args.bias + col);
-          bv = args.in_bf16 ? __uint_as_float(u << 16) : __half2float(__ushort_as_half((unsigned short)u));
-        }
-      }
-      s_bias[buf * 256 + e2] = bv;
-    }
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * EW) : "memory");
-  }
+  if (cx.has_cols) stage_columns<ESZ, BN, EW>(args, cx, buf, n0);
   const uint32_t sb0 = smem_u32(st.buf);
   const uint32_t myrow = (uint32_t)lane * 64u;
   const uint32_t swz = ((uint32_t)lane >> 1) & 3u;
@@ -525,8 +514,13 @@ __device__ __forceinline__ bool epilogue_tile_tma(const GemmArgs& args, const Ep
     if (!live || col0 >= args.N) continue;
     const int sc = buf * 256 + half * COLS + c * 32;
     float v[32];
+    if (ESZ == 1) {
 #pragma unroll
-    for (int j = 0; j < 32; j++) v[j] = __uint_as_float(rr[j]) * args.alpha;
+      for (int j = 0; j < 32; j++) v[j] = cx.q_sx * cx.s_qsw[sc + j] * (float)((int)rr[j] - cx.q_zx * cx.s_qrs[sc + j]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; j++) v[j] = __uint_as_float(rr[j]) * args.alpha;
+    }
     if (args.bias) {
 #pragma unroll
       for (int j = 0; j < 32; j++) v[j] += s_bias[sc + j];
@@ -834,7 +828,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const int m0 = u.mb * BM, n0 = u.nb * BN;
       bool done;
       if (ESZ == 2 && args.tma_epi)
-        done = epilogue_tile_tma<BN, EW>(args, cx, est, &tmC, &tmX, buf, b, m0, n0, tmem_base + buf * BN,
+        done = epilogue_tile_tma<ESZ, BN, EW>(args, cx, est, &tmC, &tmX, buf, b, m0, n0, tmem_base + buf * BN,
                                          &tfull_bar[buf], tphase[buf], abort_flag);
       else
         done = epilogue_tile<ESZ, BN, EW>(args, cx, buf, b, m0, n0, tmem_base + buf * BN, &tfull_bar[buf],
@@ -868,6 +862,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 // and a stage is 32 KB instead of 48 KB: six stages fit), and owns 128 rows of the
 // accumulator in its TMEM.  CTA 0 issues the MMAs for the pair.  Every TMA load is an
 // ordinary per-CTA load; nothing is broadcast across the cluster.
+// int8 has stages of the same bytes and twice the multiply-adds, so the one-CTA kernel's 48 KB per 128 x 256 x 128 step, 96
+// bytes a clock, was what bounded it: 8192 x 4096 x 4096 103 us (2 670 TOP/s), in pairs 79 us (3 470); 2048 x 4096 x 1024
+// 16.6 us.  Its column constants take the room of the sixth stage.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kPeerBit = 1u << 24;  // shared::cluster address bit that selects CTA 1 of a pair
 
@@ -909,6 +906,17 @@ __device__ __forceinline__ void tc_mma_f16_2sm(uint32_t d_tmem, uint64_t adesc, 
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+__device__ __forceinline__ void tc_mma_i8_2sm(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                              uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // arrive (when the issuing thread's earlier MMAs retire) on the barrier at a shared::cluster address
 __device__ __forceinline__ void tc_commit_2sm(uint32_t bar_addr) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_addr)
@@ -918,25 +926,26 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_addr) : "memory");
 }
 
+template <int ESZ>
 struct Cfg2 {
   static constexpr int BN = 256;                 // columns of the pair tile (each CTA stages 128 of them)
-  static constexpr int BK = 64;
-  static constexpr int UMMA_K = 16;
+  static constexpr int BK = kSwizzleBytes / ESZ;
+  static constexpr int UMMA_K = 32 / ESZ;
   static constexpr int A_BYTES = 128 * kSwizzleBytes;
   static constexpr int B_BYTES = 128 * kSwizzleBytes;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = 6;
+  static constexpr int STAGES = ESZ == 2 ? 6 : 5;
   static constexpr int RING_BYTES = STAGES * STAGE_BYTES;
   static constexpr int TMEM_COLS = 512;
 };
 
-template <bool A_MN, bool B_MN, int EW, bool PL>
+template <int ESZ, bool A_MN, bool B_MN, int EW, bool PL>
 __global__ void __launch_bounds__(64 + 32 * EW, 1)
 gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                          const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmX,
                          const GemmArgs args) {
-  using C = Cfg2;
-  using SL = SmemLayout<2, C::RING_BYTES, EW>;
+  using C = Cfg2<ESZ>;
+  using SL = SmemLayout<ESZ, C::RING_BYTES, EW, true>;
   extern __shared__ __align__(1024) uint8_t smem[];
   if (smem_u32(smem) & 1023u) {
     if (threadIdx.x == 0) set_status(args.status, ST_BAD_INDEX, 1024);
@@ -951,8 +960,8 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   uint64_t* aux_bar = bars + 32;               // [EW][2]   per CTA
   float* s_bias = (float*)(smem + SL::OFF_COLS);
-  float* s_qsw = s_bias;   // 8-bit constants are not used by this kernel
-  int* s_qrs = (int*)s_bias;
+  float* s_qsw = s_bias + 512;                 // 8-bit path only
+  int* s_qrs = (int*)(s_qsw + 512);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -1038,7 +1047,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
     if (cta == 0 && elect_one()) {
-      uint32_t id = make_idesc(1u, args.in_bf16 ? 1u : 0u, A_MN, B_MN, 256, 256);
+      const uint32_t id = make_idesc(ESZ == 1 ? 2u : 1u, ESZ == 1 || args.in_bf16 ? 1u : 0u, A_MN, B_MN, 256, 256);
       int stage = 0;
       uint32_t phase = 0;
       uint32_t tphase[2] = {0, 0};
@@ -1068,7 +1077,8 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
             const uint64_t bdesc =
                 B_MN ? make_smem_desc_sw128(sb + k * C::UMMA_K * kSwizzleBytes, C::BK * kSwizzleBytes, 1024)
                      : make_smem_desc_sw128(sb + k * 32, 16, 1024);
-            tc_mma_f16_2sm(d_tmem, adesc, bdesc, id, (kb > kb_begin) || k != 0);
+            if (ESZ == 1) tc_mma_i8_2sm(d_tmem, adesc, bdesc, id, (kb > kb_begin) || k != 0);
+            else tc_mma_f16_2sm(d_tmem, adesc, bdesc, id, (kb > kb_begin) || k != 0);
           }
           // free the stage in both CTAs
           const uint32_t eb = smem_u32(&empty_bar[stage]);
@@ -1086,7 +1096,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     __syncwarp();
   } else {
     // ---------------- epilogue: this CTA's 128 rows x 256 columns ----------------
-    const EpiCtx cx = make_epi_ctx<2>(args, warp, lane, threadIdx.x - 64, s_bias, s_qsw, s_qrs);
+    const EpiCtx cx = make_epi_ctx<ESZ>(args, warp, lane, threadIdx.x - 64, s_bias, s_qsw, s_qrs);
     EpiStage est;
     est.buf = smem + SL::OFF_STAGING + (warp - 2) * 2 * SL::kStageBuf;
     est.bar = aux_bar + (warp - 2) * 2;
@@ -1101,10 +1111,10 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       const int m0 = u.mb * 256 + (int)cta * 128, n0 = u.nb * 256;
       bool done;
       if (args.tma_epi)
-        done = epilogue_tile_tma<256, EW>(args, cx, est, &tmC, &tmX, buf, b, m0, n0, tmem_base + buf * 256,
+        done = epilogue_tile_tma<ESZ, 256, EW>(args, cx, est, &tmC, &tmX, buf, b, m0, n0, tmem_base + buf * 256,
                                           &tfull_bar[buf], tphase[buf], abort_flag);
       else
-        done = epilogue_tile<2, 256, EW>(args, cx, buf, b, m0, n0, tmem_base + buf * 256, &tfull_bar[buf],
+        done = epilogue_tile<ESZ, 256, EW>(args, cx, buf, b, m0, n0, tmem_base + buf * 256, &tfull_bar[buf],
                                          tphase[buf], abort_flag);
       if (!done) {
         ok = false;
@@ -1639,10 +1649,10 @@ int dispatch_major(bool a_mn, bool b_mn, const TMaps& tm, const GemmArgs& args, 
 
 int g_use_2cta = 1;
 
-template <bool A_MN, bool B_MN, bool PL>
+template <int ESZ, bool A_MN, bool B_MN, bool PL>
 int launch_2cta_t(const TMaps& tm, const GemmArgs& args, int num_sms, cudaStream_t stream) {
-  using SL = SmemLayout<2, Cfg2::RING_BYTES, 8>;
-  auto kern = gemm_tcgen05_2cta_kernel<A_MN, B_MN, 8, PL>;
+  using SL = SmemLayout<ESZ, Cfg2<ESZ>::RING_BYTES, 8, true>;
+  auto kern = gemm_tcgen05_2cta_kernel<ESZ, A_MN, B_MN, 8, PL>;
   static bool configured = false;
   if (!configured) {
     GB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SL::BYTES));
@@ -1670,8 +1680,8 @@ int launch_2cta_t(const TMaps& tm, const GemmArgs& args, int num_sms, cudaStream
 
 template <bool A_MN, bool B_MN>
 int launch_2cta(const TMaps& tm, const GemmArgs& args, int num_sms, cudaStream_t stream) {
-  return args.planes > 0 ? launch_2cta_t<A_MN, B_MN, true>(tm, args, num_sms, stream)
-                         : launch_2cta_t<A_MN, B_MN, false>(tm, args, num_sms, stream);
+  return args.planes > 0 ? launch_2cta_t<2, A_MN, B_MN, true>(tm, args, num_sms, stream)
+                         : launch_2cta_t<2, A_MN, B_MN, false>(tm, args, num_sms, stream);
 }
 
 thread_local int g_cluster_splits = 0;   // 0: by the rule of cluster_splits(); -1: off; 1, 2, 4, 8: that many CTAs per tile
@@ -1833,7 +1843,7 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
   // two-CTA 256 x 256 tiles when they fill at least four fifths of the SM pairs (measured at 2048^3: 64 pair
   // tiles on 74 pairs beat 128 one-CTA tiles on 148 SMs by 8 %); force_bn == 512 forces them
   bool use2 = false;
-  if (esz == 2) {
+  {
     long long pair_tiles = (long long)((M + 255) / 256) * ((N + 255) / 256) * batch;
     // measured: the pair kernel wins when the main loop dominates (long K, or a plain
     // epilogue); with short K and a heavy epilogue the one-CTA kernel is slightly ahead
@@ -1898,7 +1908,7 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
   // (and the auxiliary tensor) can be described by a tensor map and nothing is accumulated.
   args.tma_epi = 0;
   const bool f32_out = args.out_kind == OUT_F32;
-  if (esz == 2 && g_tma_epi && !cluster && !args.beta && !(f32_out && (args.act != ACT_NONE || args.aux_mode != AUX_NONE))) {
+  if ((esz == 2 || use2) && g_tma_epi && !cluster && !args.beta && !(f32_out && (args.act != ACT_NONE || args.aux_mode != AUX_NONE))) {
     const int osz = f32_out ? 4 : 2;
     auto mappable = [&](const void* p, long long ld, long long bs) {
       return (((uintptr_t)p & 15) == 0) && (ld * osz % 16 == 0) && (bs * osz % 16 == 0);
@@ -1968,7 +1978,8 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
     return launch_cluster<true, true>(tm, args, stream);
   }
   if (use2) {
-    if (!a_mn && !b_mn) rc = launch_2cta<false, false>(tm, args, g_num_sms, stream);
+    if (esz == 1) rc = launch_2cta_t<1, false, false, false>(tm, args, g_num_sms, stream);
+    else if (!a_mn && !b_mn) rc = launch_2cta<false, false>(tm, args, g_num_sms, stream);
     else if (!a_mn && b_mn) rc = launch_2cta<false, true>(tm, args, g_num_sms, stream);
     else if (a_mn && !b_mn) rc = launch_2cta<true, false>(tm, args, g_num_sms, stream);
     else rc = launch_2cta<true, true>(tm, args, g_num_sms, stream);

@@ -199,6 +199,23 @@ class _QLinearCore:
             else torch.empty((M, st["kp"]), dtype=torch.int8, device=x.device)
         _l.call("gb_q_quantize", _l.I(_l.dtype_code(x.dtype)), _l.ptr(x2), _l.ptr(xq), _l.L(M), _l.L(self.in_features),
                 _l.L(st["kp"]), _l.ptr(qp4[2:]), _l.ptr(zp), _l.I(0), _l.stream_ptr())
+        return self._product(x, xq, qp4, zp, st)
+
+    def forward_dynamic(self, x: torch.Tensor) -> torch.Tensor:
+        """The same with the q-parameters of ``x`` itself: one pass that observes, one that quantises."""
+        st = self._device_state(x.device)
+        x2 = x.reshape(-1, self.in_features).contiguous()
+        M = x2.shape[0]
+        xq = torch.empty((M, st["kp"]), dtype=torch.int8, device=x.device)
+        n = _l.lib().gb_q_scratch_floats()
+        scratch = torch.empty(n + 5, dtype=torch.float32, device=x.device)    # partial results, {min, max, scale, zp}, zp (int32)
+        qp4, zp = scratch[n:n + 4], scratch[n + 4:]
+        _l.call("gb_q_dynamic", _l.I(_l.dtype_code(x.dtype)), _l.ptr(x2), _l.ptr(xq), _l.L(M), _l.L(self.in_features),
+                _l.L(st["kp"]), _l.ptr(scratch), _l.ptr(qp4), _l.ptr(zp), _l.stream_ptr())
+        return self._product(x, xq, qp4, zp, st)
+
+    def _product(self, x, xq, qp4, zp, st):
+        M = xq.shape[0]
         out_dt = x.dtype if x.dtype in (torch.bfloat16, torch.float16) else torch.float32
         y = torch.empty((M, self.out_features), dtype=out_dt, device=x.device)
         _l.call("gb_gemm_i8", _l.ptr(xq), _l.ptr(st["wq"]), _l.ptr(y), _l.ptr(st["b"]), _l.I(M), _l.I(self.out_features),
@@ -233,8 +250,7 @@ class DynamicLinear(Module):
     @torch.no_grad()
     def forward(self, x):
         if _native(x):
-            qp4, zp = _observe_device(x)
-            return self.core.forward_device(x, qp4, zp)
+            return self.core.forward_dynamic(x)
         sx, zx = affine_qparams(float(x.min()), float(x.max()))
         return self.core.forward_host(x, sx, zx)
 

@@ -3,6 +3,7 @@ against the host restatement of the reference's integer loop."""
 import pytest
 import torch
 
+from gonn_b200 import lib as _l
 from gonn_b200 import quant as Q
 from gonn_b200.nn import Linear
 
@@ -10,7 +11,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("per_channel", [False, True])
-@pytest.mark.parametrize("shape", [(64, 128, 96), (300, 200, 130), (1024, 768, 3072)])
+@pytest.mark.parametrize("shape", [(64, 128, 96), (300, 200, 130), (1024, 768, 3072),
+                                   (2300, 400, 2312), (2300, 400, 2311), (2049, 16, 2304)])   # two-CTA tiles: ragged edges, unaligned rows, one k-block
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_dynamic_linear_matches_integer_reference(per_channel, shape, dtype, status_ok):
     M, K, N = shape
@@ -59,3 +61,31 @@ def test_fake_quant_kernel_matches_host(status_ok):
     yd.backward(g.cuda())
     yh.backward(g.double())
     assert (xd.grad.double().cpu() - xh.grad).abs().max().item() < 1e-6
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape", [(1, 1), (3, 5), (7, 16), (64, 256), (513, 1531), (2000, 1024)])
+@pytest.mark.parametrize("offset", [0, 1])     # 1: rows that are not 16-byte aligned
+def test_dynamic_quantisation_bytes(dtype, shape, offset, status_ok):
+    """One call that observes and quantises leaves the bytes of the two calls, zeros in the padding, and follows the rule of
+    the reference (halves away from zero) wherever x / scale is exact: steps of a half and a range of 255 make the scale 1."""
+    M, K = shape
+    pitch = (K + 15) // 16 * 16
+    torch.manual_seed(M)
+    flat = torch.randint(-256, 255, (M * K + offset,)).double() / 2
+    if M * K >= 2:
+        flat[offset], flat[-1] = -128.0, 127.0
+    x = flat.to("cuda", dtype)[offset:].view(M, K)
+    scratch = torch.empty(_l.lib().gb_q_scratch_floats(), device="cuda")
+    qp, zp = torch.empty(4, device="cuda"), torch.empty(1, dtype=torch.int32, device="cuda")
+    q = torch.full((M, pitch), 77, dtype=torch.int8, device="cuda")
+    _l.call("gb_q_dynamic", _l.I(_l.dtype_code(dtype)), _l.ptr(x), _l.ptr(q), _l.L(M), _l.L(K), _l.L(pitch), _l.ptr(scratch),
+            _l.ptr(qp), _l.ptr(zp), _l.stream_ptr())
+    qp2, zp2 = Q._observe_device(x)
+    q2 = torch.zeros((M, pitch), dtype=torch.int8, device="cuda")
+    _l.call("gb_q_quantize", _l.I(_l.dtype_code(dtype)), _l.ptr(x), _l.ptr(q2), _l.L(M), _l.L(K), _l.L(pitch), _l.ptr(qp2[2:]),
+            _l.ptr(zp2), _l.I(0), _l.stream_ptr())
+    assert torch.equal(q, q2) and torch.equal(qp, qp2) and torch.equal(zp, zp2)
+    if M * K >= 2:
+        assert qp[2].item() == 1.0 and zp.item() == 0
+        assert torch.equal(q[:, :K].cpu(), Q.quantize_value(flat[offset:].view(M, K), 1.0, 0).to(torch.int8))
