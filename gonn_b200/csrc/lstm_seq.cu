@@ -10,16 +10,18 @@
 //  * sequences are independent, so only the CTAs of one group wait for one another.  Forward: h_t travels as 64-bit
 //    words {value, step + 1} in a buffer of two steps by turns; a reader loads the words it needs and repeats those whose
 //    step is not there yet, so that no flag, fence or second round trip stands between a product and the next (a flag
-//    per CTA with release semantics: 6.3 us a step, this 4.2).  A word of step t is overwritten by step t + 2, whose writer
-//    has read step t + 1 from every CTA of its group, and each of those had read step t before.  Backward (four
-//    times the data): H / UT flags per group, one per CTA, stored with release semantics after the CTA's part of
-//    dgates_t is written, all polled by one warp;
+//    per CTA with release semantics: 6.3 us a step).  A warp receives the part of h that its share of the contraction needs
+//    and starts on it at once (4.2 -> 3.8 us against a barrier behind the whole of h).  A word of step t is overwritten by
+//    step t + 2, whose writer has read step t + 1 from every CTA of its group, and each of those had read step t before.
+//    Backward: the sums of dh_t travel the same way (lstm_seq_bwd_scatter_kernel); where their words would take too much
+//    memory, dgates_t are gathered (four times the data) behind H / UT flags per group, one per CTA, stored with release
+//    semantics after the CTA's part of dgates_t is written, all polled by one warp;
 //  * within a CTA the eight warps split the contraction, a lane accumulates 4 x 4 outputs with packed
 //    fp32 multiply-adds, and the partial sums meet in shared memory in a fixed order (deterministic);
 //  * the cell state never leaves the thread that owns it except to be saved for the backward.
 // The input projections of all steps, the weight gradients and the input gradient are single
-// GEMMs outside (ops/rnn.py).  Measured at B = 32, T = 64, H = 512: 267 us forward (4.2 us a step) and
-// 475 us backward (7.4 us a step); at H = 64 a step is 2.6 us, which is the exchange alone.
+// GEMMs outside (ops/rnn.py).  Measured at B = 32, T = 64, H = 512: 244 us forward (3.8 us a step, 1.1 of it the multiply-adds)
+// and 256 us backward (4.0); at H = 64 a step is 2.0 and 1.5 us, which is the exchange alone.
 //
 // Waiting CTAs need one another to be resident: cooperative launches only.  Every wait is bounded.
 #include "common.cuh"
@@ -101,9 +103,9 @@ __device__ __forceinline__ bool wait_group(const unsigned int* flags, int n, uns
 // a: kMB rows, w: N rows, both K floats with pitch K + 4 (16-byte rows four banks apart, so that the
 // 16-byte reads of eight neighbouring rows touch all banks once).  Lanes: two groups of four a-rows
 // x N/4 groups of w-rows (w row = i * N/4 + group: neighbouring lanes, neighbouring rows) x KQ
-// slices of the contraction.  part[warp][kMB * N] receives the warp's partial sums.
+// slices of the warp's part k0 .. k1 of the contraction.  part[warp][kMB * N] receives the warp's partial sums.
 template <int N>
-__device__ __forceinline__ void product(const float* __restrict__ a, const float* __restrict__ w, int K,
+__device__ __forceinline__ void product(const float* __restrict__ a, const float* __restrict__ w, int K, int k0, int k1,
                                         float* __restrict__ part) {
   constexpr int NG = N / 4;                  // groups of w-rows
   constexpr int KQ = 32 / (2 * NG);          // lanes that share a group pair and split k
@@ -119,7 +121,7 @@ __device__ __forceinline__ void product(const float* __restrict__ a, const float
 #pragma unroll
     for (int j = 0; j < 4; j++) acc[i][j] = 0ull;
 #pragma unroll 2
-  for (int k = (warp * KQ + kq) * 4; k < K; k += kWarps * KQ * 4) {
+  for (int k = k0 + kq * 4; k < k1; k += KQ * 4) {
     ulonglong2 av[4], wv[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) av[i] = *reinterpret_cast<const ulonglong2*>(ap + i * pitch + k);
@@ -159,18 +161,21 @@ __device__ __forceinline__ void load_tile(float* __restrict__ tile, const float*
   cp_async_wait_all();
 }
 
-// h of the step whose words carry `step` (its index + 1), rows b0 .. b0 + kMB - 1, into the tile; rows past B are zero.  False when
-// the budget of the wait ran out (for any thread of the CTA: ends with a barrier).
-__device__ __forceinline__ bool receive_tile(float* __restrict__ tile, const unsigned long long* __restrict__ xch, unsigned step, int H,
-                                             int b0, int B, int* abort_flag, int* status) {
+// The part k0 .. k1 (multiples of four) of h of the step whose words carry `step` (its index + 1), rows b0 .. b0 + kMB - 1, into the
+// tile, by one warp, which alone reads it: no barrier stands between the words and its product, and no warp waits for words of
+// another's part.  Rows past B are zero.  Gives up when the budget of the wait has run out for any thread of the CTA.
+__device__ __forceinline__ void receive_part(float* __restrict__ tile, const unsigned long long* __restrict__ xch, unsigned step, int H,
+                                             int k0, int k1, int b0, int B, int* abort_flag, int* status) {
   constexpr int U = 8;
-  const int h2 = H / 2, pitch = H + 4, total = kMB * h2;
-  for (int i0 = threadIdx.x; i0 < total; i0 += kThreads * U) {
+  const int h2 = (k1 - k0) / 2, pitch = H + 4, total = kMB * h2, lane = threadIdx.x & 31;
+  for (int i0 = lane; i0 < total; i0 += 32 * U) {
     unsigned long long w[U][2];
+    int at[U];                                     // row << 16 | column
     unsigned todo = 0;
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      const int i = i0 + u * kThreads, r = i / h2;
+      const int i = i0 + u * 32, r = i / h2;
+      at[u] = r << 16 | (k0 + 2 * (i - r * h2));
       if (i < total && b0 + r < B) todo |= 1u << u;
     }
     const unsigned mine = todo;
@@ -179,8 +184,7 @@ __device__ __forceinline__ bool receive_tile(float* __restrict__ tile, const uns
 #pragma unroll
       for (int u = 0; u < U; u++)
         if (todo >> u & 1u) {
-          const int i = i0 + u * kThreads, r = i / h2;
-          const unsigned long long* src = xch + (long long)(b0 + r) * H + 2 * (i - r * h2);
+          const unsigned long long* src = xch + (long long)(b0 + (at[u] >> 16)) * H + (at[u] & 0xffff);
           asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(w[u][0]), "=l"(w[u][1]) : "l"(src) : "memory");
         }
 #pragma unroll
@@ -197,17 +201,14 @@ __device__ __forceinline__ bool receive_tile(float* __restrict__ tile, const uns
       }
     }
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int i = i0 + u * kThreads, r = i / h2;
-      if (i < total) {
+    for (int u = 0; u < U; u++)
+      if (i0 + u * 32 < total) {
         const float2 v = mine >> u & 1u ? make_float2(__uint_as_float((unsigned)w[u][0]), __uint_as_float((unsigned)w[u][1]))
                                         : make_float2(0.f, 0.f);
-        *reinterpret_cast<float2*>(tile + r * pitch + 2 * (i - r * h2)) = v;
+        *reinterpret_cast<float2*>(tile + (at[u] >> 16) * pitch + (at[u] & 0xffff)) = v;
       }
-    }
   }
-  __syncthreads();
-  return *(volatile int*)abort_flag == 0;
+  __syncwarp();
 }
 
 // grid: (ug, groups).  UT units per CTA: N = 4 UT weight rows, row n = gate * UT + unit.  TAPE: a backward follows (a template
@@ -220,7 +221,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_fwd_kernel(const SeqArgs
   const int H = p.H, T = p.T, pitch = H + 4;
   float* ws = sm;                                  // [N][H + 4]
   float* hs = ws + N * pitch;                      // [kMB][H + 4]
-  float* part = hs + kMB * pitch;                  // [kWarps][kMB * N]
+  float* parts = hs + kMB * pitch;                 // [2][kWarps][kMB * N], by turns: a warp may be a product ahead of the cells
   const int u0 = blockIdx.x * UT;
   const int bg0 = blockIdx.y * p.sub * kMB;
   if (threadIdx.x == 0) abort_flag = 0;
@@ -235,13 +236,16 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_fwd_kernel(const SeqArgs
   const int cell_m = threadIdx.x / UT, cell_u = threadIdx.x % UT;      // the cell of threads 0 .. kMB * UT - 1
   const int u = u0 + cell_u;
   const bool cell = threadIdx.x < kMB * UT && u < H;
+  const int kper = (H / 4 + kWarps - 1) / kWarps * 4, k0 = min(H, (int)(threadIdx.x >> 5) * kper), k1 = min(H, k0 + kper);   // of this warp
   float bias[4] = {0.f, 0.f, 0.f, 0.f};
   if (cell && p.bias != nullptr) {
 #pragma unroll
     for (int g = 0; g < 4; g++) bias[g] = p.bias[g * H + u];
   }
+  int turn = 0;
   for (int t = 0; t < T; t++) {
     for (int s = 0; s < p.sub; s++) {
+      float* part = parts + (turn ^= 1) * (kWarps * kMB * N);
       const int b0 = bg0 + s * kMB, b = b0 + cell_m;
       const bool mine = cell && b < p.B;
       const long long row = (long long)b * T + t;
@@ -253,13 +257,14 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_fwd_kernel(const SeqArgs
       }
       if (t > 0 || p.h0 != nullptr) {
         if (t > 0) {
-          if (!receive_tile(hs, p.xch + (long long)((t - 1) & 1) * p.B * H, (unsigned)t, H, b0, p.B, &abort_flag, p.status)) return;
+          receive_part(hs, p.xch + (long long)((t - 1) & 1) * p.B * H, (unsigned)t, H, k0, k1, b0, p.B, &abort_flag, p.status);
         } else {
           load_tile(hs, p.h0, H, H, b0, p.B);
           __syncthreads();
         }
-        product<N>(hs, ws, H, part);
+        product<N>(hs, ws, H, k0, k1, part);
         __syncthreads();
+        if (*(volatile int*)&abort_flag != 0) return;
         if (mine) {
 #pragma unroll
           for (int g = 0; g < 4; g++) {
@@ -319,6 +324,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_bwd_kernel(const SeqArgs
       dcs[s * (kMB * N) + threadIdx.x] = (cell && b < p.B && p.dcn != nullptr) ? p.dcn[(long long)b * H + u] : 0.f;
   }
   __syncthreads();
+  const int kper = (K / 4 + kWarps - 1) / kWarps * 4;
   for (int t = T - 1; t >= 0; t--) {
     const bool chain = t < T - 1;
     if (chain && !wait_group(flags, p.ug, (unsigned)(T - 1 - t), &abort_flag, p.status)) return;
@@ -337,7 +343,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_bwd_kernel(const SeqArgs
       if (chain) {
         load_tile(ds, p.dgates + (long long)(t + 1) * K, (long long)T * K, K, b0, p.B);
         __syncthreads();
-        product<N>(ds, ws, K, part);
+        product<N>(ds, ws, K, min(K, (int)(threadIdx.x >> 5) * kper), min(K, ((int)(threadIdx.x >> 5) + 1) * kper), part);
         __syncthreads();
         if (mine) {
           float v = 0.f;
@@ -364,6 +370,170 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_bwd_kernel(const SeqArgs
   }
 }
 
+// The same chain with the exchange turned round.  The kernel above gathers all of dgates_{t+1} (4H values a sequence) in every CTA.
+// Here a CTA multiplies only the dgates of its own UT units, by the 4 UT rows of W_hh that belong to them, and sends every other
+// CTA the UT sums of dh_t that it owns: H values a sequence and CTA instead of 4H, in 64-bit words {value, step} as forward, so
+// that neither a flag nor a second round trip stands between two steps.  A CTA adds what the others sent in their order.  Slots
+// go by turns: a word of step t is overwritten by step t - 2, whose writer has the sums of step t - 1 from every CTA of its
+// group, and each of those had added up step t before it sent them.
+// us a step of 64, gathered | scattered: B = 32, H = 512 7.3 | 4.0; 32, 128 3.3 | 1.7; 4, 64 2.4 | 1.5; 8, 256 3.8 | 1.9;
+// 128, 512 24.8 | 14.4; 512, 512 86.8 | 64.2.
+// U: words in flight per thread, the senders of a cell that one thread adds up (16 at H = 512: 278 -> 256 us for 64 steps; more
+// than there are costs 5 %).  grid: (ug, groups).  Words: [slot][sub-tile][receiver][sender][kMB * UT].
+template <int UT, int U>
+__global__ void __launch_bounds__(kThreads, 1) lstm_seq_bwd_scatter_kernel(const SeqArgs p) {
+  constexpr int K = 4 * UT, pitch = K + 4, CELLS = kMB * UT;
+  constexpr int PARTS = kThreads / CELLS;          // threads that share the senders of one cell
+  extern __shared__ __align__(16) float sm[];
+  __shared__ int abort_flag;
+  const int H = p.H, T = p.T, H4 = 4 * H;
+  float* ws = sm;                                  // [H][K + 4]: W_hh of this CTA's gate rows, k = gate * UT + unit
+  float* ds = ws + (long long)H * pitch;           // [kMB][K + 4]: dgates_t of this CTA's units
+  float* part = ds + kMB * pitch;                  // [PARTS][CELLS]
+  float* dcs = part + kThreads;                    // [sub][CELLS]: dc carried from step to step
+  const int u0 = blockIdx.x * UT, ug = p.ug;
+  const int bg0 = blockIdx.y * p.sub * kMB;
+  if (threadIdx.x == 0) abort_flag = 0;
+  for (int i = threadIdx.x; i < K * H; i += kThreads) {
+    const int k = i / H, n = i - k * H, g = k / UT, uu = u0 + (k - g * UT);
+    ws[n * pitch + k] = uu < H ? p.w[((long long)g * H + uu) * H + n] : 0.f;
+  }
+  const int cell_i = threadIdx.x % CELLS, pt = threadIdx.x / CELLS;
+  const int cell_m = cell_i / UT, cell_u = cell_i % UT, u = u0 + cell_u;
+  for (int s = 0; s < p.sub; s++) {
+    const int b = bg0 + s * kMB + cell_m;
+    if (pt == 0) dcs[s * CELLS + cell_i] = (u < H && b < p.B && p.dcn != nullptr) ? p.dcn[(long long)b * H + u] : 0.f;
+  }
+  __syncthreads();
+  const int ng_all = H / 4;
+  const int lane = threadIdx.x & 31;
+  const int per = (ug + PARTS - 1) / PARTS, src0 = pt * per, src1 = min(ug, src0 + per);
+  const long long slot_words = (long long)gridDim.y * p.sub * ug * ug * CELLS;
+  for (int t = T - 1; t >= 0; t--) {
+    for (int s = 0; s < p.sub; s++) {
+      const int b0 = bg0 + s * kMB, b = b0 + cell_m;
+      const bool live = u < H && b < p.B, mine = live && pt == 0;
+      const long long row = (long long)b * T + t;
+      unsigned long long* words = p.xch + ((long long)blockIdx.y * p.sub + s) * ug * ug * CELLS;
+      float dh = 0.f, ig = 0.f, fg = 0.f, gg = 0.f, og = 0.f, ct = 0.f, cp = 0.f;
+      if (mine) {                                  // in flight while the words arrive
+        const float* a = p.act + row * H4 + u;
+        ig = __ldg(a); fg = __ldg(a + H); gg = __ldg(a + 2 * H); og = __ldg(a + 3 * H);
+        ct = __ldg(p.cseq + row * H + u);
+        cp = t > 0 ? __ldg(p.cseq + (row - 1) * H + u) : (p.c0 != nullptr ? p.c0[(long long)b * H + u] : 0.f);
+        if (p.dout != nullptr) dh = __ldg(p.dout + row * H + u);
+      }
+      if (t < T - 1) {
+        const unsigned long long* in = words + ((t + 1) & 1) * slot_words + (long long)blockIdx.x * ug * CELLS + cell_i;
+        const unsigned step = (unsigned)(T - 1 - t);
+        float v = 0.f;
+        for (int s0 = src0; s0 < src1; s0 += U) {
+          unsigned long long w[U];
+          unsigned todo = live ? (src1 - s0 >= U ? (1u << U) - 1 : (1u << (src1 - s0)) - 1) : 0u;
+          const unsigned all = todo;
+          uint64_t t0 = 0;
+          for (uint32_t spins = 0; todo != 0; spins++) {
+#pragma unroll
+            for (int i = 0; i < U; i++)
+              if (todo >> i & 1u)
+                asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(w[i]) : "l"(in + (long long)(s0 + i) * CELLS) : "memory");
+#pragma unroll
+            for (int i = 0; i < U; i++)
+              if ((unsigned)(w[i] >> 32) == step) todo &= ~(1u << i);
+            if (todo != 0 && (spins & 0xFF) == 0xFF) {
+              if (t0 == 0) t0 = globaltimer_ns();
+              if (*(volatile int*)&abort_flag) break;
+              if (globaltimer_ns() - t0 > kWaitBudgetNs) {
+                *(volatile int*)&abort_flag = 1;
+                set_status(p.status, ST_RNN_TIMEOUT, (int)step);
+                break;
+              }
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < U; i++)
+            if (all >> i & 1u) v += __uint_as_float((unsigned)w[i]);
+        }
+        part[threadIdx.x] = v;
+        __syncthreads();
+        if (*(volatile int*)&abort_flag != 0) return;
+        if (mine) {
+          v = 0.f;
+#pragma unroll
+          for (int i = 0; i < PARTS; i++) v += part[i * CELLS + cell_i];
+          dh += v;
+        }
+      } else if (s > 0) {
+        __syncthreads();                           // the product of the sub-tile before has read ds
+      }
+      if (pt == 0) {
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+        if (mine) {
+          const float tc = tanhf(ct);
+          float* dcv = dcs + s * CELLS + cell_i;
+          const float dc = *dcv + dh * og * (1.f - tc * tc);
+          d[0] = dc * gg * ig * (1.f - ig);
+          d[1] = dc * cp * fg * (1.f - fg);
+          d[2] = dc * ig * (1.f - gg * gg);
+          d[3] = dh * tc * og * (1.f - og);
+          *dcv = dc * fg;
+          if (t == 0 && p.dc0 != nullptr) p.dc0[(long long)b * H + u] = dc * fg;
+        }
+#pragma unroll
+        for (int g = 0; g < 4; g++) ds[cell_m * pitch + g * UT + cell_u] = d[g];
+        if (mine) {
+          float* o = p.dgates + row * H4 + u;
+#pragma unroll
+          for (int g = 0; g < 4; g++) o[g * H] = d[g];
+        }
+      }
+      __syncthreads();
+      if (t == 0) continue;
+      unsigned long long* out = words + (t & 1) * slot_words + (long long)blockIdx.x * CELLS;
+      const unsigned long long tag = (unsigned long long)(unsigned)(T - t) << 32;
+      // a lane takes 4 x 4 sums over all k (lanes that split the contraction cost more in shuffles than they saved, at any H):
+      // rows 4 mg .., columns ng + j H / 4, a warp 16 neighbouring columns of all eight rows
+      const int mg = lane >> 4;
+      for (int ng = (threadIdx.x >> 5) * 16 + (lane & 15); ng < ng_all; ng += kWarps * 16) {
+        const float* ap = ds + mg * 4 * pitch;
+        const float* wp = ws + ng * pitch;
+        unsigned long long acc[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) acc[i][j] = 0ull;
+#pragma unroll 4
+        for (int k = 0; k < K; k += 4) {
+          ulonglong2 av[4], wv[4];
+#pragma unroll
+          for (int i = 0; i < 4; i++) av[i] = *reinterpret_cast<const ulonglong2*>(ap + i * pitch + k);
+#pragma unroll
+          for (int j = 0; j < 4; j++) wv[j] = *reinterpret_cast<const ulonglong2*>(wp + j * ng_all * pitch + k);
+#pragma unroll
+          for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+              ffma2(acc[i][j], av[i].x, wv[j].x);
+              ffma2(acc[i][j], av[i].y, wv[j].y);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const int n = j * ng_all + ng, dest = n / UT;
+          unsigned long long* o = out + (long long)dest * ug * CELLS + (n - dest * UT);
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            const float v = __uint_as_float((unsigned)(acc[i][j] & 0xffffffffull)) + __uint_as_float((unsigned)(acc[i][j] >> 32));
+            const int m = mg * 4 + i;
+            if (b0 + m < p.B)
+              asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(o + m * UT), "l"((unsigned long long)__float_as_uint(v) | tag) : "memory");
+          }
+        }
+      }
+    }
+  }
+}
+
 constexpr int kSms = 148;       // of a whole B200; also the words of the flags' scratch
 // SMs of the current device: all CTAs of a cooperative launch need one each.  (No device, as in host-side tests: a whole B200.)
 int device_sms() {
@@ -379,12 +549,23 @@ constexpr long long kMaxSmem = 227 * 1024 - 16;      // what a block may take, l
 // step-by-step GEMMs fill the GPU themselves (forward + backward over 8 steps at H = 512: B = 1024, 32
 // sub-tiles, 3.4 ms against 4.6 ms step by step; B = 2048, 7.4 against 6.1).
 constexpr int kMaxSub = 32;
+constexpr long long kScatterBytes = 128ll << 20;
 
 long long fwd_smem(int ut, int H) {
-  return 4ll * ((4ll * ut + kMB) * (H + 4) + (long long)kWarps * kMB * 4 * ut);
+  return 4ll * ((4ll * ut + kMB) * (H + 4) + 2ll * kWarps * kMB * 4 * ut);
 }
 long long bwd_smem(int ut, int H, int sub) {
   return 4ll * (((long long)ut + kMB) * (4ll * H + 4) + (long long)kWarps * kMB * ut + (long long)sub * kMB * ut);
+}
+
+long long bwd_scatter_smem(int ut, int H, int sub) {
+  return 4ll * (((long long)H + kMB) * (4ll * ut + 4) + kThreads + (long long)sub * kMB * ut);
+}
+// Words of the exchange of the scattered backward, 0 where the gathered one runs: the scattered one is the faster at every size,
+// but its words (H = 512: 256 KB a sequence) would be a large part of the memory, and of L2, at thousands of sequences.
+long long bwd_words(int ut, int ug, int groups, int sub, int H) {
+  const long long words = 2ll * groups * sub * ug * ug * kMB * ut;
+  return 8 * words <= kScatterBytes && bwd_scatter_smem(ut, H, sub) <= kMaxSmem ? words : 0;
 }
 
 // Units per CTA, unit slices, groups of sequences and sub-tiles per group; false when the layer does
@@ -410,9 +591,9 @@ bool plan(int sms, int B, int H, bool bwd, int* ut, int* ug, int* groups, int* s
 }
 
 template <typename K>
-int launch(K kern, const SeqArgs& a, int groups, long long smem, cudaStream_t s) {
+int launch(K kern, const SeqArgs& a, int groups, long long smem, long long words, cudaStream_t s) {
   GB_CUDA_OK(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  if (a.xch != nullptr) GB_CUDA_OK(cudaMemsetAsync(a.xch, 0, 16ll * a.B * a.H, s));
+  if (words > 0) GB_CUDA_OK(cudaMemsetAsync(a.xch, 0, 8ll * words, s));
   else GB_CUDA_OK(cudaMemsetAsync(a.flags, 0, sizeof(unsigned int) * a.ug * groups, s));
   void* args[] = {(void*)&a};
   GB_CUDA_OK(cudaLaunchCooperativeKernel((const void*)kern, dim3(a.ug, groups), dim3(kThreads), args, (size_t)smem, s));
@@ -457,22 +638,30 @@ GB_EXPORT int gb_lstm_seq_fwd(void* xg, const void* bias, const void* w, const v
     gbh::set_error("gb_lstm_seq_fwd: a contiguous output is needed where a backward follows");
     return gbh::E_BAD_ARG;
   }
-  const long long smem = fwd_smem(ut, H);
+  const long long smem = fwd_smem(ut, H), words = 2ll * B * H;
   cudaStream_t s = (cudaStream_t)stream;
   if (hprev != nullptr) {
-    if (ut == 16) return launch(lstm_seq_fwd_kernel<16, true>, a, groups, smem, s);
-    if (ut == 8) return launch(lstm_seq_fwd_kernel<8, true>, a, groups, smem, s);
-    return launch(lstm_seq_fwd_kernel<4, true>, a, groups, smem, s);
+    if (ut == 16) return launch(lstm_seq_fwd_kernel<16, true>, a, groups, smem, words, s);
+    if (ut == 8) return launch(lstm_seq_fwd_kernel<8, true>, a, groups, smem, words, s);
+    return launch(lstm_seq_fwd_kernel<4, true>, a, groups, smem, words, s);
   }
-  if (ut == 16) return launch(lstm_seq_fwd_kernel<16, false>, a, groups, smem, s);
-  if (ut == 8) return launch(lstm_seq_fwd_kernel<8, false>, a, groups, smem, s);
-  return launch(lstm_seq_fwd_kernel<4, false>, a, groups, smem, s);
+  if (ut == 16) return launch(lstm_seq_fwd_kernel<16, false>, a, groups, smem, words, s);
+  if (ut == 8) return launch(lstm_seq_fwd_kernel<8, false>, a, groups, smem, words, s);
+  return launch(lstm_seq_fwd_kernel<4, false>, a, groups, smem, words, s);
 }
 
-// Backward of the above (flags: scratch of 148 words): dout (B,T,H) or null, dcn (B,H) or null; writes dgates (B,T,4H), the gradient
+// 64-bit words of scratch that gb_lstm_seq_bwd takes.
+GB_EXPORT long long gb_lstm_seq_bwd_words(int B, int H) {
+  int ut, ug, groups, sub;
+  if (B <= 0 || !plan(device_sms(), B, H, true, &ut, &ug, &groups, &sub)) return 0;
+  const long long words = bwd_words(ut, ug, groups, sub, H);
+  return words > 0 ? words : kSms / 2;
+}
+
+// Backward of the above (scratch: gb_lstm_seq_bwd_words(B, H) words): dout (B,T,H) or null, dcn (B,H) or null; writes dgates (B,T,4H), the gradient
 // of the gate pre-activations, and dc0 (B,H) when not null.
 GB_EXPORT int gb_lstm_seq_bwd(const void* w, const void* c0, const void* cseq, const void* act, const void* dout,
-                              const void* dcn, void* dgates, void* dc0, void* flags, int B, int T, int H, void* stream) {
+                              const void* dcn, void* dgates, void* dc0, void* scratch, int B, int T, int H, void* stream) {
   if (B <= 0 || T <= 0) return gbh::E_OK;
   SeqArgs a = {};
   int ut, groups;
@@ -483,10 +672,21 @@ GB_EXPORT int gb_lstm_seq_bwd(const void* w, const void* c0, const void* cseq, c
   a.B = B; a.T = T; a.H = H;
   a.w = (const float*)w; a.c0 = (const float*)c0; a.cseq = (float*)cseq; a.act = (const float*)act;
   a.dout = (const float*)dout; a.dcn = (const float*)dcn; a.dgates = (float*)dgates; a.dc0 = (float*)dc0;
-  a.flags = (unsigned int*)flags; a.status = gbh::status_ptr();
-  const long long smem = bwd_smem(ut, H, a.sub);
+  a.status = gbh::status_ptr();
   cudaStream_t s = (cudaStream_t)stream;
-  if (ut == 16) return launch(lstm_seq_bwd_kernel<16>, a, groups, smem, s);
-  if (ut == 8) return launch(lstm_seq_bwd_kernel<8>, a, groups, smem, s);
-  return launch(lstm_seq_bwd_kernel<4>, a, groups, smem, s);
+  const long long words = bwd_words(ut, a.ug, groups, a.sub, H);
+  if (words > 0) {
+    a.xch = (unsigned long long*)scratch;
+    const long long smem = bwd_scatter_smem(ut, H, a.sub);
+    const int parts = kThreads / (kMB * ut);
+    const bool deep = (a.ug + parts - 1) / parts > 8;
+    if (ut == 16) return deep ? launch(lstm_seq_bwd_scatter_kernel<16, 16>, a, groups, smem, words, s) : launch(lstm_seq_bwd_scatter_kernel<16, 8>, a, groups, smem, words, s);
+    if (ut == 8) return deep ? launch(lstm_seq_bwd_scatter_kernel<8, 16>, a, groups, smem, words, s) : launch(lstm_seq_bwd_scatter_kernel<8, 8>, a, groups, smem, words, s);
+    return deep ? launch(lstm_seq_bwd_scatter_kernel<4, 16>, a, groups, smem, words, s) : launch(lstm_seq_bwd_scatter_kernel<4, 8>, a, groups, smem, words, s);
+  }
+  a.flags = (unsigned int*)scratch;
+  const long long smem = bwd_smem(ut, H, a.sub);
+  if (ut == 16) return launch(lstm_seq_bwd_kernel<16>, a, groups, smem, words, s);
+  if (ut == 8) return launch(lstm_seq_bwd_kernel<8>, a, groups, smem, words, s);
+  return launch(lstm_seq_bwd_kernel<4>, a, groups, smem, words, s);
 }

@@ -76,7 +76,7 @@ def lib() -> ctypes.CDLL:
             l.gb_last_error.restype = ctypes.c_char_p
             l.gb_gemm_f32x3_workspace.restype = c_longlong
             l.gb_gemm_f32x3_workspace.argtypes = [c_int, c_int, c_int, c_int]
-            for name in ("gb_conv_cl_fwd_ws", "gb_conv_cl_bwd_ws", "gb_conv_cl_part", "gb_block_ws"):
+            for name in ("gb_conv_cl_fwd_ws", "gb_conv_cl_bwd_ws", "gb_conv_cl_part", "gb_block_ws", "gb_lstm_seq_bwd_words"):
                 getattr(l, name).restype = c_longlong
             for name in ("gb_bench_matmul", "gb_bench_add", "gb_bench_flash_attn"):
                 getattr(l, name).restype = c_double

@@ -155,9 +155,9 @@ class _LSTMSequence(torch.autograd.Function):
         whh = _aligned(w_hh.detach())
         dgates = torch.empty_like(act)                     # (B * T, 4H)
         dc0 = torch.empty((B, H), dtype=cseq.dtype, device=dev) if ctx.needs_input_grad[5] else None
-        flags = torch.empty(148, dtype=torch.int32, device=dev)
+        scratch = torch.empty(_l.lib().gb_lstm_seq_bwd_words(_l.I(B), _l.I(H)), dtype=torch.int64, device=dev)
         _l.call("gb_lstm_seq_bwd", _l.ptr(whh), _l.ptr(c0), _l.ptr(cseq), _l.ptr(act), _l.ptr(dout), _l.ptr(dcn),
-                _l.ptr(dgates), _l.ptr(dc0), _l.ptr(flags), _l.I(B), _l.I(T), _l.I(H), _l.stream_ptr())
+                _l.ptr(dgates), _l.ptr(dc0), _l.ptr(scratch), _l.I(B), _l.I(T), _l.I(H), _l.stream_ptr())
         dx = dwih = db = dwhh = dh0 = None
         # every read of a weight comes before its gradient is declared ready (ops/linear.py)
         if ctx.needs_input_grad[0]:

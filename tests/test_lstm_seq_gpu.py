@@ -50,6 +50,28 @@ def test_lstm_sequence_matches_float64(B, T, I, H, state):
         _close(a, b, 3e-5, n)
 
 
+@pytest.mark.parametrize("B,T,H,scattered", [(8, 9, 132, True), (300, 3, 256, True), (512, 2, 512, True), (513, 3, 512, False), (9, 5, 876, True)])
+def test_backward_either_way_round_matches_float64(B, T, H, scattered):
+    """The scattered exchange with several sub-tiles and slices that the units do not fill, up to the most words it takes, and the
+    gathered one behind that."""
+    words = L.lib().gb_lstm_seq_bwd_words(L.I(B), L.I(H))
+    assert (words > 74) == scattered and 8 * words <= 128 << 20
+    torch.manual_seed(H)
+    net = nn.LSTM(8, H, device="cuda")
+    x = torch.randn(B, T, 8, device="cuda", requires_grad=True)
+    dy = torch.randn(B, T, H, device="cuda")
+    y, (_, c) = net.ForwardWithState(x)
+    ((y * dy).sum() + c.sum()).backward()
+    L.assert_status_ok()
+    ref = copy.deepcopy(net).double().cpu()
+    ref.zero_grad()
+    xr = x.detach().double().cpu().requires_grad_()
+    yr, (_, cr) = ref.ForwardWithState(xr)
+    ((yr * dy.double().cpu()).sum() + cr.sum()).backward()
+    for n, a, b in [("y", y, yr), ("dx", x.grad, xr.grad)] + [(n, p.grad, q.grad) for (n, p), q in zip(net.named_parameters(), ref.parameters())]:
+        _close(a, b, 3e-5, n)          # as in test_lstm_sequence_matches_float64
+
+
 def test_step_path_where_the_kernel_does_not_apply():
     net = nn.LSTM(8, 16, device="cuda")
     x = torch.randn(2, 3, 8, device="cuda")
