@@ -60,6 +60,7 @@ struct AttnArgs {
   int* status;
   // optional timeline of CTA (0,0,0) of the dK/dV kernel: [3 lanes][kTraceSlots] SM clock stamps
   long long* trace;
+  float inv_scale;       // of the scale that the row statistics are folded with (see stat_row)
   int head_group;        // causal launch order, see block_of(); reciprocals, rounded up, times 2^32, of it and of H
   unsigned group_recip, head_recip;
 };
@@ -490,8 +491,7 @@ struct BwdCfg {
   static constexpr int TILE_BYTES = CH * 128 * 128;
   static constexpr int SUB_BYTES = CH * BSUB * 128;
   static constexpr int NS = 4;
-  static constexpr int STAT_BYTES = NS * 2 * BSUB * 4;  // per stage: 64 x LSE*log2(e), 64 x Delta*scale
-  static constexpr int SMEM_BYTES = 2 * TILE_BYTES + NS * 2 * SUB_BYTES + STAT_BYTES + 1024 + 256;
+  static constexpr int SMEM_BYTES = 2 * TILE_BYTES + NS * 2 * SUB_BYTES + 1024 + 256;      // of the dQ kernel
   // head_dim 64: one S/dP buffer, eight elementwise warps, 256 TMEM columns and < 113 KB of
   // shared memory, so TWO CTAs share an SM and hide each other's serial chain (S/dP MMAs ->
   // elementwise -> accumulation MMAs) as well as each other's start-up and epilogue.
@@ -503,6 +503,11 @@ struct BwdCfg {
   static constexpr int EW = 8 * NBUF;
   static constexpr int THREADS = 64 + EW * 32;
   static constexpr int CTAS_PER_SM = DUAL ? 2 : 1;
+  // dK / dV kernel: three stages make room for the row statistics (64 rows of 128 bytes: 32 a stage), the A operand that adds
+  // them, and 2 KB per elementwise warp through which dS^T leaves
+  static constexpr int NSK = 3;
+  static constexpr int STAT_BYTES = BSUB * 128, ONES_BYTES = 1024, OUT_BYTES = 2048;
+  static constexpr int SMEM_BYTES_KV = 2 * TILE_BYTES + NSK * 2 * SUB_BYTES + STAT_BYTES + ONES_BYTES + EW * OUT_BYTES + 1024 + 256;
   static constexpr int TMEM_COLS = DUAL ? 256 : 512;
   // buffer b: scores at b*128, dP at b*128 + 64; accumulators behind them
   static constexpr int COL_ACC0 = 128 * NBUF, COL_ACC1 = COL_ACC0 + HD;
@@ -554,25 +559,62 @@ __device__ __forceinline__ uint32_t pack16t(float a, float b) {
   return BF ? pack_bf16(a, b) : pack_f16(a, b);
 }
 
+// Two packed fp32 products.
+__device__ __forceinline__ unsigned long long fmul2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long pair(uint32_t lo, uint32_t hi) { return (unsigned long long)hi << 32 | lo; }
+__device__ __forceinline__ float lo_of(unsigned long long v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi_of(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
+
+// x as a sum of three bf16 values: 24 bits.
+__device__ __forceinline__ void split_bf16(float x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  const __nv_bfloat16 h = __float2bfloat16_rn(x);
+  const float r = x - __bfloat162float(h);
+  const __nv_bfloat16 m = __float2bfloat16_rn(r);
+  hi = __bfloat16_as_ushort(h);
+  mid = __bfloat16_as_ushort(m);
+  lo = __bfloat16_as_ushort(__float2bfloat16_rn(r - __bfloat162float(m)));
+}
+
+// The row statistics of the dK / dV kernel are added by the tensor core.  They belong to the columns of S^T and dP^T, so that
+// every thread would need all of them: 64 values per sub-tile and warp, and shared memory delivers one register per thread and
+// clock however they are loaded (560 of 2 360 clocks per 128 x 64 block).  Instead row q of a B operand of 16 k's holds -LSE / scale
+// and -Delta, each as three bf16 parts, and one MMA step with an A operand of ones at the parts' places adds them to every row
+// of S^T and of dP^T.  This is that row (its first eight k's; the others are zero): rows past the end and rows without any key
+// (LSE = -inf) get a statistic that makes their probabilities 0.
+__device__ __forceinline__ uint4 stat_row(float lse, float delta, float inv_scale) {
+  float x = -(lse == -INFINITY ? 1e30f : lse) * inv_scale;
+  if (fabsf(x) > 1e37f) x = copysignf(1e37f, x);     // (finite parts only; a NaN stays one)
+  uint32_t a, b, c, d, e, f;
+  split_bf16(x, a, b, c);
+  split_bf16(-delta, d, e, f);
+  return make_uint4(a | b << 16, c | d << 16, e | f << 16, 0u);
+}
+
 // dK / dV: one CTA per 128-key tile; streams 64-row query sub-tiles.  Works in the
 // transposed domain (rows = keys) so that P^T and dS^T are A operands in TMEM.
 template <int HD, bool BF, bool DUAL>
 __global__ void __launch_bounds__(BwdCfg<HD, DUAL>::THREADS, BwdCfg<HD, DUAL>::CTAS_PER_SM)
 fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                   const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
-                  const AttnArgs args) {
+                  const __grid_constant__ CUtensorMap tmDS, const AttnArgs args) {
   using C = BwdCfg<HD, DUAL>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sK = smem;
   uint8_t* sV = sK + C::TILE_BYTES;
   uint8_t* ring = sV + C::TILE_BYTES;  // [NS] x {Q sub-tile, dO sub-tile}
-  float* sStat = (float*)(ring + C::NS * 2 * C::SUB_BYTES);  // [NS][2][64]
-  uint64_t* bars = (uint64_t*)((uint8_t*)sStat + C::STAT_BYTES);
+  uint8_t* sStat = ring + C::NSK * 2 * C::SUB_BYTES;   // 64 rows of statistics, k step st of the operand for stage st
+  uint8_t* sOnes = sStat + C::STAT_BYTES;              // eight rows: k step 0 picks LSE, step 1 Delta
+  uint8_t* sOut = sOnes + C::ONES_BYTES;               // [EW][32 rows][64 B]
+  uint64_t* bars = (uint64_t*)(sOut + C::EW * C::OUT_BYTES);
   uint64_t* kv_full = bars;                 // 1
-  uint64_t* q_full = bars + 1;              // NS
-  uint64_t* q_empty = q_full + C::NS;       // NS
-  uint64_t* sdp_full = q_empty + C::NS;     // 2
+  uint64_t* q_full = bars + 1;              // NSK
+  uint64_t* q_empty = q_full + C::NSK;       // NSK
+  uint64_t* sdp_full = q_empty + C::NSK;     // 2
   uint64_t* p_full = sdp_full + 2;          // 2
   uint64_t* acc_done = p_full + 2;          // 1
   uint64_t* a_ready = acc_done + 1;         // 1: K and V copied into TMEM
@@ -591,7 +633,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
-    for (int i = 0; i < C::NS; i++) {
+    for (int i = 0; i < C::NSK; i++) {
       mbar_init(&q_full[i], 1 + 32);  // the TMA transaction + the 32 lanes that stage the row statistics
       mbar_init(&q_empty[i], 1);
     }
@@ -601,6 +643,15 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     *abort_flag = 0;
     mbar_fence_init();
   }
+  for (int i = threadIdx.x; i < C::STAT_BYTES / 16; i += C::THREADS) reinterpret_cast<uint4*>(sStat)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (threadIdx.x < 64) {
+    const uint32_t row = threadIdx.x >> 3, chunk = (threadIdx.x & 7u) ^ row;      // 16-byte chunk before the swizzle
+    constexpr uint32_t one = 0x3f80u;
+    reinterpret_cast<uint4*>(sOnes)[threadIdx.x] = chunk == 0u   ? make_uint4(one | one << 16, one, 0u, 0u)
+                                                   : chunk == 2u ? make_uint4(0u, one << 16, one | one << 16, 0u)
+                                                                 : make_uint4(0u, 0u, 0u, 0u);
+  }
+  fence_proxy_async_smem();
   if (warp == 1) { tmem_alloc(tmem_slot, C::TMEM_COLS); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
@@ -617,8 +668,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         tma_load_4d(sV + c * 128 * 128, &tmV, kv_full, c * 64, kv0, h, b);
       }
     }
-    const float* stat_g = (lane < 16 ? args.LSE : args.Delta) + ((long long)b * args.H + h) * args.Sq;
-    const bool vec = (args.Sq & 3) == 0;
+    const long long stat0 = ((long long)b * args.H + h) * args.Sq;
     int st = 0;
     uint32_t ph = 0;
     for (int it = 0; it < n_it; it++) {
@@ -637,38 +687,24 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           tma_load_4d(sdO + c * BSUB * 128, &tmdO, &q_full[st], c * 64, q0, h, b);
         }
       }
-      // lanes 0-15: LSE * log2(e) (rows past the end and fully masked rows read +inf, so
-      // their probabilities come out 0); lanes 16-31: Delta * scale
-      const int qs = q0 + (lane & 15) * 4;
-      float4 t;
-      if (vec && qs + 4 <= args.Sq) {
-        t = __ldg(reinterpret_cast<const float4*>(stat_g + qs));
-      } else {
-        const float fill = lane < 16 ? INFINITY : 0.f;
-        t.x = qs < args.Sq ? __ldg(stat_g + qs) : fill;
-        t.y = qs + 1 < args.Sq ? __ldg(stat_g + qs + 1) : fill;
-        t.z = qs + 2 < args.Sq ? __ldg(stat_g + qs + 2) : fill;
-        t.w = qs + 3 < args.Sq ? __ldg(stat_g + qs + 3) : fill;
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const int row = lane + 32 * i, q = q0 + row;
+        const bool in = q < args.Sq;
+        const uint4 v = stat_row(in ? __ldg(args.LSE + stat0 + q) : -INFINITY, in ? __ldg(args.Delta + stat0 + q) : 0.f, args.inv_scale);
+        *reinterpret_cast<uint4*>(sStat + row * 128 + (((uint32_t)(2 * st) ^ ((uint32_t)row & 7u)) << 4)) = v;
       }
-      if (lane < 16) {
-        const float k = 1.4426950408889634f;
-        t.x = t.x == -INFINITY ? INFINITY : t.x * k;
-        t.y = t.y == -INFINITY ? INFINITY : t.y * k;
-        t.z = t.z == -INFINITY ? INFINITY : t.z * k;
-        t.w = t.w == -INFINITY ? INFINITY : t.w * k;
-      } else {
-        t.x *= args.scale; t.y *= args.scale; t.z *= args.scale; t.w *= args.scale;
-      }
-      *reinterpret_cast<float4*>(sStat + st * 128 + lane * 4) = t;
+      fence_proxy_async_smem();
       mbar_arrive(&q_full[st]);
-      if (++st == C::NS) { st = 0; ph ^= 1; }
+      if (++st == C::NSK) { st = 0; ph ^= 1; }
     }
   } else if (warp == 1) {
     if (elect_one()) {
       const uint32_t fmt = BF ? 1u : 0u;
       const uint32_t idesc_s = make_idesc(1u, fmt, false, false, 128, BSUB);
       const uint32_t idesc_acc = make_idesc(1u, fmt, false, true, 128, HD);
-      const uint32_t ka = smem_u32(sK), va = smem_u32(sV);
+      const uint32_t idesc_stat = make_idesc(1u, 1u, false, false, 128, BSUB);
+      const uint32_t ka = smem_u32(sK), va = smem_u32(sV), stat = smem_u32(sStat), ones = smem_u32(sOnes);
       bool ok = mbar_wait(kv_full, 0, abort_flag, args.status, ST_ATTN_TIMEOUT, 12);
       if (ok && C::KV_IN_TMEM) {
         ok = mbar_wait(a_ready, 0, abort_flag, args.status, ST_ATTN_TIMEOUT, 18);
@@ -693,8 +729,10 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             tc_mma_f16(d + 64, kdesc(va, k), kdesc_sub(ga, k), idesc_s, k != 0);  // dP^T = V dO^T
           }
         }
+        tc_mma_f16(d, make_smem_desc_sw128(ones, 16, 0), kdesc_sub(stat, st_s), idesc_stat, 1u);             // S^T - LSE / scale
+        tc_mma_f16(d + 64, make_smem_desc_sw128(ones + 32, 16, 0), kdesc_sub(stat, st_s), idesc_stat, 1u);   // dP^T - Delta
         tc_commit(&sdp_full[it % C::NBUF]);
-        if (++st_s == C::NS) { st_s = 0; ph_s ^= 1; }
+        if (++st_s == C::NSK) { st_s = 0; ph_s ^= 1; }
         return true;
       };
       long long* tr = (blockIdx.x | blockIdx.y | blockIdx.z) == 0 ? args.trace : nullptr;
@@ -728,7 +766,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         }
         tc_commit(&q_empty[st]);
         if (it == n_it - 1) tc_commit(acc_done);
-        if (++st == C::NS) st = 0;
+        if (++st == C::NSK) st = 0;
         if (C::NBUF == 1 && it + 1 < n_it) ok = issue_sdp(it + 1);
       }
     }
@@ -756,14 +794,27 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     }
     long long* tr = ((blockIdx.x | blockIdx.y | blockIdx.z) == 0 && (e & 7) == 0 && lane == 0) ? args.trace : nullptr;
     int ntr = 0;
-    // where this thread's key row starts in the dS^T spill (its half of each 64-query sub-tile)
-    // (a byte offset from args.dS; the workspace is at most 4 GiB, so 32 bits hold it)
-    const uint32_t ds_off = (uint32_t)(((((long long)b * args.H + h) * args.ds_rows + kvrow) * args.ds_ld + half * 32) * 2);
+    uint8_t* out = sOut + e * C::OUT_BYTES;
+    const uint32_t out_row = smem_u32(out) + (uint32_t)lane * 64u, swz = ((uint32_t)lane >> 1) & 3u;
+    // this warp's 32 key rows x 32 queries of dS^T: through shared memory and one TMA store (a store of 64 bytes per thread took
+    // 55 clocks of the memory pipe per instruction, 890 per 128 x 64 block)
+    auto spill = [&](const uint32_t(&v)[16], int it) {
+      if (lane == 0) tma_store_wait_read<0>();
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(out_row + (((uint32_t)j ^ swz) << 4)), "r"(v[4 * j]),
+                     "r"(v[4 * j + 1]), "r"(v[4 * j + 2]), "r"(v[4 * j + 3])
+                     : "memory");
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_3d(&tmDS, out, (i_begin + it) * BSUB + half * 32, kv0 + quarter * 32, b * args.H + h);
+        tma_store_commit();
+      }
+    };
     for (int it = group; it < n_it; it += C::NBUF) {
-      const int st = it % C::NS;
       trace_stamp(tr, 1 + group, ntr);  // starts waiting
-      ok = mbar_wait(&q_full[st], (it / C::NS) & 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 17);
-      if (!ok) break;
       ok = mbar_wait(&sdp_full[group], (it / C::NBUF) & 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 15);
       if (!ok) break;
       trace_stamp(tr, 1 + group, ntr);  // scores ready
@@ -771,8 +822,6 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       uint32_t rs[32], rd[32];
       tmem_ld32(my, rs);
       tmem_ld32(my + 64, rd);
-      const float4* l4 = reinterpret_cast<const float4*>(sStat + st * 128 + half * 32);
-      const float4* d4 = reinterpret_cast<const float4*>(sStat + st * 128 + 64 + half * 32);
       tmem_ld_wait();
       trace_stamp(tr, 1 + group, ntr);  // loaded
       const int q0 = (i_begin + it) * BSUB + half * 32;  // first query column of this thread
@@ -790,11 +839,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         for (int i = 0; i < 16; i++) z[i] = 0u;
         tmem_st16(my, z);
         tmem_st16(my + 64, z);
-        if (args.dS) {
-          uint8_t* dst = (uint8_t*)args.dS + ds_off + (uint32_t)(i_begin + it) * (BSUB * 2);
-          st_global_v8(dst, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u);
-          st_global_v8(dst + 32, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u);
-        }
+        if (args.dS) spill(z, it);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
@@ -802,29 +847,20 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         continue;
       }
       uint32_t pp[16], pd[16];
+      const unsigned long long sl2 = pair(__float_as_uint(args.scale_log2), __float_as_uint(args.scale_log2));
+      const unsigned long long sc2 = pair(__float_as_uint(args.scale), __float_as_uint(args.scale));
       auto body = [&](auto use_mask) {
 #pragma unroll
-        for (int g = 0; g < 8; g++) {
-          const float4 l = l4[g], d = d4[g];
-          const float ls[4] = {l.x, l.y, l.z, l.w};
-          const float ds[4] = {d.x, d.y, d.z, d.w};
-          float p[4], q[4];
-#pragma unroll
-          for (int u = 0; u < 4; u++) {
-            const int j = 4 * g + u;
-            // head_dim 64: every fourth exponential runs on the FMA pipe, because there the MUFU
-            // unit is the busiest resource of this loop (at 128 the tensor core is)
-            const float e = fmaf(__uint_as_float(rs[j]), args.scale_log2, -ls[u]);
-            p[u] = (HD == 64 && u == 3 && !decltype(use_mask)::value) ? exp2_poly(e) : exp2f(e);
-            if (decltype(use_mask)::value) {
-              if (row_dead || (args.causal && kvrow > q0 + j)) p[u] = 0.f;
-            }
-            q[u] = p[u] * fmaf(__uint_as_float(rd[j]), args.scale, -ds[u]);
+        for (int g = 0; g < 16; g++) {
+          const unsigned long long x = fmul2(pair(rs[2 * g], rs[2 * g + 1]), sl2);
+          float p0 = exp2f(lo_of(x)), p1 = exp2f(hi_of(x));
+          if (decltype(use_mask)::value) {
+            if (row_dead || (args.causal && kvrow > q0 + 2 * g)) p0 = 0.f;
+            if (row_dead || (args.causal && kvrow > q0 + 2 * g + 1)) p1 = 0.f;
           }
-          pp[2 * g] = pack16t<BF>(p[0], p[1]);
-          pp[2 * g + 1] = pack16t<BF>(p[2], p[3]);
-          pd[2 * g] = pack16t<BF>(q[0], q[1]);
-          pd[2 * g + 1] = pack16t<BF>(q[2], q[3]);
+          const unsigned long long q = fmul2(pair(__float_as_uint(p0), __float_as_uint(p1)), fmul2(pair(rd[2 * g], rd[2 * g + 1]), sc2));
+          pp[g] = pack16t<BF>(p0, p1);
+          pd[g] = pack16t<BF>(lo_of(q), hi_of(q));
         }
       };
       if (masked) body(std::true_type{});
@@ -833,17 +869,12 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       trace_stamp(tr, 1 + group, ntr);  // computed
       tmem_st16(my, pp);
       tmem_st16(my + 64, pd);
-      if (args.dS) {
-        // this thread's key row, its 32 query columns: 64 contiguous bytes of dS^T
-        uint8_t* dst = (uint8_t*)args.dS + ds_off + (uint32_t)(i_begin + it) * (BSUB * 2);
-        st_global_v8(dst, pd[0], pd[1], pd[2], pd[3], pd[4], pd[5], pd[6], pd[7]);
-        st_global_v8(dst + 32, pd[8], pd[9], pd[10], pd[11], pd[12], pd[13], pd[14], pd[15]);
-      }
       tmem_st_wait();
       trace_stamp(tr, 1 + group, ntr);  // stored
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[group]);
+      if (args.dS) spill(pd, it);       // behind the arrival: the accumulation does not wait for it
     }
     if (ok && n_it > 0) ok = mbar_wait(acc_done, 0, abort_flag, args.status, ST_ATTN_TIMEOUT, 16);
     if (ok) {
@@ -873,6 +904,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       for (int i = 0; i < W; i++) v[i] = n_it > 0 ? __uint_as_float(rb[i]) : 0.f;
       if (!row_dead) store_row16_lim<W>(dkrow, v, BF, args.D - cw);
     }
+    if (args.dS && lane == 0) tma_store_wait<0>();   // shared memory must outlive the stores that read from it
   }
   tc_fence_before();
   __syncthreads();
@@ -891,7 +923,7 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint8_t* sQ = smem;
   uint8_t* sdO = sQ + C::TILE_BYTES;
   uint8_t* ring = sdO + C::TILE_BYTES;  // [NS] x {K sub-tile, V sub-tile}
-  uint64_t* bars = (uint64_t*)(ring + C::NS * 2 * C::SUB_BYTES + C::STAT_BYTES);
+  uint64_t* bars = (uint64_t*)(ring + C::NS * 2 * C::SUB_BYTES);
   uint64_t* q_full = bars;                  // 1
   uint64_t* kv_full = bars + 1;             // NS
   uint64_t* kv_empty = kv_full + C::NS;     // NS
@@ -1271,6 +1303,7 @@ struct BwdMaps {
   CUtensorMap q128, k128, v128, g128;  // 128-row boxes (resident tiles)
   CUtensorMap q64, k64, v64, g64;      // 64-row boxes (streamed sub-tiles)
   CUtensorMap ds;                      // the dS^T spill: (query, key, batch*head), boxes of 64 x 64
+  CUtensorMap ds_out;                  // the same with boxes of 32 x 32, as the dK / dV kernel's warps write it
 };
 
 int g_fa_dual = 1;
@@ -1280,12 +1313,12 @@ int launch_bwd(const BwdMaps& m, const AttnArgs& a, cudaStream_t s) {
   using C = BwdCfg<HD, DUAL>;
   static bool configured = false;
   if (!configured) {
-    GB_CUDA_OK(cudaFuncSetAttribute(fa_bwd_dkv_kernel<HD, BF, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+    GB_CUDA_OK(cudaFuncSetAttribute(fa_bwd_dkv_kernel<HD, BF, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES_KV));
     GB_CUDA_OK(cudaFuncSetAttribute(fa_bwd_dq_kernel<HD, BF, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
     configured = true;
   }
   dim3 gkv((a.Sk + BKV - 1) / BKV, a.H, a.B);
-  fa_bwd_dkv_kernel<HD, BF, DUAL><<<gkv, C::THREADS, C::SMEM_BYTES, s>>>(m.q64, m.k128, m.v128, m.g64, a);
+  fa_bwd_dkv_kernel<HD, BF, DUAL><<<gkv, C::THREADS, C::SMEM_BYTES_KV, s>>>(m.q64, m.k128, m.v128, m.g64, m.ds_out, a);
   GB_CUDA_OK(cudaGetLastError());
   dim3 gq((a.Sq + BQ - 1) / BQ, a.H, a.B);
   if (a.dS) {
@@ -1452,7 +1485,12 @@ GB_EXPORT int gb_flash_bwd_ws(int dtype, const void* q, const void* k, const voi
   a.dv_sb = strides[18]; a.dv_ss = strides[19]; a.dv_sh = strides[20];
   a.status = gbh::status_ptr();
   a.trace = g_trace;
+  // a scale so small that LSE / scale could overflow scores like 0: the statistics are folded with 2^-100 then
+  const float fold = fabsf(scale) >= 0x1p-100f ? scale : copysignf(0x1p-100f, scale);
+  a.inv_scale = 1.f / fold;
+  if (fold != scale) a.scale_log2 = fold * 1.4426950408889634f;
   BwdMaps m;
+  memset(&m, 0, sizeof(m));
   int rc;
   if ((rc = make_qkv_map(&m.q128, q, a.in_bf16, B, H, Sq, D, strides[0], strides[1], strides[2], 128))) return rc;
   if ((rc = make_qkv_map(&m.k128, k, a.in_bf16, B, H, Sk, D, strides[3], strides[4], strides[5], 128))) return rc;
@@ -1462,7 +1500,6 @@ GB_EXPORT int gb_flash_bwd_ws(int dtype, const void* q, const void* k, const voi
   if ((rc = make_qkv_map(&m.k64, k, a.in_bf16, B, H, Sk, D, strides[3], strides[4], strides[5], 64))) return rc;
   if ((rc = make_qkv_map(&m.v64, v, a.in_bf16, B, H, Sk, D, strides[6], strides[7], strides[8], 64))) return rc;
   if ((rc = make_qkv_map(&m.g64, dout, a.in_bf16, B, H, Sq, D, strides[9], strides[10], strides[11], 64))) return rc;
-  // (the kernel addresses the spill with 32-bit byte offsets: at most 4 GiB)
   if (ws != nullptr && ws_bytes >= gb_flash_bwd_ws_bytes(B, H, Sq, Sk) && !((uintptr_t)ws & 31) &&
       gb_flash_bwd_ws_bytes(B, H, Sq, Sk) <= (1LL << 32)) {
     a.dS = ws;
@@ -1473,6 +1510,10 @@ GB_EXPORT int gb_flash_bwd_ws(int dtype, const void* q, const void* k, const voi
     uint32_t box[4] = {64, 64, 1, 1};
     if ((rc = gbh::encode_tmap(&m.ds, a.in_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
                                4, ws, dims, st, box, CU_TENSOR_MAP_SWIZZLE_128B)))
+      return rc;
+    uint32_t box_out[3] = {32, 32, 1};
+    if ((rc = gbh::encode_tmap(&m.ds_out, a.in_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
+                               3, ws, dims, st, box_out, CU_TENSOR_MAP_SWIZZLE_64B)))
       return rc;
   }
   if (D > 64)
