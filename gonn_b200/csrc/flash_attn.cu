@@ -17,10 +17,8 @@
 //   warps 2-5   softmax: one thread per row; running max / sum in registers;
 //               O is rescaled only when the max moved by more than 2^8
 // Backward: a row-statistics kernel (Delta = dO . O), then one CTA per 128-key tile for
-// dK / dV and one CTA per 128-query tile for dQ; both stream 64-row sub-tiles, keep S and dP
-// in TMEM (two buffers and sixteen elementwise warps at head_dim 128; one buffer, eight
-// warps and two CTAs per SM at head_dim 64) and feed P^T / dS^T back to the tensor core as
-// TMEM A operands.
+// dK / dV, which leaves dS^T behind for one product dQ = dS K (or, without room for it, one CTA per 128-query tile that
+// computes the scores again); both stream 64-row sub-tiles and keep S and dP in TMEM.
 // Tensors are addressed through 4-D tensor maps (d, s, h, b) with arbitrary
 // strides, so (B,S,H,D) and (B,H,S,D) layouts both work without copies.
 #include "common.cuh"
@@ -86,22 +84,13 @@ __device__ __forceinline__ void block_of(const AttnArgs& args, int& rank, int& h
 
 constexpr int kTraceSlots = 512;
 // lane: 0 = MMA thread, 1 / 2 = first warp of elementwise group 0 / 1
-// Compiled in only with -DGB_FA_TRACE: the pointer and the counter cost three registers in a kernel
-// that sits at its register cap.
+// Compiled in only with -DGB_FA_TRACE: a stamp costs its warp registers and about 50 clocks.
 __device__ __forceinline__ void trace_stamp(long long* trace, int lane_id, int& n) {
 #ifdef GB_FA_TRACE
   if (trace && n < kTraceSlots) trace[lane_id * kTraceSlots + n++] = clock64();
 #else
   (void)trace; (void)lane_id; (void)n;
 #endif
-}
-
-// One 32-byte store (a whole DRAM sector) from eight registers; the address must be 32-byte aligned.
-__device__ __forceinline__ void st_global_v8(void* p, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                             uint32_t a4, uint32_t a5, uint32_t a6, uint32_t a7) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a0), "r"(a1), "r"(a2),
-               "r"(a3), "r"(a4), "r"(a5), "r"(a6), "r"(a7)
-               : "memory");
 }
 
 __device__ __forceinline__ uint32_t pack16(float a, float b, int bf) {
@@ -476,10 +465,9 @@ fa_delta_vec_kernel(const T* __restrict__ O, const T* __restrict__ dO, float* __
 // ---------------------------------------------------------------------------
 // Backward
 // ---------------------------------------------------------------------------
-constexpr int kBwdThreadsMax = 64 + 16 * 32;     // TMA warp, MMA warp, up to sixteen elementwise warps
 constexpr int BSUB = 64;                  // rows of one streamed sub-tile
 
-// Backward tiling.  The resident operand pair is a 128-row tile; the streamed pair comes in
+// Tiling of the dQ kernel that computes the scores itself.  The resident operand pair is a 128-row tile; the streamed pair comes in
 // 64-row sub-tiles through a ring of NS stages.  Scores and dP of a sub-tile are 128 x 64
 // fp32 blocks in TMEM, double buffered, so the tensor core computes sub-tile i+1 (and the
 // accumulations of sub-tile i-1) while the elementwise warps work on sub-tile i.  The
@@ -503,18 +491,11 @@ struct BwdCfg {
   static constexpr int EW = 8 * NBUF;
   static constexpr int THREADS = 64 + EW * 32;
   static constexpr int CTAS_PER_SM = DUAL ? 2 : 1;
-  // dK / dV kernel: three stages make room for the row statistics (64 rows of 128 bytes: 32 a stage), the A operand that adds
-  // them, and 2 KB per elementwise warp through which dS^T leaves
-  static constexpr int NSK = 3;
-  static constexpr int STAT_BYTES = BSUB * 128, ONES_BYTES = 1024, OUT_BYTES = 2048;
-  static constexpr int SMEM_BYTES_KV = 2 * TILE_BYTES + NSK * 2 * SUB_BYTES + STAT_BYTES + ONES_BYTES + EW * OUT_BYTES + 1024 + 256;
   static constexpr int TMEM_COLS = DUAL ? 256 : 512;
   // buffer b: scores at b*128, dP at b*128 + 64; accumulators behind them
   static constexpr int COL_ACC0 = 128 * NBUF, COL_ACC1 = COL_ACC0 + HD;
   // resident A operands kept in TMEM where the columns allow it
-  static constexpr bool KV_IN_TMEM = HD == 64 && !DUAL;
   static constexpr bool Q_IN_TMEM = !DUAL;
-  static constexpr int COL_KT = COL_ACC0 + 2 * HD, COL_VT = COL_KT + HD / 2;
   static constexpr int COL_QT = COL_ACC0 + HD, COL_GT = COL_QT + HD / 2;
 };
 
@@ -595,53 +576,147 @@ __device__ __forceinline__ uint4 stat_row(float lse, float delta, float inv_scal
 }
 
 // dK / dV: one CTA per 128-key tile; streams 64-row query sub-tiles.  Works in the
-// transposed domain (rows = keys) so that P^T and dS^T are A operands in TMEM.
+// transposed domain (rows = keys) so that P^T is an A operand in TMEM, and dS^T one in shared memory, from where a TMA store also
+// takes it to the dQ kernel (64-byte row stores by the threads took 55 clocks of the memory pipe per instruction, 890 of
+// 2 360 per block).
+//
+// One S^T and one dP^T block of 128 x 64 in TMEM, handed to and fro in two half steps, so that the tensor core and the elementwise
+// warps work at the same time on one sub-tile and the next:
+//     tensor core   dV += P^T(i) dO(i), S^T(i + 1)  |  dK += dS^T(i) Q(i), dP^T(i + 1)
+//     elementwise   dS^T(i) from P and dP^T(i)      |  P^T(i + 1) from S^T(i + 1)
+// What bounds it at head size 128 is the shared memory that feeds the tensor core (128 bytes a clock): with K and V as A operands
+// there a block moved 204 KB of it, 1 630 clocks for 1 090 of multiply-adds.  K and V therefore live in TMEM, which the single
+// S^T / dP^T pair leaves room for: 140 KB.  At head size 64 two CTAs share an SM (and hide each other's start and end), each
+// with half of TMEM, and K and V stay in shared memory.
+// What is left is the chain of an elementwise warp: per 128 x 64 block 1.01 us at 128 (1.37 with both gathered and stored by
+// the threads and two S^T / dP^T buffers), 0.67 us at 64 (1.00), where 0.57 and 0.31 are multiply-adds and 0.27 exponentials.
+// us: (8, 16, 4096, 128) causal 1 343 -> 1 100; (16, 12, 1024, 64) causal 147 -> 90; (6, 12, 1000 x 1531, 64) fp16 150 -> 84.
+template <int HD, bool DUAL_>
+struct KvCfg {
+  static constexpr bool DUAL = DUAL_;
+  static_assert(!DUAL_ || HD == 64, "two CTAs per SM need head_dim 64");
+  static constexpr int CH = HD / 64;
+  static constexpr int TILE_BYTES = CH * 128 * 128;
+  static constexpr int SUB_BYTES = CH * BSUB * 128;
+  static constexpr int NS = 3;
+  static constexpr int EW = DUAL ? 8 : 16;           // elementwise warps
+  static constexpr int CW = 4 * BSUB / EW;           // query columns of one of them: a quarter of the key rows, all EW / 4 groups
+  static constexpr int THREADS = 96 + EW * 32;       // TMA, MMA and store warps
+  static constexpr int CTAS_PER_SM = DUAL ? 2 : 1;
+  // row statistics (64 rows of 128 bytes, 32 a stage), the A operand that adds them, the tile through which dS^T leaves
+  static constexpr int STAT_BYTES = BSUB * 128, ONES_BYTES = 1024, OUT_BYTES = 128 * 128;
+  static constexpr int SMEM_BYTES = 2 * TILE_BYTES + NS * 2 * SUB_BYTES + STAT_BYTES + ONES_BYTES + OUT_BYTES + 1024 + 256;
+  static constexpr int TMEM_COLS = DUAL ? 256 : 512;
+  static constexpr int COL_S = 0, COL_DP = BSUB, COL_ACC0 = 2 * BSUB, COL_ACC1 = COL_ACC0 + HD;
+  static constexpr bool KV_IN_TMEM = !DUAL;
+  static constexpr int COL_K = COL_ACC1 + HD, COL_V = COL_K + HD / 2;
+  static_assert((KV_IN_TMEM ? COL_V + HD / 2 : COL_K) <= TMEM_COLS, "TMEM");
+};
+
+template <int N>
+__device__ __forceinline__ void tmem_ld_cols(uint32_t addr, uint32_t (&r)[N]) {
+  if constexpr (N == 32) tmem_ld32(addr, r);
+  else tmem_ld16(addr, r);
+}
+template <int N>
+__device__ __forceinline__ void tmem_st_cols(uint32_t addr, const uint32_t (&r)[N]) {
+  if constexpr (N == 16) {
+    tmem_st16(addr, r);
+  } else {
+    static_assert(N == 8, "columns");
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(addr), "r"(r[0]), "r"(r[1]),
+                 "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+  }
+}
+
 template <int HD, bool BF, bool DUAL>
-__global__ void __launch_bounds__(BwdCfg<HD, DUAL>::THREADS, BwdCfg<HD, DUAL>::CTAS_PER_SM)
+__global__ void __launch_bounds__(KvCfg<HD, DUAL>::THREADS, KvCfg<HD, DUAL>::CTAS_PER_SM)
 fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                   const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
-                  const __grid_constant__ CUtensorMap tmDS, const AttnArgs args) {
-  using C = BwdCfg<HD, DUAL>;
+                  const __grid_constant__ CUtensorMap tmDS, const __grid_constant__ CUtensorMap tmdK,
+                  const __grid_constant__ CUtensorMap tmdV, const AttnArgs args) {
+  using C = KvCfg<HD, DUAL>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sK = smem;
   uint8_t* sV = sK + C::TILE_BYTES;
-  uint8_t* ring = sV + C::TILE_BYTES;  // [NS] x {Q sub-tile, dO sub-tile}
-  uint8_t* sStat = ring + C::NSK * 2 * C::SUB_BYTES;   // 64 rows of statistics, k step st of the operand for stage st
-  uint8_t* sOnes = sStat + C::STAT_BYTES;              // eight rows: k step 0 picks LSE, step 1 Delta
-  uint8_t* sOut = sOnes + C::ONES_BYTES;               // [EW][32 rows][64 B]
-  uint64_t* bars = (uint64_t*)(sOut + C::EW * C::OUT_BYTES);
+  uint8_t* ring = sV + C::TILE_BYTES;                 // [NS] x {Q sub-tile, dO sub-tile}
+  uint8_t* sStat = ring + C::NS * 2 * C::SUB_BYTES;   // 64 rows of statistics, k step st of the operand for stage st
+  uint8_t* sOnes = sStat + C::STAT_BYTES;             // eight rows: k step 0 picks LSE, step 1 Delta
+  uint8_t* sOut = sOnes + C::ONES_BYTES;              // 128 key rows x 64 queries of dS^T
+  uint64_t* bars = (uint64_t*)(sOut + C::OUT_BYTES);
   uint64_t* kv_full = bars;                 // 1
-  uint64_t* q_full = bars + 1;              // NSK
-  uint64_t* q_empty = q_full + C::NSK;       // NSK
-  uint64_t* sdp_full = q_empty + C::NSK;     // 2
-  uint64_t* p_full = sdp_full + 2;          // 2
-  uint64_t* acc_done = p_full + 2;          // 1
-  uint64_t* a_ready = acc_done + 1;         // 1: K and V copied into TMEM
+  uint64_t* q_full = bars + 1;              // NS
+  uint64_t* q_empty = q_full + C::NS;       // NS
+  uint64_t* s_full = q_empty + C::NS;       // the rest: 1 each, completed once per sub-tile
+  uint64_t* dp_full = s_full + 1;
+  uint64_t* p_full = s_full + 2;
+  uint64_t* ds_full = s_full + 3;
+  uint64_t* out_empty = s_full + 4;
+  uint64_t* acc_done = s_full + 5;          // once
+  uint64_t* a_ready = s_full + 6;           // once: K and V copied into TMEM
   uint32_t* tmem_slot = (uint32_t*)(a_ready + 1);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // early key tiles are the longest when causal; the 128-wide kernel is at its register cap and spills with the grouped
-  // order (8 x 16 x 4096: 1.37 -> 1.5 ms), so it keeps the grid's
-  int kv_tile = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
-  if (HD == 64) block_of(args, kv_tile, h, b);
+  int kv_tile, h, b;                        // early key tiles are the longest when causal
+  block_of(args, kv_tile, h, b);
   const int kv0 = kv_tile * BKV;
   const int num_sub = (args.Sq + BSUB - 1) / BSUB;
   const int i_begin = args.causal ? kv_tile * (BKV / BSUB) : 0;
   const int n_it = max(num_sub - i_begin, 0);
 
+      const float* lse = args.LSE + ((long long)b * args.H + h) * args.Sq;
+      const float* delta = args.Delta + ((long long)b * args.H + h) * args.Sq;
+      float nl[2], nd[2];
+      auto read_stats = [&](int it) {
+  #pragma unroll
+        for (int i = 0; i < 2; i++) {
+          const int q = (i_begin + it) * BSUB + lane + 32 * i;
+          nl[i] = q < args.Sq ? __ldg(lse + q) : -INFINITY;
+          nd[i] = q < args.Sq ? __ldg(delta + q) : 0.f;
+        }
+      };
+  if (warp == 0) read_stats(0);                // (used by the producer warp only)
+  auto load_stage = [&](int it, int st) {      // Q and dO of a sub-tile, by one thread
+    const int q0 = (i_begin + it) * BSUB;
+    mbar_expect_tx(&q_full[st], 2 * C::SUB_BYTES);
+    uint8_t* sQ = ring + st * 2 * C::SUB_BYTES;
+    uint8_t* sdO = sQ + C::SUB_BYTES;
+#pragma unroll
+    for (int c = 0; c < C::CH; c++) {
+      tma_load_4d(sQ + c * BSUB * 128, &tmQ, &q_full[st], c * 64, q0, h, b);
+      tma_load_4d(sdO + c * BSUB * 128, &tmdO, &q_full[st], c * 64, q0, h, b);
+    }
+  };
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
-    for (int i = 0; i < C::NSK; i++) {
+    for (int i = 0; i < C::NS; i++) {
       mbar_init(&q_full[i], 1 + 32);  // the TMA transaction + the 32 lanes that stage the row statistics
       mbar_init(&q_empty[i], 1);
     }
-    for (int i = 0; i < 2; i++) { mbar_init(&sdp_full[i], 1); mbar_init(&p_full[i], 8); }
+    mbar_init(s_full, 1);
+    mbar_init(dp_full, 1);
+    mbar_init(p_full, C::EW);
+    mbar_init(ds_full, C::EW);
+    mbar_init(out_empty, args.dS ? 2 : 1);   // the MMAs that read the tile and its TMA store
     mbar_init(acc_done, 1);
     mbar_init(a_ready, 8);
     *abort_flag = 0;
     mbar_fence_init();
+    // the loads of the tile and of the first stages start before anything else is ready
+    fence_proxy_async_smem();
+    mbar_expect_tx(kv_full, 2 * C::TILE_BYTES);
+#pragma unroll
+    for (int c = 0; c < C::CH; c++) {
+      tma_load_4d(sK + c * 128 * 128, &tmK, kv_full, c * 64, kv0, h, b);
+      tma_load_4d(sV + c * 128 * 128, &tmV, kv_full, c * 64, kv0, h, b);
+    }
+    if (n_it > 0) load_stage(0, 0);
+  } else if (warp == 2) {
+    if (lane < 4) tma_prefetch_desc(lane == 0 ? &tmK : lane == 1 ? &tmV : lane == 2 ? &tmQ : &tmdO);
+    else if (lane < 7) tma_prefetch_desc(lane == 4 ? &tmdK : lane == 5 ? &tmdV : &tmDS);
   }
   for (int i = threadIdx.x; i < C::STAT_BYTES / 16; i += C::THREADS) reinterpret_cast<uint4*>(sStat)[i] = make_uint4(0u, 0u, 0u, 0u);
   if (threadIdx.x < 64) {
@@ -659,44 +734,29 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    // ---- producer: TMA for the tiles (lane 0), row statistics by all lanes ----
-    if (lane == 0) {
-      mbar_expect_tx(kv_full, 2 * C::TILE_BYTES);
-#pragma unroll
-      for (int c = 0; c < C::CH; c++) {
-        tma_load_4d(sK + c * 128 * 128, &tmK, kv_full, c * 64, kv0, h, b);
-        tma_load_4d(sV + c * 128 * 128, &tmV, kv_full, c * 64, kv0, h, b);
-      }
-    }
-    const long long stat0 = ((long long)b * args.H + h) * args.Sq;
+    // ---- producer: TMA for the sub-tiles (lane 0), row statistics by all lanes, read one sub-tile ahead ----
+    if (lane == 0)
+      for (int it = 1; it < min(n_it, C::NS); it++) load_stage(it, it);
     int st = 0;
     uint32_t ph = 0;
     for (int it = 0; it < n_it; it++) {
-      int ok = 1;
-      if (lane == 0) ok = mbar_wait(&q_empty[st], ph ^ 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 11);
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (!ok) break;
-      const int q0 = (i_begin + it) * BSUB;
-      if (lane == 0) {
-        mbar_expect_tx(&q_full[st], 2 * C::SUB_BYTES);
-        uint8_t* sQ = ring + st * 2 * C::SUB_BYTES;
-        uint8_t* sdO = sQ + C::SUB_BYTES;
-#pragma unroll
-        for (int c = 0; c < C::CH; c++) {
-          tma_load_4d(sQ + c * BSUB * 128, &tmQ, &q_full[st], c * 64, q0, h, b);
-          tma_load_4d(sdO + c * BSUB * 128, &tmdO, &q_full[st], c * 64, q0, h, b);
-        }
+      const float l[2] = {nl[0], nl[1]}, d[2] = {nd[0], nd[1]};
+      read_stats(it + 1);
+      if (it >= C::NS) {
+        int ok = 1;
+        if (lane == 0) ok = mbar_wait(&q_empty[st], ph ^ 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 11);
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+        if (!ok) break;
+        if (lane == 0) load_stage(it, st);
       }
 #pragma unroll
       for (int i = 0; i < 2; i++) {
-        const int row = lane + 32 * i, q = q0 + row;
-        const bool in = q < args.Sq;
-        const uint4 v = stat_row(in ? __ldg(args.LSE + stat0 + q) : -INFINITY, in ? __ldg(args.Delta + stat0 + q) : 0.f, args.inv_scale);
-        *reinterpret_cast<uint4*>(sStat + row * 128 + (((uint32_t)(2 * st) ^ ((uint32_t)row & 7u)) << 4)) = v;
+        const int row = lane + 32 * i;
+        *reinterpret_cast<uint4*>(sStat + row * 128 + (((uint32_t)(2 * st) ^ ((uint32_t)row & 7u)) << 4)) = stat_row(l[i], d[i], args.inv_scale);
       }
       fence_proxy_async_smem();
       mbar_arrive(&q_full[st]);
-      if (++st == C::NSK) { st = 0; ph ^= 1; }
+      if (++st == C::NS) { st = 0; ph ^= 1; }
     }
   } else if (warp == 1) {
     if (elect_one()) {
@@ -704,207 +764,226 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       const uint32_t idesc_s = make_idesc(1u, fmt, false, false, 128, BSUB);
       const uint32_t idesc_acc = make_idesc(1u, fmt, false, true, 128, HD);
       const uint32_t idesc_stat = make_idesc(1u, 1u, false, false, 128, BSUB);
-      const uint32_t ka = smem_u32(sK), va = smem_u32(sV), stat = smem_u32(sStat), ones = smem_u32(sOnes);
+      const uint32_t ones = smem_u32(sOnes), stat = smem_u32(sStat);
       bool ok = mbar_wait(kv_full, 0, abort_flag, args.status, ST_ATTN_TIMEOUT, 12);
       if (ok && C::KV_IN_TMEM) {
         ok = mbar_wait(a_ready, 0, abort_flag, args.status, ST_ATTN_TIMEOUT, 18);
         tc_fence_after();
       }
-      int st_s = 0;        // ring stage of the next S / dP issue
-      uint32_t ph_s = 0;
-      auto issue_sdp = [&](int it) {
-        if (!mbar_wait(&q_full[st_s], ph_s, abort_flag, args.status, ST_ATTN_TIMEOUT, 13)) return false;
-        tc_fence_after();
-        const uint32_t qa = smem_u32(ring + st_s * 2 * C::SUB_BYTES), ga = qa + C::SUB_BYTES;
-        const uint32_t d = tmem_base + (it % C::NBUF) * 128;
-        // two independent accumulation chains, interleaved so that an MMA never has to wait
-        // for the one just before it
+      // S^T = K Q^T - LSE / scale (tile sK, sub-tile at 0) or dP^T = V dO^T - Delta (sV, second sub-tile) of the sub-tile in a stage
+      auto issue = [&](int st, int which) {
+        const uint32_t sub = smem_u32(ring + st * 2 * C::SUB_BYTES) + which * C::SUB_BYTES;
+        const uint32_t tile = smem_u32(sK) + which * C::TILE_BYTES;
+        const uint32_t d = tmem_base + (which ? C::COL_DP : C::COL_S);
 #pragma unroll
         for (int k = 0; k < HD / 16; k++) {
-          if (C::KV_IN_TMEM) {
-            tc_mma_f16_ts(d, tmem_base + C::COL_KT + k * 8, kdesc_sub(qa, k), idesc_s, k != 0);
-            tc_mma_f16_ts(d + 64, tmem_base + C::COL_VT + k * 8, kdesc_sub(ga, k), idesc_s, k != 0);
-          } else {
-            tc_mma_f16(d, kdesc(ka, k), kdesc_sub(qa, k), idesc_s, k != 0);       // S^T = K Q^T
-            tc_mma_f16(d + 64, kdesc(va, k), kdesc_sub(ga, k), idesc_s, k != 0);  // dP^T = V dO^T
-          }
+          if (C::KV_IN_TMEM) tc_mma_f16_ts(d, tmem_base + (which ? C::COL_V : C::COL_K) + k * 8, kdesc_sub(sub, k), idesc_s, k != 0);
+          else tc_mma_f16(d, kdesc(tile, k), kdesc_sub(sub, k), idesc_s, k != 0);
         }
-        tc_mma_f16(d, make_smem_desc_sw128(ones, 16, 0), kdesc_sub(stat, st_s), idesc_stat, 1u);             // S^T - LSE / scale
-        tc_mma_f16(d + 64, make_smem_desc_sw128(ones + 32, 16, 0), kdesc_sub(stat, st_s), idesc_stat, 1u);   // dP^T - Delta
-        tc_commit(&sdp_full[it % C::NBUF]);
-        if (++st_s == C::NSK) { st_s = 0; ph_s ^= 1; }
-        return true;
+        tc_mma_f16(d, make_smem_desc_sw128(ones + which * 32, 16, 0), kdesc_sub(stat, st), idesc_stat, 1u);
+        tc_commit(which ? dp_full : s_full);
+      };
+      // dV += P^T dO (which = 0) or dK += dS^T Q (1).  P^T: each elementwise warp left CW / 2 packed columns at the start of its
+      // own CW, so a step of 16 queries reads from there; dS^T: from the tile in shared memory
+      auto accumulate = [&](int st, int which, bool first) {
+        const uint32_t sub = smem_u32(ring + st * 2 * C::SUB_BYTES) + (which ? 0 : C::SUB_BYTES);
+        const uint32_t d = tmem_base + (which ? C::COL_ACC1 : C::COL_ACC0);
+#pragma unroll
+        for (int k = 0; k < BSUB / 16; k++) {
+          if (which) tc_mma_f16(d, kdesc(smem_u32(sOut), k), mndesc_sub(sub, k), idesc_acc, !first || k != 0);
+          else tc_mma_f16_ts(d, tmem_base + C::COL_S + k * 16 / C::CW * C::CW + k * 16 % C::CW / 2, mndesc_sub(sub, k), idesc_acc, !first || k != 0);
+        }
       };
       long long* tr = (blockIdx.x | blockIdx.y | blockIdx.z) == 0 ? args.trace : nullptr;
       int ntr = 0;
       trace_stamp(tr, 0, ntr);
-      if (ok && n_it > 0) ok = issue_sdp(0);
-      int st = 0;
+      if (ok && n_it > 0) {
+        ok = mbar_wait(&q_full[0], 0, abort_flag, args.status, ST_ATTN_TIMEOUT, 13);
+        if (ok) {
+          tc_fence_after();
+          issue(0, 0);
+          issue(0, 1);
+        }
+      }
+      int st = 0, nst = 1;
+      uint32_t nph = 0;        // of the next sub-tile's stage
       for (int it = 0; it < n_it && ok; it++) {
-        // two buffers: the next sub-tile's S / dP are issued before this one's P / dS are
-        // awaited; one buffer: they follow this sub-tile's accumulation MMAs
-        if (C::NBUF == 2 && it + 1 < n_it) {
-          ok = issue_sdp(it + 1);
-          if (!ok) break;
-        }
-        trace_stamp(tr, 0, ntr);  // S / dP of the next sub-tile issued
-        const int bb = it % C::NBUF;
-        ok = mbar_wait(&p_full[bb], (it / C::NBUF) & 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 14);
+        const uint32_t ph = it & 1;
+        const bool more = it + 1 < n_it;
+        ok = mbar_wait(p_full, ph, abort_flag, args.status, ST_ATTN_TIMEOUT, 14);
         if (!ok) break;
-        trace_stamp(tr, 0, ntr);  // P / dS of this sub-tile ready
+        trace_stamp(tr, 0, ntr);  // P ready
         tc_fence_after();
-        const uint32_t qa = smem_u32(ring + st * 2 * C::SUB_BYTES), ga = qa + C::SUB_BYTES;
-        const uint32_t pt = tmem_base + bb * 128;
-        // each elementwise warp left 16 packed columns at the start of its own 32-column
-        // range, so MMA step k reads from (k / 2) * 32 + (k % 2) * 8
-#pragma unroll
-        for (int k = 0; k < BSUB / 16; k++) {
-          tc_mma_f16_ts(tmem_base + C::COL_ACC0, pt + (k >> 1) * 32 + (k & 1) * 8, mndesc_sub(ga, k), idesc_acc,
-                        (it | k) != 0);  // dV += P^T dO
-          tc_mma_f16_ts(tmem_base + C::COL_ACC1, pt + 64 + (k >> 1) * 32 + (k & 1) * 8, mndesc_sub(qa, k),
-                        idesc_acc, (it | k) != 0);  // dK += dS^T Q
+        accumulate(st, 0, it == 0);
+        if (more) {
+          ok = mbar_wait(&q_full[nst], nph, abort_flag, args.status, ST_ATTN_TIMEOUT, 13);
+          if (!ok) break;
+          tc_fence_after();
+          issue(nst, 0);
         }
+        ok = mbar_wait(ds_full, ph, abort_flag, args.status, ST_ATTN_TIMEOUT, 20);
+        if (!ok) break;
+        trace_stamp(tr, 0, ntr);  // dS ready
+        tc_fence_after();
+        accumulate(st, 1, it == 0);
         tc_commit(&q_empty[st]);
-        if (it == n_it - 1) tc_commit(acc_done);
-        if (++st == C::NSK) st = 0;
-        if (C::NBUF == 1 && it + 1 < n_it) ok = issue_sdp(it + 1);
+        tc_commit(out_empty);
+        if (more) issue(nst, 1);
+        else tc_commit(acc_done);
+        st = nst;
+        if (++nst == C::NS) { nst = 0; nph ^= 1; }
       }
     }
     __syncwarp();
+  } else if (warp == 2 + C::EW) {
+    // ---- dS^T out: one TMA store of 128 rows x 128 bytes per sub-tile ----
+    if (args.dS && elect_one()) {
+      for (int it = 0; it < n_it; it++) {
+        if (!mbar_wait(ds_full, it & 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 27)) break;
+        tma_store_3d(&tmDS, sOut, (i_begin + it) * BSUB, kv0, b * args.H + h);
+        tma_store_commit();
+        tma_store_wait_read<0>();
+        mbar_arrive(out_empty);
+      }
+      tma_store_wait<0>();   // shared memory must outlive the stores that read from it
+    }
+    __syncwarp();
   } else {
+    constexpr int CW = C::CW;
     const int e = warp - 2;
-    const int group = e >> 3;                // sub-tiles it with it % NBUF == group, TMEM buffer `group`
-    const int half = (e >> 2) & 1;           // which 32 of the sub-tile's 64 query columns
+    const int cg = e >> 2;                   // which CW of the sub-tile's 64 query columns
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;       // key row inside the tile
     const int kvrow = kv0 + r;
     const bool row_dead = kvrow >= args.Sk;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
-    const uint32_t my = lane_addr + group * 128 + half * 32;
+    const uint32_t s_addr = lane_addr + C::COL_S + cg * CW, dp_addr = lane_addr + C::COL_DP + cg * CW;
     bool ok = true;
-    if (C::KV_IN_TMEM && group == 0) {
-      // the eight warps of group 0 copy K (half 0) and V (half 1) into TMEM once
+    if (C::KV_IN_TMEM && cg < 2) {
       ok = mbar_wait(kv_full, 0, abort_flag, args.status, ST_ATTN_TIMEOUT, 19);
       if (ok) {
-        tile_row_to_tmem<HD>(half == 0 ? sK : sV, r, lane_addr, half == 0 ? C::COL_KT : C::COL_VT);
+        tile_row_to_tmem<HD>(cg == 0 ? sK : sV, r, lane_addr, cg == 0 ? C::COL_K : C::COL_V);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(a_ready);
       }
     }
     long long* tr = ((blockIdx.x | blockIdx.y | blockIdx.z) == 0 && (e & 7) == 0 && lane == 0) ? args.trace : nullptr;
+    const int tl = 1 + (e >> 3);
     int ntr = 0;
-    uint8_t* out = sOut + e * C::OUT_BYTES;
-    const uint32_t out_row = smem_u32(out) + (uint32_t)lane * 64u, swz = ((uint32_t)lane >> 1) & 3u;
-    // this warp's 32 key rows x 32 queries of dS^T: through shared memory and one TMA store (a store of 64 bytes per thread took
-    // 55 clocks of the memory pipe per instruction, 890 per 128 x 64 block)
-    auto spill = [&](const uint32_t(&v)[16], int it) {
-      if (lane == 0) tma_store_wait_read<0>();
-      __syncwarp();
-#pragma unroll
-      for (int j = 0; j < 4; j++)
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(out_row + (((uint32_t)j ^ swz) << 4)), "r"(v[4 * j]),
-                     "r"(v[4 * j + 1]), "r"(v[4 * j + 2]), "r"(v[4 * j + 3])
-                     : "memory");
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) {
-        tma_store_3d(&tmDS, out, (i_begin + it) * BSUB + half * 32, kv0 + quarter * 32, b * args.H + h);
-        tma_store_commit();
-      }
-    };
-    for (int it = group; it < n_it; it += C::NBUF) {
-      trace_stamp(tr, 1 + group, ntr);  // starts waiting
-      ok = mbar_wait(&sdp_full[group], (it / C::NBUF) & 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 15);
-      if (!ok) break;
-      trace_stamp(tr, 1 + group, ntr);  // scores ready
-      tc_fence_after();
-      uint32_t rs[32], rd[32];
-      tmem_ld32(my, rs);
-      tmem_ld32(my + 64, rd);
-      tmem_ld_wait();
-      trace_stamp(tr, 1 + group, ntr);  // loaded
-      const int q0 = (i_begin + it) * BSUB + half * 32;  // first query column of this thread
-      // masking is needed on the diagonal sub-tiles and for key rows past the end; the common
-      // case runs a loop without any of the compare / select instructions
-      // The warp's 32 key rows against its 32 query columns: entirely above the diagonal
-      // (everything masked: zeros, no arithmetic), entirely on or below it (no masking), or
-      // the 32 x 32 block the diagonal crosses (per-element test).
+    const unsigned long long sl2 = pair(__float_as_uint(args.scale_log2), __float_as_uint(args.scale_log2));
+    const unsigned long long sc2 = pair(__float_as_uint(args.scale), __float_as_uint(args.scale));
+    const uint32_t out_row = smem_u32(sOut) + (uint32_t)r * 128u;
+    for (int it = 0; it < n_it; it++) {
+      const uint32_t ph = it & 1;
+      const int q0 = (i_begin + it) * BSUB + cg * CW;  // first query column of this thread
+      // The warp's 32 key rows against its CW query columns: entirely above the diagonal (everything masked: zeros, no
+      // arithmetic), entirely on or below it (no masking), or a block that the diagonal crosses (per-element test).
       const int rel = kv0 + quarter * 32 - q0;  // first key row minus first query column
-      const bool all_masked = args.causal && rel > 31;
+      const bool all_masked = args.causal && rel > CW - 1;
       const bool masked = __any_sync(0xffffffffu, row_dead) || (args.causal && rel + 31 > 0);
-      if (all_masked) {
-        uint32_t z[16];
+      uint32_t in[CW], pk[CW / 2];
+      float pr[CW];
+      trace_stamp(tr, tl, ntr);
+      ok = mbar_wait(s_full, ph, abort_flag, args.status, ST_ATTN_TIMEOUT, 15);
+      if (!ok) break;
+      trace_stamp(tr, tl, ntr);  // scores ready
+      tc_fence_after();
+      if (!all_masked) {
+        tmem_ld_cols<CW>(s_addr, in);
+        tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 16; i++) z[i] = 0u;
-        tmem_st16(my, z);
-        tmem_st16(my + 64, z);
-        if (args.dS) spill(z, it);
-        tmem_st_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&p_full[group]);
-        continue;
-      }
-      uint32_t pp[16], pd[16];
-      const unsigned long long sl2 = pair(__float_as_uint(args.scale_log2), __float_as_uint(args.scale_log2));
-      const unsigned long long sc2 = pair(__float_as_uint(args.scale), __float_as_uint(args.scale));
-      auto body = [&](auto use_mask) {
-#pragma unroll
-        for (int g = 0; g < 16; g++) {
-          const unsigned long long x = fmul2(pair(rs[2 * g], rs[2 * g + 1]), sl2);
-          float p0 = exp2f(lo_of(x)), p1 = exp2f(hi_of(x));
-          if (decltype(use_mask)::value) {
-            if (row_dead || (args.causal && kvrow > q0 + 2 * g)) p0 = 0.f;
-            if (row_dead || (args.causal && kvrow > q0 + 2 * g + 1)) p1 = 0.f;
-          }
-          const unsigned long long q = fmul2(pair(__float_as_uint(p0), __float_as_uint(p1)), fmul2(pair(rd[2 * g], rd[2 * g + 1]), sc2));
-          pp[g] = pack16t<BF>(p0, p1);
-          pd[g] = pack16t<BF>(lo_of(q), hi_of(q));
+        for (int g = 0; g < CW / 2; g++) {
+          const unsigned long long x = fmul2(pair(in[2 * g], in[2 * g + 1]), sl2);
+          pr[2 * g] = exp2f(lo_of(x));
+          pr[2 * g + 1] = exp2f(hi_of(x));
         }
-      };
-      if (masked) body(std::true_type{});
-      else body(std::false_type{});
+        if (masked) {
+#pragma unroll
+          for (int g = 0; g < CW; g++)
+            if (row_dead || (args.causal && kvrow > q0 + g)) pr[g] = 0.f;
+        }
+      } else {
+#pragma unroll
+        for (int g = 0; g < CW; g++) pr[g] = 0.f;
+      }
+#pragma unroll
+      for (int g = 0; g < CW / 2; g++) pk[g] = pack16t<BF>(pr[2 * g], pr[2 * g + 1]);
       // each warp overwrites only columns it has read itself
-      trace_stamp(tr, 1 + group, ntr);  // computed
-      tmem_st16(my, pp);
-      tmem_st16(my + 64, pd);
+      tmem_st_cols<CW / 2>(s_addr, pk);
       tmem_st_wait();
-      trace_stamp(tr, 1 + group, ntr);  // stored
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[group]);
-      if (args.dS) spill(pd, it);       // behind the arrival: the accumulation does not wait for it
+      if (lane == 0) mbar_arrive(p_full);
+      trace_stamp(tr, tl, ntr);  // P stored
+      ok = mbar_wait(dp_full, ph, abort_flag, args.status, ST_ATTN_TIMEOUT, 17);
+      if (!ok) break;
+      trace_stamp(tr, tl, ntr);  // dP ready
+      tc_fence_after();
+      if (!all_masked) {
+        tmem_ld_cols<CW>(dp_addr, in);
+        tmem_ld_wait();
+#pragma unroll
+        for (int g = 0; g < CW / 2; g++) {
+          const unsigned long long q = fmul2(pair(__float_as_uint(pr[2 * g]), __float_as_uint(pr[2 * g + 1])), fmul2(pair(in[2 * g], in[2 * g + 1]), sc2));
+          pk[g] = pack16t<BF>(lo_of(q), hi_of(q));
+        }
+      }
+      ok = mbar_wait(out_empty, ph ^ 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 30);
+      if (!ok) break;
+#pragma unroll
+      for (int j = 0; j < CW / 8; j++)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(out_row + (((uint32_t)(cg * (CW / 8) + j) ^ ((uint32_t)r & 7u)) << 4)),
+                     "r"(pk[4 * j]), "r"(pk[4 * j + 1]), "r"(pk[4 * j + 2]), "r"(pk[4 * j + 3])
+                     : "memory");
+      tc_fence_before();
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ds_full);
+      trace_stamp(tr, tl, ntr);  // dS stored
     }
     if (ok && n_it > 0) ok = mbar_wait(acc_done, 0, abort_flag, args.status, ST_ATTN_TIMEOUT, 16);
     if (ok) {
       tc_fence_after();
       constexpr int W = HD * 4 / C::EW;  // columns of dV / dK per warp
-      const int cw = (group * 2 + half) * W;
-      uint16_t* dvrow = (uint16_t*)args.dV + (long long)b * args.dv_sb + (long long)kvrow * args.dv_ss +
-                        (long long)h * args.dv_sh + cw;
-      uint16_t* dkrow = (uint16_t*)args.dK + (long long)b * args.dk_sb + (long long)kvrow * args.dk_ss +
-                        (long long)h * args.dk_sh + cw;
-      uint32_t ra[W], rb[W];
-      float v[W];
-      if (n_it > 0) {
-        if constexpr (W == 32) {
-          tmem_ld32(lane_addr + C::COL_ACC0 + cw, ra);
-          tmem_ld32(lane_addr + C::COL_ACC1 + cw, rb);
+      const int cw = cg * W;
+      // through the ring, whose loads have all been consumed, and TMA stores of whole rows (rows and columns behind the tensors' ends
+      // are clipped; 16-byte stores of 32 rows at a time took 3 000 clocks)
+      static_assert(2 * C::TILE_BYTES <= C::NS * 2 * C::SUB_BYTES, "the gradient tiles reuse the ring");
+#pragma unroll
+      for (int o = 0; o < 2; o++) {
+        uint32_t in[W];
+        if (n_it > 0) {
+          tmem_ld_cols<W>(lane_addr + (o ? C::COL_ACC1 : C::COL_ACC0) + cw, in);
+          tmem_ld_wait();
         } else {
-          tmem_ld16(lane_addr + C::COL_ACC0 + cw, ra);
-          tmem_ld16(lane_addr + C::COL_ACC1 + cw, rb);
+#pragma unroll
+          for (int i = 0; i < W; i++) in[i] = 0u;
         }
-        tmem_ld_wait();
+        const uint32_t row = smem_u32(ring) + o * C::TILE_BYTES + cw / 64 * (128 * 128) + (uint32_t)r * 128u;
+#pragma unroll
+        for (int j = 0; j < W / 8; j++) {
+          uint32_t w[4];
+#pragma unroll
+          for (int i = 0; i < 4; i++) w[i] = pack16t<BF>(__uint_as_float(in[8 * j + 2 * i]), __uint_as_float(in[8 * j + 2 * i + 1]));
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row + (((uint32_t)(cw % 64 / 8 + j) ^ ((uint32_t)r & 7u)) << 4)),
+                       "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
+                       : "memory");
+        }
       }
+      fence_proxy_async_smem();
+      asm volatile("bar.sync 1, %0;" ::"n"(C::EW * 32) : "memory");
+      if (threadIdx.x == 64) {
 #pragma unroll
-      for (int i = 0; i < W; i++) v[i] = n_it > 0 ? __uint_as_float(ra[i]) : 0.f;
-      if (!row_dead) store_row16_lim<W>(dvrow, v, BF, args.D - cw);
-#pragma unroll
-      for (int i = 0; i < W; i++) v[i] = n_it > 0 ? __uint_as_float(rb[i]) : 0.f;
-      if (!row_dead) store_row16_lim<W>(dkrow, v, BF, args.D - cw);
+        for (int c = 0; c < C::CH; c++)
+          if (c * 64 < args.D) {
+            tma_store_4d(&tmdV, ring + c * 128 * 128, c * 64, kv0, h, b);
+            tma_store_4d(&tmdK, ring + C::TILE_BYTES + c * 128 * 128, c * 64, kv0, h, b);
+          }
+        tma_store_commit();
+        tma_store_wait<0>();
+      }
     }
-    if (args.dS && lane == 0) tma_store_wait<0>();   // shared memory must outlive the stores that read from it
   }
   tc_fence_before();
   __syncthreads();
@@ -1302,8 +1381,9 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
 struct BwdMaps {
   CUtensorMap q128, k128, v128, g128;  // 128-row boxes (resident tiles)
   CUtensorMap q64, k64, v64, g64;      // 64-row boxes (streamed sub-tiles)
+  CUtensorMap dk, dv;                  // 128-row boxes
   CUtensorMap ds;                      // the dS^T spill: (query, key, batch*head), boxes of 64 x 64
-  CUtensorMap ds_out;                  // the same with boxes of 32 x 32, as the dK / dV kernel's warps write it
+  CUtensorMap ds_out;                  // the same with boxes of 64 x 128, as the dK / dV kernel writes it
 };
 
 int g_fa_dual = 1;
@@ -1311,14 +1391,15 @@ int g_fa_dual = 1;
 template <int HD, bool BF, bool DUAL>
 int launch_bwd(const BwdMaps& m, const AttnArgs& a, cudaStream_t s) {
   using C = BwdCfg<HD, DUAL>;
+  using KV = KvCfg<HD, DUAL>;
   static bool configured = false;
   if (!configured) {
-    GB_CUDA_OK(cudaFuncSetAttribute(fa_bwd_dkv_kernel<HD, BF, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES_KV));
+    GB_CUDA_OK(cudaFuncSetAttribute(fa_bwd_dkv_kernel<HD, BF, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, KV::SMEM_BYTES));
     GB_CUDA_OK(cudaFuncSetAttribute(fa_bwd_dq_kernel<HD, BF, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
     configured = true;
   }
   dim3 gkv((a.Sk + BKV - 1) / BKV, a.H, a.B);
-  fa_bwd_dkv_kernel<HD, BF, DUAL><<<gkv, C::THREADS, C::SMEM_BYTES_KV, s>>>(m.q64, m.k128, m.v128, m.g64, m.ds_out, a);
+  fa_bwd_dkv_kernel<HD, BF, DUAL><<<gkv, KV::THREADS, KV::SMEM_BYTES, s>>>(m.q64, m.k128, m.v128, m.g64, m.ds_out, m.dk, m.dv, a);
   GB_CUDA_OK(cudaGetLastError());
   dim3 gq((a.Sq + BQ - 1) / BQ, a.H, a.B);
   if (a.dS) {
@@ -1500,6 +1581,8 @@ GB_EXPORT int gb_flash_bwd_ws(int dtype, const void* q, const void* k, const voi
   if ((rc = make_qkv_map(&m.k64, k, a.in_bf16, B, H, Sk, D, strides[3], strides[4], strides[5], 64))) return rc;
   if ((rc = make_qkv_map(&m.v64, v, a.in_bf16, B, H, Sk, D, strides[6], strides[7], strides[8], 64))) return rc;
   if ((rc = make_qkv_map(&m.g64, dout, a.in_bf16, B, H, Sq, D, strides[9], strides[10], strides[11], 64))) return rc;
+  if ((rc = make_qkv_map(&m.dk, dk, a.in_bf16, B, H, Sk, D, strides[15], strides[16], strides[17], 128))) return rc;
+  if ((rc = make_qkv_map(&m.dv, dv, a.in_bf16, B, H, Sk, D, strides[18], strides[19], strides[20], 128))) return rc;
   if (ws != nullptr && ws_bytes >= gb_flash_bwd_ws_bytes(B, H, Sq, Sk) && !((uintptr_t)ws & 31) &&
       gb_flash_bwd_ws_bytes(B, H, Sq, Sk) <= (1LL << 32)) {
     a.dS = ws;
@@ -1511,9 +1594,9 @@ GB_EXPORT int gb_flash_bwd_ws(int dtype, const void* q, const void* k, const voi
     if ((rc = gbh::encode_tmap(&m.ds, a.in_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
                                4, ws, dims, st, box, CU_TENSOR_MAP_SWIZZLE_128B)))
       return rc;
-    uint32_t box_out[3] = {32, 32, 1};
+    uint32_t box_out[3] = {64, 128, 1};
     if ((rc = gbh::encode_tmap(&m.ds_out, a.in_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                               3, ws, dims, st, box_out, CU_TENSOR_MAP_SWIZZLE_64B)))
+                               3, ws, dims, st, box_out, CU_TENSOR_MAP_SWIZZLE_128B)))
       return rc;
   }
   if (D > 64)

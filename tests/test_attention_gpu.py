@@ -99,3 +99,26 @@ def test_backward_with_and_without_the_dS_workspace(B, Sq, Sk, H, D, causal, sta
     for got in (g_spill[0], g_two[0]):
         assert (got.float() - qf.grad).abs().max().item() < 0.01 * qf.grad.abs().max().item() + 0.03
     assert (g_spill[0].float() - g_two[0].float()).abs().max().item() < 0.02 * qf.grad.abs().max().item() + 0.01
+
+
+@pytest.mark.parametrize("scale", [1e-33, 3e-38, 0.3, 4.0])
+@pytest.mark.parametrize("Sq,Sk,D,causal", [(1, 1, 64, False), (65, 129, 64, False), (191, 191, 128, True), (257, 63, 128, False)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_backward_folds_the_row_statistics(scale, Sq, Sk, D, causal, dtype, status_ok):
+    """The dK / dV kernel adds -LSE / scale to the scores: also where that quotient would overflow, at edges of its
+    64-query steps and 128-key tiles, and where large scores make the statistics large beside their differences."""
+    torch.manual_seed(Sq)
+    q = torch.randn(2, Sq, 2, D, device="cuda", dtype=dtype)
+    k, v = (torch.randn(2, Sk, 2, D, device="cuda", dtype=dtype) for _ in range(2))
+    out, lse = flash_fwd(q, k, v, causal, scale)
+    do = torch.randn_like(out)
+    grads = flash_bwd(q, k, v, out, do, lse, causal, scale)[:3]
+    qd, kd, vd = (t.double().requires_grad_(True) for t in (q, k, v))
+    attention_ref(qd, kd, vd, causal, scale).backward(do.double())
+    # roundings to the inputs' type of at most one unit each (2^-8 or 2^-11): P, the output inside Delta, dS and the result; the
+    # statistics take the scores, up to 4 * 4 sqrt(D) * 4 here, to fp32: 2^-24 of that in the exponent
+    unit = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    for got, want in zip(grads, (qd.grad, kd.grad, vd.grad)):
+        assert torch.isfinite(got).all()
+        floor = 1e-2 * unit * want.numel() ** 0.5          # gradients that vanish (scale 0, one key): rounding of P * (dP - Delta)
+        assert (got.double() - want).norm() <= 4 * unit * want.norm() + floor
