@@ -10,7 +10,7 @@
 // fp32 accumulation, no atomics (dQ and dK/dV are produced by two kernels so that
 // every output tile has one owner and a fixed summation order).
 //
-// Forward CTA (192 threads, two CTAs per SM) owns 128 query rows of one (batch, head):
+// Forward CTA (192 threads, two or four CTAs per SM) owns 128 query rows of one (batch, head):
 //   warp 0      TMA loads of Q once and the K / V sub-tiles of 64 keys (rings)
 //   warp 1      MMA issue: S = Q K^T into one of two TMEM score buffers, then
 //               O += P V with P read from TMEM (written there by the softmax warps)
@@ -132,28 +132,76 @@ __device__ __forceinline__ void store_row16_lim(void* dst, const float* v, int b
   }
 }
 
+// Two packed fp32 products.
+__device__ __forceinline__ unsigned long long fmul2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long pair(uint32_t lo, uint32_t hi) { return (unsigned long long)hi << 32 | lo; }
+__device__ __forceinline__ float lo_of(unsigned long long v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi_of(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ unsigned long long ffma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ unsigned long long fadd2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long pairf(float lo, float hi) { return pair(__float_as_uint(lo), __float_as_uint(hi)); }
+
+template <int N>
+__device__ __forceinline__ void tmem_ld_cols(uint32_t addr, uint32_t (&r)[N]) {
+  if constexpr (N == 32) tmem_ld32(addr, r);
+  else tmem_ld16(addr, r);
+}
+template <int N>
+__device__ __forceinline__ void tmem_st_cols(uint32_t addr, const uint32_t (&r)[N]) {
+  if constexpr (N == 16) {
+    tmem_st16(addr, r);
+  } else {
+    static_assert(N == 8, "columns");
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(addr), "r"(r[0]), "r"(r[1]),
+                 "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+  }
+}
+
+template <bool BF>
+__device__ __forceinline__ uint32_t pack16t(float a, float b) {
+  return BF ? pack_bf16(a, b) : pack_f16(a, b);
+}
+
 constexpr int BKF = 64;  // key rows per forward sub-tile
 
 // Forward tiling: 128 query rows per CTA, keys in 64-row sub-tiles.  Two score buffers of 64
 // columns and the output accumulator need 128 + HD <= 256 TMEM columns, and the shared
 // memory of one CTA stays under half an SM, so two CTAs share an SM: while the softmax warps
-// of one are busy, the tensor core serves the other.
-template <int HD>
+// of one are busy, the tensor core serves the other.  With one score buffer a head of 64 takes 128 columns, and four CTAs
+// share the SM: four softmax warps per scheduler instead of two, each with a longer chain (the next scores follow this
+// sub-tile's P V), which pays once there are CTAs enough.
+template <int HD, int NBUF_>
 struct FwdCfg {
   static constexpr int CH = HD / 64;                   // 64-column chunks per row
   static constexpr int Q_BYTES = CH * BQ * 128;        // the resident query tile
   static constexpr int SUB_BYTES = CH * BKF * 128;     // one K or V sub-tile
-  static constexpr int STAGES = HD == 64 ? 3 : 2;
+  static constexpr int NBUF = NBUF_;                   // score buffers
+  static constexpr int CTAS_PER_SM = NBUF == 1 ? 4 : 2;
+  static_assert(NBUF == 2 || HD == 64, "four CTAs share TMEM");
+  static constexpr int STAGES = NBUF == 2 && HD == 64 ? 3 : 2;
   static constexpr int SMEM_BYTES = Q_BYTES + 2 * STAGES * SUB_BYTES + 1024 + 256;
-  static constexpr int TMEM_COLS = 256;
-  static constexpr int COL_S0 = 0, COL_S1 = 64, COL_O = 128;
+  static constexpr int TMEM_COLS = NBUF == 1 ? 128 : 256;
+  static constexpr int COL_S = 0, COL_O = NBUF * BKF;
 };
 
-template <int HD, bool BF>
-__global__ void __launch_bounds__(kFwdThreads, 2)
+template <int HD, bool BF, int NBUF>
+__global__ void __launch_bounds__(kFwdThreads, FwdCfg<HD, NBUF>::CTAS_PER_SM)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-              const __grid_constant__ CUtensorMap tmV, const AttnArgs args) {
-  using C = FwdCfg<HD>;
+              const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const AttnArgs args) {
+  using C = FwdCfg<HD, NBUF>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sQ = smem;
@@ -180,6 +228,12 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   int n_kv = (args.Sk + BKF - 1) / BKF;
   if (args.causal) n_kv = min(n_kv, (q_tile + 1) * (BQ / BKF));
 
+  auto load_k = [&](int j, int st) {
+    mbar_expect_tx(&k_full[st], C::SUB_BYTES);
+#pragma unroll
+    for (int c = 0; c < C::CH; c++)
+      tma_load_4d(sK + st * C::SUB_BYTES + c * BKF * 128, &tmK, &k_full[st], c * 64, j * BKF, h, b);
+  };
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int i = 0; i < C::STAGES; i++) {
@@ -195,9 +249,14 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     }
     *abort_flag = 0;
     mbar_fence_init();
-    tma_prefetch_desc(&tmQ);
-    tma_prefetch_desc(&tmK);
-    tma_prefetch_desc(&tmV);
+    // the query tile and the first keys start before anything else is ready
+    fence_proxy_async_smem();
+    mbar_expect_tx(q_full, C::Q_BYTES);
+#pragma unroll
+    for (int c = 0; c < C::CH; c++) tma_load_4d(sQ + c * BQ * 128, &tmQ, q_full, c * 64, q0, h, b);
+    if (n_kv > 0) load_k(0, 0);
+  } else if (warp == 2 && lane < 4) {
+    tma_prefetch_desc(lane == 0 ? &tmK : lane == 1 ? &tmQ : lane == 2 ? &tmV : &tmO);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, C::TMEM_COLS);
@@ -209,18 +268,14 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (elect_one()) {
-      mbar_expect_tx(q_full, C::Q_BYTES);
-#pragma unroll
-      for (int c = 0; c < C::CH; c++) tma_load_4d(sQ + c * BQ * 128, &tmQ, q_full, c * 64, q0, h, b);
+    if (lane == 0) {
       int st = 0;
       uint32_t ph = 0;
       for (int j = 0; j < n_kv; j++) {
-        if (!mbar_wait(&k_empty[st], ph ^ 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 1)) break;
-        mbar_expect_tx(&k_full[st], C::SUB_BYTES);
-#pragma unroll
-        for (int c = 0; c < C::CH; c++)
-          tma_load_4d(sK + st * C::SUB_BYTES + c * BKF * 128, &tmK, &k_full[st], c * 64, j * BKF, h, b);
+        if (j > 0) {
+          if (!mbar_wait(&k_empty[st], ph ^ 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 1)) break;
+          load_k(j, st);
+        }
         if (!mbar_wait(&v_empty[st], ph ^ 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 2)) break;
         mbar_expect_tx(&v_full[st], C::SUB_BYTES);
 #pragma unroll
@@ -243,13 +298,13 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         if (!mbar_wait(&k_full[st_s], ph_s, abort_flag, args.status, ST_ATTN_TIMEOUT, 4)) return false;
         tc_fence_after();
         const uint32_t ka = smem_u32(sK + st_s * C::SUB_BYTES);
-        const uint32_t d = tmem_base + ((j & 1) ? C::COL_S1 : C::COL_S0);
+        const uint32_t d = tmem_base + C::COL_S + j % C::NBUF * BKF;
 #pragma unroll
         for (int k = 0; k < HD / 16; k++)
           tc_mma_f16(d, make_smem_desc_sw128(qa + (k / 4) * (BQ * 128) + (k % 4) * 32, 16, 1024),
                      make_smem_desc_sw128(ka + (k / 4) * (BKF * 128) + (k % 4) * 32, 16, 1024), idesc_s, k != 0);
         tc_commit(&k_empty[st_s]);
-        tc_commit(&s_full[j & 1]);
+        tc_commit(&s_full[j % C::NBUF]);
         if (++st_s == C::STAGES) { st_s = 0; ph_s ^= 1; }
         return true;
       };
@@ -257,128 +312,155 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       int st = 0;
       uint32_t ph = 0;
       for (int j = 0; j < n_kv && ok; j++) {
-        if (j + 1 < n_kv) {
+        if (C::NBUF == 2 && j + 1 < n_kv) {       // two buffers: the next scores before this sub-tile's P is waited for
           ok = issue_s(j + 1);
           if (!ok) break;
         }
-        const int sb = j & 1;
-        ok = mbar_wait(&p_full[sb], (j >> 1) & 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 5);
+        const int sb = j % C::NBUF;
+        ok = mbar_wait(&p_full[sb], (j / C::NBUF) & 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 5);
         if (!ok) break;
         ok = mbar_wait(&v_full[st], ph, abort_flag, args.status, ST_ATTN_TIMEOUT, 6);
         if (!ok) break;
         tc_fence_after();
         const uint32_t va = smem_u32(sV + st * C::SUB_BYTES);
-        const uint32_t p_tmem = tmem_base + (sb ? C::COL_S1 : C::COL_S0);
+        const uint32_t p_tmem = tmem_base + C::COL_S + sb * BKF;
         const uint32_t d = tmem_base + C::COL_O;
 #pragma unroll
         for (int k = 0; k < BKF / 16; k++) {
           // V is the MN-major B operand: 64-wide d chunks are BKF*128 B apart, 8-row groups
           // 1024 B apart, one MMA step covers 16 key rows.
-          tc_mma_f16_ts(d, p_tmem + k * 8, make_smem_desc_sw128(va + k * 16 * 128, BKF * 128, 1024), idesc_o,
+          tc_mma_f16_ts(d, p_tmem + (k >> 1) * 32 + (k & 1) * 8, make_smem_desc_sw128(va + k * 16 * 128, BKF * 128, 1024), idesc_o,
                         (j | k) != 0);
         }
         tc_commit(&v_empty[st]);
         tc_commit(&pv_done[sb]);
         if (++st == C::STAGES) { st = 0; ph ^= 1; }
+        if (C::NBUF == 1 && j + 1 < n_kv) ok = issue_s(j + 1);
       }
     }
     __syncwarp();
   } else {
-    // ---------------- softmax warps ----------------
+    // ---------------- softmax warps: thread = row ----------------
+    // What bounds the kernel is the chain of such a warp: the exponentials of a sub-tile, 512 clocks of its scheduler, and about
+    // as much again of waits, loads and hand-overs (MUFU 65 % busy at head size 64).  So the maximum is four chains, products and
+    // sums are packed, and the CTA's start and end are short: first loads before its barrier, O by TMA.  (Scores of the next
+    // sub-tile loaded while exponentials run, or two warps to a row: slower.)  us before -> now: (16, 12, 1024, 64) causal
+    // 66.0 -> 53.9, (6, 12, 1000 x 1531, 64) 51.9 -> 49.4, (8, 16, 4096, 128) causal 535 -> 502, (4, 16, 2048, 128) 79.7 -> 74.5.
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;  // row inside the tile
     const int qrow = q0 + r;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    const unsigned long long sl2 = pairf(args.scale_log2, args.scale_log2);
     float m_used = -INFINITY;  // in log2 units, already scaled
-    float l = 0.f;
-    bool ok = true;
-    for (int j = 0; j < n_kv; j++) {
-      const int sb = j & 1;
-      ok = mbar_wait(&s_full[sb], (j >> 1) & 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 7);
-      if (!ok) break;
+    unsigned long long l2 = 0ull;   // the row sum, as two sums
+    // sub-tiles entirely to the right of this warp's 32 rows (from q0 + 32 * quarter) contribute nothing: P = 0, running max
+    // and sum unchanged
+    const int n_live = args.causal ? min(n_kv, (q0 + quarter * 32 + 31) / BKF + 1) : n_kv;
+    uint32_t s[C::NBUF][32];
+    auto wait_scores = [&](int j) {
+      const bool ready = mbar_wait(&s_full[j % C::NBUF], (j / C::NBUF) & 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 7);
       tc_fence_after();
-      const uint32_t s_addr = lane_addr + (sb ? C::COL_S1 : C::COL_S0);
-      const int kv0 = j * BKF;
-      // this warp's 32 rows start at q0 + 32 * quarter: a sub-tile entirely to the right of
-      // them contributes nothing (P = 0, running max and sum unchanged)
-      if (args.causal && kv0 > q0 + quarter * 32 + 31) {
-        uint32_t zero[32];
-#pragma unroll
-        for (int i = 0; i < 32; i++) zero[i] = 0u;
-        tmem_st32(s_addr, zero);
-        tmem_st_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&p_full[sb]);
-        continue;
-      }
-      uint32_t rr[BKF];
-      tmem_ld32(s_addr, *reinterpret_cast<uint32_t(*)[32]>(&rr[0]));
-      tmem_ld32(s_addr + 32, *reinterpret_cast<uint32_t(*)[32]>(&rr[32]));
-      tmem_ld_wait();
-      float s[BKF];
-#pragma unroll
-      for (int i = 0; i < BKF; i++) s[i] = __uint_as_float(rr[i]);
-      const bool need_mask = (args.causal && kv0 + BKF - 1 > q0 + quarter * 32) || (kv0 + BKF > args.Sk);
-      if (need_mask) {
-#pragma unroll
-        for (int c = 0; c < BKF; c++) {
-          const int kv = kv0 + c;
-          if (kv >= args.Sk || (args.causal && kv > qrow)) s[c] = -INFINITY;
-        }
-      }
-      float mx = -INFINITY;
-#pragma unroll
-      for (int c = 0; c < BKF; c++) mx = fmaxf(mx, s[c]);
-      float m_new = fmaxf(m_used, mx * args.scale_log2);
-      if (m_new == -INFINITY) m_new = 0.f;
-      // rescale O only when the running max moved by more than 8 (a factor 256)
-      const bool need = (m_new - m_used) > 8.f;
-      float alpha = 1.f;
-      if (need) {
-        alpha = (m_used == -INFINITY) ? 0.f : exp2f(m_used - m_new);
-        m_used = m_new;
-        l *= alpha;
-      }
-      if (j > 0 && __any_sync(0xffffffffu, need)) {
-        ok = mbar_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 8);
-        if (!ok) break;
-        tc_fence_after();
-#pragma unroll
-        for (int c = 0; c < HD / 32; c++) {
-          uint32_t ro[32];
-          tmem_ld32(lane_addr + C::COL_O + c * 32, ro);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; i++) ro[i] = __float_as_uint(__uint_as_float(ro[i]) * alpha);
-          tmem_st32(lane_addr + C::COL_O + c * 32, ro);
-        }
-        tmem_st_wait();
-      }
-      float sum = 0.f;
-      uint32_t pk[BKF / 2];
-#pragma unroll
-      for (int i = 0; i < BKF / 2; i++) {
-        const float p0 = exp2f(fmaf(s[2 * i], args.scale_log2, -m_used));
-        const float p1 = exp2f(fmaf(s[2 * i + 1], args.scale_log2, -m_used));
-        sum += p0 + p1;
-        pk[i] = BF ? pack_bf16(p0, p1) : pack_f16(p0, p1);
-      }
-      tmem_st32(s_addr, *reinterpret_cast<uint32_t(*)[32]>(&pk[0]));
-      l += sum;
+      return ready;
+    };
+    auto scores_at = [&](int j) { return lane_addr + C::COL_S + j % C::NBUF * BKF; };
+    auto give_p = [&](int j) {
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[sb]);
+      if (lane == 0) mbar_arrive(&p_full[j % C::NBUF]);
+    };
+    bool ok = true;
+    for (int j = 0; j < n_live; j++) {
+      ok = wait_scores(j);
+      if (!ok) break;
+      const uint32_t s_addr = scores_at(j);
+      const int kv0 = j * BKF;
+      const bool masked = (args.causal && kv0 + BKF - 1 > q0 + quarter * 32) || kv0 + BKF > args.Sk;
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      auto load_half = [&](int g) { tmem_ld32(s_addr + g * 32, s[C::NBUF == 2 ? g : 0]); };
+      auto mask_half = [&](int g) {
+        if (masked) {
+#pragma unroll
+          for (int c = 0; c < 32; c++)
+            if (kv0 + g * 32 + c >= args.Sk || (args.causal && kv0 + g * 32 + c > qrow)) s[C::NBUF == 2 ? g : 0][c] = 0xff800000u;
+        }
+      };
+      if (C::NBUF == 2) { load_half(0); load_half(1); }
+#pragma unroll
+      for (int g = 0; g < 2; g++) {
+        if (C::NBUF == 1) load_half(g);
+        if (C::NBUF == 1 || g == 0) tmem_ld_wait();
+        mask_half(g);
+#pragma unroll
+        for (int c = 0; c < 32; c++) mx[c & 3] = fmaxf(mx[c & 3], __uint_as_float(s[C::NBUF == 2 ? g : 0][c]));
+      }
+      float m_new = fmaxf(m_used, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * args.scale_log2);
+      if (m_new == -INFINITY) m_new = 0.f;
+      // rescale O only when the running max moved by more than 8 (a factor 256)
+      const bool need = (m_new - m_used) > 8.f;
+      if (__any_sync(0xffffffffu, need)) {
+        float alpha = 1.f;
+        if (need) {
+          alpha = (m_used == -INFINITY) ? 0.f : exp2f(m_used - m_new);
+          m_used = m_new;
+          l2 = fmul2(l2, pairf(alpha, alpha));
+        }
+        if (j > 0) {
+          ok = mbar_wait(&pv_done[(j - 1) % C::NBUF], ((j - 1) / C::NBUF) & 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 8);
+          if (!ok) break;
+          tc_fence_after();
+#pragma unroll
+          for (int c = 0; c < HD / 16; c++) {
+            uint32_t ro[16];
+            tmem_ld16(lane_addr + C::COL_O + c * 16, ro);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; i++) ro[i] = __float_as_uint(__uint_as_float(ro[i]) * alpha);
+            tmem_st16(lane_addr + C::COL_O + c * 16, ro);
+          }
+          tmem_st_wait();
+        }
+      }
+      const unsigned long long nm2 = pairf(-m_used, -m_used);
+      // the second half first: it is the one in registers where they hold one.  P goes over the columns that its scores came from.
+#pragma unroll
+      for (int g = 1; g >= 0; g--) {
+        if (C::NBUF == 1 && g == 0) {
+          load_half(0);
+          tmem_ld_wait();
+          mask_half(0);
+        }
+        uint32_t pk[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+          const uint32_t* x2 = s[C::NBUF == 2 ? g : 0];
+          const unsigned long long x = ffma2(pair(x2[2 * i], x2[2 * i + 1]), sl2, nm2);
+          const float p0 = exp2f(lo_of(x)), p1 = exp2f(hi_of(x));
+          l2 = fadd2(l2, pairf(p0, p1));
+          pk[i] = pack16t<BF>(p0, p1);
+        }
+        tmem_st16(s_addr + g * 32, pk);
+      }
+      give_p(j);
+    }
+    for (int j = n_live; j < n_kv && ok; j++) {
+      ok = wait_scores(j);
+      if (!ok) break;
+      uint32_t zero[16];
+#pragma unroll
+      for (int i = 0; i < 16; i++) zero[i] = 0u;
+      tmem_st16(scores_at(j), zero);
+      tmem_st16(scores_at(j) + 32, zero);
+      give_p(j);
     }
     if (ok && n_kv > 0)
-      ok = mbar_wait(&pv_done[(n_kv - 1) & 1], ((n_kv - 1) >> 1) & 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 9);
+      ok = mbar_wait(&pv_done[(n_kv - 1) % C::NBUF], ((n_kv - 1) / C::NBUF) & 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 9);
     if (ok) {
       tc_fence_after();
+      const float l = lo_of(l2) + hi_of(l2);
       const float inv = l > 0.f ? 1.f / l : 0.f;
-      const bool row_ok = qrow < args.Sq;
-      uint16_t* orow = (uint16_t*)args.O + (long long)b * args.o_sb + (long long)qrow * args.o_ss +
-                       (long long)h * args.o_sh;
+      // through the query tile, which every MMA has read by now, and a TMA store of this warp's rows (rows and columns behind
+      // the tensor's ends are clipped)
 #pragma unroll
       for (int c = 0; c < HD / 32; c++) {
         uint32_t ro[32];
@@ -389,16 +471,32 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 #pragma unroll
           for (int i = 0; i < 32; i++) ro[i] = 0;
         }
-        float v[32];
+        const uint32_t row = smem_u32(sQ) + c / 2 * (BQ * 128) + (uint32_t)r * 128u;
 #pragma unroll
-        for (int i = 0; i < 32; i++) v[i] = __uint_as_float(ro[i]) * inv;
-        if (row_ok) store_row16_lim<32>(orow + c * 32, v, BF, args.D - c * 32);
+        for (int q = 0; q < 4; q++) {
+          uint32_t w[4];
+#pragma unroll
+          for (int i = 0; i < 4; i++)
+            w[i] = pack16t<BF>(__uint_as_float(ro[8 * q + 2 * i]) * inv, __uint_as_float(ro[8 * q + 2 * i + 1]) * inv);
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row + (((uint32_t)(c % 2 * 4 + q) ^ ((uint32_t)r & 7u)) << 4)),
+                       "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
+                       : "memory");
+        }
       }
-      if (row_ok && args.LSE) {
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0 && q0 + quarter * 32 < args.Sq) {
+#pragma unroll
+        for (int c = 0; c < C::CH; c++)
+          if (c * 64 < args.D) tma_store_4d(&tmO, sQ + c * BQ * 128 + quarter * 32 * 128, c * 64, q0 + quarter * 32, h, b);
+        tma_store_commit();
+      }
+      if (qrow < args.Sq && args.LSE) {
         // natural-log LSE of the scaled scores
         args.LSE[((long long)b * args.H + h) * args.Sq + qrow] =
             l > 0.f ? (m_used + log2f(l)) * 0.6931471805599453f : -INFINITY;
       }
+      if (lane == 0) tma_store_wait_read<0>();   // shared memory must outlive the stores that read from it
     }
   }
   tc_fence_before();
@@ -535,21 +633,6 @@ __device__ __forceinline__ void tile_row_to_tmem(const uint8_t* tile, int r, uin
   tmem_st_wait();
 }
 
-template <bool BF>
-__device__ __forceinline__ uint32_t pack16t(float a, float b) {
-  return BF ? pack_bf16(a, b) : pack_f16(a, b);
-}
-
-// Two packed fp32 products.
-__device__ __forceinline__ unsigned long long fmul2(unsigned long long a, unsigned long long b) {
-  unsigned long long d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ unsigned long long pair(uint32_t lo, uint32_t hi) { return (unsigned long long)hi << 32 | lo; }
-__device__ __forceinline__ float lo_of(unsigned long long v) { return __uint_as_float((uint32_t)v); }
-__device__ __forceinline__ float hi_of(unsigned long long v) { return __uint_as_float((uint32_t)(v >> 32)); }
-
 // x as a sum of three bf16 values: 24 bits.
 __device__ __forceinline__ void split_bf16(float x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   const __nv_bfloat16 h = __float2bfloat16_rn(x);
@@ -612,23 +695,6 @@ struct KvCfg {
   static constexpr int COL_K = COL_ACC1 + HD, COL_V = COL_K + HD / 2;
   static_assert((KV_IN_TMEM ? COL_V + HD / 2 : COL_K) <= TMEM_COLS, "TMEM");
 };
-
-template <int N>
-__device__ __forceinline__ void tmem_ld_cols(uint32_t addr, uint32_t (&r)[N]) {
-  if constexpr (N == 32) tmem_ld32(addr, r);
-  else tmem_ld16(addr, r);
-}
-template <int N>
-__device__ __forceinline__ void tmem_st_cols(uint32_t addr, const uint32_t (&r)[N]) {
-  if constexpr (N == 16) {
-    tmem_st16(addr, r);
-  } else {
-    static_assert(N == 8, "columns");
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(addr), "r"(r[0]), "r"(r[1]),
-                 "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
-  }
-}
 
 template <int HD, bool BF, bool DUAL>
 __global__ void __launch_bounds__(KvCfg<HD, DUAL>::THREADS, KvCfg<HD, DUAL>::CTAS_PER_SM)
@@ -845,7 +911,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         tma_store_wait_read<0>();
         mbar_arrive(out_empty);
       }
-      tma_store_wait<0>();   // shared memory must outlive the stores that read from it
+      tma_store_wait_read<0>();   // shared memory must outlive the stores that read from it (they complete behind the CTA)
     }
     __syncwarp();
   } else {
@@ -871,8 +937,8 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     long long* tr = ((blockIdx.x | blockIdx.y | blockIdx.z) == 0 && (e & 7) == 0 && lane == 0) ? args.trace : nullptr;
     const int tl = 1 + (e >> 3);
     int ntr = 0;
-    const unsigned long long sl2 = pair(__float_as_uint(args.scale_log2), __float_as_uint(args.scale_log2));
-    const unsigned long long sc2 = pair(__float_as_uint(args.scale), __float_as_uint(args.scale));
+    const unsigned long long sl2 = pairf(args.scale_log2, args.scale_log2);
+    const unsigned long long sc2 = pairf(args.scale, args.scale);
     const uint32_t out_row = smem_u32(sOut) + (uint32_t)r * 128u;
     for (int it = 0; it < n_it; it++) {
       const uint32_t ph = it & 1;
@@ -925,7 +991,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         tmem_ld_wait();
 #pragma unroll
         for (int g = 0; g < CW / 2; g++) {
-          const unsigned long long q = fmul2(pair(__float_as_uint(pr[2 * g]), __float_as_uint(pr[2 * g + 1])), fmul2(pair(in[2 * g], in[2 * g + 1]), sc2));
+          const unsigned long long q = fmul2(pairf(pr[2 * g], pr[2 * g + 1]), fmul2(pair(in[2 * g], in[2 * g + 1]), sc2));
           pk[g] = pack16t<BF>(lo_of(q), hi_of(q));
         }
       }
@@ -981,7 +1047,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             tma_store_4d(&tmdK, ring + C::TILE_BYTES + c * 128 * 128, c * 64, kv0, h, b);
           }
         tma_store_commit();
-        tma_store_wait<0>();
+        tma_store_wait_read<0>();
       }
     }
   }
@@ -1362,18 +1428,19 @@ void fill_head_group(AttnArgs& a, int slots) {
   a.head_recip = (unsigned)(((1ULL << 32) + a.H - 1) / a.H);
 }
 
-template <int HD, bool BF>
-int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
-               const AttnArgs& a, cudaStream_t s) {
-  using C = FwdCfg<HD>;
+template <int HD, bool BF, int NBUF>
+int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to,
+               AttnArgs& a, cudaStream_t s) {
+  using C = FwdCfg<HD, NBUF>;
   static bool configured = false;
   if (!configured) {
-    GB_CUDA_OK(cudaFuncSetAttribute(fa_fwd_kernel<HD, BF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    GB_CUDA_OK(cudaFuncSetAttribute(fa_fwd_kernel<HD, BF, NBUF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     C::SMEM_BYTES));
     configured = true;
   }
+  fill_head_group(a, C::CTAS_PER_SM * 148);
   dim3 grid((a.Sq + BQ - 1) / BQ, a.H, a.B);
-  fa_fwd_kernel<HD, BF><<<grid, kFwdThreads, C::SMEM_BYTES, s>>>(tq, tk, tv, a);
+  fa_fwd_kernel<HD, BF, NBUF><<<grid, kFwdThreads, C::SMEM_BYTES, s>>>(tq, tk, tv, to, a);
   GB_CUDA_OK(cudaGetLastError());
   return gbh::E_OK;
 }
@@ -1465,19 +1532,22 @@ GB_EXPORT int gb_flash_fwd(int dtype, const void* q, const void* k, const void* 
   a.causal = causal; a.in_bf16 = dtype == DT_BF16;
   a.O = o; a.LSE = lse; a.o_sb = o_sb; a.o_ss = o_ss; a.o_sh = o_sh;
   a.status = gbh::status_ptr();
-  fill_head_group(a, 2 * 148);
-  CUtensorMap tq, tk, tv;
+  CUtensorMap tq, tk, tv, to;
   int rc;
   if ((rc = make_qkv_map(&tq, q, a.in_bf16, B, H, Sq, D, q_sb, q_ss, q_sh, BQ))) return rc;
   if ((rc = make_qkv_map(&tk, k, a.in_bf16, B, H, Sk, D, k_sb, k_ss, k_sh, BKF))) return rc;
   if ((rc = make_qkv_map(&tv, v, a.in_bf16, B, H, Sk, D, v_sb, v_ss, v_sh, BKF))) return rc;
+  if ((rc = make_qkv_map(&to, o, a.in_bf16, B, H, Sq, D, o_sb, o_ss, o_sh, 32))) return rc;
   // head sizes other than 64 / 128 run the next larger kernel: the tensor maps describe the real
   // extent, loads beyond it are zero-filled by TMA, stores stop at the real extent
-  if (D > 64)
-    return a.in_bf16 ? launch_fwd<128, true>(tq, tk, tv, a, (cudaStream_t)stream)
-                     : launch_fwd<128, false>(tq, tk, tv, a, (cudaStream_t)stream);
-  return a.in_bf16 ? launch_fwd<64, true>(tq, tk, tv, a, (cudaStream_t)stream)
-                   : launch_fwd<64, false>(tq, tk, tv, a, (cudaStream_t)stream);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (D > 64) return a.in_bf16 ? launch_fwd<128, true, 2>(tq, tk, tv, to, a, st) : launch_fwd<128, false, 2>(tq, tk, tv, to, a, st);
+  // Four CTAs per SM from two rounds of them on.  us, two | four CTAs per SM, heads x length: causal 768 tiles 30.8 | 31.4, 1 024 (32 x
+  // 4096) 105 | 115, 1 184 (148 x 1024) 46.7 | 42.5, (74 x 2048) 72.0 | 73.1, 1 536 59.5 | 53.9, 4 096 (128 x 4096) 403 | 391;
+  // not causal 768 49.5 | 50.0, 1 184 67.9 | 64.4, 2 400 135.5 | 122.6; 12 tiles of 77 5.3 | 6.4.
+  const bool four = (long long)((Sq + BQ - 1) / BQ) * H * B >= 2 * FwdCfg<64, 1>::CTAS_PER_SM * 148;
+  if (four) return a.in_bf16 ? launch_fwd<64, true, 1>(tq, tk, tv, to, a, st) : launch_fwd<64, false, 1>(tq, tk, tv, to, a, st);
+  return a.in_bf16 ? launch_fwd<64, true, 2>(tq, tk, tv, to, a, st) : launch_fwd<64, false, 2>(tq, tk, tv, to, a, st);
 }
 
 GB_EXPORT int gb_flash_delta(int dtype, const void* o, const void* dout, float* delta, int B, int H,

@@ -122,3 +122,25 @@ def test_backward_folds_the_row_statistics(scale, Sq, Sk, D, causal, dtype, stat
         assert torch.isfinite(got).all()
         floor = 1e-2 * unit * want.numel() ** 0.5          # gradients that vanish (scale 0, one key): rounding of P * (dP - Delta)
         assert (got.double() - want).norm() <= 4 * unit * want.norm() + floor
+
+
+@pytest.mark.parametrize("B,H,Sq,Sk,D,causal", [(8, 74, 130, 130, 64, True), (8, 74, 129, 191, 64, False), (37, 32, 65, 65, 32, True),
+                                                (8, 74, 256, 64, 40, False), (4, 74, 450, 450, 64, True)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_forward_of_many_tiles(B, H, Sq, Sk, D, causal, dtype, status_ok):
+    """1 184 query tiles and more of heads up to 64 run with one score buffer and four CTAs per SM: edges of the 64-key steps, rows
+    whose last steps are masked, a single step, running maxima that grow (scores of a few tens)."""
+    torch.manual_seed(Sq)
+    q = torch.randn(B, Sq, H, D, device="cuda", dtype=dtype) * 3
+    k, v = (torch.randn(B, Sk, H, D, device="cuda", dtype=dtype) for _ in range(2))
+    k = k * torch.linspace(0.2, 3, Sk, device="cuda")[None, :, None, None].to(dtype)
+    out, lse = flash_fwd(q, k, v, causal, 0.5)
+    qd, kd, vd = (t.float().transpose(1, 2) for t in (q, k, v))
+    s = qd @ kd.transpose(-1, -2) * 0.5
+    if causal:
+        s = s.masked_fill(torch.ones(Sq, Sk, dtype=torch.bool, device="cuda").triu(1), -float("inf"))
+    assert (lse - torch.logsumexp(s, -1)).abs().max().item() < 1e-3
+    ref = (s.softmax(-1) @ vd).transpose(1, 2)
+    # P and the result are rounded to the inputs' type: half a unit of 2^-8 or 2^-11 each, relative to sum |P V| <= max |V|
+    unit = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    assert (out.float() - ref).abs().max().item() <= 2 * unit * vd.abs().max().item()
