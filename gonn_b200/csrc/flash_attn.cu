@@ -529,34 +529,42 @@ __global__ void fa_delta_kernel(const T* __restrict__ O, const T* __restrict__ d
 }
 
 
-// The same for 16-byte aligned rows of D = 8 * TPR elements: TPR threads per row, one
-// 16-byte load of O and of dO each.
-template <typename T, int TPR>
+// The same for 16-byte aligned rows of D = 8 * TPR elements: TPR threads per row, one 16-byte load of O and of dO each for four rows
+// at a time.  Rows are visited in (b, s, h) order so that neighbouring threads read neighbouring memory; I: the type that rows
+// are counted in (the 64-bit divisions of one row at a time kept the loads waiting: (8, 16, 4096, 128) 72 -> 56 us, (16, 12, 1024,
+// 64) 15.2 -> 10.2).
+template <typename T, int TPR, typename I>
 __global__ void __launch_bounds__(256)
 fa_delta_vec_kernel(const T* __restrict__ O, const T* __restrict__ dO, float* __restrict__ delta, int B,
                     int H, int S, long long o_sb, long long o_ss, long long o_sh, long long g_sb,
                     long long g_ss, long long g_sh) {
-  const long long total = (long long)B * H * S;
+  constexpr int R = 4;
+  const I total = (I)B * (I)H * (I)S;
   const int sub = threadIdx.x % TPR;
-  constexpr int RPB = 256 / TPR;  // rows per CTA pass; every thread of the CTA runs the same trip count
-  for (long long base = (long long)blockIdx.x * RPB; base < total; base += (long long)gridDim.x * RPB) {
-    const long long i = base + threadIdx.x / TPR;
-    // rows are visited in (b, s, h) order so that neighbouring threads read neighbouring memory
-    const bool live = i < total;
-    const long long ii = live ? i : 0;
-    const int h = (int)(ii % H);
-    const int q = (int)((ii / H) % S);
-    const int b = (int)(ii / ((long long)S * H));
-    const uint4 uo = *reinterpret_cast<const uint4*>(O + b * o_sb + q * o_ss + h * o_sh + sub * 8);
-    const uint4 ug = *reinterpret_cast<const uint4*>(dO + b * g_sb + q * g_ss + h * g_sh + sub * 8);
-    const T* eo = reinterpret_cast<const T*>(&uo);
-    const T* eg = reinterpret_cast<const T*>(&ug);
-    float s = 0.f;
+  constexpr int RPB = 256 / TPR;  // rows per CTA and load; every thread of the CTA runs the same trip count
+  for (I base = (I)blockIdx.x * (RPB * R); base < total; base += (I)gridDim.x * (RPB * R)) {
+    uint4 uo[R], ug[R];
+    I at[R];
 #pragma unroll
-    for (int j = 0; j < 8; j++) s += (float)eo[j] * (float)eg[j];
+    for (int k = 0; k < R; k++) {
+      const I i = base + (I)(k * RPB + threadIdx.x / TPR);
+      const I ii = i < total ? i : 0;
+      const I bs = ii / (I)H, h = ii - bs * (I)H, b = bs / (I)S, q = bs - b * (I)S;
+      at[k] = i < total ? (b * (I)H + h) * (I)S + q : total;
+      uo[k] = *reinterpret_cast<const uint4*>(O + (long long)b * o_sb + (long long)q * o_ss + (long long)h * o_sh + sub * 8);
+      ug[k] = *reinterpret_cast<const uint4*>(dO + (long long)b * g_sb + (long long)q * g_ss + (long long)h * g_sh + sub * 8);
+    }
 #pragma unroll
-    for (int o = TPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (live && sub == 0) delta[((long long)b * H + h) * S + q] = s;
+    for (int k = 0; k < R; k++) {
+      const T* eo = reinterpret_cast<const T*>(&uo[k]);
+      const T* eg = reinterpret_cast<const T*>(&ug[k]);
+      float s = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; j++) s += (float)eo[j] * (float)eg[j];
+#pragma unroll
+      for (int o = TPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (at[k] < total && sub == 0) delta[at[k]] = s;
+    }
   }
 }
 
@@ -1558,14 +1566,21 @@ GB_EXPORT int gb_flash_delta(int dtype, const void* o, const void* dout, float* 
   const bool vec = (D == 64 || D == 128) && !((o_sb | o_ss | o_sh | g_sb | g_ss | g_sh) & 7) &&
                    !(((uintptr_t)o | (uintptr_t)dout) & 15);
   if (vec) {
-    const int tpr = D / 8, rpb = 256 / tpr;
-    int grid = (int)((total + rpb - 1) / rpb < 148 * 8 ? (total + rpb - 1) / rpb : 148 * 8);
+    const int rows = 4 * 256 / (D / 8);         // of a CTA pass
+    const int grid = (int)((total + rows - 1) / rows < 148 * 8 ? (total + rows - 1) / rows : 148 * 8);
     cudaStream_t st = (cudaStream_t)stream;
-#define GB_DELTA(T, TPR)                                                                               \
-  fa_delta_vec_kernel<T, TPR><<<grid, 256, 0, st>>>((const T*)o, (const T*)dout, delta, B, H, S, o_sb, \
-                                                    o_ss, o_sh, g_sb, g_ss, g_sh)
+    const bool small = total < (1LL << 31) - (long long)rows * 148 * 8;      // no sum of rows overflows
+#define GB_DELTA_I(T, TPR, I)                                                                             \
+  fa_delta_vec_kernel<T, TPR, I><<<grid, 256, 0, st>>>((const T*)o, (const T*)dout, delta, B, H, S, o_sb, \
+                                                       o_ss, o_sh, g_sb, g_ss, g_sh)
+#define GB_DELTA(T, TPR)                            \
+  do {                                              \
+    if (small) GB_DELTA_I(T, TPR, unsigned);        \
+    else GB_DELTA_I(T, TPR, long long);             \
+  } while (0)
     if (dtype == DT_BF16) { if (D == 64) GB_DELTA(__nv_bfloat16, 8); else GB_DELTA(__nv_bfloat16, 16); }
     else { if (D == 64) GB_DELTA(__half, 8); else GB_DELTA(__half, 16); }
+#undef GB_DELTA_I
 #undef GB_DELTA
     GB_CUDA_OK(cudaGetLastError());
     return gbh::E_OK;
