@@ -185,6 +185,8 @@ struct alignas(sizeof(T) * N) Vec { T v[N]; };
 template <typename T, int MODE, int OP>
 __global__ void unary_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __restrict__ y,
                              long long n, int vec_ok, double p0d, double p1d) {
+  pdl_trigger();
+  pdl_wait();
   using CT = typename Conv<T>::CT;
   constexpr int V = 16 / sizeof(T);
   const CT p0 = (CT)p0d, p1 = (CT)p1d;
@@ -229,6 +231,8 @@ __device__ __forceinline__ CT bin(int op, CT a, CT b) {
 template <typename T, int OP>
 __global__ void binary_same_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ c,
                                    long long n, int vec_ok) {
+  pdl_trigger();
+  pdl_wait();
   using CT = typename Conv<T>::CT;
   constexpr int V = 16 / sizeof(T);
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -263,6 +267,8 @@ struct BcastDims {
 template <typename T, int OP>
 __global__ void binary_bcast_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ c,
                                     long long n, BcastDims d) {
+  pdl_trigger();
+  pdl_wait();
   using CT = typename Conv<T>::CT;
   const long long nth = (long long)gridDim.x * blockDim.x;
   if (n <= 0x7fffffffLL) {
@@ -307,6 +313,8 @@ __global__ void binary_bcast_kernel(const T* __restrict__ a, const T* __restrict
 template <typename T, int OP, bool SWAP>
 __global__ void binary_rowvec_kernel(const T* __restrict__ full, const T* __restrict__ row, T* __restrict__ c,
                                      long long nvec, long long inner_vec) {
+  pdl_trigger();
+  pdl_wait();
   using CT = typename Conv<T>::CT;
   constexpr int V = 16 / sizeof(T);
   const Vec<T, V>* fv = reinterpret_cast<const Vec<T, V>*>(full);
@@ -371,9 +379,10 @@ int launch_unary(int op, const void* x, const void* dy, void* y, long long n, do
   constexpr int V = 16 / sizeof(T);
   int vec_ok = (((uintptr_t)x | (uintptr_t)y | (uintptr_t)dy) & 15) == 0;
   int grid = grid_for((n + V - 1) / V, 256);
+  cudaError_t rc = cudaSuccess;
 #define GB_U(OPID)                                                                            \
   case OPID:                                                                                  \
-    unary_kernel<T, MODE, OPID><<<grid, 256, 0, s>>>((const T*)x, (const T*)dy, (T*)y, n, vec_ok, p0, p1); \
+    rc = gbh::launch(unary_kernel<T, MODE, OPID>, dim3(grid), dim3(256), 0, s, 1, (const T*)x, (const T*)dy, (T*)y, n, vec_ok, p0, p1); \
     break;
   switch (op) {
     GB_U(U_EXP) GB_U(U_LOG) GB_U(U_SQRT) GB_U(U_SIN) GB_U(U_COS) GB_U(U_TAN) GB_U(U_ABS)
@@ -388,7 +397,7 @@ int launch_unary(int op, const void* x, const void* dy, void* y, long long n, do
       return gbh::E_BAD_ARG;
   }
 #undef GB_U
-  GB_CUDA_OK(cudaGetLastError());
+  GB_CUDA_OK(rc);
   return gbh::E_OK;
 }
 
@@ -411,17 +420,18 @@ int launch_binary(int op, const void* a, const void* b, void* c, long long n, co
       if (inner % V == 0 && n % V == 0 && inner >= V) { rv_mode = side; rv_inner = inner; }
     }
   }
+  cudaError_t rc = cudaSuccess;
 #define GB_B(OPID)                                                                                 \
   case OPID:                                                                                       \
     if (d == nullptr) {                                                                            \
       int vec_ok = (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15) == 0;                       \
-      binary_same_kernel<T, OPID><<<grid_for((n + V - 1) / V, 256), 256, 0, s>>>((const T*)a, (const T*)b, (T*)c, n, vec_ok); \
+      rc = gbh::launch(binary_same_kernel<T, OPID>, dim3(grid_for((n + V - 1) / V, 256)), dim3(256), 0, s, 1, (const T*)a, (const T*)b, (T*)c, n, vec_ok); \
     } else if (rv_mode == 1) {                                                                     \
-      binary_rowvec_kernel<T, OPID, false><<<grid_for(n / V, 256), 256, 0, s>>>((const T*)a, (const T*)b, (T*)c, n / V, rv_inner / V); \
+      rc = gbh::launch(binary_rowvec_kernel<T, OPID, false>, dim3(grid_for(n / V, 256)), dim3(256), 0, s, 1, (const T*)a, (const T*)b, (T*)c, n / V, rv_inner / V); \
     } else if (rv_mode == 2) {                                                                     \
-      binary_rowvec_kernel<T, OPID, true><<<grid_for(n / V, 256), 256, 0, s>>>((const T*)b, (const T*)a, (T*)c, n / V, rv_inner / V); \
+      rc = gbh::launch(binary_rowvec_kernel<T, OPID, true>, dim3(grid_for(n / V, 256)), dim3(256), 0, s, 1, (const T*)b, (const T*)a, (T*)c, n / V, rv_inner / V); \
     } else {                                                                                       \
-      binary_bcast_kernel<T, OPID><<<grid_for(n, 256), 256, 0, s>>>((const T*)a, (const T*)b, (T*)c, n, *d); \
+      rc = gbh::launch(binary_bcast_kernel<T, OPID>, dim3(grid_for(n, 256)), dim3(256), 0, s, 1, (const T*)a, (const T*)b, (T*)c, n, *d); \
     }                                                                                              \
     break;
   switch (op) {
@@ -431,7 +441,7 @@ int launch_binary(int op, const void* a, const void* b, void* c, long long n, co
       return gbh::E_BAD_ARG;
   }
 #undef GB_B
-  GB_CUDA_OK(cudaGetLastError());
+  GB_CUDA_OK(rc);
   return gbh::E_OK;
 }
 

@@ -18,6 +18,8 @@ template <typename T>
 __global__ void gather_rows_kernel(const T* __restrict__ w, const long long* __restrict__ idx,
                                    T* __restrict__ out, long long n, int D, long long V, int vec_ok,
                                    int* status) {
+  pdl_trigger();
+  pdl_wait();
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (long long r = (long long)blockIdx.x * warps + warp; r < n; r += (long long)gridDim.x * warps) {
     long long v = idx[r];
@@ -192,13 +194,13 @@ GB_EXPORT int gb_gather_rows(int dtype, const void* w, const long long* idx, voi
   int* st = gbh::status_ptr();
   switch (dtype) {
     case DT_BF16: case DT_F16:
-      gather_rows_kernel<uint16_t><<<(int)g, 256, 0, s>>>((const uint16_t*)w, idx, (uint16_t*)out, n, D, V, vec_ok, st);
+      GB_CUDA_OK(gbh::launch(gather_rows_kernel<uint16_t>, dim3((unsigned)g), dim3(256), 0, s, 1, (const uint16_t*)w, idx, (uint16_t*)out, n, D, V, vec_ok, st));
       break;
     case DT_F32:
-      gather_rows_kernel<float><<<(int)g, 256, 0, s>>>((const float*)w, idx, (float*)out, n, D, V, vec_ok, st);
+      GB_CUDA_OK(gbh::launch(gather_rows_kernel<float>, dim3((unsigned)g), dim3(256), 0, s, 1, (const float*)w, idx, (float*)out, n, D, V, vec_ok, st));
       break;
     case DT_F64:
-      gather_rows_kernel<double><<<(int)g, 256, 0, s>>>((const double*)w, idx, (double*)out, n, D, V, vec_ok, st);
+      GB_CUDA_OK(gbh::launch(gather_rows_kernel<double>, dim3((unsigned)g), dim3(256), 0, s, 1, (const double*)w, idx, (double*)out, n, D, V, vec_ok, st));
       break;
     default:
       gbh::set_error("gb_gather_rows: bad dtype %d", dtype);

@@ -228,12 +228,6 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   int n_kv = (args.Sk + BKF - 1) / BKF;
   if (args.causal) n_kv = min(n_kv, (q_tile + 1) * (BQ / BKF));
 
-  auto load_k = [&](int j, int st) {
-    mbar_expect_tx(&k_full[st], C::SUB_BYTES);
-#pragma unroll
-    for (int c = 0; c < C::CH; c++)
-      tma_load_4d(sK + st * C::SUB_BYTES + c * BKF * 128, &tmK, &k_full[st], c * 64, j * BKF, h, b);
-  };
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int i = 0; i < C::STAGES; i++) {
@@ -249,12 +243,6 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     }
     *abort_flag = 0;
     mbar_fence_init();
-    // the query tile and the first keys start before anything else is ready
-    fence_proxy_async_smem();
-    mbar_expect_tx(q_full, C::Q_BYTES);
-#pragma unroll
-    for (int c = 0; c < C::CH; c++) tma_load_4d(sQ + c * BQ * 128, &tmQ, q_full, c * 64, q0, h, b);
-    if (n_kv > 0) load_k(0, 0);
   } else if (warp == 2 && lane < 4) {
     tma_prefetch_desc(lane == 0 ? &tmK : lane == 1 ? &tmQ : lane == 2 ? &tmV : &tmO);
   }
@@ -266,16 +254,21 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
 
   if (warp == 0) {
     if (lane == 0) {
+      mbar_expect_tx(q_full, C::Q_BYTES);
+#pragma unroll
+      for (int c = 0; c < C::CH; c++) tma_load_4d(sQ + c * BQ * 128, &tmQ, q_full, c * 64, q0, h, b);
       int st = 0;
       uint32_t ph = 0;
       for (int j = 0; j < n_kv; j++) {
-        if (j > 0) {
-          if (!mbar_wait(&k_empty[st], ph ^ 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 1)) break;
-          load_k(j, st);
-        }
+        if (!mbar_wait(&k_empty[st], ph ^ 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 1)) break;
+        mbar_expect_tx(&k_full[st], C::SUB_BYTES);
+#pragma unroll
+        for (int c = 0; c < C::CH; c++)
+          tma_load_4d(sK + st * C::SUB_BYTES + c * BKF * 128, &tmK, &k_full[st], c * 64, j * BKF, h, b);
         if (!mbar_wait(&v_empty[st], ph ^ 1, abort_flag, args.status, ST_ATTN_TIMEOUT, 2)) break;
         mbar_expect_tx(&v_full[st], C::SUB_BYTES);
 #pragma unroll
@@ -1448,8 +1441,7 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
   }
   fill_head_group(a, C::CTAS_PER_SM * 148);
   dim3 grid((a.Sq + BQ - 1) / BQ, a.H, a.B);
-  fa_fwd_kernel<HD, BF, NBUF><<<grid, kFwdThreads, C::SMEM_BYTES, s>>>(tq, tk, tv, to, a);
-  GB_CUDA_OK(cudaGetLastError());
+  GB_CUDA_OK(gbh::launch(fa_fwd_kernel<HD, BF, NBUF>, grid, dim3(kFwdThreads), C::SMEM_BYTES, s, 1, tq, tk, tv, to, a));
   return gbh::E_OK;
 }
 

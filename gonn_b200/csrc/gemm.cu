@@ -699,6 +699,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
+  pdl_wait();
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -999,6 +1001,8 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   cluster_sync_all();   // barriers of both CTAs are initialised before anyone touches the peer's
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
+  pdl_wait();
 
   if (warp == 0) {
     // ---------------- TMA producer (one per CTA) ----------------
@@ -1199,6 +1203,8 @@ gemm_tcgen05_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __gri
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
+  pdl_wait();
   if (warp == 0) {
     if (lane == 0) {
       bool ok = true;
@@ -1620,8 +1626,7 @@ int launch_tc_ew(const TMaps& tm, const GemmArgs& args, int num_sms, cudaStream_
   }
   int tiles = args.num_m * args.num_n * args.batch * args.splits;
   int grid = tiles < num_sms ? tiles : num_sms;
-  kern<<<grid, 64 + 32 * EW, SL::BYTES, stream>>>(tm.a, tm.b, tm.c, tm.x, args);
-  GB_CUDA_OK(cudaGetLastError());
+  GB_CUDA_OK(gbh::launch(kern, dim3(grid), dim3(64 + 32 * EW), SL::BYTES, stream, 1, tm.a, tm.b, tm.c, tm.x, args));
   return gbh::E_OK;
 }
 
@@ -1661,20 +1666,7 @@ int launch_2cta_t(const TMaps& tm, const GemmArgs& args, int num_sms, cudaStream
   int tiles = args.num_m * args.num_n * args.batch * args.splits;
   int pairs = num_sms / 2;
   if (tiles < pairs) pairs = tiles;
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(2 * pairs);
-  cfg.blockDim = dim3(64 + 32 * 8);
-  cfg.dynamicSmemBytes = SL::BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  GB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tm.a, tm.b, tm.c, tm.x, args));
+  GB_CUDA_OK(gbh::launch(kern, dim3(2 * pairs), dim3(64 + 32 * 8), SL::BYTES, stream, 2, tm.a, tm.b, tm.c, tm.x, args));
   return gbh::E_OK;
 }
 
@@ -1718,20 +1710,7 @@ int launch_cluster_t(const TMaps& tm, const GemmArgs& args, cudaStream_t stream)
     GB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CfgS::BYTES));
     configured = true;
   }
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(args.num_m * args.num_n * args.splits, args.batch);
-  cfg.blockDim = dim3(CfgS::THREADS);
-  cfg.dynamicSmemBytes = CfgS::BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = args.splits;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = args.splits > 1 ? 1 : 0;
-  GB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tm.a, tm.b, args));
+  GB_CUDA_OK(gbh::launch(kern, dim3(args.num_m * args.num_n * args.splits, args.batch), dim3(CfgS::THREADS), CfgS::BYTES, stream, args.splits, tm.a, tm.b, args));
   return gbh::E_OK;
 }
 
@@ -1745,6 +1724,8 @@ int launch_cluster(const TMaps& tm, const GemmArgs& args, cudaStream_t stream) {
 template <typename TO>
 __global__ void splitk_finish_kernel(const float* __restrict__ ws, TO* __restrict__ C, const float* __restrict__ bias, int M, int N,
                                      int batch, int splits, long long ldc, long long strideC, int beta) {
+  pdl_trigger();
+  pdl_wait();
   const long long per = (long long)M * N;
   const long long total = per * batch;
   for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < total;
@@ -1996,15 +1977,14 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
     const int grid = (int)(quads + 255) / 256 < g_num_sms * 8 ? (int)((quads + 255) / 256) : g_num_sms * 8;
     const float* ws = (const float*)workspace;
     if (user_out == OUT_F32)
-      splitk_finish_kernel<float><<<grid, 256, 0, stream>>>(ws, (float*)user_C, user_bias, M, N, batch, splits, user_ldc,
-                                                            user_strideC, user_beta);
+      GB_CUDA_OK(gbh::launch(splitk_finish_kernel<float>, dim3(grid), dim3(256), 0, stream, 1, ws, (float*)user_C, user_bias, M, N, batch, splits, user_ldc,
+                                                            user_strideC, user_beta));
     else if (user_out == OUT_BF16)
-      splitk_finish_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(ws, (__nv_bfloat16*)user_C, user_bias, M, N, batch,
-                                                                    splits, user_ldc, user_strideC, user_beta);
+      GB_CUDA_OK(gbh::launch(splitk_finish_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, stream, 1, ws, (__nv_bfloat16*)user_C, user_bias, M, N, batch,
+                                                                    splits, user_ldc, user_strideC, user_beta));
     else
-      splitk_finish_kernel<__half><<<grid, 256, 0, stream>>>(ws, (__half*)user_C, user_bias, M, N, batch, splits,
-                                                             user_ldc, user_strideC, user_beta);
-    GB_CUDA_OK(cudaGetLastError());
+      GB_CUDA_OK(gbh::launch(splitk_finish_kernel<__half>, dim3(grid), dim3(256), 0, stream, 1, ws, (__half*)user_C, user_bias, M, N, batch, splits,
+                                                             user_ldc, user_strideC, user_beta));
   }
   return gbh::E_OK;
 }

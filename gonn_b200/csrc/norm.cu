@@ -696,6 +696,8 @@ template <typename T, typename TW, int VPT, bool RMS, bool STAGED>
 __global__ void __launch_bounds__(128)
 norm_fwd_warp_kernel(const T* __restrict__ x, const TW* __restrict__ w, const TW* __restrict__ b, T* __restrict__ y,
                      float* __restrict__ mean_out, float* __restrict__ rstd_out, long long rows, int D, float eps) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int V = IO<T>::V;
   constexpr int NP2 = Pairs<T>::NP2;
   using Raw = typename IO<T>::Raw;
@@ -1006,8 +1008,8 @@ int norm_fwd_t(const void* x, const void* w, const void* b, void* y, float* mean
     const long long blocks = (rows + 3) / 4, most = staged ? 148 * (nvec <= 128 ? 16 : 8) : 1 << 20;
     const size_t smem = staged ? 2 * (size_t)D * sizeof(TW) : 0;
 #define GB_FWDW_(VPT, STAGED)                                                                              \
-  norm_fwd_warp_kernel<T, TW, VPT, RMS, STAGED><<<(unsigned)(blocks < most ? blocks : most), 128, smem, s>>>( \
-      (const T*)x, (const TW*)w, (const TW*)b, (T*)y, mean, rstd, rows, D, eps)
+  GB_CUDA_OK(gbh::launch(norm_fwd_warp_kernel<T, TW, VPT, RMS, STAGED>, dim3((unsigned)(blocks < most ? blocks : most)), dim3(128), \
+                         smem, s, 1, (const T*)x, (const TW*)w, (const TW*)b, (T*)y, mean, rstd, rows, D, eps))
 #define GB_FWDW(VPT)              \
   if (staged) GB_FWDW_(VPT, true); \
   else GB_FWDW_(VPT, false)
@@ -1019,7 +1021,6 @@ int norm_fwd_t(const void* x, const void* w, const void* b, void* y, float* mean
     else { GB_FWDW(8); }
 #undef GB_FWDW_
 #undef GB_FWDW
-    GB_CUDA_OK(cudaGetLastError());
     return gbh::E_OK;
   }
   if (aligned && nvec > 256 && nvec <= 1024 && g_norm_pipe) {
