@@ -199,3 +199,43 @@ def test_cnn_trains(status_ok):
         ddp.step()
         losses.append(loss.item())
     assert losses[-1] < losses[0] - 0.3, losses
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("include", [0, 1])
+@pytest.mark.parametrize("B,S,nwin,taps", [(64, 9, 5, 1), (67, 50, 257, 4), (130, 33, 7, 5), (1200, 20, 3, 8), (5, 300, 1, 64), (3, 700, 9, 257), (2401, 90, 4, 70)])
+def test_pool_kernels_on_any_map(mode, include, B, S, nwin, taps, status_ok):
+    """Maps with padding anywhere (also a window of nothing else), ties, NaNs and planes that the unrolled loops leave over."""
+    import numpy as np
+    from gonn_b200 import lib as L
+    rng = np.random.default_rng(taps)
+    idx = rng.integers(0, S, (nwin, taps))
+    idx[rng.random((nwin, taps)) < 0.3] = -1
+    idx[0, 0] = -1
+    if nwin > 2:
+        idx[2] = -1
+    x = torch.from_numpy(rng.integers(-4, 5, (B, S))).float()
+    if taps <= 8:                      # (over wide windows a NaN may lose to a number of another lane)
+        x[B // 2, ::3] = float("nan")
+    xd, it = x.cuda(), torch.from_numpy(idx.astype(np.int32)).cuda()
+    y = torch.empty(B, nwin, device="cuda")
+    arg = torch.empty(B, nwin, dtype=torch.int32, device="cuda")
+    L.call("gb_pool_fwd", L.I(2), L.ptr(xd), L.ptr(it), L.ptr(y), L.ptr(arg) if mode == 0 else None, L.L(B), L.L(S), L.I(nwin), L.I(taps),
+           L.I(mode), L.I(include), L.F(2.0), L.stream_ptr())
+    want, warg = np.zeros((B, nwin), np.float32), np.full((B, nwin), -1)
+    xn = x.numpy()
+    for w in range(nwin):
+        ok = [t for t in range(taps) if idx[w, t] >= 0]
+        if mode == 1:
+            if ok:
+                want[:, w] = xn[:, idx[w, ok]].sum(1) / (taps if include else len(ok))
+            continue
+        for n, t in enumerate(ok):
+            v = xn[:, idx[w, t]]
+            new = v > want[:, w] if n else np.ones(B, bool)
+            want[new, w], warg[new, w] = v[new], t
+    nan = torch.from_numpy(np.isnan(want))
+    assert torch.equal(y.cpu()[~nan], torch.from_numpy(want)[~nan]) if mode == 0 else torch.allclose(y.cpu()[~nan], torch.from_numpy(want)[~nan], rtol=1e-6, atol=1e-6)
+    assert bool(y.cpu()[nan].isnan().all())
+    if mode == 0:
+        assert torch.equal(arg.cpu()[~nan], torch.from_numpy(warg).int()[~nan])
