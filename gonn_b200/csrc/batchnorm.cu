@@ -69,58 +69,101 @@ __device__ __forceinline__ bool planes_vectorisable(long long S, const void* p0,
   return (S & 3) == 0 && (((uintptr_t)p0 | (uintptr_t)p1 | (uintptr_t)p2) & m) == 0;
 }
 
-// partial[c][split][0..1]; mode 0: (x, x^2); mode 1: (dy, dy * xhat).  CTA (c, split):
-// the samples of the split, one warp per sample plane at a time.
-template <typename T>
+// Planes that cannot be read in vectors (S odd: 13 x 13, ...) go element by element, several of them in flight per lane.  With one in
+// flight and the channel's constants worked out for every plane, us forward, backward, sums of one tensor: 256 x 128 x 169 bf16 20.6,
+// 27.4, 13.2, so 15.4, 24.0, 10.2; 256 x 64 x 900 18.2, 36.7, 10.3, so 15.3, 34.7, 8.8; 64 x 512 x 49 34.2, 36.1, 28.9, so 14.6,
+// 13.6, 9.6.
+constexpr int kBatch = 8;
+template <int NB, typename T>
+__device__ __forceinline__ void load_batch(const T* __restrict__ p, long long i0, long long S, float (&v)[NB]) {
+#pragma unroll
+  for (int j = 0; j < NB; j++) v[j] = i0 + 32 * j < S ? (float)p[i0 + 32 * j] : 0.f;
+}
+
+// The same in vectors of four.
+template <int NB, typename T>
+__device__ __forceinline__ void load_vec_batch(const T* __restrict__ p, long long i0, long long S, float (&v)[NB][4]) {
+#pragma unroll
+  for (int j = 0; j < NB; j++) {
+    if (i0 + 128 * j < S) Vec4<T>::ld(p + i0 + 128 * j, v[j]);
+    else v[j][0] = v[j][1] = v[j][2] = v[j][3] = 0.f;
+  }
+}
+
+// partial[c][split][0..1]; mode 0: (x, x^2); mode 1: (dy, dy * xhat).  PER_WARP 0: CTA (c, split), one warp per sample plane of the
+// split at a time; 1: a warp takes all planes of its (c, split), eight channels to a CTA, and no barrier.
+template <typename T, bool PER_WARP, int MODE>
 __global__ void __launch_bounds__(256)
-bn_partial_kernel(const T* __restrict__ a, const T* __restrict__ xin,
-                                  const float* __restrict__ mean, const float* __restrict__ invstd,
-                                  float* __restrict__ part, int N, int C, long long S, int mode,
-                                  const T* __restrict__ yrelu) {
+bn_partial_kernel(const T* __restrict__ a, const T* __restrict__ xin, const float* __restrict__ mean, const float* __restrict__ invstd,
+                  float* __restrict__ part, int N, int C, long long S, const T* __restrict__ yrelu) {
   // yrelu (backward only, may be null): the forward's output after its fused ReLU; the incoming
   // gradient counts as zero wherever that output is zero
+  constexpr int VB = MODE ? 1 : 4, SB = MODE ? 2 : 8;      // in flight of each tensor: a backward that holds more registers is slower
   __shared__ float red[32];
-  const int c = blockIdx.x, sp = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c = PER_WARP ? blockIdx.x * 8 + warp : blockIdx.x, sp = blockIdx.y;
+  if (PER_WARP && c >= C) return;
   const int per = (N + kSplits - 1) / kSplits;
   const int n0 = sp * per, n1 = min(n0 + per, N);
   float s0 = 0.f, s1 = 0.f;
-  const float mu = mode ? mean[c] : 0.f, is = mode ? invstd[c] : 0.f;
-  const bool vec = planes_vectorisable<T>(S, a, mode ? xin : a, yrelu ? yrelu : a);
-  for (int n = n0 + warp; n < n1; n += 8) {
+  const float mu = MODE ? mean[c] : 0.f, is = MODE ? invstd[c] : 0.f;
+  const bool vec = planes_vectorisable<T>(S, a, MODE ? xin : a, yrelu ? yrelu : a);
+  auto add = [&](float v, float xv, float yv) {
+    if (MODE && yrelu && !(yv > 0.f)) v = 0.f;
+    s0 += v;
+    s1 += MODE ? v * ((xv - mu) * is) : v * v;
+  };
+  for (int n = PER_WARP ? n0 : n0 + warp; n < n1; n += PER_WARP ? 1 : 8) {
     const long long base = ((long long)n * C + c) * S;
     if (vec) {
-      for (long long i = lane * 4; i < S; i += 128) {
-        float v[4], xv[4];
-        Vec4<T>::ld(a + base + i, v);
-        if (mode) Vec4<T>::ld(xin + base + i, xv);
-        if (yrelu) {
-          float yv[4];
-          Vec4<T>::ld(yrelu + base + i, yv);
+      for (long long i = lane * 4; i < S; i += 128 * VB) {
+        float v[VB][4], xv[VB][4], yv[VB][4];
+        load_vec_batch(a + base, i, S, v);
+        if (MODE) load_vec_batch(xin + base, i, S, xv);
+        if (MODE && yrelu) load_vec_batch(yrelu + base, i, S, yv);
 #pragma unroll
-          for (int j = 0; j < 4; j++) v[j] = yv[j] > 0.f ? v[j] : 0.f;
-        }
+        for (int j = 0; j < VB; j++)
+          if (!MODE || i + 128 * j < S) {
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-          s0 += v[j];
-          s1 += mode ? v[j] * ((xv[j] - mu) * is) : v[j] * v[j];
-        }
+            for (int q = 0; q < 4; q++) add(v[j][q], xv[j][q], yv[j][q]);
+          }
       }
     } else {
-      for (long long i = lane; i < S; i += 32) {
-        float v = (float)a[base + i];
-        if (yrelu && !((float)yrelu[base + i] > 0.f)) v = 0.f;
-        s0 += v;
-        s1 += mode ? v * (((float)xin[base + i] - mu) * is) : v * v;
+      for (long long i = lane; i < S; i += 32 * SB) {
+        float v[SB], xv[SB], yv[SB];
+        load_batch(a + base, i, S, v);
+        if (MODE) load_batch(xin + base, i, S, xv);
+        if (MODE && yrelu) load_batch(yrelu + base, i, S, yv);
+#pragma unroll
+        for (int j = 0; j < SB; j++)
+          if (!MODE || i + 32 * j < S) add(v[j], xv[j], yv[j]);
       }
     }
   }
-  s0 = block_sum(s0, red);
-  s1 = block_sum(s1, red);
-  if (threadIdx.x == 0) {
+  if (PER_WARP) {
+    s0 = warp_sum(s0);
+    s1 = warp_sum(s1);
+  } else {
+    s0 = block_sum(s0, red);
+    s1 = block_sum(s1, red);
+  }
+  if (PER_WARP ? lane == 0 : threadIdx.x == 0) {
     part[((long long)c * kSplits + sp) * 2] = s0;
     part[((long long)c * kSplits + sp) * 2 + 1] = s1;
   }
+}
+
+// A warp per (channel, split) where its planes are few elements and there are pairs enough for every SM.  us, forward, backward, sums
+// of one tensor: 64 x 512 x 49 a CTA each 26, 31, 21, a warp each 14.6, 13.6, 9.6; 32 x 256 x 196 13.5, 18, 13 and 7.1, 9.9, 6.5;
+// 256 x 128 x 169 (1 352 elements) 16.3, 24.1, 11.2 and 15.3, 24.0, 10.2; 256 x 64 x 900 (7 200) 15.8, 39.1, 9.3 and 16.3, 49, 9.7.
+template <typename T, int MODE>
+void launch_partial(const void* a, const void* xin, const float* mean, const float* invstd, float* part, int N, int C, long long S,
+                    const void* yrelu, cudaStream_t s) {
+  const long long elements = (long long)((N + kSplits - 1) / kSplits) * S;
+  if (C >= 64 && elements <= 2048)
+    bn_partial_kernel<T, true, MODE><<<dim3((C + 7) / 8, kSplits), 256, 0, s>>>((const T*)a, (const T*)xin, mean, invstd, part, N, C, S, (const T*)yrelu);
+  else
+    bn_partial_kernel<T, false, MODE><<<dim3(C, kSplits), 256, 0, s>>>((const T*)a, (const T*)xin, mean, invstd, part, N, C, S, (const T*)yrelu);
 }
 
 struct BnArgs {
@@ -288,6 +331,10 @@ __global__ void __launch_bounds__(256) bn_finalise_kernel(const BnArgs a, float*
   else bn_fwd_finalise(a, &sm_flag, &s_count);
 }
 
+__device__ __forceinline__ int channel_of(long long plane, int C) {
+  return plane <= 0xffffffffll ? (int)((unsigned)plane % (unsigned)C) : (int)(plane % C);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256)
 bn_apply_kernel(const T* __restrict__ x, T* __restrict__ y, const BnArgs a) {
@@ -310,38 +357,44 @@ bn_apply_kernel(const T* __restrict__ x, T* __restrict__ y, const BnArgs a) {
   const long long S = a.S;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool vec = planes_vectorisable<T>(S, x, y, x);
+  // The launch strides by whole images where it can (grid_planes), so a warp mostly stays with its channel.
+  int known = -1;
+  float scale = 0.f, shift = 0.f;
   for (long long pl = (long long)blockIdx.x * 8 + warp; pl < planes; pl += (long long)gridDim.x * 8) {
-    const int c = (int)(pl % C);
-    float mean, is;
-    if (a.training && a.split == 2) {
-      // single rank: mean and 1/std straight from the partial sums; the planes of the first image
-      // publish them for the backward and update the running statistics (one writer per channel)
-      float s0, s1;
-      local_sums(a, c, s0, s1);
-      const float n = (float)a.N * (float)a.S;
-      mean = s0 / n;
-      float var = s1 / n - mean * mean;
-      var = var > 0.f ? var : 0.f;
-      is = rsqrtf(var + a.eps);
-      if (pl < C && lane == 0) {
-        a.stats[c] = mean;
-        a.stats[C + c] = is;
-        if (a.running_mean) {
-          const float unbiased = n > 1.f ? var * n / (n - 1.f) : var;
-          a.running_mean[c] = (1.f - a.momentum) * a.running_mean[c] + a.momentum * mean;
-          a.running_var[c] = (1.f - a.momentum) * a.running_var[c] + a.momentum * unbiased;
+    const int c = channel_of(pl, C);
+    if (c != known) {
+      known = c;
+      float mean, is;
+      if (a.training && a.split == 2) {
+        // single rank: mean and 1/std straight from the partial sums; the planes of the first image
+        // publish them for the backward and update the running statistics (one writer per channel)
+        float s0, s1;
+        local_sums(a, c, s0, s1);
+        const float n = (float)a.N * (float)a.S;
+        mean = s0 / n;
+        float var = s1 / n - mean * mean;
+        var = var > 0.f ? var : 0.f;
+        is = rsqrtf(var + a.eps);
+        if (pl < C && lane == 0) {
+          a.stats[c] = mean;
+          a.stats[C + c] = is;
+          if (a.running_mean) {
+            const float unbiased = n > 1.f ? var * n / (n - 1.f) : var;
+            a.running_mean[c] = (1.f - a.momentum) * a.running_mean[c] + a.momentum * mean;
+            a.running_var[c] = (1.f - a.momentum) * a.running_var[c] + a.momentum * unbiased;
+          }
         }
+      } else if (a.training) {
+        mean = __ldcg(a.stats + c);
+        is = __ldcg(a.stats + C + c);
+      } else {
+        mean = a.running_mean[c];
+        is = rsqrtf(a.running_var[c] + a.eps);
       }
-    } else if (a.training) {
-      mean = __ldcg(a.stats + c);
-      is = __ldcg(a.stats + C + c);
-    } else {
-      mean = a.running_mean[c];
-      is = rsqrtf(a.running_var[c] + a.eps);
+      // y = x * scale + shift
+      scale = w ? is * w[c] : is;
+      shift = (b ? b[c] : 0.f) - mean * scale;
     }
-    // y = x * scale + shift
-    const float scale = w ? is * w[c] : is;
-    const float shift = (b ? b[c] : 0.f) - mean * scale;
     const T* xp = x + pl * S;
     T* yp = y + pl * S;
     if (vec) {
@@ -356,10 +409,15 @@ bn_apply_kernel(const T* __restrict__ x, T* __restrict__ y, const BnArgs a) {
         Vec4<T>::st(yp + i, v);
       }
     } else {
-      for (long long i = lane; i < S; i += 32) {
-        float v = fmaf((float)xp[i], scale, shift);
-        if (a.relu) v = fmaxf(v, 0.f);
-        yp[i] = (T)v;
+      for (long long i = lane; i < S; i += 32 * kBatch) {
+        float v[kBatch];
+        load_batch(xp, i, S, v);
+#pragma unroll
+        for (int j = 0; j < kBatch; j++) {
+          v[j] = fmaf(v[j], scale, shift);
+          if (a.relu) v[j] = fmaxf(v[j], 0.f);
+          if (i + 32 * j < S) yp[i + 32 * j] = (T)v[j];
+        }
       }
     }
   }
@@ -371,6 +429,7 @@ __global__ void __launch_bounds__(256)
 bn_bwd_apply_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __restrict__ dx,
                     float* __restrict__ dgamma, float* __restrict__ dbeta, const BnArgs a,
                     const T* __restrict__ yrelu) {
+  constexpr int SB = 2;      // (three tensors: see bn_partial_kernel)
   __shared__ int sm_flag;
   __shared__ float s_count;
   const int C = a.C;
@@ -389,25 +448,30 @@ bn_bwd_apply_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __rest
   const long long S = a.S;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool vec = planes_vectorisable<T>(S, x, dy, dx) && (yrelu == nullptr || planes_vectorisable<T>(S, yrelu, dy, dx));
+  int known = -1;
+  float mean = 0.f, is = 0.f, m1 = 0.f, m2 = 0.f, k = 0.f;
   for (long long pl = (long long)blockIdx.x * 8 + warp; pl < planes; pl += (long long)gridDim.x * 8) {
-    const int c = (int)(pl % C);
-    const float mean = a.stats[c], is = a.stats[C + c];
-    float m1, m2;
-    if (a.split == 2) {
-      float s0, s1;
-      local_sums(a, c, s0, s1);
-      if (pl < C && lane == 0) {
-        if (dbeta) dbeta[c] = s0;
-        if (dgamma) dgamma[c] = s1;
+    const int c = channel_of(pl, C);
+    if (c != known) {
+      known = c;
+      mean = a.stats[c];
+      is = a.stats[C + c];
+      if (a.split == 2) {
+        float s0, s1;
+        local_sums(a, c, s0, s1);
+        if (pl < C && lane == 0) {
+          if (dbeta) dbeta[c] = s0;
+          if (dgamma) dgamma[c] = s1;
+        }
+        const float n = (float)a.N * (float)a.S;
+        m1 = s0 / n;
+        m2 = s1 / n;
+      } else {
+        m1 = __ldcg(a.sums + c);
+        m2 = __ldcg(a.sums + C + c);
       }
-      const float n = (float)a.N * (float)a.S;
-      m1 = s0 / n;
-      m2 = s1 / n;
-    } else {
-      m1 = __ldcg(a.sums + c);
-      m2 = __ldcg(a.sums + C + c);
+      k = w ? is * w[c] : is;
     }
-    const float k = w ? is * w[c] : is;
     const T* xp = x + pl * S;
     const T* gp = dy + pl * S;
     T* op = dx + pl * S;
@@ -427,10 +491,16 @@ bn_bwd_apply_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __rest
         Vec4<T>::st(op + i, g);
       }
     } else {
-      for (long long i = lane; i < S; i += 32) {
-        float g = (float)gp[i];
-        if (yrelu && !((float)yrelu[pl * S + i] > 0.f)) g = 0.f;
-        op[i] = (T)(k * (g - m1 - ((float)xp[i] - mean) * is * m2));
+      for (long long i = lane; i < S; i += 32 * SB) {
+        float xv[SB], g[SB], yv[SB];
+        load_batch(xp, i, S, xv);
+        load_batch(gp, i, S, g);
+        if (yrelu) load_batch(yrelu + pl * S, i, S, yv);
+#pragma unroll
+        for (int j = 0; j < SB; j++) {
+          if (yrelu && !(yv[j] > 0.f)) g[j] = 0.f;
+          if (i + 32 * j < S) op[i + 32 * j] = (T)(k * (g[j] - m1 - (xv[j] - mean) * is * m2));
+        }
       }
     }
   }
@@ -451,6 +521,14 @@ inline int grid_for(long long work) {
   if (g > 148 * 8) g = 148 * 8;
   if (g < 1) g = 1;
   return (int)g;
+}
+
+// CTAs of the apply kernels: a multiple of C / 8 where that keeps a warp, which takes every eighth plane of a CTA, with one channel.
+inline int grid_planes(long long total, int C) {
+  int g = grid_for(total);
+  const int unit = C % 8 == 0 ? C / 8 : C;
+  if (unit <= g) g = g / unit * unit;
+  return g;
 }
 
 void fill_comm(BnArgs& a, int sync, long long slot_off) {
@@ -502,9 +580,9 @@ GB_EXPORT int gb_bn_fwd(int dtype, const void* x, void* y, const float* w, const
 #define GB_BN(T)                                                                                      \
   {                                                                                                   \
     if (training)                                                                                     \
-      bn_partial_kernel<T><<<dim3(C, kSplits), 256, 0, s>>>((const T*)x, nullptr, nullptr, nullptr, work, N, C, S, 0, nullptr); \
+      launch_partial<T, 0>(x, nullptr, nullptr, nullptr, work, N, C, S, nullptr, s);                  \
     if (training && a.split == 1) bn_finalise_kernel<<<1, 256, 0, s>>>(a, nullptr, nullptr, 0);       \
-    bn_apply_kernel<T><<<grid_for(total), 256, 0, s>>>((const T*)x, (T*)y, a);                        \
+    bn_apply_kernel<T><<<grid_planes(total, C), 256, 0, s>>>((const T*)x, (T*)y, a);                        \
   }
   switch (dtype) {
     case DT_BF16: GB_BN(__nv_bfloat16) break;
@@ -532,8 +610,7 @@ GB_EXPORT int gb_channel_sum(int dtype, const void* x, void* out, float* work, i
   cudaStream_t s = (cudaStream_t)stream;
 #define GB_CS(T)                                                                                              \
   {                                                                                                           \
-    bn_partial_kernel<T><<<dim3(C, kSplits), 256, 0, s>>>((const T*)x, nullptr, nullptr, nullptr, work, N, C, S, 0, \
-                                                          nullptr);                                           \
+    launch_partial<T, 0>(x, nullptr, nullptr, nullptr, work, N, C, S, nullptr, s);                            \
     channel_sum_finish_kernel<T><<<(C + 127) / 128, 128, 0, s>>>(work, (T*)out, C);                           \
   }
   switch (dtype) {
@@ -573,9 +650,9 @@ GB_EXPORT int gb_bn_bwd(int dtype, const void* x, const void* dy, void* dx, cons
   const long long total = (long long)N * C * S;
 #define GB_BN(T)                                                                                      \
   {                                                                                                   \
-    bn_partial_kernel<T><<<dim3(C, kSplits), 256, 0, s>>>((const T*)dy, (const T*)x, stats, stats + C, work, N, C, S, 1, (const T*)yrelu); \
+    launch_partial<T, 1>(dy, x, stats, stats + C, work, N, C, S, yrelu, s);                           \
     if (a.split == 1) bn_finalise_kernel<<<1, 256, 0, s>>>(a, dgamma, dbeta, 1);                      \
-    bn_bwd_apply_kernel<T><<<grid_for(total), 256, 0, s>>>((const T*)x, (const T*)dy, (T*)dx, dgamma, dbeta, a, (const T*)yrelu); \
+    bn_bwd_apply_kernel<T><<<grid_planes(total, C), 256, 0, s>>>((const T*)x, (const T*)dy, (T*)dx, dgamma, dbeta, a, (const T*)yrelu); \
   }
   switch (dtype) {
     case DT_BF16: GB_BN(__nv_bfloat16) break;

@@ -239,3 +239,28 @@ def test_pool_kernels_on_any_map(mode, include, B, S, nwin, taps, status_ok):
     assert bool(y.cpu()[nan].isnan().all())
     if mode == 0:
         assert torch.equal(arg.cpu()[~nan], torch.from_numpy(warg).int()[~nan])
+
+
+@pytest.mark.parametrize("N,C,H,W", [(5, 64, 7, 7), (33, 72, 13, 13), (64, 64, 1, 1), (3, 100, 23, 89), (40, 64, 30, 30), (2, 65, 1, 3), (33, 9, 13, 13), (70, 3, 32, 32)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_batchnorm_of_odd_and_even_planes(N, C, H, W, dtype, status_ok):
+    """A warp or a CTA per channel and split, vectors or single elements, images that the splits and the launch's stride leave over."""
+    from gonn_b200.nn.batchnorm import BatchNorm2d
+    torch.manual_seed(C)
+    bn = BatchNorm2d(C, fused_relu=True, device="cuda", dtype=dtype)
+    with torch.no_grad():
+        bn.weight.uniform_(0.5, 1.5)
+        bn.bias.uniform_(-0.5, 0.5)
+    x = (torch.randn(N, C, H, W, device="cuda") * 2 + 1).to(dtype).requires_grad_()
+    dy = torch.randn(N, C, H, W, device="cuda").to(dtype)
+    y = bn(x)
+    y.backward(dy)
+    xd = x.detach().double().requires_grad_()
+    w, b = (p.detach().double().requires_grad_() for p in (bn.weight, bn.bias))
+    yd = F.relu(F.batch_norm(xd, None, None, w, b, True, 0.1, bn.eps if hasattr(bn, "eps") else 1e-5))
+    # the mask of the fused ReLU is that of the rounded output
+    yd.backward(torch.where(y > 0, dy, 0).double())
+    unit = 2.0 ** (-8 if dtype == torch.bfloat16 else -20)      # the result's type; fp32: sums of up to 36 000 terms
+    for name, got, want in (("y", y, yd), ("dx", x.grad, xd.grad), ("dw", bn.weight.grad, w.grad), ("db", bn.bias.grad, b.grad)):
+        err = (got.double() - want).norm() / want.norm().clamp_min(1e-3 * want.numel() ** 0.5)
+        assert err.item() < 2 * unit, (name, err.item())
