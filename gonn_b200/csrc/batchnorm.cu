@@ -96,6 +96,8 @@ template <typename T, bool PER_WARP, int MODE>
 __global__ void __launch_bounds__(256)
 bn_partial_kernel(const T* __restrict__ a, const T* __restrict__ xin, const float* __restrict__ mean, const float* __restrict__ invstd,
                   float* __restrict__ part, int N, int C, long long S, const T* __restrict__ yrelu) {
+  pdl_trigger();
+  pdl_wait();
   // yrelu (backward only, may be null): the forward's output after its fused ReLU; the incoming
   // gradient counts as zero wherever that output is zero
   constexpr int VB = MODE ? 1 : 4, SB = MODE ? 2 : 8;      // in flight of each tensor: a backward that holds more registers is slower
@@ -161,9 +163,9 @@ void launch_partial(const void* a, const void* xin, const float* mean, const flo
                     const void* yrelu, cudaStream_t s) {
   const long long elements = (long long)((N + kSplits - 1) / kSplits) * S;
   if (C >= 64 && elements <= 2048)
-    bn_partial_kernel<T, true, MODE><<<dim3((C + 7) / 8, kSplits), 256, 0, s>>>((const T*)a, (const T*)xin, mean, invstd, part, N, C, S, (const T*)yrelu);
+    gbh::launch(bn_partial_kernel<T, true, MODE>, dim3(dim3((C + 7) / 8, kSplits)), dim3(256), 0, s, 1, (const T*)a, (const T*)xin, mean, invstd, part, N, C, S, (const T*)yrelu);
   else
-    bn_partial_kernel<T, false, MODE><<<dim3(C, kSplits), 256, 0, s>>>((const T*)a, (const T*)xin, mean, invstd, part, N, C, S, (const T*)yrelu);
+    gbh::launch(bn_partial_kernel<T, false, MODE>, dim3(dim3(C, kSplits)), dim3(256), 0, s, 1, (const T*)a, (const T*)xin, mean, invstd, part, N, C, S, (const T*)yrelu);
 }
 
 struct BnArgs {
@@ -338,6 +340,8 @@ __device__ __forceinline__ int channel_of(long long plane, int C) {
 template <typename T>
 __global__ void __launch_bounds__(256)
 bn_apply_kernel(const T* __restrict__ x, T* __restrict__ y, const BnArgs a) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ int sm_flag;
   __shared__ float s_count;
   const int C = a.C;
@@ -429,6 +433,8 @@ __global__ void __launch_bounds__(256)
 bn_bwd_apply_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __restrict__ dx,
                     float* __restrict__ dgamma, float* __restrict__ dbeta, const BnArgs a,
                     const T* __restrict__ yrelu) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int SB = 2;      // (three tensors: see bn_partial_kernel)
   __shared__ int sm_flag;
   __shared__ float s_count;
@@ -509,6 +515,8 @@ bn_bwd_apply_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __rest
 
 template <typename T>
 __global__ void channel_sum_finish_kernel(const float* __restrict__ part, T* __restrict__ out, int C) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= C) return;
   float s = 0.f;
@@ -582,7 +590,7 @@ GB_EXPORT int gb_bn_fwd(int dtype, const void* x, void* y, const float* w, const
     if (training)                                                                                     \
       launch_partial<T, 0>(x, nullptr, nullptr, nullptr, work, N, C, S, nullptr, s);                  \
     if (training && a.split == 1) bn_finalise_kernel<<<1, 256, 0, s>>>(a, nullptr, nullptr, 0);       \
-    bn_apply_kernel<T><<<grid_planes(total, C), 256, 0, s>>>((const T*)x, (T*)y, a);                        \
+    gbh::launch(bn_apply_kernel<T>, dim3(grid_planes(total, C)), dim3(256), 0, s, 1, (const T*)x, (T*)y, a);                        \
   }
   switch (dtype) {
     case DT_BF16: GB_BN(__nv_bfloat16) break;
@@ -611,7 +619,7 @@ GB_EXPORT int gb_channel_sum(int dtype, const void* x, void* out, float* work, i
 #define GB_CS(T)                                                                                              \
   {                                                                                                           \
     launch_partial<T, 0>(x, nullptr, nullptr, nullptr, work, N, C, S, nullptr, s);                            \
-    channel_sum_finish_kernel<T><<<(C + 127) / 128, 128, 0, s>>>(work, (T*)out, C);                           \
+    gbh::launch(channel_sum_finish_kernel<T>, dim3((C + 127) / 128), dim3(128), 0, s, 1, work, (T*)out, C);                           \
   }
   switch (dtype) {
     case DT_BF16: GB_CS(__nv_bfloat16) break;
@@ -652,7 +660,7 @@ GB_EXPORT int gb_bn_bwd(int dtype, const void* x, const void* dy, void* dx, cons
   {                                                                                                   \
     launch_partial<T, 1>(dy, x, stats, stats + C, work, N, C, S, yrelu, s);                           \
     if (a.split == 1) bn_finalise_kernel<<<1, 256, 0, s>>>(a, dgamma, dbeta, 1);                      \
-    bn_bwd_apply_kernel<T><<<grid_planes(total, C), 256, 0, s>>>((const T*)x, (const T*)dy, (T*)dx, dgamma, dbeta, a, (const T*)yrelu); \
+    gbh::launch(bn_bwd_apply_kernel<T>, dim3(grid_planes(total, C)), dim3(256), 0, s, 1, (const T*)x, (const T*)dy, (T*)dx, dgamma, dbeta, a, (const T*)yrelu); \
   }
   switch (dtype) {
     case DT_BF16: GB_BN(__nv_bfloat16) break;

@@ -343,6 +343,8 @@ conv_igemm_kernel(const ConvArgs a) {
 __global__ void __launch_bounds__(256) conv_wgrad_finish_kernel(const float* __restrict__ part, uint16_t* __restrict__ dW,
                                                                 long long n, int C, int T, int splits, int bf16, int beta,
                                                                 int tap_major) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float sm[8][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (long long b = blockIdx.x; b * 32 < n; b += gridDim.x) {
@@ -517,6 +519,8 @@ __global__ void __launch_bounds__(kSmallWarps * 32)
 conv_direct_small_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w, const int* __restrict__ idx,
                          const uint16_t* __restrict__ bias, uint16_t* __restrict__ y, int Nimg, int C, int S, int L, int T,
                          int M, int bf16) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) uint32_t dsm[];
   const int MT = (M + 15) / 16, K = C * T;
   uint32_t* wf = dsm;                                    // [MT][2 k-steps][32 lanes][4]
@@ -613,6 +617,8 @@ template <int MT, int V>
 __global__ void __launch_bounds__(kSmallWarps * 32, 2)
 conv_wgrad_small_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ dy, const int* __restrict__ idx,
                         float* __restrict__ part, int Nimg, int C, int S, int L, int T, int M, int bf16) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) uint32_t dsm[];
   const int K = C * T, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   int* si = reinterpret_cast<int*>(dsm) + warp * 32 * (T + 17);
@@ -710,7 +716,7 @@ int set_attr_once() {
 int gbc::launch_wgrad_finish(const float* part, uint16_t* dW, int M, int C, int T, int splits, int bf16, int beta, bool tap_major,
                              cudaStream_t s) {
   const long long n = (long long)M * C * T, blocks = (n + 31) / 32;
-  conv_wgrad_finish_kernel<<<(int)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, s>>>(part, dW, n, C, T, splits, bf16, beta, tap_major);
+  gbh::launch(conv_wgrad_finish_kernel, dim3((int)(blocks < 148 * 16 ? blocks : 148 * 16)), dim3(256), 0, s, 1, part, dW, n, C, T, splits, bf16, beta, tap_major);
   GB_CUDA_OK(cudaGetLastError());
   return gbh::E_OK;
 }
@@ -776,7 +782,7 @@ GB_EXPORT int gb_conv_direct_small(int dtype, const void* x, const void* w, cons
 #define GB_DS(V)                                                                                                          \
   {                                                                                                                       \
     GB_CUDA_OK(cudaFuncSetAttribute(conv_direct_small_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem)); \
-    conv_direct_small_kernel<V><<<grid, kSmallWarps * 32, smem, (cudaStream_t)stream>>>(                                  \
+    gbh::launch(conv_direct_small_kernel<V>, dim3(grid), dim3(kSmallWarps * 32), smem, (cudaStream_t)stream, 1,                                   \
         (const uint16_t*)x, (const uint16_t*)w, idx, (const uint16_t*)bias, (uint16_t*)y, Nimg, C, S, L, T, M, dtype == DT_BF16); \
   }
   switch (run_width(L, y)) {
@@ -825,7 +831,7 @@ GB_EXPORT int gb_conv_wgrad(int dtype, const void* x, const void* dy, const int*
   {                                                                                                                \
     const size_t red = (size_t)MT * 16 * kDirectK * 4, smem = idx_bytes > red ? idx_bytes : red;                   \
     GB_CUDA_OK(cudaFuncSetAttribute(conv_wgrad_small_kernel<MT, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem)); \
-    conv_wgrad_small_kernel<MT, V><<<dim3(splits, M / (MT * 16)), kSmallWarps * 32, smem, (cudaStream_t)stream>>>( \
+    gbh::launch(conv_wgrad_small_kernel<MT, V>, dim3(dim3(splits, M / (MT * 16))), dim3(kSmallWarps * 32), smem, (cudaStream_t)stream, 1,  \
         (const uint16_t*)x, (const uint16_t*)dy, idx, part, Nimg, C, S, L, T, M, bf);                              \
   }
 #define GB_WV(MT)                    \

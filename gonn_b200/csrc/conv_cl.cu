@@ -67,6 +67,7 @@ __global__ void __launch_bounds__(THREADS, 2) conv_cl_kernel(const ClArgs a) {
     tmem_alloc(tmem_slot, BN);
     tmem_relinquish();
   }
+  pdl_wait();
   const int m0 = blockIdx.y * BM;
   const long long n0 = (long long)blockIdx.x * BN;        // MODE 0: position; MODE 1: (tap, c) column
   if (MODE == 0) {
@@ -86,6 +87,7 @@ __global__ void __launch_bounds__(THREADS, 2) conv_cl_kernel(const ClArgs a) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
   long long k_begin = 0, k_end = K;                       // contraction range: k (MODE 0) or positions (MODE 1)
   if (MODE == 1) {
     k_begin = (long long)blockIdx.z * a.per_split;
@@ -275,6 +277,8 @@ struct PackArgs {
 // A block of 256 threads turns a 64 x 64 tile.  Two-byte loads along the contiguous dimension, pairs of rows
 // packed into one word of shared memory (pitch 33 words: free of conflicts both ways), 16-byte stores.
 __global__ void __launch_bounds__(256) conv_pack_kernel(const PackArgs a) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ uint32_t sm[64 * 33];
   int ji = 0;
   while (ji + 1 < a.jobs && (long long)blockIdx.x >= a.job[ji + 1].first) ji++;
@@ -383,13 +387,13 @@ GB_EXPORT int gb_conv_cl_fwd(int dtype, const void* x, const void* w, const int*
     gbh::set_error("gb_conv_cl_fwd: problem too large");
     return gbh::E_TOO_LARGE;
   }
-  conv_pack_kernel<<<(unsigned)blocks, 256, 0, s>>>(pa);
+  gbh::launch(conv_pack_kernel, dim3((unsigned)blocks), dim3(256), 0, s, 1, pa);
   ClArgs a;
   memset(&a, 0, sizeof(a));
   a.W = wp; a.X = xt; a.idx = idx; a.Y = y; a.bias = (const uint16_t*)bias;
   a.Nimg = Nimg; a.C = C; a.S = S; a.L = L; a.T = T; a.M = M; a.bf16 = dtype == 0;
   a.status = gbh::status_ptr();
-  conv_cl_kernel<0><<<dim3((unsigned)(((long long)Nimg * L + BN - 1) / BN), (M + BM - 1) / BM), THREADS, smem_bytes(T), s>>>(a);
+  gbh::launch(conv_cl_kernel<0>, dim3(dim3((unsigned)(((long long)Nimg * L + BN - 1) / BN), (M + BM - 1) / BM)), dim3(THREADS), smem_bytes(T), s, 1, a);
   GB_CUDA_OK(cudaGetLastError());
   return gbh::E_OK;
 }
@@ -424,14 +428,14 @@ GB_EXPORT int gb_conv_cl_bwd(int dtype, const void* x, const void* w, const void
     gbh::set_error("gb_conv_cl_bwd: problem too large");
     return gbh::E_TOO_LARGE;
   }
-  conv_pack_kernel<<<(unsigned)blocks, 256, 0, s>>>(pa);
+  gbh::launch(conv_pack_kernel, dim3((unsigned)blocks), dim3(256), 0, s, 1, pa);
   ClArgs a;
   memset(&a, 0, sizeof(a));
   a.bf16 = dtype == 0; a.Nimg = Nimg; a.T = T; a.status = gbh::status_ptr();
   if (dx != nullptr) {
     a.W = wp; a.X = dyt; a.idx = inv; a.Y = dx;
     a.C = M; a.S = L; a.L = S; a.M = C;
-    conv_cl_kernel<0><<<dim3((unsigned)(((long long)Nimg * S + BN - 1) / BN), (C + BM - 1) / BM), THREADS, smem_bytes(T), s>>>(a);
+    gbh::launch(conv_cl_kernel<0>, dim3(dim3((unsigned)(((long long)Nimg * S + BN - 1) / BN), (C + BM - 1) / BM)), dim3(THREADS), smem_bytes(T), s, 1, a);
   }
   if (dw != nullptr) {
     const long long P = (long long)Nimg * L;
@@ -439,7 +443,7 @@ GB_EXPORT int gb_conv_cl_bwd(int dtype, const void* x, const void* w, const void
     a.W = nullptr; a.X = xt; a.DY = dyt; a.idx = idx; a.Y = part;
     a.C = C; a.S = S; a.L = L; a.M = M;
     a.per_split = ((P + splits - 1) / splits + BK - 1) / BK * BK;
-    conv_cl_kernel<1><<<dim3((C * T + BN - 1) / BN, (M + BM - 1) / BM, splits), THREADS, smem_bytes(0), s>>>(a);
+    gbh::launch(conv_cl_kernel<1>, dim3(dim3((C * T + BN - 1) / BN, (M + BM - 1) / BM, splits)), dim3(THREADS), smem_bytes(0), s, 1, a);
     rc = gbc::launch_wgrad_finish(part, (uint16_t*)dw, M, C, T, splits, a.bf16, beta, true, s);
     if (rc) return rc;
   }

@@ -104,6 +104,8 @@ template <typename T, typename TO, int OP>
 __global__ void col_reduce_kernel(const T* __restrict__ x, TO* __restrict__ y,
                                   typename Acc<T>::CT* __restrict__ part, long long R, long long inner,
                                   int splits, int to_part) {
+  pdl_trigger();
+  pdl_wait();
   using CT = typename Acc<T>::CT;
   __shared__ CT sm[8][33];
   const long long col = (long long)blockIdx.x * 32 + threadIdx.x;
@@ -136,6 +138,8 @@ template <typename T, typename TO, int OP>
 __global__ void __launch_bounds__(256)
 col_reduce_vec_kernel(const T* __restrict__ x, TO* __restrict__ y, float* __restrict__ part, long long R,
                       long long inner, int splits, int to_part) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float sm[8][8 * 32];
   const int tx = threadIdx.x, ty = threadIdx.y;
   const long long col0 = ((long long)blockIdx.x * 32 + tx) * 8;
@@ -196,6 +200,8 @@ col_reduce_vec_kernel(const T* __restrict__ x, TO* __restrict__ y, float* __rest
 template <typename CT, typename TO, int OP>
 __global__ void col_finish_kernel(const CT* __restrict__ part, TO* __restrict__ y, long long R,
                                   long long inner, int splits, long long outer, int accumulate) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ CT sm[8][33];
   const long long col = (long long)blockIdx.x * 32 + threadIdx.x;
   const long long o = blockIdx.y;
@@ -254,7 +260,7 @@ template <typename T, typename TO, int OP>
 void launch_col_vec(dim3 grid, dim3 blk, cudaStream_t s, const void* x, void* y, void* scratch, long long R,
                     long long inner, int splits, int to_part) {
   if constexpr (sizeof(T) == 2) {
-    col_reduce_vec_kernel<T, TO, OP><<<grid, blk, 0, s>>>((const T*)x, (TO*)y, (float*)scratch, R, inner, splits,
+    gbh::launch(col_reduce_vec_kernel<T, TO, OP>, dim3(grid), dim3(blk), 0, s, 1, (const T*)x, (TO*)y, (float*)scratch, R, inner, splits,
                                                           to_part);
   }
 }
@@ -303,10 +309,10 @@ int reduce_t(int op, const void* x, void* y, void* scratch, long long scratch_by
       }                                                                                              \
       dim3 grid((unsigned)tiles, splits, (unsigned)outer), blk(32, 8);                               \
       if (vec) launch_col_vec<T, TO, OPID>(grid, blk, s, x, y, scratch, R, inner, splits, two ? 1 : 0); \
-      else col_reduce_kernel<T, TO, OPID><<<grid, blk, 0, s>>>((const T*)x, (TO*)y, (CT*)scratch, R, inner, splits, two ? 1 : 0); \
+      else gbh::launch(col_reduce_kernel<T, TO, OPID>, dim3(grid), dim3(blk), 0, s, 1, (const T*)x, (TO*)y, (CT*)scratch, R, inner, splits, two ? 1 : 0); \
       if (two) {                                                                                     \
         dim3 fgrid((unsigned)((inner + 31) / 32), (unsigned)outer);                                  \
-        col_finish_kernel<CT, TO, OPID><<<fgrid, dim3(32, 8), 0, s>>>((const CT*)scratch, (TO*)y, R, inner, splits, outer, accumulate); \
+        gbh::launch(col_finish_kernel<CT, TO, OPID>, dim3(fgrid), dim3(dim3(32, 8)), 0, s, 1, (const CT*)scratch, (TO*)y, R, inner, splits, outer, accumulate); \
       }                                                                                              \
     }                                                                                                \
     break;

@@ -154,6 +154,8 @@ __global__ void ce_fwd_kernel(const T* __restrict__ x, const long long* __restri
                               float* __restrict__ lse_out, float* __restrict__ w_row, int C,
                               long long ignore_index, int has_ignore, float eps, float cw_sum,
                               int use_smem, int* status) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ float red[32];
   const long long row = blockIdx.x;
@@ -198,6 +200,8 @@ __global__ void __launch_bounds__(256)
 ce_fwd_vec_kernel(const T* __restrict__ x, const long long* __restrict__ tgt, const float* __restrict__ cw,
                   float* __restrict__ loss_row, float* __restrict__ lse_out, float* __restrict__ w_row, int C,
                   long long ignore_index, int has_ignore, int* status) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * C);
@@ -248,6 +252,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 ce_fused_vec_kernel(T* x, const long long* __restrict__ tgt, float* __restrict__ loss_row,
                     float* __restrict__ w_row, int C, float scale, int* status) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[32];
   __shared__ float s_lse;
   const long long row = blockIdx.x;
@@ -316,6 +322,8 @@ __global__ void scale_unless_one_kernel(T* x, long long nvec, const float* __res
 // writes out[0] = total loss (mean: / denom), out[1] = denom.
 __global__ void ce_reduce_kernel(const float* __restrict__ loss_row, const float* __restrict__ w_row,
                                  long long rows, int mean, float* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[32];
   float a = 0.f, b = 0.f;
   for (long long i = threadIdx.x; i < rows; i += blockDim.x) { a += loss_row[i]; b += w_row[i]; }
@@ -336,6 +344,8 @@ __global__ void ce_bwd_kernel(const T* x, const long long* __restrict__ tgt,
                               const float* __restrict__ gscalar, const float* __restrict__ grow,
                               const float* __restrict__ denom, T* dx, int C, long long ignore_index,
                               int has_ignore, float eps, float cw_sum) {
+  pdl_trigger();
+  pdl_wait();
   const long long row = blockIdx.x;
   const long long t = tgt[row];
   const bool ignored = (has_ignore && t == ignore_index) || t < 0 || t >= C;
@@ -442,7 +452,7 @@ int ce_fwd_t(const void* x, const long long* tgt, const float* cw, float* loss_r
              float cw_sum, cudaStream_t s) {
   if constexpr (sizeof(T) == 2) {
     if (eps == 0.f && (C & 7) == 0 && (((uintptr_t)x & 15) == 0)) {
-      ce_fwd_vec_kernel<T><<<(unsigned)rows, 256, 0, s>>>((const T*)x, tgt, cw, loss_row, lse, w_row, C,
+      gbh::launch(ce_fwd_vec_kernel<T>, dim3((unsigned)rows), dim3(256), 0, s, 1, (const T*)x, tgt, cw, loss_row, lse, w_row, C,
                                                           ignore_index, has_ignore, gbh::status_ptr());
       GB_CUDA_OK(cudaGetLastError());
       return gbh::E_OK;
@@ -452,7 +462,7 @@ int ce_fwd_t(const void* x, const long long* tgt, const float* cw, float* loss_r
   size_t bytes;
   int rc = set_smem<T>((const void*)ce_fwd_kernel<T>, C, &use_smem, &bytes);
   if (rc) return rc;
-  ce_fwd_kernel<T><<<(unsigned)rows, block_for(C), bytes, s>>>((const T*)x, tgt, cw, loss_row, lse, w_row, C,
+  gbh::launch(ce_fwd_kernel<T>, dim3((unsigned)rows), dim3(block_for(C)), bytes, s, 1, (const T*)x, tgt, cw, loss_row, lse, w_row, C,
                                                               ignore_index, has_ignore, eps, cw_sum,
                                                               use_smem, gbh::status_ptr());
   GB_CUDA_OK(cudaGetLastError());
@@ -509,7 +519,7 @@ GB_EXPORT int gb_ce_fwd(int dtype, const void* logits, const long long* targets,
       return gbh::E_BAD_ARG;
   }
   if (rc) return rc;
-  ce_reduce_kernel<<<1, 1024, 0, s>>>(loss_row, w_row, rows, reduction == 0, out2);
+  gbh::launch(ce_reduce_kernel, dim3(1), dim3(1024), 0, s, 1, loss_row, w_row, rows, reduction == 0, out2);
   GB_CUDA_OK(cudaGetLastError());
   return gbh::E_OK;
 }
@@ -527,11 +537,11 @@ GB_EXPORT int gb_ce_fused(int dtype, void* logits, const long long* targets, flo
   }
   const float scale = reduction == 0 ? 1.f / (float)rows : 1.f;
   if (dtype == DT_BF16)
-    ce_fused_vec_kernel<__nv_bfloat16><<<(unsigned)rows, 256, 0, s>>>((__nv_bfloat16*)logits, targets, loss_row, w_row, C, scale, gbh::status_ptr());
+    gbh::launch(ce_fused_vec_kernel<__nv_bfloat16>, dim3((unsigned)rows), dim3(256), 0, s, 1, (__nv_bfloat16*)logits, targets, loss_row, w_row, C, scale, gbh::status_ptr());
   else
-    ce_fused_vec_kernel<__half><<<(unsigned)rows, 256, 0, s>>>((__half*)logits, targets, loss_row, w_row, C, scale, gbh::status_ptr());
+    gbh::launch(ce_fused_vec_kernel<__half>, dim3((unsigned)rows), dim3(256), 0, s, 1, (__half*)logits, targets, loss_row, w_row, C, scale, gbh::status_ptr());
   GB_CUDA_OK(cudaGetLastError());
-  ce_reduce_kernel<<<1, 1024, 0, s>>>(loss_row, w_row, rows, reduction == 0, out2);
+  gbh::launch(ce_reduce_kernel, dim3(1), dim3(1024), 0, s, 1, loss_row, w_row, rows, reduction == 0, out2);
   GB_CUDA_OK(cudaGetLastError());
   return gbh::E_OK;
 }
@@ -565,7 +575,7 @@ GB_EXPORT int gb_ce_bwd(int dtype, const void* logits, const long long* targets,
   if (!class_w) class_w_sum = (float)C;
   int blk = block_for(C);
 #define GB_CE(T)                                                                                   \
-  ce_bwd_kernel<T><<<(unsigned)rows, blk, 0, s>>>((const T*)logits, targets, class_w, lse, g_scalar, g_row, \
+  gbh::launch(ce_bwd_kernel<T>, dim3((unsigned)rows), dim3(blk), 0, s, 1, (const T*)logits, targets, class_w, lse, g_scalar, g_row, \
                                                   denom, (T*)dlogits, C, ignore_index, has_ignore,  \
                                                   label_smoothing, class_w_sum)
   switch (dtype) {

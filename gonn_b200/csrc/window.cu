@@ -88,6 +88,8 @@ template <typename T>
 __global__ void pool_fwd_kernel(const T* __restrict__ x, const int* __restrict__ idx,
                                 T* __restrict__ y, int* __restrict__ arg, long long B, long long S,
                                 int nwin, int T_, int mode, int count_include_pad, float p) {
+  pdl_trigger();
+  pdl_wait();
   const long long total = B * nwin;
   const bool small = total <= 0x7fffffffLL && B * S <= 0x7fffffffLL;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -137,6 +139,8 @@ template <typename T, int TAPS, bool MAX>
 __global__ void __launch_bounds__(256)
 pool_fwd_small_kernel(const T* __restrict__ x, const int* __restrict__ idx, T* __restrict__ y, int* __restrict__ arg, long long B,
                       long long S, int nwin, int T_, int count_include_pad) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int U = 16 / TAPS;
   for (int win = blockIdx.x * blockDim.x + threadIdx.x; win < nwin; win += gridDim.x * blockDim.x) {
     int src[TAPS], first = -1, cnt = 0;
@@ -212,6 +216,8 @@ template <typename T, bool MAX>
 __global__ void __launch_bounds__(256)
 pool_fwd_wide_kernel(const T* __restrict__ x, const int* __restrict__ idx, T* __restrict__ y, int* __restrict__ arg, long long B,
                      long long S, int nwin, int T_, int count_include_pad) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int U = 2;
   const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
   const long long warps = (long long)gridDim.x * wpb, w0 = (long long)blockIdx.x * wpb + (threadIdx.x >> 5);
@@ -294,6 +300,8 @@ __global__ void pool_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ 
                                 const int* __restrict__ cols, T* __restrict__ dx, long long B,
                                 long long S, int nwin, int T_, int mode, int count_include_pad,
                                 float p) {
+  pdl_trigger();
+  pdl_wait();
   const long long total = B * S;
   const bool small = total <= 0x7fffffffLL;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -335,6 +343,8 @@ template <typename T, bool MAX>
 __global__ void __launch_bounds__(256)
 pool_bwd_disjoint_kernel(const T* __restrict__ dy, const int* __restrict__ arg, const int2* __restrict__ p2w, const int* __restrict__ wcnt,
                          T* __restrict__ dx, long long B, int S, int nwin, int T_, int count_include_pad) {
+  pdl_trigger();
+  pdl_wait();
   // A thread keeps its positions' table entries in registers and walks the planes (b) of its blockIdx.y slice, U at a time so that
   // their loads are in flight together (a position outside every window reads window 0 and stores 0).  16384 x 900, 2 x 2 windows,
   // bf16: four at a time 31 us, so 19.9.
@@ -427,7 +437,7 @@ GB_EXPORT int gb_pool_fwd(int dtype, const void* x, const int* idx, void* y, int
     const int bx = (nwin + 255) / 256 < 64 ? (nwin + 255) / 256 : 64;
     long long by = (148 * 8 + bx - 1) / bx;
     if (by > B) by = B;
-#define GB_POOL(TAPS, MAX) pool_fwd_small_kernel<T, TAPS, MAX><<<dim3(bx, (unsigned)by), 256, 0, s>>>((const T*)x, idx, (T*)y, arg, B, S, nwin, T_, count_include_pad)
+#define GB_POOL(TAPS, MAX) gbh::launch(pool_fwd_small_kernel<T, TAPS, MAX>, dim3(dim3(bx, (unsigned)by)), dim3(256), 0, s, 1, (const T*)x, idx, (T*)y, arg, B, S, nwin, T_, count_include_pad)
     GB_DISPATCH_T(({
       if (T_ <= 4) { if (mode == POOL_MAX) GB_POOL(4, true); else GB_POOL(4, false); }
       else { if (mode == POOL_MAX) GB_POOL(8, true); else GB_POOL(8, false); }
@@ -441,13 +451,13 @@ GB_EXPORT int gb_pool_fwd(int dtype, const void* x, const int* idx, void* y, int
     const long long most = 148 * 8 > (nwin + 7) / 8 ? 148 * 8 : (nwin + 7) / 8;
     const unsigned grid = (unsigned)((total + 7) / 8 < most ? (total + 7) / 8 : most);
     GB_DISPATCH_T(({
-      if (mode == POOL_MAX) pool_fwd_wide_kernel<T, true><<<grid, 256, 0, s>>>((const T*)x, idx, (T*)y, arg, B, S, nwin, T_, count_include_pad);
-      else pool_fwd_wide_kernel<T, false><<<grid, 256, 0, s>>>((const T*)x, idx, (T*)y, arg, B, S, nwin, T_, count_include_pad);
+      if (mode == POOL_MAX) gbh::launch(pool_fwd_wide_kernel<T, true>, dim3(grid), dim3(256), 0, s, 1, (const T*)x, idx, (T*)y, arg, B, S, nwin, T_, count_include_pad);
+      else gbh::launch(pool_fwd_wide_kernel<T, false>, dim3(grid), dim3(256), 0, s, 1, (const T*)x, idx, (T*)y, arg, B, S, nwin, T_, count_include_pad);
     }));
     GB_CUDA_OK(cudaGetLastError());
     return gbh::E_OK;
   }
-  GB_DISPATCH_T((pool_fwd_kernel<T><<<grid_for(total), 256, 0, s>>>((const T*)x, idx, (T*)y, arg, B, S, nwin, T_, mode, count_include_pad, p)));
+  GB_DISPATCH_T((gbh::launch(pool_fwd_kernel<T>, dim3(grid_for(total)), dim3(256), 0, s, 1, (const T*)x, idx, (T*)y, arg, B, S, nwin, T_, mode, count_include_pad, p)));
   GB_CUDA_OK(cudaGetLastError());
   return gbh::E_OK;
 }
@@ -469,8 +479,8 @@ GB_EXPORT int gb_pool_bwd_disjoint(int dtype, const void* dy, const int* arg, co
   if (by > B) by = B;
   if (by < 1) by = 1;
   GB_DISPATCH_T(({
-    if (mode == POOL_MAX) pool_bwd_disjoint_kernel<T, true><<<dim3(bx, (unsigned)by), 256, 0, s>>>((const T*)dy, arg, (const int2*)p2w, wcnt, (T*)dx, B, (int)S, nwin, T_, count_include_pad);
-    else pool_bwd_disjoint_kernel<T, false><<<dim3(bx, (unsigned)by), 256, 0, s>>>((const T*)dy, arg, (const int2*)p2w, wcnt, (T*)dx, B, (int)S, nwin, T_, count_include_pad);
+    if (mode == POOL_MAX) gbh::launch(pool_bwd_disjoint_kernel<T, true>, dim3(dim3(bx, (unsigned)by)), dim3(256), 0, s, 1, (const T*)dy, arg, (const int2*)p2w, wcnt, (T*)dx, B, (int)S, nwin, T_, count_include_pad);
+    else gbh::launch(pool_bwd_disjoint_kernel<T, false>, dim3(dim3(bx, (unsigned)by)), dim3(256), 0, s, 1, (const T*)dy, arg, (const int2*)p2w, wcnt, (T*)dx, B, (int)S, nwin, T_, count_include_pad);
   }));
   GB_CUDA_OK(cudaGetLastError());
   return gbh::E_OK;
@@ -484,7 +494,7 @@ GB_EXPORT int gb_pool_bwd(int dtype, const void* dy, const void* x, const void* 
   if (total <= 0) return gbh::E_OK;
   cudaStream_t s = (cudaStream_t)stream;
   GB_BOUNDS_BIND();
-  GB_DISPATCH_T((pool_bwd_kernel<T><<<grid_for(total), 256, 0, s>>>((const T*)dy, (const T*)x, (const T*)y, arg, idx, offs, cols, (T*)dx, B, S, nwin, T_, mode, count_include_pad, p)));
+  GB_DISPATCH_T((gbh::launch(pool_bwd_kernel<T>, dim3(grid_for(total)), dim3(256), 0, s, 1, (const T*)dy, (const T*)x, (const T*)y, arg, idx, offs, cols, (T*)dx, B, S, nwin, T_, mode, count_include_pad, p)));
   GB_CUDA_OK(cudaGetLastError());
   return gbh::E_OK;
 }
