@@ -95,3 +95,12 @@ GB_EXPORT int gb_block_fwd(const long long* words, int n, float eps1, float eps2
   if ((rc = linear(buf_w, a.w2, a.b2, buf_x, E, F, 0, buf_n))) return rc;
   return norm(buf_x, a.n2w, a.n2b, P(a.y), eps2);
 }
+
+// Blocks one after another: argument words and (eps1, eps2, scale) of each, as gb_block_fwd takes them.
+GB_EXPORT int gb_stack_fwd(const long long* words, const float* scalars, int blocks, int n, void* stream) {
+  for (int i = 0; i < blocks; i++) {
+    const int rc = gb_block_fwd(words + (long long)i * n, n, scalars[3 * i], scalars[3 * i + 1], scalars[3 * i + 2], stream);
+    if (rc) return rc;
+  }
+  return gbh::E_OK;
+}

@@ -17,7 +17,7 @@ from ..nn.embedding import Embedding
 from ..nn.linear import Linear
 from ..nn.module import Module, ModuleList
 from ..nn.norm import LayerNorm, RMSNorm
-from ..nn.transformer import TransformerEncoderLayer
+from ..nn.transformer import ENCODER_FORWARD, TransformerEncoderLayer
 from ..ops.elementwise import binary as _binary
 from ..ops.linear import feed_forward as _feed_forward
 from ..ops.softmax import cross_entropy
@@ -44,8 +44,7 @@ class TransformerLM(Module):
         B, S = ids.shape
         pos = torch.arange(S, device=ids.device)
         x = _binary("add", self.tok(ids), self.pos(pos)[None])
-        for l in self.layers:
-            x = l(x)
+        x = _block.chain(x, self.layers, TransformerEncoderLayer, ENCODER_FORWARD)
         return self.head(self.norm(x))
 
     def loss(self, ids, targets):
@@ -65,10 +64,13 @@ class GPTBlock(Module):
         self.ff1 = Linear(d_model, d_ff, True, **kw)
         self.ff2 = Linear(d_ff, d_model, True, **kw)
 
+    def _parts(self):
+        m = self._modules
+        return m["attn"], m["norm1"], m["norm2"], m["ff1"], m["ff2"], "gelu", True, True
+
     def forward(self, x):
         if not torch.is_grad_enabled() and type(self) is GPTBlock:
-            m = self._modules
-            y = _block.evaluate(x, m["attn"], m["norm1"], m["norm2"], m["ff1"], m["ff2"], "gelu", True, True)
+            y = _block.evaluate(x, *self._parts())
             if y is not None:
                 return y
         f1 = self.norm1.fork(x, self.attn.outproj.bias) if torch.is_grad_enabled() else None
@@ -83,6 +85,9 @@ class GPTBlock(Module):
                                  "gelu", f2[1], False)
         return _feed_forward(self.norm2(x), self.ff1.weight, self.ff1.bias, self.ff2.weight, self.ff2.bias,
                              "gelu", x)
+
+
+GPT_FORWARD = GPTBlock.forward
 
 
 class GPT(Module):
@@ -106,8 +111,7 @@ class GPT(Module):
         B, S = ids.shape
         pos = torch.arange(S, device=ids.device)
         x = _binary("add", self.tok(ids), self.pos(pos)[None])
-        for l in self.layers:
-            x = l(x)
+        x = _block.chain(x, self.layers, GPTBlock, GPT_FORWARD)
         return self.head(self.norm(x))
 
     def loss(self, ids, targets):

@@ -62,10 +62,17 @@ class TransformerEncoderLayer(Module):
         y = self.ff2(self.dropff(self.act(self.ff1(x))))
         return y if residual is None else residual + y
 
+    def _parts(self):
+        """What a native evaluation of the layer needs, or None where a dropout is in the way."""
+        if not self._no_dropout():
+            return None
+        m = self._modules
+        return m["attn"], m["norm1"], m["norm2"], m["ff1"], m["ff2"], m["act"], self.pre_norm, self.causal
+
     def forward(self, x):
-        if not torch.is_grad_enabled() and type(self) is TransformerEncoderLayer and self._no_dropout():
-            m = self._modules
-            y = _block.evaluate(x, m["attn"], m["norm1"], m["norm2"], m["ff1"], m["ff2"], m["act"], self.pre_norm, self.causal)
+        if not torch.is_grad_enabled() and type(self) is TransformerEncoderLayer:
+            parts = self._parts()
+            y = _block.evaluate(x, *parts) if parts is not None else None
             if y is not None:
                 return y
         nodrop = not (self.training and self.drop1.p > 0)
@@ -95,6 +102,9 @@ class TransformerEncoderLayer(Module):
         return self.norm2(x + self.drop2(self._ff(x)))
 
 
+ENCODER_FORWARD = TransformerEncoderLayer.forward      # what a native evaluation of a chain of layers stands for
+
+
 class TransformerEncoder(Module):
     def __init__(self, num_layers: int, embed_dim: int, num_heads: int, dim_ff: int, **opts):
         super().__init__()
@@ -102,9 +112,7 @@ class TransformerEncoder(Module):
                                   for _ in range(num_layers)])
 
     def forward(self, x):
-        for l in self.layers:
-            x = l(x)
-        return x
+        return _block.chain(x, self.layers, TransformerEncoderLayer, ENCODER_FORWARD)
 
 
 class TransformerDecoderLayer(Module):

@@ -87,3 +87,45 @@ def test_what_runs_operator_by_operator():
     d.eval()
     assert _calls(lambda: d(x))[1] == 1
     assert block.evaluate(x, base.attn, base.norm1, base.norm2, base.ff1, base.ff2, base.act, True, True) is None   # tape on
+
+
+@pytest.mark.parametrize("layers", [1, 2, 5])
+def test_a_chain_of_blocks_is_one_call(layers):
+    """The models' chains: the same bits as block by block, an input that stays as it is, and block by block as soon as one of
+    them is observed, replaced or cannot be taken."""
+    from gonn_b200.models.lm import GPT
+    torch.manual_seed(layers)
+    enc = nn.TransformerEncoder(layers, 128, 4, 264, pre_norm=True, activation=nn.GELU(), dtype=torch.bfloat16, device="cuda")
+    gpt = GPT(64, 128, layers, 4, 256, 64, dtype=torch.bfloat16, device="cuda").layers
+    for stack, run in ((enc.layers, enc), (gpt, lambda x: block.chain(x, gpt, GPTBlock, GPTBlock.forward))):
+        for p in stack.parameters():
+            p.data += 0.05 * torch.randn_like(p)
+        x = torch.randn(2, 33, 128, device="cuda").bfloat16()
+        keep = x.clone()
+        y, n = _calls(lambda: run(x))
+        assert n == 1 and torch.equal(x, keep)
+        want = x
+        with torch.no_grad():
+            for l in stack:
+                want = l(want)
+        assert torch.equal(y, want)
+        last = stack[layers - 1]
+        h = last.register_forward_hook(lambda *a: None)
+        y2, n = _calls(lambda: run(x))
+        h.remove()
+        assert n == layers and torch.equal(y2, want)              # each by itself still one call
+        last.forward = last.forward
+        assert _calls(lambda: run(x))[1] == layers
+        del last.__dict__["forward"]
+        last.norm2.float()
+        assert _calls(lambda: run(x))[1] > layers
+        last.norm2.to(torch.bfloat16)
+        assert _calls(lambda: run(x))[1] == 1
+    seen = []
+    original = nn.TransformerEncoderLayer.forward
+    try:
+        nn.TransformerEncoderLayer.forward = lambda self, x: seen.append(1) or original(self, x)
+        _calls(lambda: enc(x))
+    finally:
+        nn.TransformerEncoderLayer.forward = original
+    assert len(seen) == layers
