@@ -1793,9 +1793,10 @@ int g_tma_epi = 1;
 // Builds the two tensor maps and launches.  esz: 2 (bf16/fp16) or 1 (int8).
 int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, int transB,
             long long lda, long long ldb, long long sA, long long sB, int force_bn,
-            cudaStream_t stream, void* workspace = nullptr, long long workspace_bytes = 0, int planes = 0) {
+            cudaStream_t stream, void* workspace = nullptr, long long workspace_bytes = 0, int planes = 0, int chain = 0) {
   // planes > 0: A and B are stacks of three planes, sA / sB elements apart (batch entries 3 sA / 3 sB apart, 0: shared), and
-  // `planes` plane products run along K
+  // `planes` plane products run along K.  chain > 0: no accumulator takes more than `chain` (a multiple of an atom) of K;
+  // the slices meet in the workspace
   if (g_num_sms == 0) {
     int dev = 0;
     GB_CUDA_OK(cudaGetDevice(&dev));
@@ -1839,6 +1840,16 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
   int splits = 1;
   const bool plain = (args.bias == nullptr || (planes > 0 && args.bias_f32)) && args.act == ACT_NONE && args.aux_mode == AUX_NONE;
   const bool big = 2.0 * M * N * (double)K * batch >= 8e9;  // below this the second launch costs more than it saves
+  const int cut = chain > 0 ? (kb_plane * atom_k + chain - 1) / chain : 1;       // slices that the chain asks for
+  if (cut > 1) {
+    if (workspace == nullptr || (N & 3) != 0 || !plain || (long long)M * N * batch * 4 * cut > workspace_bytes) {
+      gbh::set_error("gemm: no workspace for %d slices of K", cut);
+      return gbh::E_BAD_ARG;
+    }
+    splits = cut;
+    use2 = g_use_2cta && M >= 256 && N >= 256 &&
+           (long long)((M + 255) / 256) * ((N + 255) / 256) * batch * cut * 5 >= (long long)(g_num_sms / 2) * 4;
+  }
   if (esz == 2 && g_splitk && force_bn == 0 && plain && big && workspace != nullptr && (N & 3) == 0 &&
       M >= 128 && N >= 128) {
     const int num_kb = (K + atom - 1) / atom;
@@ -1848,8 +1859,8 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
     const bool pair_ok = g_use_2cta && M >= 256 && N >= 256;
     const int s2 = pair_ok ? pick_splits(t2, g_num_sms / 2, num_kb, slice_bytes, workspace_bytes) : 1;
     const int s1 = pick_splits(t1, g_num_sms, num_kb, slice_bytes, workspace_bytes);
-    if (s2 > 1) { splits = s2; use2 = true; }
-    else if (s1 > 1) { splits = s1; use2 = false; bn = 256; }
+    if (s2 > cut) { splits = s2; use2 = true; }
+    else if (s1 > cut) { splits = s1; use2 = false; bn = 256; }
   }
   void* user_C = args.C;
   const long long user_ldc = args.ldc, user_strideC = args.strideC;
@@ -2062,11 +2073,12 @@ GB_EXPORT int gb_gemm16(const void* A, const void* B, void* C, const void* bias,
 
 // fp32 C = alpha * op(A) op(B) (+ C) (+ bias[N]) from stacks of three bf16 planes: A (batch or 1, 3, rows, lda), B likewise,
 // plane_a / plane_b elements between planes.  `planes` products, product p of planes (order_a >> 4p) & 15 and
-// (order_b >> 4p) & 15, are added in that order into one fp32 accumulator.  (Called by gb_gemm_f32x3.)
+// (order_b >> 4p) & 15, are added in that order into one fp32 accumulator, which takes at most `chain` of K (a multiple of 64;
+// 0: all of it).  (Called by gb_gemm_f32x3.)
 int gemm_bf16_planes(const void* A, const void* B, float* C, const float* bias, int M, int N, int K, int batch, int transA,
                      int transB, long long lda, long long ldb, long long ldc, long long plane_a, long long plane_b, int bcastA,
                      int bcastB, long long sC, int planes, uint32_t order_a, uint32_t order_b, float alpha, int beta,
-                     void* workspace, long long workspace_bytes, cudaStream_t stream) {
+                     void* workspace, long long workspace_bytes, cudaStream_t stream, int chain) {
   GemmArgs a;
   memset(&a, 0, sizeof(a));
   a.M = M; a.N = N; a.K = K; a.batch = batch;
@@ -2074,7 +2086,7 @@ int gemm_bf16_planes(const void* A, const void* B, float* C, const float* bias, 
   a.ldc = ldc; a.strideC = sC; a.alpha = alpha; a.beta = beta;
   a.out_kind = OUT_F32; a.in_bf16 = 1;
   a.bcastA = bcastA; a.bcastB = bcastB; a.plane_a = order_a; a.plane_b = order_b;
-  return gemm_tc(2, A, B, a, transA, transB, lda, ldb, plane_a, plane_b, 0, stream, workspace, workspace_bytes, planes);
+  return gemm_tc(2, A, B, a, transA, transB, lda, ldb, plane_a, plane_b, 0, stream, workspace, workspace_bytes, planes, chain);
 }
 
 // int8 x int8 -> int32 GEMM with the dequantising epilogue of the reference's

@@ -27,7 +27,7 @@ extern "C" int gb_gemm16(const void* A, const void* B, void* C, const void* bias
 int gemm_bf16_planes(const void* A, const void* B, float* C, const float* bias, int M, int N, int K, int batch, int transA,
                      int transB, long long lda, long long ldb, long long ldc, long long plane_a, long long plane_b, int bcastA,
                      int bcastB, long long sC, int planes, uint32_t order_a, uint32_t order_b, float alpha, int beta,
-                     void* workspace, long long workspace_bytes, cudaStream_t stream);
+                     void* workspace, long long workspace_bytes, cudaStream_t stream, int chain);
 extern "C" int gb_binary(int op, int dtype, const void* a, const void* b, void* c, long long n, int rank,
                          const long long* shape, const long long* sa, const long long* sb, void* stream);
 extern "C" int gb_flash_fwd(int dtype, const void* q, const void* k, const void* v, void* o, float* lse, int B, int H,
@@ -339,11 +339,12 @@ GB_EXPORT long long gb_gemm_f32x3_workspace(int M, int N, int K, int batch) {
 }
 
 // fp32 GEMM through three bf16 planes per operand (see the file header).  bias: fp32 [N] or null.  workspace:
-// gb_gemm_f32x3_workspace() bytes; split_ws / split_ws_bytes: optional split-K scratch handed on to the bf16 GEMM.
+// gb_gemm_f32x3_workspace() bytes; split_ws / split_ws_bytes: optional split-K scratch handed on to the bf16 GEMM.  chain: the most
+// of K that one accumulator takes (a multiple of 64, with room for every slice in split_ws; 0: any length).
 GB_EXPORT int gb_gemm_f32x3(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int batch, int transA,
                             int transB, long long lda, long long ldb, long long ldc, long long sA, long long sB,
                             long long sC, float alpha, int beta, void* workspace, long long workspace_bytes,
-                            void* split_ws, long long split_ws_bytes, void* stream) {
+                            void* split_ws, long long split_ws_bytes, int chain, void* stream) {
   if (workspace == nullptr || workspace_bytes < gb_gemm_f32x3_workspace(M, N, K, batch)) {
     gbh::set_error("gb_gemm_f32x3: workspace too small");
     return gbh::E_BAD_ARG;
@@ -371,7 +372,7 @@ GB_EXPORT int gb_gemm_f32x3(const void* A, const void* B, void* C, const void* b
   // (relative to 64 bits at 3000 x 4096 x 1024: 1.0e-6 in this order in one accumulator, in two and in three).
   // A slice of a split K runs all six products over its part of K, which shortens that chain.
   return gemm_bf16_planes(a3, b3, (float*)C, (const float*)bias, M, N, K, batch, transA, transB, acp, bcp, ldc, plane_a, plane_b,
-                          share_a, share_b, sC, 6, 0x001102u, 0x010120u, alpha, beta, split_ws, split_ws_bytes, s);
+                          share_a, share_b, sC, 6, 0x001102u, 0x010120u, alpha, beta, split_ws, split_ws_bytes, s, chain);
 }
 
 // ---------------------------------------------------------------------------
@@ -420,7 +421,7 @@ GB_EXPORT double gb_bench_matmul(int m, int k, int n, int iters, int dtype) {
     ms = bench_loop(iters, [&] { return gb_gemm_f64(A, B, C, m, n, k, 1, 0, 0, k, n, n, 0, 0, 0, 1.0, 0, nullptr); });
   else if (dtype == DT_F32)
     ms = bench_loop(iters, [&] {
-      return gb_gemm_f32x3(A, B, C, nullptr, m, n, k, 1, 0, 0, k, n, n, 0, 0, 0, 1.f, 0, ws, ws_bytes, nullptr, 0, nullptr);
+      return gb_gemm_f32x3(A, B, C, nullptr, m, n, k, 1, 0, 0, k, n, n, 0, 0, 0, 1.f, 0, ws, ws_bytes, nullptr, 0, 0, nullptr);
     });
   else
     ms = bench_loop(iters, [&] {

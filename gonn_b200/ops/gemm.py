@@ -77,6 +77,19 @@ def _plane_chain(M: int, N: int, K: int, batch: int) -> int:
     return min(K, 512 if K >= 4096 else 256 if K >= 1024 else 128)
 
 
+def _ragged_part(M: int, N: int, K: int, batch: int) -> int:
+    """How much of K one accumulator of the plane kernel takes where K is no multiple of 8 and an operand is not stored
+    along K (the weight gradient of an odd number of rows), 0: the FMA kernel.  Short enough that the error stays below
+    that of an FMA chain of K; the slices run in one launch and meet in fp32.  FMA and planes, us, and relative error
+    against 64 bits on inputs of one sign (|normal| where the two are closest):
+    4096 x 1024 x 3001 721 -> 177, 7.4e-7 -> 5.6e-7; 4096 x 2048 x 4095 1927 -> 393, 9.9e-7 -> 8.9e-7; 2048 x 512 x 1001 91 -> 43,
+    4.9e-7 -> 3.7e-7; 4096 x 2048 x 259 137 -> 84; 384 x 384 x 999 59 -> 31; 512 x 512 x 513 34 -> 31.  Five launches cost
+    what the smallest products take: 4096 x 256 x 391 40 -> 31, but 4096 x 256 x 257 30 -> 32 and 1024 x 512 x 333 25 -> 41."""
+    if N % 4 or (K < 512 and M * N * K * batch < 400e6):
+        return 0
+    return 512 if K >= 3584 else 384 if K >= 2048 else 256 if K >= 1024 else 192 if K >= 512 else 128
+
+
 def _x3_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     key = (device.index, _l.current_stream_handle())
     buf = _x3_cache.get(key)
@@ -187,13 +200,18 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         raise ValueError(f"gemm: out has shape {tuple(out.shape)}, expected {oshape}")
 
     if native_simt:
-        need = 0                        # scratch of the plane path, 0 = another kernel
+        need = part = 0                 # scratch of the plane path, 0 = another kernel; longest accumulator, 0 = any
+        ragged = bool(K % 8) and (trans_a or not trans_b)
         if (a.dtype == torch.float32 and out.dtype == torch.float32 and _FP32_MODE == "bf16x3"
                 and 2.0 * M * N * K * batch >= 2.0 ** 28 and M >= 128 and N >= 128
-                and (K % 8 == 0 or (not trans_a and trans_b)) and out.stride(-2) % 4 == 0
-                and out.data_ptr() % 16 == 0):
+                and out.stride(-2) % 4 == 0 and out.data_ptr() % 16 == 0):
             chain = _plane_chain(M, N, K, batch)
-            need = int(_l.lib().gb_gemm_f32x3_workspace(M, N, chain, batch))
+            if ragged:
+                part = _ragged_part(M, N, K, batch)
+                slices = _WS_BYTES // (4 * M * N * batch)
+                chain = min(chain, part * max(slices, 1)) if part else 0
+                part = part if slices > 1 else 0          # no room for slices: pieces alone
+            need = int(_l.lib().gb_gemm_f32x3_workspace(M, N, chain, batch)) if chain else 0
             need = need if need <= (4 << 30) else 0
         f64_mma = a.dtype == torch.float64 and M >= 64 and N >= 64 and K >= 16
         # the plane and SIMT kernels add a bias of the operands' type in their epilogue (as separate tensor
@@ -215,15 +233,21 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
                     _l.L(sB), _l.L(sC), _l.D(alpha), _l.I(int(beta)), _l.stream_ptr())
             return out
         if need:
-            ws3 = _x3_workspace(a.device, need)
-            ws = _workspace(a.device) if M * N * batch * 4 * 2 <= _WS_BYTES else None
+            try:
+                ws3 = _x3_workspace(a.device, need)
+                ws = _workspace(a.device) if part or M * N * batch * 4 * 2 <= _WS_BYTES else None
+            except torch.OutOfMemoryError:
+                if not ragged:
+                    raise
+                need = 0                # the FMA kernel needs none
+        if need:
             for k in range(0, K, chain):
                 ak, bk = a2.data_ptr() + 4 * k * (lda if trans_a else 1), b2.data_ptr() + 4 * k * (1 if trans_b else ldb)
                 _l.call("gb_gemm_f32x3", _l.P(ak), _l.P(bk), _l.ptr(out), _l.ptr(bias if k == 0 else None), _l.I(M), _l.I(N),
                         _l.I(min(chain, K - k)), _l.I(batch), _l.I(int(trans_a)), _l.I(int(trans_b)), _l.L(lda), _l.L(ldb),
                         _l.L(out.stride(-2)), _l.L(sA), _l.L(sB), _l.L(sC), _l.F(alpha), _l.I(int(beta or k > 0)),
                         _l.ptr(ws3), _l.L(ws3.numel()), _l.ptr(ws), _l.L(_WS_BYTES if ws is not None else 0),
-                        _l.stream_ptr())
+                        _l.I(part), _l.stream_ptr())
             return out
         _l.call("gb_gemm_simt", _l.ptr(a2), _l.ptr(b2), _l.ptr(out), _l.ptr(bias), _l.I(M), _l.I(N), _l.I(K),
                 _l.I(batch), _l.I(int(trans_a)), _l.I(int(trans_b)), _l.L(lda), _l.L(ldb),

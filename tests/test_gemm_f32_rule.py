@@ -71,3 +71,56 @@ def test_error_relative_to_the_fma_kernel(M, N, K, factor):
         finally:
             G.set_fp32_gemm_mode(old)
     assert err["bf16x3"] <= factor * err["simt"], err
+
+
+@pytest.mark.parametrize("M,N,K,batch,part", [(4096, 1024, 3001, 1, 384), (4096, 1024, 3583, 1, 384), (4096, 2048, 4095, 1, 512),
+                                              (2048, 512, 1001, 1, 192), (1024, 1024, 1025, 1, 256), (512, 512, 513, 1, 192),
+                                              (1024, 512, 333, 1, 0), (4096, 256, 391, 1, 128), (4096, 1023, 3001, 1, 0)])
+def test_ragged_rule(M, N, K, batch, part):
+    assert G._ragged_part(M, N, K, batch) == part
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("draw", [torch.randn, torch.rand])
+@pytest.mark.parametrize("M,N,K,ta,tb", [(1031, 516, 513, True, False), (130, 1000, 1537, False, False), (2050, 128, 1025, True, True),
+                                         (516, 260, 4097, True, False), (1030, 1028, 2305, True, False), (2048, 1024, 257, True, False),
+                                         (512, 3000, 386, True, True)])
+def test_ragged_contractions_are_no_less_exact_than_fma(draw, M, N, K, ta, tb):
+    assert G._ragged_part(M, N, K, 1) > 0
+    a, b = draw(*((K, M) if ta else (M, K)), device="cuda"), draw(*((N, K) if tb else (K, N)), device="cuda")
+    want = (a.t() if ta else a).double() @ (b.t() if tb else b).double()
+    err = {}
+    for mode in ("bf16x3", "simt"):
+        old = G.set_fp32_gemm_mode(mode)
+        try:
+            err[mode] = float((G.gemm(a, b, trans_a=ta, trans_b=tb).double() - want).norm() / want.norm())
+        finally:
+            G.set_fp32_gemm_mode(old)
+    L.assert_status_ok()
+    assert err["bf16x3"] <= err["simt"], err
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("room", ["slices", "two slices", "pieces", "none"])
+@pytest.mark.parametrize("ta,tb,batch", [(True, False, 1), (False, False, 3), (True, True, 1)])
+def test_ragged_scratch(monkeypatch, room, ta, tb, batch):
+    """Slices in one launch, two slices a launch, pieces without slices, and the FMA kernel where memory is short: bias and the
+    old result once, alpha in every slice."""
+    M, N, K = 333, 516, 1001
+    if room == "two slices":
+        monkeypatch.setattr(G, "_WS_BYTES", 2 * 4 * M * N * batch + 64)
+    if room == "pieces":
+        monkeypatch.setattr(G, "_WS_BYTES", 4 * M * N * batch - 4)
+    if room == "none":
+        def short(*_):
+            raise torch.OutOfMemoryError("short")
+        monkeypatch.setattr(G, "_x3_workspace", short)
+    one = (lambda *s: torch.randn(batch, *s)) if batch > 1 else torch.randn
+    a, b, bv = one(*((K, M) if ta else (M, K))), one(*((N, K) if tb else (K, N))), 30 * torch.randn(N)
+    out = 30 * one(M, N)
+    want = -0.5 * ((a.transpose(-1, -2) if ta else a).double() @ (b.transpose(-1, -2) if tb else b).double())
+    want = want + bv.double() + out.double()
+    got = G.gemm(a.cuda(), b.cuda(), trans_a=ta, trans_b=tb, alpha=-0.5, bias=bv.cuda(), out=out.cuda(), beta=True)
+    L.assert_status_ok()
+    # as in test_pieces: every accumulator truncates 6 x 12 sums, every slice is rounded once; an FMA chain of 1001 is below too
+    assert float((got.double().cpu() - want).norm() / want.norm()) < 2.0 ** -20
