@@ -103,8 +103,9 @@ __device__ __forceinline__ bool wait_group(const unsigned int* flags, int n, uns
 // a: kMB rows, w: N rows, both K floats with pitch K + 4 (16-byte rows four banks apart, so that the
 // 16-byte reads of eight neighbouring rows touch all banks once).  Lanes: two groups of four a-rows
 // x N/4 groups of w-rows (w row = i * N/4 + group: neighbouring lanes, neighbouring rows) x KQ
-// slices of the warp's part k0 .. k1 of the contraction.  part[warp][kMB * N] receives the warp's partial sums.
-template <int N>
+// slices of the warp's share of the contraction: every kWarps-th step of it, or (OWN) its part k0 .. k1.  part[warp][kMB * N]
+// receives the warp's partial sums.
+template <int N, bool OWN>
 __device__ __forceinline__ void product(const float* __restrict__ a, const float* __restrict__ w, int K, int k0, int k1,
                                         float* __restrict__ part) {
   constexpr int NG = N / 4;                  // groups of w-rows
@@ -121,7 +122,7 @@ __device__ __forceinline__ void product(const float* __restrict__ a, const float
 #pragma unroll
     for (int j = 0; j < 4; j++) acc[i][j] = 0ull;
 #pragma unroll 2
-  for (int k = k0 + kq * 4; k < k1; k += KQ * 4) {
+  for (int k = OWN ? k0 + kq * 4 : (warp * KQ + kq) * 4; k < (OWN ? k1 : K); k += (OWN ? 1 : kWarps) * KQ * 4) {
     ulonglong2 av[4], wv[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) av[i] = *reinterpret_cast<const ulonglong2*>(ap + i * pitch + k);
@@ -163,20 +164,28 @@ __device__ __forceinline__ void load_tile(float* __restrict__ tile, const float*
 
 // The part k0 .. k1 (multiples of four) of h of the step whose words carry `step` (its index + 1), rows b0 .. b0 + kMB - 1, into the
 // tile, by one warp, which alone reads it: no barrier stands between the words and its product, and no warp waits for words of
-// another's part.  Rows past B are zero.  Gives up when the budget of the wait has run out for any thread of the CTA.
+// another's part.  OWN = false: k0 .. k1 by all threads of the CTA, a barrier follows (and the places of the words are worked out
+// again where they are needed: kept in registers, 64 x 64 steps at H = 720 take 1 190 us instead of 1 142).  Rows past B are zero.
+// Gives up when the budget of the wait has run out for any thread of the CTA.
+template <bool OWN>
 __device__ __forceinline__ void receive_part(float* __restrict__ tile, const unsigned long long* __restrict__ xch, unsigned step, int H,
                                              int k0, int k1, int b0, int B, int* abort_flag, int* status) {
   constexpr int U = 8;
-  const int h2 = (k1 - k0) / 2, pitch = H + 4, total = kMB * h2, lane = threadIdx.x & 31;
-  for (int i0 = lane; i0 < total; i0 += 32 * U) {
+  constexpr int W = OWN ? 32 : kThreads;
+  const int h2 = (k1 - k0) / 2, pitch = H + 4, total = kMB * h2;
+  for (int i0 = OWN ? threadIdx.x & 31 : threadIdx.x; i0 < total; i0 += W * U) {
     unsigned long long w[U][2];
-    int at[U];                                     // row << 16 | column
+    int at[OWN ? U : 1];
+    auto place = [&](int u) {                      // row << 16 | column
+      const int i = i0 + u * W, r = i / h2;
+      return r << 16 | (k0 + 2 * (i - r * h2));
+    };
     unsigned todo = 0;
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      const int i = i0 + u * 32, r = i / h2;
-      at[u] = r << 16 | (k0 + 2 * (i - r * h2));
-      if (i < total && b0 + r < B) todo |= 1u << u;
+      const int to = place(u);
+      if (OWN) at[u] = to;
+      if (i0 + u * W < total && b0 + (to >> 16) < B) todo |= 1u << u;
     }
     const unsigned mine = todo;
     uint64_t t0 = 0;
@@ -184,7 +193,8 @@ __device__ __forceinline__ void receive_part(float* __restrict__ tile, const uns
 #pragma unroll
       for (int u = 0; u < U; u++)
         if (todo >> u & 1u) {
-          const unsigned long long* src = xch + (long long)(b0 + (at[u] >> 16)) * H + (at[u] & 0xffff);
+          const int from = OWN ? at[u] : place(u);
+          const unsigned long long* src = xch + (long long)(b0 + (from >> 16)) * H + (from & 0xffff);
           asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(w[u][0]), "=l"(w[u][1]) : "l"(src) : "memory");
         }
 #pragma unroll
@@ -202,18 +212,23 @@ __device__ __forceinline__ void receive_part(float* __restrict__ tile, const uns
     }
 #pragma unroll
     for (int u = 0; u < U; u++)
-      if (i0 + u * 32 < total) {
+      if (i0 + u * W < total) {
         const float2 v = mine >> u & 1u ? make_float2(__uint_as_float((unsigned)w[u][0]), __uint_as_float((unsigned)w[u][1]))
                                         : make_float2(0.f, 0.f);
-        *reinterpret_cast<float2*>(tile + (at[u] >> 16) * pitch + (at[u] & 0xffff)) = v;
+        const int to = OWN ? at[u] : place(u);
+        *reinterpret_cast<float2*>(tile + (to >> 16) * pitch + (to & 0xffff)) = v;
       }
   }
   __syncwarp();
 }
 
 // grid: (ug, groups).  UT units per CTA: N = 4 UT weight rows, row n = gate * UT + unit.  TAPE: a backward follows (a template
-// parameter and the stores in this order: with strides and flags at run time a step takes 0.2 us longer).
-template <int UT, bool TAPE>
+// parameter and the stores in this order: with strides and flags at run time a step takes 0.2 us longer).  PARTS: buffers of partial
+// sums.  With two a warp may be a product ahead of the cells; where the weights leave room for one (16 units, H from 692 to 744), a
+// barrier stands before each product instead of half the units a CTA and, for many sequences, three times the dependent
+// exchanges.  64 steps, us, 8 units and two buffers | 16 units and one:
+// B = 64, H = 720 2 443 | 1 142, 256, 720 9 790 | 4 185, 64, 692 2 143 | 1 347, 64, 744 2 441 | 1 158.
+template <int UT, bool TAPE, int PARTS>
 __global__ void __launch_bounds__(kThreads, 1) lstm_seq_fwd_kernel(const SeqArgs p) {
   constexpr int N = 4 * UT;
   extern __shared__ __align__(16) float sm[];
@@ -221,7 +236,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_fwd_kernel(const SeqArgs
   const int H = p.H, T = p.T, pitch = H + 4;
   float* ws = sm;                                  // [N][H + 4]
   float* hs = ws + N * pitch;                      // [kMB][H + 4]
-  float* parts = hs + kMB * pitch;                 // [2][kWarps][kMB * N], by turns: a warp may be a product ahead of the cells
+  float* parts = hs + kMB * pitch;                 // [PARTS][kWarps][kMB * N], by turns
   const int u0 = blockIdx.x * UT;
   const int bg0 = blockIdx.y * p.sub * kMB;
   if (threadIdx.x == 0) abort_flag = 0;
@@ -245,7 +260,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_fwd_kernel(const SeqArgs
   int turn = 0;
   for (int t = 0; t < T; t++) {
     for (int s = 0; s < p.sub; s++) {
-      float* part = parts + (turn ^= 1) * (kWarps * kMB * N);
+      float* part = parts + (turn = (turn + 1) % PARTS) * (kWarps * kMB * N);
       const int b0 = bg0 + s * kMB, b = b0 + cell_m;
       const bool mine = cell && b < p.B;
       const long long row = (long long)b * T + t;
@@ -257,12 +272,14 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_fwd_kernel(const SeqArgs
       }
       if (t > 0 || p.h0 != nullptr) {
         if (t > 0) {
-          receive_part(hs, p.xch + (long long)((t - 1) & 1) * p.B * H, (unsigned)t, H, k0, k1, b0, p.B, &abort_flag, p.status);
+          receive_part<PARTS == 2>(hs, p.xch + (long long)((t - 1) & 1) * p.B * H, (unsigned)t, H, PARTS == 2 ? k0 : 0, PARTS == 2 ? k1 : H, b0,
+                                   p.B, &abort_flag, p.status);
         } else {
           load_tile(hs, p.h0, H, H, b0, p.B);
           __syncthreads();
         }
-        product<N>(hs, ws, H, k0, k1, part);
+        if (PARTS == 1) __syncthreads();           // the cells have read the sums of the product before; h is whole
+        product<N, PARTS == 2>(hs, ws, H, k0, k1, part);
         __syncthreads();
         if (*(volatile int*)&abort_flag != 0) return;
         if (mine) {
@@ -343,7 +360,7 @@ __global__ void __launch_bounds__(kThreads, 1) lstm_seq_bwd_kernel(const SeqArgs
       if (chain) {
         load_tile(ds, p.dgates + (long long)(t + 1) * K, (long long)T * K, K, b0, p.B);
         __syncthreads();
-        product<N>(ds, ws, K, min(K, (int)(threadIdx.x >> 5) * kper), min(K, ((int)(threadIdx.x >> 5) + 1) * kper), part);
+        product<N, true>(ds, ws, K, min(K, (int)(threadIdx.x >> 5) * kper), min(K, ((int)(threadIdx.x >> 5) + 1) * kper), part);
         __syncthreads();
         if (mine) {
           float v = 0.f;
@@ -551,9 +568,10 @@ constexpr long long kMaxSmem = 227 * 1024 - 16;      // what a block may take, l
 constexpr int kMaxSub = 32;
 constexpr long long kScatterBytes = 128ll << 20;
 
-long long fwd_smem(int ut, int H) {
-  return 4ll * ((4ll * ut + kMB) * (H + 4) + 2ll * kWarps * kMB * 4 * ut);
+long long fwd_smem(int ut, int H, int parts) {
+  return 4ll * ((4ll * ut + kMB) * (H + 4) + (long long)parts * kWarps * kMB * 4 * ut);
 }
+int fwd_parts(int ut, int H) { return ut == 16 && fwd_smem(ut, H, 2) > kMaxSmem ? 1 : 2; }
 long long bwd_smem(int ut, int H, int sub) {
   return 4ll * (((long long)ut + kMB) * (4ll * H + 4) + (long long)kWarps * kMB * ut + (long long)sub * kMB * ut);
 }
@@ -581,7 +599,7 @@ bool plan(int sms, int B, int H, bool bwd, int* ut, int* ug, int* groups, int* s
     if (slices > sms) break;                      // smaller u only makes more slices
     const int g = tiles < sms / slices ? tiles : sms / slices;
     const int s = (tiles + g - 1) / g;
-    const long long need = bwd ? bwd_smem(u, H, s) : fwd_smem(u, H);
+    const long long need = bwd ? bwd_smem(u, H, s) : fwd_smem(u, H, fwd_parts(u, H));
     if (need > kMaxSmem || s > kMaxSub) continue;
     *ut = u; *ug = slices; *sub = s; *groups = (tiles + s - 1) / s;
     best = u;
@@ -606,7 +624,7 @@ int launch(K kern, const SeqArgs& a, int groups, long long smem, long long words
 GB_EXPORT int gb_lstm_seq_smem(int B, int H, int bwd) {
   int ut, ug, groups, sub;
   if (B <= 0 || !plan(kSms, B, H, bwd != 0, &ut, &ug, &groups, &sub)) return 0;
-  return (int)(bwd ? bwd_smem(ut, H, sub) : fwd_smem(ut, H));
+  return (int)(bwd ? bwd_smem(ut, H, sub) : fwd_smem(ut, H, fwd_parts(ut, H)));
 }
 // 1 when both directions of an LSTM layer of this size run as persistent kernels on that many SMs ...
 GB_EXPORT int gb_lstm_seq_fits_on(int sms, int B, int H) {
@@ -638,16 +656,19 @@ GB_EXPORT int gb_lstm_seq_fwd(void* xg, const void* bias, const void* w, const v
     gbh::set_error("gb_lstm_seq_fwd: a contiguous output is needed where a backward follows");
     return gbh::E_BAD_ARG;
   }
-  const long long smem = fwd_smem(ut, H), words = 2ll * B * H;
+  const int parts = fwd_parts(ut, H);
+  const long long smem = fwd_smem(ut, H, parts), words = 2ll * B * H;
   cudaStream_t s = (cudaStream_t)stream;
   if (hprev != nullptr) {
-    if (ut == 16) return launch(lstm_seq_fwd_kernel<16, true>, a, groups, smem, words, s);
-    if (ut == 8) return launch(lstm_seq_fwd_kernel<8, true>, a, groups, smem, words, s);
-    return launch(lstm_seq_fwd_kernel<4, true>, a, groups, smem, words, s);
+    if (ut == 16 && parts == 1) return launch(lstm_seq_fwd_kernel<16, true, 1>, a, groups, smem, words, s);
+    if (ut == 16) return launch(lstm_seq_fwd_kernel<16, true, 2>, a, groups, smem, words, s);
+    if (ut == 8) return launch(lstm_seq_fwd_kernel<8, true, 2>, a, groups, smem, words, s);
+    return launch(lstm_seq_fwd_kernel<4, true, 2>, a, groups, smem, words, s);
   }
-  if (ut == 16) return launch(lstm_seq_fwd_kernel<16, false>, a, groups, smem, words, s);
-  if (ut == 8) return launch(lstm_seq_fwd_kernel<8, false>, a, groups, smem, words, s);
-  return launch(lstm_seq_fwd_kernel<4, false>, a, groups, smem, words, s);
+  if (ut == 16 && parts == 1) return launch(lstm_seq_fwd_kernel<16, false, 1>, a, groups, smem, words, s);
+  if (ut == 16) return launch(lstm_seq_fwd_kernel<16, false, 2>, a, groups, smem, words, s);
+  if (ut == 8) return launch(lstm_seq_fwd_kernel<8, false, 2>, a, groups, smem, words, s);
+  return launch(lstm_seq_fwd_kernel<4, false, 2>, a, groups, smem, words, s);
 }
 
 // 64-bit words of scratch that gb_lstm_seq_bwd takes.

@@ -37,3 +37,14 @@ def test_fewer_sms_fit_fewer_layers():
     assert fits(1, 1, 16) and not fits(1, 300, 16)                                # one CTA, 32 tiles of 8 sequences at most
     for H in (64, 512, 800):
         assert [fits(s, 64, H) for s in range(1, 149)] == sorted(fits(s, 64, H) for s in range(1, 149))
+
+
+@pytest.mark.parametrize("H", [4 * h for h in range(160, 187)])
+def test_sixteen_units_a_cta_as_long_as_their_weights_fit(H):
+    """Forward: 16 units and the exchange tile are 72 rows of H + 4 floats, and a buffer of partial sums beside them takes 16 KB.  Up to
+    H = 744 that fits, and so 16 units it is where many sequences would otherwise wait for one another in a single group."""
+    need = 4 * 72 * (H + 4) + (16 << 10)
+    assert need <= BLOCK - 16
+    got = int(L.lib().gb_lstm_seq_smem(L.I(256), L.I(H), L.I(0)))
+    assert got in (need, need + (16 << 10))
+    assert got == need + (16 << 10) or need + (16 << 10) > BLOCK - 16          # two buffers wherever there is room

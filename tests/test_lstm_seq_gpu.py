@@ -185,3 +185,9 @@ def test_tangents_and_transforms_are_not_dropped_without_a_tape():
         torch.func.vmap(net)(torch.randn(2, 3, 5, 12, device="cuda"))
     with torch.no_grad():
         assert net(x).isfinite().all()
+
+
+@pytest.mark.parametrize("B,T,H", [(9, 5, 692), (70, 4, 720), (200, 3, 744)])
+def test_forward_with_one_buffer_of_partial_sums(B, T, H):
+    """Widths at which 16 units leave room for one: alone, several sub-tiles to a group, the widest."""
+    test_lstm_sequence_matches_float64(B, T, 8, H, True)
