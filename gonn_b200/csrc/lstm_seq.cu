@@ -672,18 +672,20 @@ GB_EXPORT int gb_lstm_seq_fwd(void* xg, const void* bias, const void* w, const v
   return launch(lstm_seq_fwd_kernel<4, false, 2>, a, groups, smem, words, s);
 }
 
-// 64-bit words of scratch that gb_lstm_seq_bwd takes.
+// 64-bit words of scratch with which gb_lstm_seq_bwd runs at its fastest (it runs with kSms / 2, too).
 GB_EXPORT long long gb_lstm_seq_bwd_words(int B, int H) {
   int ut, ug, groups, sub;
   if (B <= 0 || !plan(device_sms(), B, H, true, &ut, &ug, &groups, &sub)) return 0;
   const long long words = bwd_words(ut, ug, groups, sub, H);
-  return words > 0 ? words : kSms / 2;
+  return words > kSms / 2 ? words : kSms / 2;
 }
 
-// Backward of the above (scratch: gb_lstm_seq_bwd_words(B, H) words): dout (B,T,H) or null, dcn (B,H) or null; writes dgates (B,T,4H), the gradient
+// Backward of the above (scratch: gb_lstm_seq_bwd_words(B, H) 64-bit words, or kSms / 2 where memory is short: then dgates are
+// gathered): dout (B,T,H) or null, dcn (B,H) or null; writes dgates (B,T,4H), the gradient
 // of the gate pre-activations, and dc0 (B,H) when not null.
 GB_EXPORT int gb_lstm_seq_bwd(const void* w, const void* c0, const void* cseq, const void* act, const void* dout,
-                              const void* dcn, void* dgates, void* dc0, void* scratch, int B, int T, int H, void* stream) {
+                              const void* dcn, void* dgates, void* dc0, void* scratch, long long scratch_words, int B, int T,
+                              int H, void* stream) {
   if (B <= 0 || T <= 0) return gbh::E_OK;
   SeqArgs a = {};
   int ut, groups;
@@ -697,7 +699,11 @@ GB_EXPORT int gb_lstm_seq_bwd(const void* w, const void* c0, const void* cseq, c
   a.status = gbh::status_ptr();
   cudaStream_t s = (cudaStream_t)stream;
   const long long words = bwd_words(ut, a.ug, groups, a.sub, H);
-  if (words > 0) {
+  if (scratch_words < kSms / 2) {
+    gbh::set_error("gb_lstm_seq_bwd: %d words of scratch are needed", kSms / 2);
+    return gbh::E_BAD_ARG;
+  }
+  if (words > 0 && scratch_words >= words) {
     a.xch = (unsigned long long*)scratch;
     const long long smem = bwd_scatter_smem(ut, H, a.sub);
     const int parts = kThreads / (kMB * ut);
@@ -708,7 +714,7 @@ GB_EXPORT int gb_lstm_seq_bwd(const void* w, const void* c0, const void* cseq, c
   }
   a.flags = (unsigned int*)scratch;
   const long long smem = bwd_smem(ut, H, a.sub);
-  if (ut == 16) return launch(lstm_seq_bwd_kernel<16>, a, groups, smem, words, s);
-  if (ut == 8) return launch(lstm_seq_bwd_kernel<8>, a, groups, smem, words, s);
-  return launch(lstm_seq_bwd_kernel<4>, a, groups, smem, words, s);
+  if (ut == 16) return launch(lstm_seq_bwd_kernel<16>, a, groups, smem, 0, s);
+  if (ut == 8) return launch(lstm_seq_bwd_kernel<8>, a, groups, smem, 0, s);
+  return launch(lstm_seq_bwd_kernel<4>, a, groups, smem, 0, s);
 }

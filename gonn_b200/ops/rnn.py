@@ -102,6 +102,7 @@ def _aligned(t):
 # Without a tape the projections of the whole input (four times the output) live for a moment only: longer sequences go in
 # pieces of at most this many bytes, each from the state that the one before it left.
 PROJECTION_BYTES = 256 << 20
+LEAST_WORDS = 74       # 64-bit words: a flag per CTA of the backward that gathers (the one that scatters takes up to 128 MiB)
 
 
 def _lstm_forward(x, w_ih, b_ih, w_hh, h0, c0, tape: bool):
@@ -155,9 +156,14 @@ class _LSTMSequence(torch.autograd.Function):
         whh = _aligned(w_hh.detach())
         dgates = torch.empty_like(act)                     # (B * T, 4H)
         dc0 = torch.empty((B, H), dtype=cseq.dtype, device=dev) if ctx.needs_input_grad[5] else None
-        scratch = torch.empty(_l.lib().gb_lstm_seq_bwd_words(_l.I(B), _l.I(H)), dtype=torch.int64, device=dev)
+        words = _l.lib().gb_lstm_seq_bwd_words(_l.I(B), _l.I(H))
+        try:
+            scratch = torch.empty(words, dtype=torch.int64, device=dev)
+        except torch.OutOfMemoryError:
+            words = LEAST_WORDS
+            scratch = torch.empty(words, dtype=torch.int64, device=dev)
         _l.call("gb_lstm_seq_bwd", _l.ptr(whh), _l.ptr(c0), _l.ptr(cseq), _l.ptr(act), _l.ptr(dout), _l.ptr(dcn),
-                _l.ptr(dgates), _l.ptr(dc0), _l.ptr(scratch), _l.I(B), _l.I(T), _l.I(H), _l.stream_ptr())
+                _l.ptr(dgates), _l.ptr(dc0), _l.ptr(scratch), _l.L(words), _l.I(B), _l.I(T), _l.I(H), _l.stream_ptr())
         dx = dwih = db = dwhh = dh0 = None
         # every read of a weight comes before its gradient is declared ready (ops/linear.py)
         if ctx.needs_input_grad[0]:

@@ -191,3 +191,24 @@ def test_tangents_and_transforms_are_not_dropped_without_a_tape():
 def test_forward_with_one_buffer_of_partial_sums(B, T, H):
     """Widths at which 16 units leave room for one: alone, several sub-tiles to a group, the widest."""
     test_lstm_sequence_matches_float64(B, T, 8, H, True)
+
+
+def _no_words(monkeypatch, asked):
+    """Memory for the words of the scattered exchange (more than any other whole-number buffer here) is short."""
+    real = torch.empty
+
+    def empty(*size, **kw):
+        if kw.get("dtype") is torch.int64 and size[0] > 1 << 16:
+            asked.append(size[0])
+            raise torch.OutOfMemoryError("short")
+        return real(*size, **kw)
+    monkeypatch.setattr(torch, "empty", empty)
+
+
+@pytest.mark.parametrize("B,H", [(16, 256), (200, 132)])
+def test_backward_where_memory_for_the_exchange_is_short(monkeypatch, B, H):
+    assert L.lib().gb_lstm_seq_bwd_words(L.I(B), L.I(H)) > 1 << 16 > 2 * B * H
+    asked = []
+    _no_words(monkeypatch, asked)
+    test_lstm_sequence_matches_float64(B, 5, 8, H, True)
+    assert asked
