@@ -698,7 +698,8 @@ GB_EXPORT int gb_lstm_seq_bwd(const void* w, const void* c0, const void* cseq, c
   a.dout = (const float*)dout; a.dcn = (const float*)dcn; a.dgates = (float*)dgates; a.dc0 = (float*)dc0;
   a.status = gbh::status_ptr();
   cudaStream_t s = (cudaStream_t)stream;
-  const long long words = bwd_words(ut, a.ug, groups, a.sub, H);
+  // (a single step exchanges nothing: no words to clear)
+  const long long words = T > 1 ? bwd_words(ut, a.ug, groups, a.sub, H) : 0;
   if (scratch_words < kSms / 2) {
     gbh::set_error("gb_lstm_seq_bwd: %d words of scratch are needed", kSms / 2);
     return gbh::E_BAD_ARG;

@@ -212,3 +212,10 @@ def test_backward_where_memory_for_the_exchange_is_short(monkeypatch, B, H):
     _no_words(monkeypatch, asked)
     test_lstm_sequence_matches_float64(B, 5, 8, H, True)
     assert asked
+
+
+def test_one_step_takes_no_words(monkeypatch):
+    asked = []
+    _no_words(monkeypatch, asked)
+    test_lstm_sequence_matches_float64(70, 1, 8, 256, True)
+    assert not asked
