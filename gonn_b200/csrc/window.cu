@@ -433,7 +433,8 @@ GB_EXPORT int gb_pool_fwd(int dtype, const void* x, const int* idx, void* y, int
   if (total <= 0) return gbh::E_OK;
   cudaStream_t s = (cudaStream_t)stream;
   GB_BOUNDS_BIND();
-  if (mode != POOL_LP && T_ <= 8 && B >= 64) {
+  // (an empty plane under padding alone has no element that a tap of padding could read again)
+  if (mode != POOL_LP && T_ <= 8 && B >= 64 && S > 0) {
     const int bx = (nwin + 255) / 256 < 64 ? (nwin + 255) / 256 : 64;
     long long by = (148 * 8 + bx - 1) / bx;
     if (by > B) by = B;

@@ -264,3 +264,15 @@ def test_batchnorm_of_odd_and_even_planes(N, C, H, W, dtype, status_ok):
     for name, got, want in (("y", y, yd), ("dx", x.grad, xd.grad), ("dw", bn.weight.grad, w.grad), ("db", bn.bias.grad, b.grad)):
         err = (got.double() - want).norm() / want.norm().clamp_min(1e-3 * want.numel() ** 0.5)
         assert err.item() < 2 * unit, (name, err.item())
+
+
+@pytest.mark.parametrize("pool", [MaxPool2d(2, padding=1), AvgPool2d(2, padding=1), AvgPool2d(2, 1, 1, count_include_pad=False),
+                                  MaxPool2d((2, 4), padding=(1, 2)), AvgPool2d(16, padding=8)])
+@pytest.mark.parametrize("H,W", [(0, 0), (0, 5), (4, 0)])
+def test_pooling_of_empty_planes_is_padding(pool, H, W, status_ok):
+    """Windows of padding alone give 0 and read nothing: there is nothing to read."""
+    x = torch.empty(64, 2, H, W, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    y = pool(x)
+    assert y.numel() > 0 and not y.any()
+    y.sum().backward()
+    assert x.grad.shape == x.shape
