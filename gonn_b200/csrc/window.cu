@@ -209,68 +209,99 @@ pool_fwd_small_kernel(const T* __restrict__ x, const int* __restrict__ idx, T* _
 // Max / average pooling over wide windows (global pooling: one window of H * W taps): one warp per
 // output, lanes along the taps, then a shuffle reduction.  The arg-max is the first tap that holds the
 // maximum, as in the one-thread-per-output kernel.
-// A warp stays with one window: its lanes keep the first kWideTaps * 32 taps' offsets in registers and have the loads of two planes
-// in flight together (an offset and a load at a time: 32768 x 169, one window, average, bf16 15.6 us, so 12.3).
-constexpr int kWideTaps = 8;
-template <typename T, bool MAX>
+template <typename T>
+__global__ void pool_fwd_wide_kernel(const T* __restrict__ x, const int* __restrict__ idx, T* __restrict__ y,
+                                     int* __restrict__ arg, long long B, long long S, int nwin, int T_, int mode,
+                                     int count_include_pad) {
+  pdl_trigger();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+  const long long total = B * nwin;
+  for (long long o = (long long)blockIdx.x * wpb + (threadIdx.x >> 5); o < total; o += (long long)gridDim.x * wpb) {
+    const long long b = o / nwin;
+    const int win = (int)(o - b * nwin);
+    const T* xb = x + b * S;
+    const int* iw = idx + (long long)win * T_;
+    float best = -INFINITY, sum = 0.f;
+    int bt = 0x7fffffff, cnt = 0;
+    for (int t = lane; t < T_; t += 32) {
+      const int src = __ldg(iw + t);
+      if (src < 0 || !GB_IN_BOUNDS(src, S, 109)) continue;
+      const float v = (float)xb[src];
+      sum += v;
+      cnt++;
+      if (v > best || bt == 0x7fffffff) { best = v; bt = t; }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, best, off);
+      const int ot = __shfl_xor_sync(0xffffffffu, bt, off);
+      sum += __shfl_xor_sync(0xffffffffu, sum, off);
+      cnt += __shfl_xor_sync(0xffffffffu, cnt, off);
+      // a lane that saw no tap holds (-inf, INT_MAX) and always loses; equal values keep the earlier tap
+      if (ot != 0x7fffffff && (bt == 0x7fffffff || ov > best || (ov == best && ot < bt))) { best = ov; bt = ot; }
+    }
+    if (lane == 0) {
+      if (mode == POOL_MAX) {
+        y[o] = (T)(bt == 0x7fffffff ? 0.f : best);
+        if (arg) arg[o] = bt == 0x7fffffff ? -1 : bt;
+      } else {
+        y[o] = (T)(sum / (float)(count_include_pad ? T_ : (cnt > 0 ? cnt : 1)));
+      }
+    }
+  }
+}
+
+// The same for windows of at most 32 NT taps where there are many planes: a warp stays with one window, keeps the taps' offsets in
+// registers and has the loads of U planes in flight together (a maximum one plane's: its selections are what a warp waits for, and
+// with more planes fewer warps fit).
+template <typename T, int NT, bool MAX>
 __global__ void __launch_bounds__(256)
-pool_fwd_wide_kernel(const T* __restrict__ x, const int* __restrict__ idx, T* __restrict__ y, int* __restrict__ arg, long long B,
+pool_fwd_stay_kernel(const T* __restrict__ x, const int* __restrict__ idx, T* __restrict__ y, int* __restrict__ arg, long long B,
                      long long S, int nwin, int T_, int count_include_pad) {
   pdl_trigger();
   pdl_wait();
-  constexpr int U = 2;
+  constexpr int U = MAX ? 1 : 16 / NT;
   const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
   const long long warps = (long long)gridDim.x * wpb, w0 = (long long)blockIdx.x * wpb + (threadIdx.x >> 5);
   const long long per = warps / nwin;            // warps of a window (the launch has at least one each)
   if (w0 >= per * nwin) return;
   const int win = (int)(w0 % nwin);
-  const int* iw = idx + (long long)win * T_;
-  int off[kWideTaps], cnt = 0;
+  int off[NT], cnt = 0;
 #pragma unroll
-  for (int k = 0; k < kWideTaps; k++) {
+  for (int k = 0; k < NT; k++) {
     const int t = lane + 32 * k;
-    off[k] = t < T_ ? __ldg(iw + t) : -1;
+    off[k] = t < T_ ? __ldg(idx + (long long)win * T_ + t) : -1;
     if (off[k] >= 0 && !GB_IN_BOUNDS(off[k], S, 109)) off[k] = -1;
     cnt += off[k] >= 0;
   }
-  for (int t = lane + 32 * kWideTaps; t < T_; t += 32) {
-    const int src = __ldg(iw + t);
-    cnt += src >= 0 && GB_IN_BOUNDS(src, S, 109);
+  float div = (float)T_;
+  if (!MAX && !count_include_pad) {
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    div = (float)(cnt > 0 ? cnt : 1);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-  const float div = (float)(count_include_pad ? T_ : (cnt > 0 ? cnt : 1));
   for (long long b = w0 / nwin; b < B; b += per * U) {
-    float v[U][kWideTaps];
+    float v[U][NT];
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const T* xb = x + (b + u * per) * S;
 #pragma unroll
-      for (int k = 0; k < kWideTaps; k++) v[u][k] = off[k] >= 0 && b + u * per < B ? (float)xb[off[k]] : 0.f;
+      for (int k = 0; k < NT; k++) v[u][k] = off[k] >= 0 && b + u * per < B ? (float)xb[off[k]] : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < U; u++) {
       if (b + u * per >= B) break;               // (the same for the whole warp)
-      const T* xb = x + (b + u * per) * S;
       const long long o = (b + u * per) * nwin + win;
       if (MAX) {
         float best = -INFINITY;
         int bt = 0x7fffffff;
-        auto take = [&](float f, int t) {
-          if (f > best || bt == 0x7fffffff) { best = f; bt = t; }
-        };
 #pragma unroll
-        for (int k = 0; k < kWideTaps; k++)
-          if (off[k] >= 0) take(v[u][k], lane + 32 * k);
-        for (int t = lane + 32 * kWideTaps; t < T_; t += 32) {
-          const int src = __ldg(iw + t);
-          if (src >= 0 && GB_IN_BOUNDS(src, S, 109)) take((float)xb[src], t);
-        }
+        for (int k = 0; k < NT; k++)
+          if (off[k] >= 0 && (v[u][k] > best || bt == 0x7fffffff)) { best = v[u][k]; bt = lane + 32 * k; }
 #pragma unroll
         for (int q = 16; q > 0; q >>= 1) {
           const float ov = __shfl_xor_sync(0xffffffffu, best, q);
           const int ot = __shfl_xor_sync(0xffffffffu, bt, q);
-          // a lane that saw no tap holds (-inf, INT_MAX) and always loses; equal values keep the earlier tap
           if (ot != 0x7fffffff && (bt == 0x7fffffff || ov > best || (ov == best && ot < bt))) { best = ov; bt = ot; }
         }
         if (lane == 0) {
@@ -280,11 +311,7 @@ pool_fwd_wide_kernel(const T* __restrict__ x, const int* __restrict__ idx, T* __
       } else {
         float sum = 0.f;
 #pragma unroll
-        for (int k = 0; k < kWideTaps; k++) sum += v[u][k];
-        for (int t = lane + 32 * kWideTaps; t < T_; t += 32) {
-          const int src = __ldg(iw + t);
-          if (src >= 0 && GB_IN_BOUNDS(src, S, 109)) sum += (float)xb[src];
-        }
+        for (int k = 0; k < NT; k++) sum += v[u][k];
         sum = warp_sum(sum);
         if (lane == 0) y[o] = (T)(sum / div);
       }
@@ -448,13 +475,28 @@ GB_EXPORT int gb_pool_fwd(int dtype, const void* x, const int* idx, void* y, int
     return gbh::E_OK;
   }
   if (mode != POOL_LP && T_ >= 64) {
-    // (every window has a warp, or several that share its planes)
-    const long long most = 148 * 8 > (nwin + 7) / 8 ? 148 * 8 : (nwin + 7) / 8;
+    const long long most = 148 * 8;
     const unsigned grid = (unsigned)((total + 7) / 8 < most ? (total + 7) / 8 : most);
+    // Staying pays where a warp has several planes of its window (bf16, us, walking | staying: average over 64 taps, 8 192 outputs 10.2 |
+    // 10.4, 32 768 18.3 | 12.4, 1.2 M 424 | 184; maximum over 169 taps, 2 048 outputs 8.3 | 10.1, 8 192 10.4 | 10.2, 295 K 139 | 100), and
+    // where the warps divide among the windows (6 400 windows of 64 taps on 64 planes 548 | 566).  More than 256 taps would not stay
+    // in registers: 1 024 taps on 8 192 planes 22 | 37, 3 136 on 2 048 29 | 56 with the rest read behind them.
+    const int nt = (T_ + 31) / 32;
+    const bool stay = T_ <= 256 && nwin * 4ll <= grid * 8ll && total >= (mode == POOL_MAX ? 4096 : 16384);
+#define GB_STAY_(NT, MAX) gbh::launch(pool_fwd_stay_kernel<T, NT, MAX>, dim3(grid), dim3(256), 0, s, 1, (const T*)x, idx, (T*)y, arg, B, S, nwin, T_, count_include_pad)
+#define GB_STAY(NT) { if (mode == POOL_MAX) GB_STAY_(NT, true); else GB_STAY_(NT, false); }
     GB_DISPATCH_T(({
-      if (mode == POOL_MAX) gbh::launch(pool_fwd_wide_kernel<T, true>, dim3(grid), dim3(256), 0, s, 1, (const T*)x, idx, (T*)y, arg, B, S, nwin, T_, count_include_pad);
-      else gbh::launch(pool_fwd_wide_kernel<T, false>, dim3(grid), dim3(256), 0, s, 1, (const T*)x, idx, (T*)y, arg, B, S, nwin, T_, count_include_pad);
+      if (!stay) gbh::launch(pool_fwd_wide_kernel<T>, dim3(grid), dim3(256), 0, s, 1, (const T*)x, idx, (T*)y, arg, B, S, nwin, T_, mode, count_include_pad);
+      else if (nt <= 2) GB_STAY(2)
+      else if (nt == 3) GB_STAY(3)
+      else if (nt == 4) GB_STAY(4)
+      else if (nt == 5) GB_STAY(5)
+      else if (nt == 6) GB_STAY(6)
+      else if (nt == 7) GB_STAY(7)
+      else GB_STAY(8)
     }));
+#undef GB_STAY
+#undef GB_STAY_
     GB_CUDA_OK(cudaGetLastError());
     return gbh::E_OK;
   }

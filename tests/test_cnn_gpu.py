@@ -276,3 +276,18 @@ def test_pooling_of_empty_planes_is_padding(pool, H, W, status_ok):
     assert y.numel() > 0 and not y.any()
     y.sum().backward()
     assert x.grad.shape == x.shape
+
+
+@pytest.mark.parametrize("mode,B", [(0, 2100), (1, 8300)])
+@pytest.mark.parametrize("taps", [64, 65, 97, 129, 161, 193, 225, 256, 257])
+def test_pool_kernels_that_stay_with_a_window(mode, B, taps, status_ok):
+    """Two windows, outputs enough for the kernel that keeps a window's taps in registers, each of its sizes and one tap more."""
+    for include in (0, 1):
+        test_pool_kernels_on_any_map(B=B, S=300, nwin=2, taps=taps, include=include, mode=mode, status_ok=status_ok)
+
+
+def test_pool_kernels_that_stay_with_one_of_many_windows(status_ok):
+    """As many windows as divide the warps among them, and one more."""
+    for nwin in (148 * 8 * 2, 148 * 8 * 2 + 1):
+        for mode in (0, 1):
+            test_pool_kernels_on_any_map(B=9, S=40, nwin=nwin, taps=70, include=1, mode=mode, status_ok=status_ok)
