@@ -158,14 +158,15 @@ bn_partial_kernel(const T* __restrict__ a, const T* __restrict__ xin, const floa
 // A warp per (channel, split) where its planes are few elements and there are pairs enough for every SM.  us, forward, backward, sums
 // of one tensor: 64 x 512 x 49 a CTA each 26, 31, 21, a warp each 14.6, 13.6, 9.6; 32 x 256 x 196 13.5, 18, 13 and 7.1, 9.9, 6.5;
 // 256 x 128 x 169 (1 352 elements) 16.3, 24.1, 11.2 and 15.3, 24.0, 10.2; 256 x 64 x 900 (7 200) 15.8, 39.1, 9.3 and 16.3, 49, 9.7.
-// A warp takes its planes one after another, so they have to be few for the channels there are.  A warp's time by a CTA's, forward
-// and backward of any plane from 25 to 900 elements: 64 channels, 1, 2, 4, 8, 32 planes to a split 0.8, 0.9, 1.0, 1.1, 1.3; 128
-// channels, 4, 8, 16 planes 0.9, 1.0, 1.1; 256 channels, 8, 16, 32 planes 0.9, 0.97, 1.03; 1 024 channels, 8, 32 planes 0.85, 0.97.
+// A warp takes its planes one after another, so they have to be few for the channels there are; the line is drawn where both took the
+// same.  A warp's time by a CTA's, of any plane from 25 to 900 elements, backward: 64 channels, 1, 2, 4, 8 planes to a split 0.83, 0.89,
+// 1.01, 1.13; 96 channels, 4, 8 planes 0.95, 1.06; 128, 4, 8 0.91, 1.02; 256, 4, 8, 16 0.81, 0.91, 0.94; 512, 8, 16 0.87, 0.94; forward 64,
+// 2, 4, 8, 32 planes 0.9, 1.0, 1.1, 1.3; 256, 16, 32 0.97, 1.03; 1 024, 8, 32 0.85, 0.97 (and 128 x 64 x 400 one call behind another 12.4 us, a CTA each 14.4).
 template <typename T, int MODE>
 void launch_partial(const void* a, const void* xin, const float* mean, const float* invstd, float* part, int N, int C, long long S,
                     const void* yrelu, cudaStream_t s) {
   const long long per = (N + kSplits - 1) / kSplits;
-  if (C >= 64 && C >= 32 * per && per * S <= 2048)
+  if (C >= 64 && C >= (MODE ? 14 * per + 24 : 16 * per) && per * S <= 2048)
     gbh::launch(bn_partial_kernel<T, true, MODE>, dim3(dim3((C + 7) / 8, kSplits)), dim3(256), 0, s, 1, (const T*)a, (const T*)xin, mean, invstd, part, N, C, S, (const T*)yrelu);
   else
     gbh::launch(bn_partial_kernel<T, false, MODE>, dim3(dim3(C, kSplits)), dim3(256), 0, s, 1, (const T*)a, (const T*)xin, mean, invstd, part, N, C, S, (const T*)yrelu);
