@@ -352,6 +352,12 @@ __device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t smem_addr, uin
   return d;
 }
 
+// The same without a swizzle, K-major: eight rows of 16 bytes lie together, sbo bytes to the next eight rows, lbo bytes to the second
+// half of a 32-byte step.
+__device__ __forceinline__ uint64_t make_smem_desc_plain(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  return make_smem_desc_sw128(smem_addr, lbo_bytes, sbo_bytes) & ~((uint64_t)7 << 61);
+}
+
 // Instruction descriptor (32 bit): accumulator format at [4,6) (1 = f32,
 // 2 = s32), A format at [7,10), B format at [10,13) (f16 = 0, bf16 = 1; for
 // kind::i8 signed = 1), A/B major at bits 15/16 (1 = MN-major), N>>3 at

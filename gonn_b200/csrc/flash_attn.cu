@@ -634,29 +634,27 @@ __device__ __forceinline__ void tile_row_to_tmem(const uint8_t* tile, int r, uin
   tmem_st_wait();
 }
 
-// x as a sum of three bf16 values: 24 bits.
-__device__ __forceinline__ void split_bf16(float x, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  const __nv_bfloat16 h = __float2bfloat16_rn(x);
-  const float r = x - __bfloat162float(h);
-  const __nv_bfloat16 m = __float2bfloat16_rn(r);
-  hi = __bfloat16_as_ushort(h);
-  mid = __bfloat16_as_ushort(m);
-  lo = __bfloat16_as_ushort(__float2bfloat16_rn(r - __bfloat162float(m)));
-}
-
 // The row statistics of the dK / dV kernel are added by the tensor core.  They belong to the columns of S^T and dP^T, so that
 // every thread would need all of them: 64 values per sub-tile and warp, and shared memory delivers one register per thread and
 // clock however they are loaded (560 of 2 360 clocks per 128 x 64 block).  Instead row q of a B operand of 16 k's holds -LSE / scale
-// and -Delta, each as three bf16 parts, and one MMA step with an A operand of ones at the parts' places adds them to every row
-// of S^T and of dP^T.  This is that row (its first eight k's; the others are zero): rows past the end and rows without any key
-// (LSE = -inf) get a statistic that makes their probabilities 0.
-__device__ __forceinline__ uint4 stat_row(float lse, float delta, float inv_scale) {
+// or -Delta as three bf16 parts, 24 bits, and one MMA step with an A operand of ones at their places adds it to every row of S^T or
+// dP^T.  LSE and Delta have an operand each: what is infinite in one would be NaN in the other's product with the zeros at its
+// places.  This is the row's first eight k's (the others are zero).  A value that is not finite has one part; a finite one that
+// would round to infinity in bf16 is cut and keeps the rest in the other parts.
+__device__ __forceinline__ uint4 three_parts(float x) {
+  const bool fin = (__float_as_uint(x) & 0x7fffffffu) < 0x7f800000u;
+  const float top = __uint_as_float(0x7f7f0000u);                 // bf16's largest value
+  const __nv_bfloat16 h = __float2bfloat16_rn(fin ? fminf(fmaxf(x, -top), top) : x);
+  const float r = fin ? x - __bfloat162float(h) : 0.f;
+  const __nv_bfloat16 m = __float2bfloat16_rn(r);
+  const __nv_bfloat16 l = __float2bfloat16_rn(r - __bfloat162float(m));
+  return make_uint4(__bfloat16_as_ushort(h) | (uint32_t)__bfloat16_as_ushort(m) << 16, __bfloat16_as_ushort(l), 0u, 0u);
+}
+// Rows past the end and rows without any key (LSE = -inf) get a statistic that makes their probabilities 0.
+__device__ __forceinline__ uint4 lse_parts(float lse, float inv_scale) {
   float x = -(lse == -INFINITY ? 1e30f : lse) * inv_scale;
-  if (fabsf(x) > 1e37f) x = copysignf(1e37f, x);     // (finite parts only; a NaN stays one)
-  uint32_t a, b, c, d, e, f;
-  split_bf16(x, a, b, c);
-  split_bf16(-delta, d, e, f);
-  return make_uint4(a | b << 16, c | d << 16, e | f << 16, 0u);
+  if (fabsf(x) > 1e37f) x = copysignf(1e37f, x);     // (a NaN stays one)
+  return three_parts(x);
 }
 
 // dK / dV: one CTA per 128-key tile; streams 64-row query sub-tiles.  Works in the
@@ -687,8 +685,9 @@ struct KvCfg {
   static constexpr int CW = 4 * BSUB / EW;           // query columns of one of them: a quarter of the key rows, all EW / 4 groups
   static constexpr int THREADS = 96 + EW * 32;       // TMA, MMA and store warps
   static constexpr int CTAS_PER_SM = DUAL ? 2 : 1;
-  // row statistics (64 rows of 128 bytes, 32 a stage), the A operand that adds them, the tile through which dS^T leaves
-  static constexpr int STAT_BYTES = BSUB * 128, ONES_BYTES = 1024, OUT_BYTES = 128 * 128;
+  // row statistics (64 rows of 16 bytes for LSE and for Delta of each stage, and once the zeros behind them), the A operand that adds
+  // them, the tile through which dS^T leaves
+  static constexpr int STAT_ROWS = BSUB * 16, STAT_BYTES = (2 * NS + 1) * STAT_ROWS, ONES_BYTES = 1024, OUT_BYTES = 128 * 128;
   static constexpr int SMEM_BYTES = 2 * TILE_BYTES + NS * 2 * SUB_BYTES + STAT_BYTES + ONES_BYTES + OUT_BYTES + 1024 + 256;
   static constexpr int TMEM_COLS = DUAL ? 256 : 512;
   static constexpr int COL_S = 0, COL_DP = BSUB, COL_ACC0 = 2 * BSUB, COL_ACC1 = COL_ACC0 + HD;
@@ -709,8 +708,8 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   uint8_t* sK = smem;
   uint8_t* sV = sK + C::TILE_BYTES;
   uint8_t* ring = sV + C::TILE_BYTES;                 // [NS] x {Q sub-tile, dO sub-tile}
-  uint8_t* sStat = ring + C::NS * 2 * C::SUB_BYTES;   // 64 rows of statistics, k step st of the operand for stage st
-  uint8_t* sOnes = sStat + C::STAT_BYTES;             // eight rows: k step 0 picks LSE, step 1 Delta
+  uint8_t* sStat = ring + C::NS * 2 * C::SUB_BYTES;   // [NS][LSE, Delta] rows, then rows of zeros
+  uint8_t* sOnes = sStat + C::STAT_BYTES;             // eight rows: ones for the three parts
   uint8_t* sOut = sOnes + C::ONES_BYTES;              // 128 key rows x 64 queries of dS^T
   uint64_t* bars = (uint64_t*)(sOut + C::OUT_BYTES);
   uint64_t* kv_full = bars;                 // 1
@@ -785,13 +784,11 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     if (lane < 4) tma_prefetch_desc(lane == 0 ? &tmK : lane == 1 ? &tmV : lane == 2 ? &tmQ : &tmdO);
     else if (lane < 7) tma_prefetch_desc(lane == 4 ? &tmdK : lane == 5 ? &tmdV : &tmDS);
   }
-  for (int i = threadIdx.x; i < C::STAT_BYTES / 16; i += C::THREADS) reinterpret_cast<uint4*>(sStat)[i] = make_uint4(0u, 0u, 0u, 0u);
   if (threadIdx.x < 64) {
     const uint32_t row = threadIdx.x >> 3, chunk = (threadIdx.x & 7u) ^ row;      // 16-byte chunk before the swizzle
     constexpr uint32_t one = 0x3f80u;
-    reinterpret_cast<uint4*>(sOnes)[threadIdx.x] = chunk == 0u   ? make_uint4(one | one << 16, one, 0u, 0u)
-                                                   : chunk == 2u ? make_uint4(0u, one << 16, one | one << 16, 0u)
-                                                                 : make_uint4(0u, 0u, 0u, 0u);
+    reinterpret_cast<uint4*>(sOnes)[threadIdx.x] = chunk == 0u ? make_uint4(one | one << 16, one, 0u, 0u) : make_uint4(0u, 0u, 0u, 0u);
+    reinterpret_cast<uint4*>(sStat + 2 * C::NS * C::STAT_ROWS)[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
   }
   fence_proxy_async_smem();
   if (warp == 1) { tmem_alloc(tmem_slot, C::TMEM_COLS); tmem_relinquish(); }
@@ -818,8 +815,9 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       }
 #pragma unroll
       for (int i = 0; i < 2; i++) {
-        const int row = lane + 32 * i;
-        *reinterpret_cast<uint4*>(sStat + row * 128 + (((uint32_t)(2 * st) ^ ((uint32_t)row & 7u)) << 4)) = stat_row(l[i], d[i], args.inv_scale);
+        uint4* row = reinterpret_cast<uint4*>(sStat + 2 * st * C::STAT_ROWS) + lane + 32 * i;
+        row[0] = lse_parts(l[i], args.inv_scale);
+        row[C::STAT_ROWS / 16] = three_parts(-d[i]);
       }
       fence_proxy_async_smem();
       mbar_arrive(&q_full[st]);
@@ -847,7 +845,8 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           if (C::KV_IN_TMEM) tc_mma_f16_ts(d, tmem_base + (which ? C::COL_V : C::COL_K) + k * 8, kdesc_sub(sub, k), idesc_s, k != 0);
           else tc_mma_f16(d, kdesc(tile, k), kdesc_sub(sub, k), idesc_s, k != 0);
         }
-        tc_mma_f16(d, make_smem_desc_sw128(ones + which * 32, 16, 0), kdesc_sub(stat, st), idesc_stat, 1u);
+        const int at = (2 * st + which) * C::STAT_ROWS;
+        tc_mma_f16(d, make_smem_desc_sw128(ones, 16, 0), make_smem_desc_plain(stat + at, 2 * C::NS * C::STAT_ROWS - at, 128), idesc_stat, 1u);
         tc_commit(which ? dp_full : s_full);
       };
       // dV += P^T dO (which = 0) or dK += dS^T Q (1).  P^T: each elementwise warp left CW / 2 packed columns at the start of its

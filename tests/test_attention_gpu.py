@@ -144,3 +144,34 @@ def test_forward_of_many_tiles(B, H, Sq, Sk, D, causal, dtype, status_ok):
     # P and the result are rounded to the inputs' type: half a unit of 2^-8 or 2^-11 each, relative to sum |P V| <= max |V|
     unit = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
     assert (out.float() - ref).abs().max().item() <= 2 * unit * vd.abs().max().item()
+
+
+@pytest.mark.parametrize("bad", [float("inf"), -float("inf"), float("nan")])
+@pytest.mark.parametrize("D,causal", [(64, True), (64, False), (128, True), (32, False)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_what_an_infinity_reaches_in_the_backward(bad, D, causal, dtype, status_ok):
+    """One infinity or NaN in dO: its column of dV, its query's dQ and the keys that this query sees in dK.  One in V makes the output
+    and Delta of many queries infinite, but dV depends on neither.  Everything else keeps its bits."""
+    torch.manual_seed(D)
+    q, k, v = (torch.randn(1, 200, 2, D, device="cuda", dtype=dtype) for _ in range(3))
+    scale = D ** -0.5
+    out, lse = flash_fwd(q, k, v, causal, scale)
+    do = torch.randn_like(out)
+    do[0, 70, 1, 5] = 0
+    dq, dk, dv = flash_bwd(q, k, v, out, do, lse, causal, scale)[:3]
+    g = do.clone()
+    g[0, 70, 1, 5] = bad
+    gq, gk, gv = flash_bwd(q, k, v, out, g, lse, causal, scale)[:3]
+    seen = 71 if causal else 200
+    other = [d for d in range(D) if d != 5]
+    assert torch.equal(gv[..., other], dv[..., other]) and not torch.isfinite(gv[0, :seen, 1, 5]).any()
+    rows = [r for r in range(200) if r != 70]
+    assert torch.equal(gq[0, rows, 1], dq[0, rows, 1]) and not torch.isfinite(gq[0, 70, 1]).any()
+    assert not torch.isfinite(gk[0, :seen, 1]).any()
+    for a, b in ((gq, dq), (gk, dk), (gv, dv)):
+        assert torch.equal(a[:, :, 0], b[:, :, 0])
+    w = v.clone()
+    w[0, 30, 1, 3] = bad
+    o2, lse2 = flash_fwd(q, k, w, causal, scale)
+    assert torch.equal(lse, lse2) and not torch.isfinite(o2[0, 30:, 1, 3]).any()
+    assert torch.equal(flash_bwd(q, k, w, o2, do, lse2, causal, scale)[2], dv)
