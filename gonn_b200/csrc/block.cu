@@ -96,11 +96,19 @@ GB_EXPORT int gb_block_fwd(const long long* words, int n, float eps1, float eps2
   return norm(buf_x, a.n2w, a.n2b, P(a.y), eps2);
 }
 
-// Blocks one after another: argument words and (eps1, eps2, scale) of each, as gb_block_fwd takes them.
-GB_EXPORT int gb_stack_fwd(const long long* words, const float* scalars, int blocks, int n, void* stream) {
-  for (int i = 0; i < blocks; i++) {
-    const int rc = gb_block_fwd(words + (long long)i * n, n, scalars[3 * i], scalars[3 * i + 1], scalars[3 * i + 2], stream);
-    if (rc) return rc;
+// Blocks one after another, as gb_block_fwd takes them: argument words and (eps1, eps2, scale) of counts[0] of them in `words` and
+// `scalars`, which have room for `room`.  While counts[2] says that there are more, `more` is called once these are launched and leaves
+// the next ones there (none of them by not coming so far).  So the first kernel starts when the first block is known, and the GPU
+// works while the caller looks at the others.  counts[1]: how many are launched.
+GB_EXPORT int gb_stack_fwd(void (*more)(), int* counts, const long long* words, const float* scalars, int n, int room, void* stream) {
+  for (counts[1] = 0; counts[0] > 0 && counts[0] <= room;) {
+    for (int i = 0; i < counts[0]; i++, counts[1]++) {
+      const int rc = gb_block_fwd(words + (long long)i * n, n, scalars[3 * i], scalars[3 * i + 1], scalars[3 * i + 2], stream);
+      if (rc) return rc;
+    }
+    if (counts[2] == 0) break;
+    counts[0] = counts[2] = 0;
+    more();
   }
   return gbh::E_OK;
 }

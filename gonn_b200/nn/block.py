@@ -26,6 +26,9 @@ _DTYPES = {torch.bfloat16: 0, torch.float16: 1}
 _fwd_ad = torch.autograd.forward_ad
 _tm = torch.nn.modules.module
 _ABSENT = object()
+_WORDS = 26                 # argument words of a block
+_GROUP = 4                  # blocks that a native call asks for at most at a time
+_More = ctypes.CFUNCTYPE(None)
 
 
 def plain(m, cls) -> bool:
@@ -124,54 +127,97 @@ def _block_words(B, S, E, dt, dev, parts):
     return F, H, code, rms, bool(pre_norm), bool(causal), (*n1, *n2, wq, bq, *rest), norm1.eps, norm2.eps, 1.0 / math.sqrt(D)
 
 
+class _Run:
+    """How far a native call over a chain of blocks has come."""
+    __slots__ = ("group", "done", "y", "spare", "sized", "ws", "keep", "error")
+
+    def __init__(self, group):
+        self.group, self.done, self.keep = group, 0, []
+        self.y = self.spare = self.sized = self.ws = self.error = None
+
+
 def evaluate_stack(x, blocks):
-    """The output of a chain of blocks for ``x`` (B, S, E) from one native call, or None (see the module docstring).  ``blocks``:
-    the parts of each (attn, norm1, norm2, ff1, ff2, act, pre_norm, causal); ``act``: an Activation module, or the name of a
-    fusable activation."""
-    if not _input_ok(x):
-        return None
+    """The output of a chain of blocks for ``x`` (B, S, E) and how many of them it stands for: one native call, up to the first
+    block that it cannot take (see the module docstring).  ``blocks``: the parts of each (attn, norm1, norm2, ff1, ff2, act,
+    pre_norm, causal); ``act``: an Activation module, or the name of a fusable activation.
+
+    It starts with the first one and asks for the others by and by, so that the first kernel waits for the checks of one block only
+    (about 20 us of the host) and the GPU works while the others are checked: one, three, then four at a time, since going to and
+    fro costs the host 5 to 10 us.  One call on an idle GPU, us, all checked first | so: 12 layers, 1 x 77 858 | 711; 24 layers, 4 x 512
+    2 440 | 2 083; 24 layers of 2 048, 1 x 1024 3 880 | 3 560; 4 layers, 4 x 512 621 | 577; calls back to back the same.  A few
+    blocks that the host alone bounds go at once (4 layers, 1 x 77 384 | 369, but back to back 307 | 321)."""
+    if not blocks or not _input_ok(x):
+        return x, 0
     B, S, E = x.shape
-    dt, dev = x.dtype, x.get_device()
-    found = []
-    for parts in blocks:
-        w = _block_words(B, S, E, dt, dev, parts)
-        if w is None:
-            return None
-        found.append(w)
-    if not found:
-        return None
-    widest = max(found, key=lambda w: w[0])[0]
-    need = max(int(_l.lib().gb_block_ws(B, S, E, H, widest)) for H in {w[1] for w in found})
-    ws = torch.empty(need, dtype=torch.uint8, device=x.device)
-    y = torch.empty_like(x)
-    other = torch.empty_like(x) if len(found) > 1 else y
-    last = len(found) - 1
-    words, scalars, at = [], [], x.data_ptr()
-    code_dt, ws_at, ya, oa = _DTYPES[dt], ws.data_ptr(), y.data_ptr(), other.data_ptr()
-    for i, (F, H, code, rms, pre_norm, causal, weights, eps1, eps2, scale) in enumerate(found):
-        to = ya if (last - i) % 2 == 0 else oa                 # by turns, the last one in y
-        words += (code_dt, B, S, E, H, F, rms, pre_norm, causal, code, at, to, *weights, ws_at, need)
-        scalars += (eps1, eps2, scale)
-        at = to
-    _l.call("gb_stack_fwd", (_l.L * len(words))(*words), (_l.F * len(scalars))(*scalars), _l.I(len(found)), _l.I(26), _l.stream_ptr())
-    _l.kernel_count += 7 * len(found)
-    return y
+    dt, dev, code_dt = x.dtype, x.get_device(), _DTYPES[x.dtype]
+    counts, words, scalars = (ctypes.c_int * 3)(), (_l.L * (_WORDS * _GROUP))(), (_l.F * (3 * _GROUP))()
+    run = _Run(len(blocks) if len(blocks) <= _GROUP and B * S < 512 else 1)
+
+    def more():
+        try:
+            n = 0
+            while n < run.group and run.done < len(blocks):
+                w = _block_words(B, S, E, dt, dev, blocks[run.done])
+                if w is None:
+                    run.group = 0
+                    break
+                F, H, code, rms, pre_norm, causal, weights, eps1, eps2, scale = w
+                if run.sized != (H, F):
+                    run.sized = H, F
+                    need = int(_l.lib().gb_block_ws(B, S, E, H, F))
+                    if run.ws is None or run.ws.numel() < need:
+                        run.keep.append(run.ws)        # (blocks of this group may use it)
+                        run.ws = torch.empty(need, dtype=torch.uint8, device=x.device)
+                frm, to = (x if run.y is None else run.y), (torch.empty_like(x) if run.spare is None else run.spare)
+                words[_WORDS * n:_WORDS * (n + 1)] = (code_dt, B, S, E, H, F, rms, pre_norm, causal, code, frm.data_ptr(), to.data_ptr(), *weights,
+                                                      run.ws.data_ptr(), run.ws.numel())
+                scalars[3 * n:3 * (n + 1)] = eps1, eps2, scale
+                run.spare, run.y = run.y, to           # by turns
+                run.done += 1
+                n += 1
+            run.group = 0 if run.group == 0 else 3 if run.done == 1 else _GROUP
+            counts[2] = run.group > 0 and run.done < len(blocks)
+            counts[0] = n
+        except BaseException as e:                     # (nothing passes through the native call)
+            run.error = e
+
+    more()
+    if run.done == 0 and run.error is None:
+        return x, 0
+    _l.call("gb_stack_fwd", _More(more), counts, words, scalars, _l.I(_WORDS), _l.I(_GROUP), _l.stream_ptr())
+    _l.kernel_count += 7 * counts[1]
+    if run.error is not None or counts[1] != run.done:
+        raise run.error or RuntimeError("the checks of a transformer block were interrupted")
+    return (x if run.y is None else run.y), run.done
 
 
 def evaluate(x, *parts):
-    """``evaluate_stack`` of a single block."""
-    return evaluate_stack(x, (parts,))
+    """The output of a single block, or None."""
+    if not _input_ok(x):
+        return None
+    B, S, E = x.shape
+    w = _block_words(B, S, E, x.dtype, x.get_device(), parts)
+    if w is None:
+        return None
+    F, H, code, rms, pre_norm, causal, weights, eps1, eps2, scale = w
+    need = int(_l.lib().gb_block_ws(B, S, E, H, F))
+    ws = torch.empty(need, dtype=torch.uint8, device=x.device)
+    y = torch.empty_like(x)
+    words = (_l.L * _WORDS)(_DTYPES[x.dtype], B, S, E, H, F, rms, pre_norm, causal, code, x.data_ptr(), y.data_ptr(), *weights,
+                            ws.data_ptr(), need)
+    _l.call("gb_block_fwd", words, _l.I(_WORDS), _l.F(eps1), _l.F(eps2), _l.F(scale), _l.stream_ptr())
+    return y
 
 
 def chain(x, layers, cls, forward):
     """``layers`` (a ModuleList) applied one after another: without a tape in one native call, if all of them are plain ``cls``
-    layers, whose class's forward is still ``forward``, that it can take."""
+    layers whose class's forward is still ``forward``, as far as it can take them, and layer by layer from there."""
+    done = 0
     if not torch.is_grad_enabled() and type(layers) is ModuleList and cls.forward is forward:
         blocks = [l._parts() if plain(l, cls) else None for l in layers]
-        if blocks and None not in blocks:
-            y = evaluate_stack(x, blocks)
-            if y is not None:
-                return y
-    for l in layers:
-        x = l(x)
+        if None not in blocks:
+            x, done = evaluate_stack(x, blocks)
+    for i, l in enumerate(layers):
+        if i >= done:
+            x = l(x)
     return x

@@ -129,3 +129,54 @@ def test_a_chain_of_blocks_is_one_call(layers):
     finally:
         nn.TransformerEncoderLayer.forward = original
     assert len(seen) == layers
+
+
+def test_a_chain_up_to_a_block_that_it_cannot_take(monkeypatch):
+    """One native call up to that block, whose output goes on from there; nothing is computed or looked at twice."""
+    torch.manual_seed(0)
+    enc = nn.TransformerEncoder(9, 128, 4, 264, pre_norm=True, activation=nn.GELU(), dtype=torch.bfloat16, device="cuda")
+    x = torch.randn(2, 33, 128, device="cuda").bfloat16()
+    looked = []
+    real = block._block_words
+    monkeypatch.setattr(block, "_block_words", lambda *a: looked.append(1) or real(*a))
+    for at in (0, 1, 2, 5, 8):
+        layer = enc.layers[at]
+        layer.norm2.float()
+        want = [x]
+        with torch.no_grad():
+            for l in enc.layers:
+                want.append(l(want[-1]))
+        alone = _calls(lambda: layer(want[at]))[1]
+        looked.clear()
+        y, n = _calls(lambda: enc(x))
+        # the chain (if it has a first block), the block operator by operator, the others each by itself
+        assert n == (at > 0) + alone + (8 - at) and len(looked) == 10 and torch.equal(y, want[-1])
+        layer.norm2.to(torch.bfloat16)
+    L.assert_status_ok()
+
+
+def test_a_chain_of_unlike_blocks():
+    """Feed-forward layers and heads that differ: the workspace grows on the way."""
+    torch.manual_seed(1)
+    stack = nn.ModuleList([nn.TransformerEncoderLayer(128, h, f, pre_norm=i % 2 == 0, causal=i % 3 == 0, activation=nn.ReLU(), dtype=torch.bfloat16,
+                                                      device="cuda") for i, (h, f) in enumerate([(4, 64), (8, 512), (2, 128), (4, 1024), (4, 1024), (1, 8)])])
+    x = torch.randn(3, 70, 128, device="cuda").bfloat16()
+    cls = nn.TransformerEncoderLayer
+    y, n = _calls(lambda: block.chain(x, stack, cls, cls.forward))
+    want = x
+    with torch.no_grad():
+        for l in stack:
+            want = l(want)
+    assert n == 1 and torch.equal(y, want)
+
+
+def test_an_error_among_the_checks_reaches_the_caller(monkeypatch):
+    enc = nn.TransformerEncoder(4, 128, 4, 264, pre_norm=True, activation=nn.GELU(), dtype=torch.bfloat16, device="cuda")
+    x = torch.randn(1, 5, 128, device="cuda").bfloat16()
+    with torch.no_grad():
+        want = enc(x)
+        q = enc.layers[2].attn._modules.pop("qproj")
+        with pytest.raises(KeyError):
+            enc(x)
+        enc.layers[2].attn._modules["qproj"] = q
+        assert torch.equal(enc(x), want)
