@@ -337,6 +337,18 @@ __device__ __forceinline__ void tmem_st_wait() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+// Whether a product of two fp32 operands may run as products of their bf16 planes (csrc/gemm_exact.cu) with the results that FMA
+// gives.  w: the largest magnitude (as bits) and minus the smallest that is not zero, of A and of B, maxima over zeros.  No sum may
+// overflow between the planes, whose parts have signs of their own (`top`: the largest exponent of a product), and no part
+// of an operand or of a product may be subnormal.
+__device__ __forceinline__ bool planes_hold(const unsigned* w, int top) {
+  const uint4 v = __ldcg(reinterpret_cast<const uint4*>(w));
+  const int a1 = v.x >> 23, b1 = v.z >> 23, a0 = (0u - v.y) >> 23, b0 = (0u - v.w) >> 23;      // biased exponents, largest and smallest
+  if (a1 == 255 || b1 == 255) return false;
+  if (v.x == 0u || v.z == 0u) return true;                                                    // zeros alone
+  return a1 + b1 - 254 <= top && a0 >= 25 && b0 >= 25 && a0 + b0 - 254 >= -102;
+}
+
 // Shared-memory matrix descriptor for tcgen05.mma.  Bit layout: start address
 // >>4 at [0,14), leading byte offset >>4 at [16,30), stride byte offset >>4 at
 // [32,46), descriptor version 1 at [46,48), swizzle mode at [61,64)

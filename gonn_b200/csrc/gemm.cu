@@ -72,6 +72,8 @@ struct GemmArgs {
   // plane product p, planes (plane_a >> 4p) & 15 and (plane_b >> 4p) & 15, one after another (csrc/gemm_exact.cu)
   int planes, kb_plane;
   uint32_t plane_a, plane_b;
+  const unsigned* guard;   // null, or the words of planes_hold(): a launch does nothing where the planes do not hold
+  int guard_top;
   int* status;
 };
 
@@ -670,7 +672,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int num_tiles = args.num_m * args.num_n * args.batch * args.splits;
+  int num_tiles = args.num_m * args.num_n * args.batch * args.splits;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; s++) {
@@ -701,6 +703,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   const uint32_t tmem_base = *tmem_slot;
   pdl_trigger();
   pdl_wait();
+  if (PL && args.guard != nullptr && !planes_hold(args.guard, args.guard_top)) num_tiles = 0;   // (the same in every CTA)
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
@@ -971,7 +974,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   const int pair = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
   // num_m / num_n count 256 x 256 pair tiles here
-  const int num_tiles = args.num_m * args.num_n * args.batch * args.splits;
+  int num_tiles = args.num_m * args.num_n * args.batch * args.splits;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; s++) {
@@ -1003,6 +1006,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   const uint32_t tmem_base = *tmem_slot;
   pdl_trigger();
   pdl_wait();
+  if (PL && args.guard != nullptr && !planes_hold(args.guard, args.guard_top)) num_tiles = 0;   // (the same in every CTA)
 
   if (warp == 0) {
     // ---------------- TMA producer (one per CTA) ----------------
@@ -1457,10 +1461,9 @@ __global__ void gemm_simt_kernel(const T* __restrict__ A, const T* __restrict__ 
 // 16 threads writes 256 contiguous bytes of C.  Tiles are staged k-major in two shared-memory
 // buffers; the next tile travels global -> registers while the current one is multiplied.
 template <typename T, int TM, int TN, int BK, bool BIAS>
-__global__ void __launch_bounds__(256, 2)
-gemm_simt_tiled_kernel(const T* __restrict__ A, const T* __restrict__ B, T* __restrict__ C, int M,
-                       int N, int K, int transA, int transB, long long lda, long long ldb,
-                       long long ldc, long long sA, long long sB, long long sC, T alpha, int beta, const T* __restrict__ bias) {
+__device__ __forceinline__ void simt_tile(const T* __restrict__ A, const T* __restrict__ B, T* __restrict__ C, int M, int N, int K, int transA,
+                                          int transB, long long lda, long long ldb, long long ldc, long long sA, long long sB,
+                                          long long sC, T alpha, int beta, const T* __restrict__ bias, int nb, int mb, int b) {
   constexpr int VEC = 16 / (int)sizeof(T);
   constexpr int BM = 16 * TM, BN = 16 * TN, PAD = VEC;
   constexpr int LA = BM * BK / 256, LB = BN * BK / 256;
@@ -1470,12 +1473,11 @@ gemm_simt_tiled_kernel(const T* __restrict__ A, const T* __restrict__ B, T* __re
   __shared__ __align__(16) T As[2][BK][BM + PAD];
   __shared__ __align__(16) T Bs[2][BK][BN + PAD];
 
-  const int b = blockIdx.z;
   A += (long long)b * sA;
   B += (long long)b * sB;
   C += (long long)b * sC;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  const int m0 = mb * BM, n0 = nb * BN;
 
   T acc[TM][TN];
 #pragma unroll
@@ -1592,6 +1594,30 @@ gemm_simt_tiled_kernel(const T* __restrict__ A, const T* __restrict__ B, T* __re
         }
       }
     }
+  }
+}
+
+template <typename T, int TM, int TN, int BK, bool BIAS>
+__global__ void __launch_bounds__(256, 2)
+gemm_simt_tiled_kernel(const T* __restrict__ A, const T* __restrict__ B, T* __restrict__ C, int M,
+                       int N, int K, int transA, int transB, long long lda, long long ldb,
+                       long long ldc, long long sA, long long sB, long long sC, T alpha, int beta, const T* __restrict__ bias) {
+  simt_tile<T, TM, TN, BK, BIAS>(A, B, C, M, N, K, transA, transB, lda, ldb, ldc, sA, sB, sC, alpha, beta, bias, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+// The same where the planes of this product do not hold (see planes_hold), otherwise nothing: few CTAs, which take tile after tile,
+// since one for each would be thousands that only look (8192 x 8192 x 257: 22 us).
+template <int TM, int TN, bool BIAS>
+__global__ void __launch_bounds__(256, 2)
+gemm_fma_guarded_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C, int M, int N, int K, int transA, int transB,
+                        long long lda, long long ldb, long long ldc, long long sA, long long sB, long long sC, float alpha, int beta,
+                        const float* __restrict__ bias, int nx, int ny, long long tiles, const unsigned* guard, int guard_top) {
+  pdl_wait();
+  if (planes_hold(guard, guard_top)) return;
+  for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const long long row = t / nx;
+    simt_tile<float, TM, TN, 16, BIAS>(A, B, C, M, N, K, transA, transB, lda, ldb, ldc, sA, sB, sC, alpha, beta, bias, (int)(t - row * nx),
+                                       (int)(row % ny), (int)(row / ny));
   }
 }
 
@@ -1723,9 +1749,11 @@ int launch_cluster(const TMaps& tm, const GemmArgs& args, cudaStream_t stream) {
 // caller's type: C = (beta ? C : 0) + sum_s ws[s] (+ an fp32 bias).
 template <typename TO>
 __global__ void splitk_finish_kernel(const float* __restrict__ ws, TO* __restrict__ C, const float* __restrict__ bias, int M, int N,
-                                     int batch, int splits, long long ldc, long long strideC, int beta) {
+                                     int batch, int splits, long long ldc, long long strideC, int beta, const unsigned* __restrict__ guard,
+                                     int guard_top) {
   pdl_trigger();
   pdl_wait();
+  if (guard != nullptr && !planes_hold(guard, guard_top)) return;
   const long long per = (long long)M * N;
   const long long total = per * batch;
   for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < total;
@@ -1877,7 +1905,7 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
     args.out_kind = OUT_F32;
     args.beta = 0;
   }
-  const int cluster = esz == 2 && force_bn == 0 && splits == 1 && !use2 ? cluster_splits(M, N, K, batch, g_num_sms) : 0;
+  const int cluster = esz == 2 && force_bn == 0 && splits == 1 && !use2 && args.guard == nullptr ? cluster_splits(M, N, K, batch, g_num_sms) : 0;
   if (cluster) {
     bn = CfgS::BN;
     args.splits = cluster;
@@ -1989,13 +2017,13 @@ int gemm_tc(int esz, const void* A, const void* B, GemmArgs& args, int transA, i
     const float* ws = (const float*)workspace;
     if (user_out == OUT_F32)
       GB_CUDA_OK(gbh::launch(splitk_finish_kernel<float>, dim3(grid), dim3(256), 0, stream, 1, ws, (float*)user_C, user_bias, M, N, batch, splits, user_ldc,
-                                                            user_strideC, user_beta));
+                                                            user_strideC, user_beta, args.guard, args.guard_top));
     else if (user_out == OUT_BF16)
       GB_CUDA_OK(gbh::launch(splitk_finish_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, stream, 1, ws, (__nv_bfloat16*)user_C, user_bias, M, N, batch,
-                                                                    splits, user_ldc, user_strideC, user_beta));
+                                                                    splits, user_ldc, user_strideC, user_beta, nullptr, 0));
     else
       GB_CUDA_OK(gbh::launch(splitk_finish_kernel<__half>, dim3(grid), dim3(256), 0, stream, 1, ws, (__half*)user_C, user_bias, M, N, batch, splits,
-                                                             user_ldc, user_strideC, user_beta));
+                                                             user_ldc, user_strideC, user_beta, nullptr, 0));
   }
   return gbh::E_OK;
 }
@@ -2078,7 +2106,7 @@ GB_EXPORT int gb_gemm16(const void* A, const void* B, void* C, const void* bias,
 int gemm_bf16_planes(const void* A, const void* B, float* C, const float* bias, int M, int N, int K, int batch, int transA,
                      int transB, long long lda, long long ldb, long long ldc, long long plane_a, long long plane_b, int bcastA,
                      int bcastB, long long sC, int planes, uint32_t order_a, uint32_t order_b, float alpha, int beta,
-                     void* workspace, long long workspace_bytes, cudaStream_t stream, int chain) {
+                     void* workspace, long long workspace_bytes, cudaStream_t stream, int chain, const unsigned* guard, int guard_top) {
   GemmArgs a;
   memset(&a, 0, sizeof(a));
   a.M = M; a.N = N; a.K = K; a.batch = batch;
@@ -2086,7 +2114,25 @@ int gemm_bf16_planes(const void* A, const void* B, float* C, const float* bias, 
   a.ldc = ldc; a.strideC = sC; a.alpha = alpha; a.beta = beta;
   a.out_kind = OUT_F32; a.in_bf16 = 1;
   a.bcastA = bcastA; a.bcastB = bcastB; a.plane_a = order_a; a.plane_b = order_b;
+  a.guard = guard; a.guard_top = guard_top;
   return gemm_tc(2, A, B, a, transA, transB, lda, ldb, plane_a, plane_b, 0, stream, workspace, workspace_bytes, planes, chain);
+}
+
+// The same product by FMA, as gb_gemm_simt computes it, where the planes do not hold; otherwise nothing.
+int gemm_fma_unless_planes(const void* A, const void* B, float* C, const float* bias, int M, int N, int K, int batch, int transA, int transB,
+                           long long lda, long long ldb, long long ldc, long long sA, long long sB, long long sC, float alpha, int beta,
+                           const unsigned* guard, int guard_top, cudaStream_t stream) {
+  auto go = [&](auto kern, int tile) {
+    const int nx = (N + tile - 1) / tile, ny = (M + tile - 1) / tile;
+    const long long tiles = (long long)nx * ny * batch;
+    return gbh::launch(kern, dim3((unsigned)(tiles < 2 * 148 ? tiles : 2 * 148)), dim3(256), 0, stream, 1, (const float*)A, (const float*)B, C, M, N, K,
+                       transA, transB, lda, ldb, ldc, sA, sB, sC, alpha, beta, bias, nx, ny, tiles, guard, guard_top);
+  };
+  if (((M + 127) / 128) * ((N + 127ll) / 128) * batch >= 120)      // (the tiles of gb_gemm_simt)
+    GB_CUDA_OK(bias != nullptr ? go(gemm_fma_guarded_kernel<8, 8, true>, 128) : go(gemm_fma_guarded_kernel<8, 8, false>, 128));
+  else
+    GB_CUDA_OK(bias != nullptr ? go(gemm_fma_guarded_kernel<4, 4, true>, 64) : go(gemm_fma_guarded_kernel<4, 4, false>, 64));
+  return gbh::E_OK;
 }
 
 // int8 x int8 -> int32 GEMM with the dequantising epilogue of the reference's

@@ -27,7 +27,10 @@ extern "C" int gb_gemm16(const void* A, const void* B, void* C, const void* bias
 int gemm_bf16_planes(const void* A, const void* B, float* C, const float* bias, int M, int N, int K, int batch, int transA,
                      int transB, long long lda, long long ldb, long long ldc, long long plane_a, long long plane_b, int bcastA,
                      int bcastB, long long sC, int planes, uint32_t order_a, uint32_t order_b, float alpha, int beta,
-                     void* workspace, long long workspace_bytes, cudaStream_t stream, int chain);
+                     void* workspace, long long workspace_bytes, cudaStream_t stream, int chain, const unsigned* guard, int guard_top);
+int gemm_fma_unless_planes(const void* A, const void* B, float* C, const float* bias, int M, int N, int K, int batch, int transA, int transB,
+                           long long lda, long long ldb, long long ldc, long long sA, long long sB, long long sC, float alpha, int beta,
+                           const unsigned* guard, int guard_top, cudaStream_t stream);
 extern "C" int gb_binary(int op, int dtype, const void* a, const void* b, void* c, long long n, int rank,
                          const long long* shape, const long long* sa, const long long* sb, void* stream);
 extern "C" int gb_flash_fwd(int dtype, const void* q, const void* k, const void* v, void* o, float* lse, int B, int H,
@@ -265,24 +268,30 @@ int launch_f64(const void* A, const void* B, void* C, int M, int N, int K, int b
 // lo or mid part of the other sign turns it into NaN; the hi plane holds +-1 in its place, with which an infinity of the other
 // operand gets its sign.  (In the hi plane an infinity times an ordinary row gave NaN.)  A finite value that would round
 // to infinity in bf16 is cut to bf16's largest value and keeps the rest in the other planes.
-__global__ void __launch_bounds__(256) split3_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, int rows, int cols,
-                                                     long long ld, int cols_p, long long src_batch, int vec) {
-  src += (long long)blockIdx.z * src_batch;
-  const long long plane = (long long)rows * cols_p;
-  dst += (long long)blockIdx.z * 3 * plane;
-  const int per_row = cols_p / 8;
-  const unsigned total = (unsigned)rows * (unsigned)per_row;      // < 2^31: the operands' 16-bit planes fit 4 GiB
+struct SplitArgs {
+  const float* src;
+  __nv_bfloat16* dst;
+  int rows, cols, cols_p, vec, batch;
+  long long ld, src_batch;
+};
+template <bool GUARD>
+__device__ __forceinline__ void split3(const SplitArgs& a, int z, unsigned& most, unsigned& least) {
+  const float* src = a.src + (long long)z * a.src_batch;
+  const long long plane = (long long)a.rows * a.cols_p;
+  __nv_bfloat16* dst = a.dst + (long long)z * 3 * plane;
+  const int per_row = a.cols_p / 8;
+  const unsigned total = (unsigned)a.rows * (unsigned)per_row;      // < 2^31: the operands' 16-bit planes fit 4 GiB
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const unsigned r = i / (unsigned)per_row;
     const int c = (int)(i - r * per_row) * 8;
-    const float* s = src + (long long)r * ld + c;
+    const float* s = src + (long long)r * a.ld + c;
     float x[8];
-    if (vec && c + 8 <= cols) {
+    if (a.vec && c + 8 <= a.cols) {
       const float4 u = __ldg(reinterpret_cast<const float4*>(s)), v = __ldg(reinterpret_cast<const float4*>(s) + 1);
       x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
     } else {
 #pragma unroll
-      for (int j = 0; j < 8; j++) x[j] = c + j < cols ? __ldg(s + j) : 0.f;
+      for (int j = 0; j < 8; j++) x[j] = c + j < a.cols ? __ldg(s + j) : 0.f;
     }
     __align__(16) __nv_bfloat16 pl[3][8];
 #pragma unroll
@@ -293,10 +302,42 @@ __global__ void __launch_bounds__(256) split3_kernel(const float* __restrict__ s
       const float r1 = fin ? x[j] - __bfloat162float(pl[0][j]) : 0.f;
       pl[1][j] = __float2bfloat16_rn(r1);
       pl[2][j] = __float2bfloat16_rn(fin ? r1 - __bfloat162float(pl[1][j]) : x[j]);
+      if (GUARD) {
+        const unsigned u = __float_as_uint(x[j]) & 0x7fffffffu;
+        most = max(most, u);
+        least = max(least, 0u - u);
+      }
     }
-    __nv_bfloat16* d = dst + (long long)r * cols_p + c;
+    __nv_bfloat16* d = dst + (long long)r * a.cols_p + c;
 #pragma unroll
     for (int p = 0; p < 3; p++) *reinterpret_cast<uint4*>(d + p * plane) = *reinterpret_cast<const uint4*>(pl[p]);
+  }
+}
+__global__ void __launch_bounds__(256) split3_kernel(const SplitArgs a) {
+  unsigned most = 0u, least = 0u;
+  split3<false>(a, blockIdx.z, most, least);
+}
+
+// Both operands of a product in one launch (blockIdx.y), and into guard[2 y] and [2 y + 1] the largest magnitude and minus the smallest
+// one that is not zero, as bits (see planes_hold).
+__global__ void __launch_bounds__(256) split3_both_kernel(const SplitArgs a, const SplitArgs b, unsigned* guard) {
+  __shared__ unsigned sm[2][8];
+  if ((int)blockIdx.z >= (blockIdx.y == 0 ? a.batch : b.batch)) return;
+  unsigned most = 0u, least = 0u;
+  if (blockIdx.y == 0) split3<true>(a, blockIdx.z, most, least);
+  else split3<true>(b, blockIdx.z, most, least);
+  most = __reduce_max_sync(0xffffffffu, most);
+  least = __reduce_max_sync(0xffffffffu, least);
+  if ((threadIdx.x & 31) == 0) {
+    sm[0][threadIdx.x >> 5] = most;
+    sm[1][threadIdx.x >> 5] = least;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    unsigned v = 0u, *word = guard + 2 * blockIdx.y + threadIdx.x;
+#pragma unroll
+    for (int i = 0; i < 8; i++) v = max(v, sm[threadIdx.x][i]);
+    if (v > *(volatile unsigned*)word) atomicMax(word, v);     // (few blocks raise it)
   }
 }
 
@@ -340,11 +381,13 @@ GB_EXPORT long long gb_gemm_f32x3_workspace(int M, int N, int K, int batch) {
 
 // fp32 GEMM through three bf16 planes per operand (see the file header).  bias: fp32 [N] or null.  workspace:
 // gb_gemm_f32x3_workspace() bytes; split_ws / split_ws_bytes: optional split-K scratch handed on to the bf16 GEMM.  chain: the most
-// of K that one accumulator takes (a multiple of 64, with room for every slice in split_ws; 0: any length).
+// of K that one accumulator takes (a multiple of 64, with room for every slice in split_ws; 0: any length).  guarded: operands that
+// could overflow between the planes, or whose parts would be subnormal, are multiplied by FMA instead; the splits find out, the plane
+// kernels then do nothing, and the FMA kernel else.
 GB_EXPORT int gb_gemm_f32x3(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int batch, int transA,
                             int transB, long long lda, long long ldb, long long ldc, long long sA, long long sB,
                             long long sC, float alpha, int beta, void* workspace, long long workspace_bytes,
-                            void* split_ws, long long split_ws_bytes, int chain, void* stream) {
+                            void* split_ws, long long split_ws_bytes, int chain, int guarded, void* stream) {
   if (workspace == nullptr || workspace_bytes < gb_gemm_f32x3_workspace(M, N, K, batch)) {
     gbh::set_error("gb_gemm_f32x3: workspace too small");
     return gbh::E_BAD_ARG;
@@ -357,22 +400,38 @@ GB_EXPORT int gb_gemm_f32x3(const void* A, const void* B, void* C, const void* b
   const long long plane_a = ar * acp, plane_b = br * bcp;
   __nv_bfloat16* a3 = (__nv_bfloat16*)workspace;
   __nv_bfloat16* b3 = a3 + 3 * plane_a * (share_a ? 1 : batch);
-  auto split = [&](const void* src, __nv_bfloat16* dst, int rows, int cols, long long ld, long long cols_p, long long sb, int n) {
-    const int vec = (ld & 3) == 0 && (sb & 3) == 0 && (((uintptr_t)src) & 15) == 0;
-    const long long blocks = (rows * (cols_p / 8) + 255) / 256;
-    split3_kernel<<<dim3((unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 1, n), 256, 0, s>>>((const float*)src, dst, rows, cols, ld,
-                                                                                               (int)cols_p, sb, vec);
+  auto operand = [&](const void* src, __nv_bfloat16* dst, int rows, int cols, long long ld, long long cols_p, long long sb, int n) {
+    return SplitArgs{(const float*)src, dst, rows, cols, (int)cols_p, (ld & 3) == 0 && (sb & 3) == 0 && (((uintptr_t)src) & 15) == 0, n, ld, sb};
   };
-  split(A, a3, ar, ac, lda, acp, sA, share_a ? 1 : batch);
-  split(B, b3, br, bc, ldb, bcp, sB, share_b ? 1 : batch);
+  auto blocks_of = [](const SplitArgs& o) {
+    const long long blocks = (o.rows * (o.cols_p / 8ll) + 255) / 256;
+    return (unsigned)(blocks < 148 * 16 ? blocks : 148 * 16);
+  };
+  const SplitArgs sa = operand(A, a3, ar, ac, lda, acp, sA, share_a ? 1 : batch), sb = operand(B, b3, br, bc, ldb, bcp, sB, share_b ? 1 : batch);
+  unsigned* guard = nullptr;
+  int top = 0;
+  if (guarded) {
+    guard = (unsigned*)(((uintptr_t)(b3 + 3 * plane_b * sb.batch) + 15) & ~(uintptr_t)15);   // (256 bytes of the workspace are left over)
+    // so far the products and their sums (of fewer than 2^26) stay finite, and what alpha makes of them
+    top = 100 - (fabsf(alpha) > 1.f ? ilogbf(alpha) : 0);
+    GB_CUDA_OK(cudaMemsetAsync(guard, 0, 16, s));
+    const unsigned most = blocks_of(sa) > blocks_of(sb) ? blocks_of(sa) : blocks_of(sb);
+    split3_both_kernel<<<dim3(most, 2, sa.batch > sb.batch ? sa.batch : sb.batch), 256, 0, s>>>(sa, sb, guard);
+  } else {
+    split3_kernel<<<dim3(blocks_of(sa), 1, sa.batch), 256, 0, s>>>(sa);
+    split3_kernel<<<dim3(blocks_of(sb), 1, sb.batch), 256, 0, s>>>(sb);
+  }
   GB_CUDA_OK(cudaGetLastError());
   // Planes 0, 1, 2 = hi, mid, lo.  One launch and one accumulator for all six products, from the smallest to the largest:
   // lo hi, hi lo, mid mid, then mid hi, hi mid, then hi hi.  The tensor core truncates each sum at its accumulator's last
   // bit, so the small products must be in before the large ones; the error is then that of the hi hi chain alone
   // (relative to 64 bits at 3000 x 4096 x 1024: 1.0e-6 in this order in one accumulator, in two and in three).
   // A slice of a split K runs all six products over its part of K, which shortens that chain.
-  return gemm_bf16_planes(a3, b3, (float*)C, (const float*)bias, M, N, K, batch, transA, transB, acp, bcp, ldc, plane_a, plane_b,
-                          share_a, share_b, sC, 6, 0x001102u, 0x010120u, alpha, beta, split_ws, split_ws_bytes, s, chain);
+  const int rc = gemm_bf16_planes(a3, b3, (float*)C, (const float*)bias, M, N, K, batch, transA, transB, acp, bcp, ldc, plane_a, plane_b,
+                                  share_a, share_b, sC, 6, 0x001102u, 0x010120u, alpha, beta, split_ws, split_ws_bytes, s, chain, guard, top);
+  if (rc || guard == nullptr) return rc;
+  return gemm_fma_unless_planes(A, B, (float*)C, (const float*)bias, M, N, K, batch, transA, transB, lda, ldb, ldc, sA, sB, sC, alpha, beta,
+                                guard, top, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -421,7 +480,7 @@ GB_EXPORT double gb_bench_matmul(int m, int k, int n, int iters, int dtype) {
     ms = bench_loop(iters, [&] { return gb_gemm_f64(A, B, C, m, n, k, 1, 0, 0, k, n, n, 0, 0, 0, 1.0, 0, nullptr); });
   else if (dtype == DT_F32)
     ms = bench_loop(iters, [&] {
-      return gb_gemm_f32x3(A, B, C, nullptr, m, n, k, 1, 0, 0, k, n, n, 0, 0, 0, 1.f, 0, ws, ws_bytes, nullptr, 0, 0, nullptr);
+      return gb_gemm_f32x3(A, B, C, nullptr, m, n, k, 1, 0, 0, k, n, n, 0, 0, 0, 1.f, 0, ws, ws_bytes, nullptr, 0, 0, 0, nullptr);
     });
   else
     ms = bench_loop(iters, [&] {

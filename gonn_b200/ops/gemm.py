@@ -84,7 +84,10 @@ def _ragged_part(M: int, N: int, K: int, batch: int) -> int:
     against 64 bits on inputs of one sign (|normal| where the two are closest):
     4096 x 1024 x 3001 721 -> 177, 7.4e-7 -> 5.6e-7; 4096 x 2048 x 4095 1927 -> 393, 9.9e-7 -> 8.9e-7; 2048 x 512 x 1001 91 -> 43,
     4.9e-7 -> 3.7e-7; 4096 x 2048 x 259 137 -> 84; 384 x 384 x 999 59 -> 31; 512 x 512 x 513 34 -> 31.  Five launches cost
-    what the smallest products take: 4096 x 256 x 391 40 -> 31, but 4096 x 256 x 257 30 -> 32 and 1024 x 512 x 333 25 -> 41."""
+    what the smallest products take: 4096 x 256 x 391 40 -> 31, but 4096 x 256 x 257 30 -> 32 and 1024 x 512 x 333 25 -> 41.
+    That is for operands from about 2^-50 to 2^50 (``planes_hold`` in csrc/common.cuh).  Others, found while they are split, take the
+    FMA kernel after all, and its results: what overflows is infinite and not NaN, and magnitudes below 2^-102 keep their bits.
+    The check costs 1 to 4 us of the times above; with one value of 1e-36, 4096 x 1024 x 3001 takes 813 us, 718 by FMA alone."""
     if N % 4 or (K < 512 and M * N * K * batch < 400e6):
         return 0
     return 512 if K >= 3584 else 384 if K >= 2048 else 256 if K >= 1024 else 192 if K >= 512 else 128
@@ -247,7 +250,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
                         _l.I(min(chain, K - k)), _l.I(batch), _l.I(int(trans_a)), _l.I(int(trans_b)), _l.L(lda), _l.L(ldb),
                         _l.L(out.stride(-2)), _l.L(sA), _l.L(sB), _l.L(sC), _l.F(alpha), _l.I(int(beta or k > 0)),
                         _l.ptr(ws3), _l.L(ws3.numel()), _l.ptr(ws), _l.L(_WS_BYTES if ws is not None else 0),
-                        _l.I(part), _l.stream_ptr())
+                        _l.I(part), _l.I(int(ragged)), _l.stream_ptr())
             return out
         _l.call("gb_gemm_simt", _l.ptr(a2), _l.ptr(b2), _l.ptr(out), _l.ptr(bias), _l.I(M), _l.I(N), _l.I(K),
                 _l.I(batch), _l.I(int(trans_a)), _l.I(int(trans_b)), _l.L(lda), _l.L(ldb),

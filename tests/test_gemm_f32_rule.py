@@ -124,3 +124,74 @@ def test_ragged_scratch(monkeypatch, room, ta, tb, batch):
     L.assert_status_ok()
     # as in test_pieces: every accumulator truncates 6 x 12 sums, every slice is rounded once; an FMA chain of 1001 is below too
     assert float((got.double().cpu() - want).norm() / want.norm()) < 2.0 ** -20
+
+
+def _both_ways(a, b, **kw):
+    got = {}
+    for mode in ("bf16x3", "simt"):
+        old = G.set_fp32_gemm_mode(mode)
+        try:
+            out = kw["out"].clone() if "out" in kw else None
+            got[mode] = G.gemm(a, b, **{**kw, "out": out})
+        finally:
+            G.set_fp32_gemm_mode(old)
+    L.assert_status_ok()
+    return got["bf16x3"], got["simt"]
+
+
+def _same(x, y):
+    return bool(((x == y) | (x.isnan() & y.isnan())).all())
+
+
+_ODD_OPERANDS = {
+    "overflow": lambda t: t.mul_(3e37), "one large": lambda t: t[7, 5].fill_(1e35), "tiny": lambda t: t.mul_(1e-36),
+    "one tiny": lambda t: t[7, 5].fill_(2e-33), "a tiny row": lambda t: t[:, 3].mul_(1e-34), "one infinity": lambda t: t[7, 5].fill_(float("inf")),
+    "one nan": lambda t: t[7, 5].fill_(float("nan")), "one subnormal": lambda t: t[7, 5].fill_(1e-40), "products that vanish": lambda t: t.mul_(1e-17),
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what", sorted(_ODD_OPERANDS))
+@pytest.mark.parametrize("M,N,K,ta,tb", [(516, 260, 1001, True, False), (384, 1024, 2049, False, False), (1031, 516, 513, True, True)])
+def test_ragged_operands_outside_the_planes_range(what, M, N, K, ta, tb):
+    """What would overflow between the planes, or whose parts would be subnormal: the bits of the FMA kernel."""
+    assert G._ragged_part(M, N, K, 1) > 0
+    torch.manual_seed(K)
+    a, b = torch.randn(*((K, M) if ta else (M, K)), device="cuda"), torch.randn(*((N, K) if tb else (K, N)), device="cuda")
+    bias, out = torch.randn(N, device="cuda"), torch.randn(M, N, device="cuda")
+    change = _ODD_OPERANDS[what]
+    if what in ("overflow", "tiny", "products that vanish"):
+        change(a)
+    change(b)
+    for kw in (dict(), dict(bias=bias, alpha=0.5), dict(out=out, beta=True)):
+        x, y = _both_ways(a, b, trans_a=ta, trans_b=tb, **kw)
+        assert _same(x, y)
+    assert what != "overflow" or bool(y.isinf().any())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("room", ["slices", "two slices", "pieces"])
+def test_ragged_infinities_with_little_scratch(monkeypatch, room):
+    M, N, K = 333, 516, 1001
+    if room != "slices":
+        monkeypatch.setattr(G, "_WS_BYTES", 2 * 4 * M * N + 64 if room == "two slices" else 4 * M * N - 4)
+    a, b, out = torch.rand(K, M, device="cuda") + 0.5, torch.rand(K, N, device="cuda") + 0.5, torch.randn(M, N, device="cuda")
+    a[K - 3, 9], b[K - 3, 11], a[5, 20] = 1e30, -1e30, 1e30
+    x, y = _both_ways(a, b, trans_a=True, out=out, beta=True, bias=torch.ones(N, device="cuda"))
+    assert x[9, 11] == y[9, 11] == -float("inf") and torch.equal(x.isinf(), y.isinf()) and not x.isnan().any()
+    # FMA sums of 1001 products and of the pieces
+    ok = y.isfinite()
+    assert float((x[ok].double() - y[ok].double()).norm() / y[ok].double().norm()) < 2.0 ** -20
+
+
+@pytest.mark.gpu
+def test_ragged_ordinary_operands_are_products_of_planes():
+    """Zeros, and magnitudes from 2^-50 to 2^48, do not send a product to the FMA kernel."""
+    torch.manual_seed(3)
+    a, b = torch.randn(1001, 516, device="cuda"), torch.randn(1001, 260, device="cuda")
+    a[:, ::3], b[5] = 0, 0
+    a[3, 1], b[9, 9] = 2.0 ** 48, 2.0 ** -50
+    x, y = _both_ways(a, b, trans_a=True)
+    assert not torch.equal(x, y)
+    want = a.double().t() @ b.double()
+    assert float((x.double() - want).norm()) <= float((y.double() - want).norm())
