@@ -92,7 +92,14 @@ __device__ __forceinline__ float exp2_poly(float x) {
 // kernel leave SMs empty.  16-bit products back to back, us: 77 x 2304 x 768 7.0 -> 6.3, 512 x 2304 x 768 7.6 -> 6.6, 2048^3 17.7 -> 16.9,
 // 4096^3 95.7 -> 93.1, 16384 x 2304 x 768 50.9 -> 49.8; the 12-layer model on 77 tokens, replayed, 539 -> 492 (without triggers 534;
 // with one in the attention kernel as well 541: more kernels waiting in a row are slower than fewer, so that one has none).
+//
+// Thousands of CTAs that take a few hundred clocks each feel it; kernels that may be launched so ask starts_early() first, on the host
+// and before the trigger.  us, in full order | so, one call behind another (and alone behind cold caches): bf16 RMSNorm, four rows a
+// CTA, 100 000 of 64 18.5 (22.9) | 27.0 (31.2), 65 536 of 256 14.4 (19.2) | 17.8 (22.9); fp32 LayerNorm 300 000 of 128 64 (68) | 79
+// (84); fp32 cross-entropy, a row a CTA, 200 000 of 16 129 | 227 and its gradient 112 | 212, 50 000 of 512 55 | 60; wider ones gain: bf16 LayerNorm 32 768 of
+// 512 14.4 | 12.6, fp32 65 536 of 256 26.6 | 23.5, cross-entropy 20 000 of 1 024 38.9 | 35.0.
 // ---------------------------------------------------------------------------
+__host__ __device__ constexpr bool starts_early(long long bytes_per_cta, long long ctas) { return bytes_per_cta > 2048 || ctas <= 8 * 148; }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -503,6 +510,14 @@ inline cudaError_t launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem
   cfg.attrs = attr;
   cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<A&&>(args)...);
+}
+
+// The same, or in full order.
+template <typename... P, typename... A>
+inline cudaError_t launch_if(bool early, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  if (early) return launch(kern, grid, block, smem, stream, 1, static_cast<A&&>(args)...);
+  kern<<<grid, block, smem, stream>>>(static_cast<A&&>(args)...);
+  return cudaGetLastError();
 }
 
 #define GB_CUDA_OK(expr)                                                           \

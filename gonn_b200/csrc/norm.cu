@@ -696,7 +696,7 @@ template <typename T, typename TW, int VPT, bool RMS, bool STAGED>
 __global__ void __launch_bounds__(128)
 norm_fwd_warp_kernel(const T* __restrict__ x, const TW* __restrict__ w, const TW* __restrict__ b, T* __restrict__ y,
                      float* __restrict__ mean_out, float* __restrict__ rstd_out, long long rows, int D, float eps) {
-  pdl_trigger();
+  if (starts_early(4ll * D * sizeof(T), gridDim.x)) pdl_trigger();
   pdl_wait();
   constexpr int V = IO<T>::V;
   constexpr int NP2 = Pairs<T>::NP2;
@@ -1007,11 +1007,15 @@ int norm_fwd_t(const void* x, const void* w, const void* b, void* y, float* mean
     const bool staged = (((uintptr_t)w | (uintptr_t)b) & 15) != 0;
     const long long blocks = (rows + 3) / 4, most = staged ? 148 * (nvec <= 128 ? 16 : 8) : 1 << 20;
     const size_t smem = staged ? 2 * (size_t)D * sizeof(TW) : 0;
+    const unsigned grid = (unsigned)(blocks < most ? blocks : most);
+    const bool early = starts_early(4ll * D * sizeof(T), grid);
 #define GB_FWDW_(VPT, STAGED)                                                                              \
-  GB_CUDA_OK(gbh::launch(norm_fwd_warp_kernel<T, TW, VPT, RMS, STAGED>, dim3((unsigned)(blocks < most ? blocks : most)), dim3(128), \
-                         smem, s, 1, (const T*)x, (const TW*)w, (const TW*)b, (T*)y, mean, rstd, rows, D, eps))
+  {                                                                                                        \
+    auto kern = norm_fwd_warp_kernel<T, TW, VPT, RMS, STAGED>;                                             \
+    GB_CUDA_OK(gbh::launch_if(early, kern, dim3(grid), dim3(128), smem, s, (const T*)x, (const TW*)w, (const TW*)b, (T*)y, mean, rstd, rows, D, eps)); \
+  }
 #define GB_FWDW(VPT)              \
-  if (staged) GB_FWDW_(VPT, true); \
+  if (staged) GB_FWDW_(VPT, true) \
   else GB_FWDW_(VPT, false)
     if (nvec <= 32) { GB_FWDW(1); }
     else if (nvec <= 64) { GB_FWDW(2); }
