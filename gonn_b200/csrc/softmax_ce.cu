@@ -154,7 +154,7 @@ __global__ void ce_fwd_kernel(const T* __restrict__ x, const long long* __restri
                               float* __restrict__ lse_out, float* __restrict__ w_row, int C,
                               long long ignore_index, int has_ignore, float eps, float cw_sum,
                               int use_smem, int* status) {
-  pdl_trigger();
+  if (starts_early((long long)C * sizeof(T), gridDim.x)) pdl_trigger();
   pdl_wait();
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ float red[32];
@@ -344,7 +344,7 @@ __global__ void ce_bwd_kernel(const T* x, const long long* __restrict__ tgt,
                               const float* __restrict__ gscalar, const float* __restrict__ grow,
                               const float* __restrict__ denom, T* dx, int C, long long ignore_index,
                               int has_ignore, float eps, float cw_sum) {
-  pdl_trigger();
+  if (starts_early((long long)C * sizeof(T), gridDim.x)) pdl_trigger();
   pdl_wait();
   const long long row = blockIdx.x;
   const long long t = tgt[row];
@@ -462,7 +462,7 @@ int ce_fwd_t(const void* x, const long long* tgt, const float* cw, float* loss_r
   size_t bytes;
   int rc = set_smem<T>((const void*)ce_fwd_kernel<T>, C, &use_smem, &bytes);
   if (rc) return rc;
-  gbh::launch(ce_fwd_kernel<T>, dim3((unsigned)rows), dim3(block_for(C)), bytes, s, 1, (const T*)x, tgt, cw, loss_row, lse, w_row, C,
+  gbh::launch_if(starts_early((long long)C * sizeof(T), rows), ce_fwd_kernel<T>, dim3((unsigned)rows), dim3(block_for(C)), bytes, s, (const T*)x, tgt, cw, loss_row, lse, w_row, C,
                                                               ignore_index, has_ignore, eps, cw_sum,
                                                               use_smem, gbh::status_ptr());
   GB_CUDA_OK(cudaGetLastError());
@@ -575,7 +575,7 @@ GB_EXPORT int gb_ce_bwd(int dtype, const void* logits, const long long* targets,
   if (!class_w) class_w_sum = (float)C;
   int blk = block_for(C);
 #define GB_CE(T)                                                                                   \
-  gbh::launch(ce_bwd_kernel<T>, dim3((unsigned)rows), dim3(blk), 0, s, 1, (const T*)logits, targets, class_w, lse, g_scalar, g_row, \
+  gbh::launch_if(starts_early((long long)C * sizeof(T), rows), ce_bwd_kernel<T>, dim3((unsigned)rows), dim3(blk), 0, s, (const T*)logits, targets, class_w, lse, g_scalar, g_row, \
                                                   denom, (T*)dlogits, C, ignore_index, has_ignore,  \
                                                   label_smoothing, class_w_sum)
   switch (dtype) {
