@@ -96,12 +96,8 @@ __device__ __forceinline__ float exp2_poly(float x) {
 // Thousands of CTAs that take a few hundred clocks each feel it; kernels that may be launched so ask starts_early() first, on the host
 // and before the trigger.  us, in full order | so, one call behind another (and alone behind cold caches): bf16 RMSNorm, four rows a
 // CTA, 100 000 of 64 18.5 (22.9) | 27.0 (31.2), 65 536 of 256 14.4 (19.2) | 17.8 (22.9); fp32 LayerNorm 300 000 of 128 64 (68) | 79
-<<<<<<< Updated upstream
-// (84); fp32 cross-entropy, a row a CTA, 200 000 of 16 129 | 227 and its gradient 112 | 212, 50 000 of 512 55 | 60; wider ones gain: bf16 LayerNorm 32 768 of
-=======
-// (84); fp32 cross-entropy, a row a CTA, 200 000 of 16 129 | 227, 50 000 of 512 55 | 60; wider ones gain: bf16 LayerNorm 32 768 of
->>>>>>> Stashed changes
-// 512 14.4 | 12.6, fp32 65 536 of 256 26.6 | 23.5, cross-entropy 20 000 of 1 024 38.9 | 35.0.
+// (84); fp32 cross-entropy, a row a CTA, 200 000 of 16 129 | 227 and its gradient 112 | 212, 50 000 of 512 55 | 60; wider ones
+// gain: bf16 LayerNorm 32 768 of 512 14.4 | 12.6, fp32 65 536 of 256 26.6 | 23.5, cross-entropy 20 000 of 1 024 38.9 | 35.0.
 // ---------------------------------------------------------------------------
 __host__ __device__ constexpr bool starts_early(long long bytes_per_cta, long long ctas) { return bytes_per_cta > 2048 || ctas <= 8 * 148; }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
