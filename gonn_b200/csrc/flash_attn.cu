@@ -40,16 +40,11 @@ struct AttnArgs {
   float scale;
   int causal;
   int in_bf16;
-  // element strides of O / dO / dQ / dK / dV style tensors: (b, s, h); d is contiguous
-  long long o_sb, o_ss, o_sh;
-  void* O;
   float* LSE;  // [B, H, Sq]
   // backward
   const float* Delta;  // [B, H, Sq]
-  void* dQ; void* dK; void* dV;
-  long long dq_sb, dq_ss, dq_sh;
-  long long dk_sb, dk_ss, dk_sh;
-  long long dv_sb, dv_ss, dv_sh;
+  void* dQ;
+  long long dq_sb, dq_ss, dq_sh;  // element strides (b, s, h); d is contiguous
   // optional spill of dS^T from the dK/dV kernel: [B*H][ds_rows keys][ds_ld queries], 16-bit, already
   // multiplied by the softmax scale.  When set, dQ is one product of this matrix with K
   // (fa_bwd_dq_ds_kernel) instead of a second pass that recomputes S, P and dP.
@@ -336,7 +331,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     // ---------------- softmax warps: thread = row ----------------
     // What bounds the kernel is the chain of such a warp: the exponentials of a sub-tile, 512 clocks of its scheduler, and about
     // as much again of waits, loads and hand-overs (MUFU 65 % busy at head size 64).  So the maximum is four chains, products and
-    // sums are packed, and the CTA's start and end are short: first loads before its barrier, O by TMA.  (Scores of the next
+    // sums are packed, and O leaves by TMA.  (Scores of the next
     // sub-tile loaded while exponentials run, or two warps to a row: slower.)  us before -> now: (16, 12, 1024, 64) causal
     // 66.0 -> 53.9, (6, 12, 1000 x 1531, 64) 51.9 -> 49.4, (8, 16, 4096, 128) causal 535 -> 502, (4, 16, 2048, 128) 79.7 -> 74.5.
     const int quarter = warp & 3;
@@ -572,7 +567,7 @@ constexpr int BSUB = 64;                  // rows of one streamed sub-tile
 // accumulations of sub-tile i-1) while the elementwise warps work on sub-tile i.  The
 // elementwise warps form two groups of eight; group g owns TMEM buffer g and every second
 // sub-tile, so the TMEM round trips of one group hide behind the arithmetic of the other.
-template <int HD, bool DUAL_>
+template <int HD>
 struct BwdCfg {
   static constexpr int CH = HD / 64;
   static constexpr int TILE_BYTES = CH * 128 * 128;
@@ -584,8 +579,7 @@ struct BwdCfg {
   // elementwise -> accumulation MMAs) as well as each other's start-up and epilogue.
   // head_dim 128: the accumulators alone need 256 columns, so one CTA per SM with two S/dP
   // buffers and two groups of eight elementwise warps that own alternate sub-tiles.
-  static constexpr bool DUAL = DUAL_;
-  static_assert(!DUAL_ || HD == 64, "two CTAs per SM need head_dim 64");
+  static constexpr bool DUAL = HD == 64;             // two CTAs per SM
   static constexpr int NBUF = DUAL ? 1 : 2;
   static constexpr int EW = 8 * NBUF;
   static constexpr int THREADS = 64 + EW * 32;
@@ -673,10 +667,9 @@ __device__ __forceinline__ uint4 lse_parts(float lse, float inv_scale) {
 // What is left is the chain of an elementwise warp: per 128 x 64 block 1.01 us at 128 (1.37 with both gathered and stored by
 // the threads and two S^T / dP^T buffers), 0.67 us at 64 (1.00), where 0.57 and 0.31 are multiply-adds and 0.27 exponentials.
 // us: (8, 16, 4096, 128) causal 1 343 -> 1 100; (16, 12, 1024, 64) causal 147 -> 90; (6, 12, 1000 x 1531, 64) fp16 150 -> 84.
-template <int HD, bool DUAL_>
+template <int HD>
 struct KvCfg {
-  static constexpr bool DUAL = DUAL_;
-  static_assert(!DUAL_ || HD == 64, "two CTAs per SM need head_dim 64");
+  static constexpr bool DUAL = HD == 64;             // two CTAs per SM
   static constexpr int CH = HD / 64;
   static constexpr int TILE_BYTES = CH * 128 * 128;
   static constexpr int SUB_BYTES = CH * BSUB * 128;
@@ -696,13 +689,13 @@ struct KvCfg {
   static_assert((KV_IN_TMEM ? COL_V + HD / 2 : COL_K) <= TMEM_COLS, "TMEM");
 };
 
-template <int HD, bool BF, bool DUAL>
-__global__ void __launch_bounds__(KvCfg<HD, DUAL>::THREADS, KvCfg<HD, DUAL>::CTAS_PER_SM)
+template <int HD, bool BF>
+__global__ void __launch_bounds__(KvCfg<HD>::THREADS, KvCfg<HD>::CTAS_PER_SM)
 fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                   const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                   const __grid_constant__ CUtensorMap tmDS, const __grid_constant__ CUtensorMap tmdK,
                   const __grid_constant__ CUtensorMap tmdV, const AttnArgs args) {
-  using C = KvCfg<HD, DUAL>;
+  using C = KvCfg<HD>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sK = smem;
@@ -733,17 +726,17 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const int i_begin = args.causal ? kv_tile * (BKV / BSUB) : 0;
   const int n_it = max(num_sub - i_begin, 0);
 
-      const float* lse = args.LSE + ((long long)b * args.H + h) * args.Sq;
-      const float* delta = args.Delta + ((long long)b * args.H + h) * args.Sq;
-      float nl[2], nd[2];
-      auto read_stats = [&](int it) {
-  #pragma unroll
-        for (int i = 0; i < 2; i++) {
-          const int q = (i_begin + it) * BSUB + lane + 32 * i;
-          nl[i] = q < args.Sq ? __ldg(lse + q) : -INFINITY;
-          nd[i] = q < args.Sq ? __ldg(delta + q) : 0.f;
-        }
-      };
+  const float* lse = args.LSE + ((long long)b * args.H + h) * args.Sq;
+  const float* delta = args.Delta + ((long long)b * args.H + h) * args.Sq;
+  float nl[2], nd[2];
+  auto read_stats = [&](int it) {
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const int q = (i_begin + it) * BSUB + lane + 32 * i;
+      nl[i] = q < args.Sq ? __ldg(lse + q) : -INFINITY;
+      nd[i] = q < args.Sq ? __ldg(delta + q) : 0.f;
+    }
+  };
   if (warp == 0) read_stats(0);                // (used by the producer warp only)
   auto load_stage = [&](int it, int st) {      // Q and dO of a sub-tile, by one thread
     const int q0 = (i_begin + it) * BSUB;
@@ -1057,12 +1050,12 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 }
 
 // dQ: one CTA per 128-row query tile; streams 64-row key sub-tiles.
-template <int HD, bool BF, bool DUAL>
-__global__ void __launch_bounds__(BwdCfg<HD, DUAL>::THREADS, BwdCfg<HD, DUAL>::CTAS_PER_SM)
+template <int HD, bool BF>
+__global__ void __launch_bounds__(BwdCfg<HD>::THREADS, BwdCfg<HD>::CTAS_PER_SM)
 fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                  const AttnArgs args) {
-  using C = BwdCfg<HD, DUAL>;
+  using C = BwdCfg<HD>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sQ = smem;
@@ -1452,20 +1445,19 @@ struct BwdMaps {
   CUtensorMap ds_out;                  // the same with boxes of 64 x 128, as the dK / dV kernel writes it
 };
 
-int g_fa_dual = 1;
 
-template <int HD, bool BF, bool DUAL>
+template <int HD, bool BF>
 int launch_bwd(const BwdMaps& m, const AttnArgs& a, cudaStream_t s) {
-  using C = BwdCfg<HD, DUAL>;
-  using KV = KvCfg<HD, DUAL>;
+  using C = BwdCfg<HD>;
+  using KV = KvCfg<HD>;
   static bool configured = false;
   if (!configured) {
-    GB_CUDA_OK(cudaFuncSetAttribute(fa_bwd_dkv_kernel<HD, BF, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, KV::SMEM_BYTES));
-    GB_CUDA_OK(cudaFuncSetAttribute(fa_bwd_dq_kernel<HD, BF, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+    GB_CUDA_OK(cudaFuncSetAttribute(fa_bwd_dkv_kernel<HD, BF>, cudaFuncAttributeMaxDynamicSharedMemorySize, KV::SMEM_BYTES));
+    GB_CUDA_OK(cudaFuncSetAttribute(fa_bwd_dq_kernel<HD, BF>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
     configured = true;
   }
   dim3 gkv((a.Sk + BKV - 1) / BKV, a.H, a.B);
-  fa_bwd_dkv_kernel<HD, BF, DUAL><<<gkv, KV::THREADS, KV::SMEM_BYTES, s>>>(m.q64, m.k128, m.v128, m.g64, m.ds_out, m.dk, m.dv, a);
+  fa_bwd_dkv_kernel<HD, BF><<<gkv, KV::THREADS, KV::SMEM_BYTES, s>>>(m.q64, m.k128, m.v128, m.g64, m.ds_out, m.dk, m.dv, a);
   GB_CUDA_OK(cudaGetLastError());
   dim3 gq((a.Sq + BQ - 1) / BQ, a.H, a.B);
   if (a.dS) {
@@ -1477,7 +1469,7 @@ int launch_bwd(const BwdMaps& m, const AttnArgs& a, cudaStream_t s) {
     }
     fa_bwd_dq_ds_kernel<HD, BF><<<gq, D::THREADS, D::SMEM_BYTES, s>>>(m.ds, m.k64, a);
   } else {
-    fa_bwd_dq_kernel<HD, BF, DUAL><<<gq, C::THREADS, C::SMEM_BYTES, s>>>(m.q128, m.k64, m.v64, m.g128, a);
+    fa_bwd_dq_kernel<HD, BF><<<gq, C::THREADS, C::SMEM_BYTES, s>>>(m.q128, m.k64, m.v64, m.g128, a);
   }
   GB_CUDA_OK(cudaGetLastError());
   return gbh::E_OK;
@@ -1491,13 +1483,6 @@ enum { DT_BF16 = 0, DT_F16 = 1 };
 
 // Timeline tracing of the dK/dV kernel (builds with -DGB_FA_TRACE only): `buf` is a device buffer of
 // 3 * 512 int64 (zeroed by the caller) that CTA (0,0,0) fills with SM clock stamps; null switches it off.
-// head_dim 64 backward: 1 = two CTAs per SM with one S/dP buffer each, 0 = one CTA per SM
-// with two buffers and sixteen elementwise warps.
-GB_EXPORT int gb_flash_tune(int dual) {
-  g_fa_dual = dual;
-  return 0;
-}
-
 GB_EXPORT int gb_flash_trace(long long* buf) {
   g_trace = buf;
   return 0;
@@ -1529,7 +1514,7 @@ GB_EXPORT int gb_flash_fwd(int dtype, const void* q, const void* k, const void* 
   a.B = B; a.H = H; a.Sq = Sq; a.Sk = Sk; a.D = D;
   a.scale = scale; a.scale_log2 = scale * 1.4426950408889634f;
   a.causal = causal; a.in_bf16 = dtype == DT_BF16;
-  a.O = o; a.LSE = lse; a.o_sb = o_sb; a.o_ss = o_ss; a.o_sh = o_sh;
+  a.LSE = lse;
   a.status = gbh::status_ptr();
   CUtensorMap tq, tk, tv, to;
   int rc;
@@ -1610,7 +1595,8 @@ GB_EXPORT int gb_flash_bwd(int dtype, const void* q, const void* k, const void* 
 
 // The same with an optional workspace (32-byte aligned, gb_flash_bwd_ws_bytes bytes, contents
 // arbitrary).  With it the dK/dV kernel also writes dS^T and dQ is one product dS K read back
-// from it; without it (null, or too small) a second kernel recomputes the scores for dQ.
+// from it; without it (null, too small, or a problem of more than 4 GiB, the most that the caller keeps for it) a second kernel
+// recomputes the scores for dQ.
 GB_EXPORT int gb_flash_bwd_ws(int dtype, const void* q, const void* k, const void* v, const void* dout,
                               const float* lse, const float* delta, void* dq, void* dk, void* dv,
                               int B, int H, int Sq, int Sk, int D, const long long* strides,
@@ -1636,10 +1622,8 @@ GB_EXPORT int gb_flash_bwd_ws(int dtype, const void* q, const void* k, const voi
   a.causal = causal; a.in_bf16 = dtype == DT_BF16;
   fill_head_group(a, 148);
   a.LSE = const_cast<float*>(lse); a.Delta = delta;
-  a.dQ = dq; a.dK = dk; a.dV = dv;
+  a.dQ = dq;
   a.dq_sb = strides[12]; a.dq_ss = strides[13]; a.dq_sh = strides[14];
-  a.dk_sb = strides[15]; a.dk_ss = strides[16]; a.dk_sh = strides[17];
-  a.dv_sb = strides[18]; a.dv_ss = strides[19]; a.dv_sh = strides[20];
   a.status = gbh::status_ptr();
   a.trace = g_trace;
   // a scale so small that LSE / scale could overflow scores like 0: the statistics are folded with 2^-100 then
@@ -1676,11 +1660,6 @@ GB_EXPORT int gb_flash_bwd_ws(int dtype, const void* q, const void* k, const voi
       return rc;
   }
   if (D > 64)
-    return a.in_bf16 ? launch_bwd<128, true, false>(m, a, (cudaStream_t)stream)
-                     : launch_bwd<128, false, false>(m, a, (cudaStream_t)stream);
-  if (g_fa_dual)
-    return a.in_bf16 ? launch_bwd<64, true, true>(m, a, (cudaStream_t)stream)
-                     : launch_bwd<64, false, true>(m, a, (cudaStream_t)stream);
-  return a.in_bf16 ? launch_bwd<64, true, false>(m, a, (cudaStream_t)stream)
-                   : launch_bwd<64, false, false>(m, a, (cudaStream_t)stream);
+    return a.in_bf16 ? launch_bwd<128, true>(m, a, (cudaStream_t)stream) : launch_bwd<128, false>(m, a, (cudaStream_t)stream);
+  return a.in_bf16 ? launch_bwd<64, true>(m, a, (cudaStream_t)stream) : launch_bwd<64, false>(m, a, (cudaStream_t)stream);
 }

@@ -236,7 +236,7 @@ def flash_fwd(q, k, v, causal: bool, scale: float, out=None):
 # The backward keeps one workspace per device and stream for the spilled dS^T (see gb_flash_bwd_ws): with it the
 # dK / dV kernel also writes dS and dQ is a single product read back from it, instead of a second pass
 # that recomputes the scores.  Problems whose dS^T is larger than the limit take the two-pass path.
-DS_SPILL_LIMIT_BYTES = 1 << 32          # the kernel's 32-bit offsets allow no more
+DS_SPILL_LIMIT_BYTES = 1 << 32          # a bound on the memory that a stream keeps (8 x 16 heads of 4096 x 4096 just fit)
 _ds_ws = {}
 DS_MIN_SCORES = 3 << 19                 # fp64: smaller problems recompute the scores
 
