@@ -698,8 +698,10 @@ GB_EXPORT int gb_lstm_seq_bwd(const void* w, const void* c0, const void* cseq, c
   a.dout = (const float*)dout; a.dcn = (const float*)dcn; a.dgates = (float*)dgates; a.dc0 = (float*)dc0;
   a.status = gbh::status_ptr();
   cudaStream_t s = (cudaStream_t)stream;
-  // (a single step exchanges nothing: no words to clear)
-  const long long words = T > 1 ? bwd_words(ut, a.ug, groups, a.sub, H) : 0;
+  // A single step exchanges nothing, and of two the words' clear costs more than one exchange gains.  us, scattered | gathered: two steps
+  // B = H = 512 132 | 118, 256 x 512 76 | 68, 32 x 512 27.0 | 24.1, 64 x 64 11.5 | 9.8, 256 x 256 26.6 | 28.6; three 203 | 213, 105 | 117,
+  // 31.1 | 30.9, 11.5 | 12.6, 34.8 | 43.2.
+  const long long words = T > 2 ? bwd_words(ut, a.ug, groups, a.sub, H) : 0;
   if (scratch_words < kSms / 2) {
     gbh::set_error("gb_lstm_seq_bwd: %d words of scratch are needed", kSms / 2);
     return gbh::E_BAD_ARG;

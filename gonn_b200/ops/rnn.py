@@ -156,8 +156,8 @@ class _LSTMSequence(torch.autograd.Function):
         whh = _aligned(w_hh.detach())
         dgates = torch.empty_like(act)                     # (B * T, 4H)
         dc0 = torch.empty((B, H), dtype=cseq.dtype, device=dev) if ctx.needs_input_grad[5] else None
-        # (one step exchanges nothing: B = H = 512, 160 us with the words allocated and cleared, 131 without)
-        words = _l.lib().gb_lstm_seq_bwd_words(_l.I(B), _l.I(H)) if T > 1 else LEAST_WORDS
+        # (sequences of up to two steps gather: one step of B = H = 512 takes 160 us with the words allocated and cleared, 131 without)
+        words = _l.lib().gb_lstm_seq_bwd_words(_l.I(B), _l.I(H)) if T > 2 else LEAST_WORDS
         try:
             scratch = torch.empty(words, dtype=torch.int64, device=dev)
         except torch.OutOfMemoryError:

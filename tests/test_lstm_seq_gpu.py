@@ -219,3 +219,23 @@ def test_one_step_takes_no_words(monkeypatch):
     _no_words(monkeypatch, asked)
     test_lstm_sequence_matches_float64(70, 1, 8, 256, True)
     assert not asked
+
+
+@pytest.mark.parametrize("B,H", [(70, 256), (9, 132)])
+def test_two_steps_take_no_words(monkeypatch, B, H):
+    asked = []
+    real = torch.empty
+
+    def empty(*size, **kw):
+        if kw.get("dtype") is torch.int64 and size[0] > max(2 * B * H, 74):      # (the forward's words are 2 B H)
+            asked.append(size[0])
+        return real(*size, **kw)
+    monkeypatch.setattr(torch, "empty", empty)
+    test_lstm_sequence_matches_float64(B, 2, 8, H, True)
+    assert not asked
+    test_lstm_sequence_matches_float64(B, 3, 8, H, True)
+    assert asked
+
+
+def test_backward_with_the_most_words_it_takes():
+    test_backward_either_way_round_matches_float64(512, 3, 512, True)
